@@ -13,6 +13,7 @@ that doubles as the numerical oracle in the tests.
 """
 from __future__ import annotations
 
+import weakref
 from typing import Optional, Sequence
 
 import torch
@@ -243,19 +244,23 @@ _wcache: dict = {}
 
 
 def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
-    """bf16 (optionally transposed) copy of a parameter, cached until the parameter changes."""
+    """bf16 (optionally transposed) copy of a parameter, cached until the parameter changes.
+
+    An entry belongs to ONE tensor object (the parameter itself, or the one that ``w`` is a view of), held by a weak reference:
+    a later parameter may get the id, the address and the version of one that is gone."""
     if w.dtype == torch.bfloat16 and not transpose:
         return w.detach()
-    key = (id(w), transpose)
-    ver = (w._version, w.data_ptr(), tuple(w.shape))
+    owner = w if w._base is None else w._base
+    key = (id(owner), transpose)
+    ver = (w._version, w.data_ptr(), tuple(w.shape), w.stride())
     hit = _wcache.get(key)
-    if hit is not None and hit[0] == ver:
+    if hit is not None and hit[2]() is owner and hit[0] == ver:
         return hit[1]
     src = w.detach()
     val = (src.t() if transpose else src).to(torch.bfloat16).contiguous()
     if len(_wcache) > 4096:
         _wcache.clear()
-    _wcache[key] = (ver, val)
+    _wcache[key] = (ver, val, weakref.ref(owner))
     return val
 
 

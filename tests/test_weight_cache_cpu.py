@@ -1,0 +1,24 @@
+"""The cached bf16 copy of a parameter belongs to that parameter alone."""
+import torch
+
+from physicsnemo_b200.ops import gemm as G
+
+
+def test_a_new_parameter_never_gets_the_copy_of_one_that_is_gone(monkeypatch):
+    a = torch.nn.Parameter(torch.full((8, 8), 1.0))
+    assert G._bf16_weight(a) is G._bf16_weight(a)
+    b = torch.nn.Parameter(torch.full((8, 8), 2.0))
+    # as if `a` had been freed and `b` had been given its id, address and version
+    (ver, val, ref), = [G._wcache[k] for k in G._wcache if k == (id(a), False)]
+    monkeypatch.setitem(G._wcache, (id(b), False), ((b._version, b.data_ptr(), tuple(b.shape), b.stride()), val, ref))
+    assert float(G._bf16_weight(b).float().mean()) == 2.0
+    with torch.no_grad():
+        b.mul_(2)                                    # a changed parameter is converted again
+    assert float(G._bf16_weight(b, transpose=True).float().mean()) == 4.0
+
+
+def test_views_of_one_parameter_share_its_life():
+    a = torch.nn.Parameter(torch.arange(32.0).reshape(4, 2, 4))
+    first = G._bf16_weight(a.reshape(4, 8))
+    assert G._bf16_weight(a.reshape(4, 8)) is first and first.shape == (4, 8)
+    assert G._bf16_weight(a.reshape(8, 4)).shape == (8, 4)
