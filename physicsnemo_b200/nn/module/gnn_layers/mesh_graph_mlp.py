@@ -7,7 +7,8 @@ split into ``lin_efeat / lin_src / lin_dst`` + ``bias``).  The reference's
 ``recompute_activation`` option trades memory for a recomputed SiLU; here the fused chain
 (``ops.mlp_chain``) already keeps only the pre-activations, and the flag is accepted.
 
-Fused path (CUDA, bf16): the whole ``Linear → act → … → Linear`` chain runs on tcgen05 GEMMs
+Fused path (CUDA, bf16): 128-wide MLPs of three linear layers with a LayerNorm are one kernel (``ops.mlp_fused``), which
+also gathers the node rows of an edge and adds the residual.  Otherwise the whole ``Linear → act → … → Linear`` chain runs on tcgen05 GEMMs
 with activations in the epilogues, the K-concatenated edge input ``[efeat | src | dst]`` is
 never materialised, and the trailing LayerNorm kernel adds the block's residual.
 """
@@ -21,13 +22,14 @@ import torch.nn.functional as F
 from torch import Tensor
 
 from .... import ops
+from ....ops import mlp_fused as _mlp_fused
 from ..activations import activation_code
 from ..layer_norm import get_layer_norm_class
-from .utils import concat_efeat, concat_efeat_hetero, gather_src_dst, sum_efeat
+from .utils import concat_efeat, concat_efeat_hetero, edge_sources, sum_efeat
 
 
-def _chain(model: nn.Sequential, x, post: Optional[Tensor] = None) -> Optional[Tensor]:
-    """Run ``model`` (Linear/act…/[LayerNorm]) on the fused kernels; ``None`` if it cannot be fused."""
+def _layers(model: nn.Sequential):
+    """``(weights, biases, activation codes, LayerNorm or None)`` of Linear/act…/[LayerNorm]; ``None`` for another structure."""
     mods = list(model)
     norm = mods[-1] if isinstance(mods[-1], nn.LayerNorm) else None
     body = mods[:-1] if norm is not None else mods
@@ -46,6 +48,29 @@ def _chain(model: nn.Sequential, x, post: Optional[Tensor] = None) -> Optional[T
         biases.append(body[i - (1 if code else 0)].bias)
         acts.append(code)
         i += 1
+    return weights, biases, acts, norm
+
+
+def _one_kernel(layers, srcs, segs, post: Optional[Tensor]) -> Optional[Tensor]:
+    """The whole MLP (three 128-wide layers, LayerNorm, residual) as one kernel that reads source ``j`` through the rows of
+    ``segs[j]``; ``None`` where that kernel does not apply."""
+    weights, biases, acts, norm = layers
+    at = None if post is None else next((j for j, t in enumerate(srcs) if t is post), -1)
+    if norm is None or at == -1 or not _mlp_fused.supported(srcs, segs, weights, biases, acts, norm.weight, norm.bias, at):
+        return None
+    return _mlp_fused.mlp3_ln(srcs, segs, weights, biases, acts[0], norm.weight, norm.bias, norm.eps, at)
+
+
+def _chain(model: nn.Sequential, x, post: Optional[Tensor] = None) -> Optional[Tensor]:
+    """Run ``model`` (Linear/act…/[LayerNorm]) on the fused kernels; ``None`` if it cannot be fused."""
+    layers = _layers(model)
+    if layers is None:
+        return None
+    srcs = list(x) if isinstance(x, (tuple, list)) else [x]
+    y = _one_kernel(layers, srcs, [None] * len(srcs), post)
+    if y is not None:
+        return y
+    weights, biases, acts, norm = layers
     if norm is None:
         return ops.mlp_chain(x, weights, biases, acts, residual=post)
     h = ops.mlp_chain(x, weights, biases, acts)
@@ -101,8 +126,13 @@ class MeshGraphEdgeMLPConcat(MeshGraphMLP):
 
     def forward(self, efeat: Tensor, nfeat, graph, post: Optional[Tensor] = None) -> Tensor:
         if ops.fused_path_enabled(efeat) and efeat.dtype == torch.bfloat16:
-            gs, gd = gather_src_dst(nfeat, graph)
-            return super().forward((efeat, gs, gd), post=post)
+            srcs, segs = edge_sources(nfeat, graph)
+            layers = _layers(self.model) if isinstance(self.model, nn.Sequential) else None
+            y = None if layers is None else _one_kernel(layers, [efeat, *srcs], [None, *segs], post)
+            if y is not None:
+                return y
+            gathered = [t if s is None else ops.gather_rows(t, s) for t, s in zip(srcs, segs)]
+            return super().forward((efeat, *gathered), post=post)
         return super().forward(concat_efeat(efeat, nfeat, graph), post=post)
 
 

@@ -43,6 +43,18 @@ def gather_src_dst(nfeat: Union[Tensor, Tuple[Tensor, Tensor]], graph) -> Tuple[
             ops.gather_rows(dst_feat, segments(graph, "dst", dst_feat.shape[0])))
 
 
+def edge_sources(nfeat: Union[Tensor, Tuple[Tensor, Tensor]], graph):
+    """``([src table, dst table], [rows, rows])`` for kernels that gather by themselves.  A table split over ranks cannot be
+    read that way: its gathered rows (rows ``None``) stand for it."""
+    src_feat, dst_feat = _src_dst(nfeat)
+    dst = segments(graph, "dst", dst_feat.shape[0])
+    if hasattr(graph, "gather_src"):
+        if getattr(graph, "world", 0) == 1 and graph.src_segments.num_segments == src_feat.shape[0]:
+            return [src_feat, dst_feat], [graph.src_segments, dst]
+        return [graph.gather_src(src_feat), dst_feat], [None, dst]
+    return [src_feat, dst_feat], [segments(graph, "src", src_feat.shape[0]), dst]
+
+
 def concat_efeat(efeat: Tensor, nfeat: Union[Tensor, Tuple[Tensor, Tensor]], graph) -> Tensor:
     """``cat(efeat, src_feat[src], dst_feat[dst])`` along the feature dimension."""
     gs, gd = gather_src_dst(nfeat, graph)

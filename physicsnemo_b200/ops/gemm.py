@@ -33,7 +33,14 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _lib.stream()
+
+
+def _f32(t: torch.Tensor) -> torch.Tensor:
+    """fp32 contiguous values of a parameter vector, for a launch (no autograd): the parameter itself where it is that already."""
+    if t.dtype == torch.float32 and t.is_contiguous():
+        return t
+    return t.detach().float().contiguous()
 
 
 def _check(code: int, what: str):

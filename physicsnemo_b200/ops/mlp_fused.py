@@ -1,0 +1,184 @@
+"""Three linear layers, two activations, LayerNorm and residual of a 128-wide message-passing MLP as one kernel.
+
+``mlp3_ln``: ``LayerNorm(act(act(x W1^T + b1) W2^T + b2) W3^T + b3) (+ post)`` where ``x`` is the concatenation of up to
+three 128-wide tables, each read through an optional row index (``csrc/mlp_fused.cuh``): the edge update of a
+MeshGraphNet step reads its node rows by TMA gathers, the node update reads (aggregate, node).  Layer by layer the same
+chain (``ops.gather_rows``, ``ops.mlp_chain``, ``ops.layer_norm``) writes and re-reads every intermediate row.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional, Sequence
+
+import torch
+
+from . import _lib
+from . import gemm as _g
+from . import graph as _graph
+
+WIDTH = 128
+_ACTS = (_g.ACT_GELU, _g.ACT_SILU, _g.ACT_RELU)
+
+
+def _lib_mlp():
+    lib = _lib.load(required=True)
+    if not getattr(lib, "_mlp3_declared", False):
+        c = ctypes
+        vp, i, l, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
+        lib.pnm_mlp3_ln_fwd.argtypes = [i, c.POINTER(vp), c.POINTER(l), c.POINTER(i), c.POINTER(vp), vp, vp, vp, vp, vp, vp, vp, vp, f, i,
+                                        vp, l, vp, l, vp, vp, vp, vp, vp, l, vp]
+        lib.pnm_mlp3_bwd.argtypes = [vp, vp, vp, vp, vp, i, vp, vp, vp, vp, vp, l, vp]
+        lib.pnm_segment_sum_split.argtypes = [vp, vp, vp, vp, l, l, i, vp]
+        lib.pnm_mlp3_ln_fwd.restype = lib.pnm_mlp3_bwd.restype = lib.pnm_segment_sum_split.restype = i
+        lib._mlp3_declared = True
+    return lib
+
+
+def _row_table(t: torch.Tensor) -> bool:
+    """A bf16 table of 128 columns whose rows start on 32-byte boundaries (the kernel moves whole sectors)."""
+    return (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == WIDTH
+            and t.shape[0] > 0 and t.stride(1) == 1 and t.stride(0) >= WIDTH and t.stride(0) % 16 == 0 and t.data_ptr() % 32 == 0)
+
+
+def supported(srcs: Sequence[torch.Tensor], segs: Sequence, weights, biases, acts, gamma, beta, post: Optional[int]) -> bool:
+    """Three 128-wide layers with the same activation after the first two and a 128-wide affine LayerNorm, on aligned
+    bf16 tables of one device."""
+    if not 1 <= len(srcs) <= 3 or len(weights) != 3 or list(acts) != [acts[0], acts[0], _g.ACT_NONE] or acts[0] not in _ACTS:
+        return False
+    if any(tuple(w.shape) != (WIDTH, k) for w, k in zip(weights, (WIDTH * len(srcs), WIDTH, WIDTH))):
+        return False
+    if gamma is None or gamma.numel() != WIDTH or not all(_row_table(t) for t in srcs):
+        return False
+    rows = {s.num_items if s is not None else t.shape[0] for t, s in zip(srcs, segs)}
+    if len(rows) != 1 or 0 in rows or any(s is not None and s.num_segments != t.shape[0] for t, s in zip(srcs, segs)):
+        return False
+    if post is not None and segs[post] is not None:
+        return False
+    params = [*weights, *[b for b in biases if b is not None], gamma] + ([beta] if beta is not None else [])
+    return all(type(p) in (torch.Tensor, torch.nn.Parameter) and p.device == srcs[0].device for p in params)
+
+
+def _vec(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """fp32 contiguous, 16-byte aligned copy (or view) of a parameter vector."""
+    if t is None:
+        return None
+    t = t.detach().float().contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _forward(srcs, segs, weights, biases, act, gamma, beta, eps, post, save: bool):
+    lib = _lib_mlp()
+    n = len(srcs)
+    m = segs[0].num_items if segs[0] is not None else srcs[0].shape[0]
+    dev = srcs[0].device
+    w16 = [_g._bf16_weight(w) for w in weights]
+    vecs = [_vec(t) for t in (*biases, gamma, beta)]
+    y = torch.empty((m, WIDTH), dtype=torch.bfloat16, device=dev)
+    kept = ()
+    if save:
+        kept = (*torch.empty((3, m, WIDTH), dtype=torch.bfloat16, device=dev).unbind(0),
+                *torch.empty((2, m), dtype=torch.float32, device=dev).unbind(0))
+    vp = ctypes.c_void_p
+    code = lib.pnm_mlp3_ln_fwd(
+        n, (vp * n)(*[t.data_ptr() for t in srcs]), (ctypes.c_longlong * n)(*[t.shape[0] for t in srcs]),
+        (ctypes.c_int * n)(*[t.stride(0) for t in srcs]), (vp * n)(*[None if s is None else s.index32.data_ptr() for s in segs]),
+        *[w.data_ptr() for w in w16], *[_g._ptr(v) for v in vecs], float(eps), act, _g._ptr(post), 0 if post is None else post.stride(0),
+        y.data_ptr(), WIDTH, *([t.data_ptr() for t in kept] if save else [None] * 5), m, _g._stream())
+    _g._check(code, "pnm_mlp3_ln_fwd")
+    _g.launch_count += 1
+    return y, kept
+
+
+def _w_t(w: torch.Tensor) -> torch.Tensor:
+    return _g._bf16_weight(w, transpose=True)
+
+
+class _Mlp3LnFn(torch.autograd.Function):
+    """``srcs`` come first among the tensor arguments; ``post`` names the (un-indexed) source that is added to the result."""
+
+    @staticmethod
+    def forward(ctx, segs, tables, act, eps, post, *tensors):
+        n = len(segs)
+        srcs, (w1, w2, w3, b1, b2, b3, gamma, beta) = tensors[:n], tensors[n:]
+        y, kept = _forward(srcs, segs, (w1, w2, w3), (b1, b2, b3), act, gamma, beta, eps, None if post is None else srcs[post], True)
+        ctx.save_for_backward(*srcs, w1, w2, w3, gamma, *kept)
+        ctx.segs, ctx.tables, ctx.act, ctx.post = segs, tables, act, post
+        ctx.dtypes = [None if t is None else t.dtype for t in (w1, w2, w3, b1, b2, b3, gamma, beta)]
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        segs, post = ctx.segs, ctx.post
+        n = len(segs)
+        srcs, (w1, w2, w3, gamma, z1, z2, x3, mean, rstd) = ctx.saved_tensors[:n], ctx.saved_tensors[n:]
+        m, dev = z1.shape[0], z1.device
+        dy = dy.contiguous()
+        lib = _lib_mlp()
+        # dW3, dW2, their biases, db1 and the blocks of dW1 in one zeroed buffer
+        sizes = [WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 3 + [WIDTH * WIDTH] * n
+        acc = torch.zeros(sum(sizes), dtype=torch.float32, device=dev).split(sizes)
+        dw3, dw2 = acc[0].view(WIDTH, WIDTH), acc[1].view(WIDTH, WIDTH)
+        db3, db2, db1 = acc[2:5]
+        rows = torch.empty((2, m, WIDTH), dtype=torch.bfloat16, device=dev)
+        dx3, g1 = rows[0], rows[1]
+        norm = torch.empty(2 * WIDTH + lib.pnm_layernorm_bwd_scratch_floats(m, WIDTH), dtype=torch.float32, device=dev)
+        dgamma, dbeta = norm[:WIDTH], norm[WIDTH:2 * WIDTH]
+        code = lib.pnm_layernorm_bwd(dy.data_ptr(), x3.data_ptr(), _vec(gamma).data_ptr(), mean.data_ptr(), rstd.data_ptr(), None,
+                                     dx3.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), norm[2 * WIDTH:].data_ptr(), m, WIDTH,
+                                     _g._stream())
+        _g._check(code, "pnm_layernorm_bwd")
+        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), _w_t(w3).data_ptr(), _w_t(w2).data_ptr(), ctx.act,
+                                g1.data_ptr(), dw3.data_ptr(), dw2.data_ptr(), db3.data_ptr(), db2.data_ptr(), m, _g._stream())
+        _g._check(code, "pnm_mlp3_bwd")
+        _g.launch_count += 3
+        need = ctx.needs_input_grad[5:]
+        w1t = _w_t(w1)                                       # [128 n, 128]: rows j * 128 .. belong to source j
+        dsrc = [None] * n
+        dw1 = [acc[5 + j].view(WIDTH, WIDTH) for j in range(n)]
+        summed_bias = False
+        for j in range(n):
+            if segs[j] is None:
+                if need[j]:
+                    own = {"aux": dy, "aux_mode": _g.AUX_ADD} if post == j else {}
+                    dsrc[j] = _g.gemm_tn(g1, w1t[j * WIDTH:(j + 1) * WIDTH], **own)
+                _g.gemm_nt(g1, srcs[j], out=dw1[j], colsum_out=None if summed_bias else db1)
+                summed_bias = True
+        # An indexed source: sum g1 over the rows that read a table row FIRST (the products are linear), then one small product
+        # per table instead of one per row of M.  The fp32 sums go into the products as a bf16 pair (hi + lo).
+        for js in ctx.tables:
+            src, rows = srcs[js[0]], segs[js[0]].num_segments
+            pairs = torch.empty((rows, 2 * WIDTH * len(js)), dtype=torch.bfloat16, device=dev)
+            for k, j in enumerate(js):
+                part = pairs[:, 2 * k * WIDTH:]
+                code = lib.pnm_segment_sum_split(g1.data_ptr(), segs[j].perm.data_ptr(), segs[j].offsets.data_ptr(), part.data_ptr(),
+                                                 pairs.stride(0), rows, WIDTH, _g._stream())
+                _g._check(code, "pnm_segment_sum_split")
+                _g.launch_count += 1
+            for k, j in enumerate(js):
+                for h in (2 * k, 2 * k + 1):
+                    hl = pairs[:, h * WIDTH:(h + 1) * WIDTH]
+                    if summed_bias:
+                        _g.gemm_nt(hl, src, out=dw1[j])
+                    else:
+                        _g.gemm_nt(hl, src, out=dw1[j], colsum_out=db1)
+                summed_bias = True
+            if any(need[j] for j in js):
+                wt = torch.cat([w1t[j * WIDTH:(j + 1) * WIDTH] for j in js for _ in range(2)], 1)
+                dsrc[js[0]] = _g.gemm_tn(pairs, wt)
+        grads = [torch.cat(dw1, 1) if n > 1 else dw1[0], dw2, dw3, db1, db2, db3, dgamma, dbeta]
+        grads = [None if dt is None else (t if t.dtype == dt else t.to(dt)) for t, dt in zip(grads, ctx.dtypes)]
+        return (None, None, None, None, None, *dsrc, *grads)
+
+
+def mlp3_ln(srcs: Sequence[torch.Tensor], segs: Sequence[Optional["_graph.SegmentIndex"]], weights, biases, act: int, gamma, beta,
+            eps: float, post: Optional[int]) -> torch.Tensor:
+    """See the module docstring; ``segs[j]`` names the rows of ``srcs[j]`` (``None``: row by row), ``post`` the source that is
+    added to the result.  Call after ``supported``."""
+    params = (*weights, *biases, gamma, beta)
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (*srcs, *params)):
+        tables = {}                                          # indexed sources that read the same tensor
+        for j, (t, s) in enumerate(zip(srcs, segs)):
+            if s is not None:
+                tables.setdefault(id(t), []).append(j)
+        return _Mlp3LnFn.apply(tuple(segs), tuple(tables.values()), act, float(eps), post, *srcs, *params)
+    return _forward(srcs, segs, weights, biases, act, gamma, beta, eps, None if post is None else srcs[post], False)[0]

@@ -1,0 +1,75 @@
+"""The one-kernel message-passing MLP (``ops.mlp_fused``) against plain torch in 64 bits."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+W = 128
+ACTS = {1: F.gelu, 2: F.silu, 3: F.relu}
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,nodes,nsrc,act", [(1, 3, 3, 2), (127, 5, 3, 3), (128, 40, 2, 2), (129, 1, 3, 2), (148 * 128 + 1, 2000, 3, 1),
+                                                 (2 * 148 * 128 + 77, 999, 1, 3), (60001, 10007, 3, 2)])
+def test_mlp3_ln_forward_backward(rows, nodes, nsrc, act):
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    g = torch.Generator().manual_seed(rows + act)
+    rn = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    edge, node = rn(rows, W).bfloat16(), rn(nodes, W).bfloat16()
+    idx = [torch.randint(0, nodes, (rows,), generator=g) for _ in range(2)]      # nodes without a row and repeated ones occur
+    params = [rn(W, W * nsrc) / (W * nsrc) ** 0.5, rn(W, W) / W ** 0.5, rn(W, W) / W ** 0.5, *(0.1 * rn(W) for _ in range(3)),
+              1 + 0.1 * rn(W), 0.1 * rn(W)]
+    up = rn(rows, W).bfloat16()
+
+    leaves = [t.double().requires_grad_() for t in (edge, node, *params)]
+    e, v, w1, w2, w3, b1, b2, b3, ga, be = leaves
+    x = torch.cat([e, v[idx[0]], v[idx[1]]][:nsrc], 1)
+    h = ACTS[act](F.linear(ACTS[act](F.linear(x, w1, b1)), w2, b2))
+    ref = F.layer_norm(F.linear(h, w3, b3), (W,), ga, be) + e
+    ref.backward(up.double())
+
+    dev = [t.cuda().requires_grad_() for t in (edge, node, *params)]
+    e, v, *p = dev
+    segs = [None] + [ops.SegmentIndex(i.cuda(), nodes) for i in idx]
+    srcs, segs = [e, v, v][:nsrc], segs[:nsrc]
+    assert mf.supported(srcs, segs, p[:3], p[3:6], [act, act, 0], p[6], p[7], 0)
+    out = mf.mlp3_ln(srcs, segs, p[:3], p[3:6], act, p[6], p[7], 1e-5, 0)
+    with torch.no_grad():
+        plain = mf.mlp3_ln(srcs, segs, p[:3], p[3:6], act, p[6], p[7], 1e-5, 0)
+    out.backward(up.cuda())
+    assert torch.equal(out, plain)                       # keeping the pre-activations does not change the result
+    # bf16 operands (2^-9 each) through three products and one rounding of the result: measured 3e-3
+    assert _rel(out.cpu(), ref.detach()) < 8e-3
+    for name, a, b in zip("edge node w1 w2 w3 b1 b2 b3 gamma beta".split(), dev, leaves):
+        if b.grad is None or float(b.grad.norm()) == 0.0:
+            continue
+        # gradients see two more roundings per layer; ReLU also flips the sign of pre-activations near zero (one row in 100),
+        # and a single row has no averaging over rows
+        tol = 0.06 if rows < 64 or act == 3 else 0.02
+        assert _rel(a.grad.cpu(), b.grad) < tol, name
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+def test_mlp3_ln_takes_the_same_calls_as_the_layered_path():
+    """Strided tables, odd alignments and other widths keep their answers: by the one kernel or layer by layer."""
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_graph_mlp import MeshGraphMLP
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    torch.manual_seed(0)
+    m = MeshGraphMLP(W, W, W, 2, torch.nn.SiLU()).cuda()
+    wide = torch.randn(300, 2 * W + 8, device="cuda").bfloat16()
+    for x, one in ((wide[:, :W].contiguous(), True), (torch.randn(300, 3 * W, device="cuda").bfloat16()[:, W:2 * W], True),
+                   (wide[:, 8:8 + W], False), (wide[:0, :W].contiguous(), False)):
+        layers = [m.model[0].weight, m.model[2].weight, m.model[4].weight], [m.model[i].bias for i in (0, 2, 4)]
+        assert mf.supported([x], [None], *layers, [2, 2, 0], m.model[5].weight, m.model[5].bias, None) is one
+        if x.shape[0]:
+            with torch.autocast("cuda", dtype=torch.bfloat16), torch.no_grad():
+                y = m(x)
+            assert _rel(y.cpu(), m.double()(x.double()).detach().cpu()) < 1e-2
+            m.float()
