@@ -29,15 +29,6 @@ float* scratch_for_current_device() {
   return g_scratch_ptr[dev];
 }
 
-template <int VEC>
-int launch(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
-           const void* dres, void* dx, float* scratch, long long M, int C, int grid, cudaStream_t st) {
-  pnm::layernorm_bwd_kernel<VEC><<<grid, pnm::kLnWarps * 32, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), gamma, mean, rstd,
-      static_cast<const __nv_bfloat16*>(dres), static_cast<__nv_bfloat16*>(dx), scratch, M, C);
-  return cudaGetLastError() == cudaSuccess ? 0 : PNM_NOALLOC_E_LAUNCH;
-}
-
 }  // namespace
 
 extern "C" int pnm_layernorm_bwd_noalloc(const void* dy, const void* x, const float* gamma, const float* mean,
@@ -54,17 +45,14 @@ extern "C" int pnm_layernorm_bwd_noalloc(const void* dy, const void* x, const fl
     fprintf(stderr, "pnm_layernorm_bwd_noalloc: could not resolve the scratch array on the current device\n");
     return PNM_NOALLOC_E_SETUP;
   }
-  long long want = (M + pnm::kLnWarps - 1) / pnm::kLnWarps;
-  const int grid = static_cast<int>(want < kMaxBlocks ? want : kMaxBlocks);
+  int* err = pnm::error_word_ptr();
+  const int sms = pnm::num_sms();
+  if (!err || sms <= 0) return PNM_NOALLOC_E_SETUP;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int rc;
-  switch (pnm::ln_vec_for(C)) {
-    case 1: rc = launch<1>(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, grid, st); break;
-    case 2: rc = launch<2>(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, grid, st); break;
-    case 3: rc = launch<3>(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, grid, st); break;
-    default: rc = launch<4>(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, grid, st); break;
-  }
-  if (rc) return rc;
+  pnm::LnStream plan;
+  if (pnm::launch_layernorm_bwd_rows(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, kMaxBlocks, sms, err, st, plan))
+    return PNM_NOALLOC_E_LAUNCH;
+  const int grid = plan.grid;
   // every scratch row [0, grid) was fully written above; the fold reads exactly those rows
   pnm::layernorm_bwd_finalize_kernel<<<(2 * C + 31) / 32, 32 * pnm::kLnFoldRows, 0, st>>>(scratch, grid, C, dgamma, dbeta);
   return cudaGetLastError() == cudaSuccess ? 0 : PNM_NOALLOC_E_LAUNCH;

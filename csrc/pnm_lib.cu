@@ -310,20 +310,20 @@ int pnm_conv2d_wgrad_nhwc(const void* dy, const void* x, float* out, float* cols
 int pnm_layernorm_fwd(const void* x, const void* r, const float* gamma, const float* beta, void* y, void* sum_out,
                       float* mean, float* rstd, const void* post, long long M, int C, float eps, void* stream) {
   if (ensure_init()) return -1;
-  return pnm::launch_layernorm_fwd(x, r, gamma, beta, y, sum_out, mean, rstd, post, M, C, eps, g_num_sms,
+  return pnm::launch_layernorm_fwd(x, r, gamma, beta, y, sum_out, mean, rstd, post, M, C, eps, g_num_sms, g_err_ptr,
                                    reinterpret_cast<cudaStream_t>(stream));
 }
 
 long long pnm_layernorm_bwd_scratch_floats(long long M, int C) {
   if (ensure_init()) return -1;
-  return (long long)pnm::layernorm_bwd_grid(M, g_num_sms) * 2 * C;
+  return (long long)pnm::layernorm_bwd_grid(M, g_num_sms, C) * 2 * C;
 }
 
 int pnm_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                       const void* dres, void* dx, float* dgamma, float* dbeta, float* scratch, long long M, int C,
                       void* stream) {
   if (ensure_init()) return -1;
-  return pnm::launch_layernorm_bwd(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, scratch, M, C, g_num_sms,
+  return pnm::launch_layernorm_bwd(dy, x, gamma, mean, rstd, dres, dx, dgamma, dbeta, scratch, M, C, g_num_sms, g_err_ptr,
                                    reinterpret_cast<cudaStream_t>(stream));
 }
 
