@@ -3,7 +3,9 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0      TMA producer (A and B k-blocks of 64 -> 128-byte-swizzled shared tiles)
 //   warp 1      tcgen05.mma issuer (one lane), owns the TMEM allocation
-//   warps 2..9  epilogue: TMEM -> registers -> fused math -> swizzled staging -> TMA store
+//   warps 2..   epilogue: TMEM -> registers -> fused math -> swizzled staging -> TMA store; one warp per 32 x 64 block of the
+//               tile, i.e. 8 warps for 128 columns and 16 for 256.  With 8 warps on 256 columns (two blocks each) the products
+//               with a heavy epilogue were bound by the latency of its instructions, not by memory or the tensor cores.
 // Two TMEM accumulators let the epilogue of tile i overlap the main loop of tile i+1.
 //
 // Fused epilogues (all optional, all applied on fp32 values):
@@ -103,16 +105,19 @@ __device__ __forceinline__ bool wait_remote_flag(const uint32_t* flag, uint32_t 
   }
 }
 
-constexpr int kGemmThreads = 320;
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kChunkBytes = 32 * 128;  // 32 rows x 64 bf16
 
 template <int BN, int MODE>
 struct GemmCfg {
-  static constexpr int NBUF = (MODE == MODE_AUX) ? 3 : 2;
+  static constexpr int EPI = BN / 16;         // epilogue warps: 4 lane quarters x (BN / 64) column blocks
+  static constexpr int THREADS = 64 + 32 * EPI;
+  // staging buffers of a warp: the auxiliary tile of the next block is prefetched while this one is worked on (128 columns: two
+  // ahead); two outputs alternate.  256 columns without either leave the shared memory to the operand stages.
+  static constexpr int NBUF = BN == 256 ? (MODE == MODE_PLAIN ? 1 : 2) : (MODE == MODE_AUX ? 3 : 2);
   static constexpr int STAGE_BYTES = kBM * kBK * 2 + BN * kBK * 2;
-  static constexpr int STAGING = 8 * NBUF * kChunkBytes;
+  static constexpr int STAGING = EPI * NBUF * kChunkBytes;
   static constexpr int BUDGET = 232448 - 1024 /*align*/ - 512 /*barriers*/;
   static constexpr int STAGES_RAW = (BUDGET - STAGING) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 6 ? 6 : STAGES_RAW;
@@ -133,6 +138,25 @@ __device__ __forceinline__ void stage_write_row(uint8_t* buf, int lane, const fl
     *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = u;
   }
 }
+__device__ __forceinline__ void stage_write16(uint8_t* buf, int lane, int k, const float* x) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    *reinterpret_cast<uint4*>(buf + lane * 128 + (((2 * k + j) ^ (lane & 7)) << 4)) =
+        make_uint4(pack_bf16x2(x[8 * j], x[8 * j + 1]), pack_bf16x2(x[8 * j + 2], x[8 * j + 3]), pack_bf16x2(x[8 * j + 4], x[8 * j + 5]),
+                   pack_bf16x2(x[8 * j + 6], x[8 * j + 7]));
+}
+// columns [16 k, 16 k + 16) of a staged row
+__device__ __forceinline__ void stage_read16(const uint8_t* buf, int lane, int k, float* a) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint4 u = *reinterpret_cast<const uint4*>(buf + lane * 128 + (((2 * k + j) ^ (lane & 7)) << 4));
+    float2 f;
+    f = unpack_bf16x2(u.x); a[8 * j + 0] = f.x; a[8 * j + 1] = f.y;
+    f = unpack_bf16x2(u.y); a[8 * j + 2] = f.x; a[8 * j + 3] = f.y;
+    f = unpack_bf16x2(u.z); a[8 * j + 4] = f.x; a[8 * j + 5] = f.y;
+    f = unpack_bf16x2(u.w); a[8 * j + 6] = f.x; a[8 * j + 7] = f.y;
+  }
+}
 __device__ __forceinline__ void stage_read_row(const uint8_t* buf, int lane, float* a) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -146,7 +170,7 @@ __device__ __forceinline__ void stage_read_row(const uint8_t* buf, int lane, flo
 }
 
 template <int BN, int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(GemmCfg<BN, MODE>::THREADS, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2,
                const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                const __grid_constant__ CUtensorMap tmX /* Z (store) or aux (load) */, const GemmArgs g) {
@@ -161,8 +185,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* empty = bars + STAGES;
   uint64_t* tfull = bars + 2 * STAGES;
   uint64_t* tempty = tfull + 2;
-  uint64_t* auxbar = tempty + 2;                      // [8 warps][NBUF]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(auxbar + 8 * 3);
+  uint64_t* auxbar = tempty + 2;                      // [epilogue warps][NBUF]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(auxbar + Cfg::EPI * NBUF);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -171,8 +195,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], 8); }
-    for (int i = 0; i < 8 * 3; ++i) mbar_init(&auxbar[i], 1);
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], Cfg::EPI); }
+    for (int i = 0; i < Cfg::EPI * NBUF; ++i) mbar_init(&auxbar[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmC);
@@ -286,24 +310,23 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    const int e = warp - 2, q = warp & 3, h = e >> 2;
-    constexpr int CH = BN / 128;  // 64-column chunks per warp per tile
+    const int e = warp - 2, q = warp & 3, h = e >> 2;   // lane quarter, 64-column block
     uint8_t* stg = staging + e * NBUF * kChunkBytes;
-    uint64_t* mybar = auxbar + e * 3;
+    uint64_t* mybar = auxbar + e * NBUF;
     uint32_t use = 0, tc = 0;
     bool ok = true;
 
     auto item_coords = [&](uint32_t item, int& r0, int& c0) -> bool {
-      const int tile = blockIdx.x + int(item / CH) * gridDim.x;
+      const int tile = blockIdx.x + int(item) * gridDim.x;
       if (tile >= num_tiles) return false;
       const int mt = tile / g.num_n_tiles, nt = tile % g.num_n_tiles;
-      if (BN == 256 && g.split_m) {             // warp half h owns the rows of sub-tile h, all 128 columns
-        r0 = (2 * mt + h) * kBM + q * 32;
-        c0 = nt * 128 + int(item % CH) * 64;
+      if (BN == 256 && g.split_m) {             // blocks 0, 1 are the columns of the first sub-tile, 2, 3 those of the second
+        r0 = (2 * mt + (h >> 1)) * kBM + q * 32;
+        c0 = nt * 128 + (h & 1) * 64;
         return true;
       }
       r0 = mt * kBM + q * 32;
-      c0 = nt * BN + h * (BN / 2) + int(item % CH) * 64;
+      c0 = nt * BN + h * 64;
       return true;
     };
     auto issue_aux = [&](uint32_t item) {
@@ -324,21 +347,120 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t aph = (tc >> 1) & 1;
       if (!mbar_wait(&tfull[acc], aph, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
-#pragma unroll 1
-      for (int ci = 0; ci < CH; ++ci, ++item) {
+      {
         int r0, c0;
         item_coords(item, r0, c0);
         if (MODE == MODE_AUX) issue_aux(item + 1);
+        const uint32_t taddr = tmem_base + acc * BN + h * 64 + (uint32_t(q * 32) << 16);
+        if constexpr (BN == 256 && MODE == MODE_AUX) {
+          // 16 columns at a time, straight from TMEM into the staged auxiliary tile (which the result replaces): a row of 64 and
+          // its auxiliary values do not fit the 96 registers of a thread.  The softmax backward reads the accumulator twice.
+          const bool store_ok = (r0 < g.M) && (c0 < g.N), full_cols = (c0 + 64 <= g.N);
+          uint8_t* arow = stg + (item % NBUF) * kChunkBytes;
+          auto load16 = [&](int k, float* x) {
+            tmem_ld16(taddr + 16 * k, x);
+            tmem_ld_wait();
+            const int c = c0 + 16 * k;
+            if (g.bias) {
+              if (full_cols) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + c) + j);
+                  x[4 * j] += b.x; x[4 * j + 1] += b.y; x[4 * j + 2] += b.z; x[4 * j + 3] += b.w;
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) if (c + j < g.N) x[j] += __ldg(g.bias + c + j);
+              }
+            }
+            if (g.scale && !g.scale_post) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) if (c + j < g.N) x[j] *= __ldg(g.scale + c + j);
+            }
+            if (g.act == ACT_GELU) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) x[j] = gelu_f(x[j]);
+            } else if (g.act == ACT_SILU) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) x[j] = silu_f(x[j]);
+            } else if (g.act == ACT_RELU) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) x[j] = fmaxf(x[j], 0.f);
+            }
+          };
+          if (!mbar_wait(&mybar[item % NBUF], (item / NBUF) & 1, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
+          float dot = 0.f, gs = 0.f;
+          if (g.aux_mode == AUX_DSOFTMAX) {
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+              float x[16], a[16];
+              load16(k, x);
+              stage_read16(arow, lane, k, a);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) dot += x[j] * a[j];
+            }
+          }
+#pragma unroll 1
+          for (int k = 0; k < 4; ++k) {
+            float x[16], a[16];
+            load16(k, x);
+            stage_read16(arow, lane, k, a);
+            switch (g.aux_mode) {
+              case AUX_ADD:
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] += a[j];
+                break;
+              case AUX_DGELU:
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] *= gelu_grad_f(a[j]);
+                break;
+              case AUX_DSILU:
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] *= silu_grad_f(a[j]);
+                break;
+              case AUX_DRELU:
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = a[j] > 0.f ? x[j] : 0.f;
+                break;
+              case AUX_DSOFTMAX:
+#pragma unroll
+                for (int j = 0; j < 16; ++j) x[j] = a[j] * (x[j] - dot);
+                if (g.group_out) {
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) gs += (a[j] > 0.f) ? x[j] * __logf(a[j]) : 0.f;
+                }
+                break;
+              default: break;
+            }
+            if (g.scale && g.scale_post) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) if (c0 + 16 * k + j < g.N) x[j] *= __ldg(g.scale + c0 + 16 * k + j);
+            }
+            stage_write16(arow, lane, k, x);
+          }
+          tc_fence_before();
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&tempty[acc]);
+            if (store_ok) tma_store_2d(arow, &tmC, c0, r0);
+            tma_store_commit();
+          }
+          if (g.group_out) {                     // only the softmax backward has one
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+            if (lane == 0 && c0 < g.N && g.aux_mode == AUX_DSOFTMAX) atomicAdd(g.group_out + (c0 >> 6), gs);
+          }
+          ++item;
+          continue;
+        }
         float v[64];
-        const uint32_t taddr = tmem_base + acc * BN + h * (BN / 2) + ci * 64 + (uint32_t(q * 32) << 16);
         tmem_ld32(taddr, v);
         tmem_ld32(taddr + 32, v + 32);
         tmem_ld_wait();
-        if (ci == CH - 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[acc]);
-        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[acc]);
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
         const bool full_cols = (c0 + 64 <= g.N);
         const int vo = g.batch_m_tiles ? (r0 / (kBM * g.batch_m_tiles)) * g.N : 0;   // offset of the problem's bias / scale
@@ -406,34 +528,64 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           b = item % NBUF;
           const uint32_t bph = (item / NBUF) & 1;
           if (!mbar_wait(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
-          float a[64];
-          stage_read_row(stg + b * kChunkBytes, lane, a);
+          // read back 16 columns at a time: all 64 next to v[64] would not fit the registers of a 16-warp epilogue
+          const uint8_t* arow = stg + b * kChunkBytes;
           switch (g.aux_mode) {
             case AUX_ADD:
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] += a[j];
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[16 * k + j] += a[j];
+              }
               break;
             case AUX_DGELU:
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] *= gelu_grad_f(a[j]);
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[16 * k + j] *= gelu_grad_f(a[j]);
+              }
               break;
             case AUX_DSILU:
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] *= silu_grad_f(a[j]);
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[16 * k + j] *= silu_grad_f(a[j]);
+              }
               break;
             case AUX_DRELU:
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] = a[j] > 0.f ? v[j] : 0.f;
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[16 * k + j] = a[j] > 0.f ? v[16 * k + j] : 0.f;
+              }
               break;
             case AUX_DSOFTMAX: {
               float dot = 0.f;
 #pragma unroll
-              for (int j = 0; j < 64; ++j) dot += v[j] * a[j];
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) dot += v[16 * k + j] * a[j];
+              }
               float gs = 0.f;
 #pragma unroll
-              for (int j = 0; j < 64; ++j) {
-                v[j] = a[j] * (v[j] - dot);
-                gs += (a[j] > 0.f) ? v[j] * __logf(a[j]) : 0.f;
+              for (int k = 0; k < 4; ++k) {
+                float a[16];
+                stage_read16(arow, lane, k, a);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  v[16 * k + j] = a[j] * (v[16 * k + j] - dot);
+                  gs += (a[j] > 0.f) ? v[16 * k + j] * __logf(a[j]) : 0.f;
+                }
               }
               if (g.group_out) {
 #pragma unroll
@@ -465,6 +617,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tma_store_commit();
         }
         ++use;
+        ++item;
       }
     }
     if (lane == 0) tma_store_wait_all<0>();
@@ -564,7 +717,7 @@ inline int launch_gemm_tn(const GemmCall& c, int num_sms, int* err_word, cudaStr
   int tiles = g.num_m_tiles * g.num_n_tiles;
   int cap = c.max_ctas > 0 ? c.max_ctas : num_sms;
   int grid = tiles < cap ? tiles : cap;
-  gemm_tn_kernel<BN, MODE><<<grid, kGemmThreads, Cfg::SMEM, stream>>>(tA, tA2, tA3, tB, tC, tX, g);
+  gemm_tn_kernel<BN, MODE><<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(tA, tA2, tA3, tB, tC, tX, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
 }
 

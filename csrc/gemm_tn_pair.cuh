@@ -29,6 +29,8 @@ namespace pnm {
 
 // Two staging buffers per epilogue warp in every mode: a third buffer for the auxiliary operand costs a stage and
 // measured slower on K = 3072 (132 vs 124 us) and no faster on K = 768.
+constexpr int kPairThreads = 320;
+
 template <int BN, int MODE>
 struct PairCfg {
   static constexpr int NBUF = 2;
@@ -104,7 +106,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 // The kernel reads GemmArgs with num_m_tiles counting 256-row PAIR tiles; in convolution mode M is the number of valid
 // 128-pixel tiles x 128 (the last pair may own a single tile) and halo is 0.
 template <int BN, int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kPairThreads, 1)
 gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2 /* halo: 7-row box */,
                     const __grid_constant__ CUtensorMap tmA3 /* halo: upper neighbour's row */,
                     const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
@@ -462,7 +464,7 @@ inline int launch_gemm_tn_pair(const GemmCall& c, int num_sms, int* err_word, cu
   if (clusters < 1) return -17;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(kGemmThreads);
+  cfg.blockDim = dim3(kPairThreads);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
