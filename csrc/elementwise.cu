@@ -216,3 +216,51 @@ extern "C" int pnm_add_scale_bf16(const void* a, const void* b, void* out, long 
       (const uint4*)a, (const uint4*)b, (uint4*)out, nvec, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
+
+// ------------------------------------------------------------------------------------------------ convolution weights
+namespace pnm {
+
+// w [cout, cin, k, k] (fp32 or bf16) -> out [rows_p, k * k, cols_p] bf16, tap-major and zero-padded: rows are output channels, or,
+// with `flip`, input channels of the mirrored filter (the operand of the input gradient).  Tensor operations take a padded,
+// permuted copy, a cast and, for the gradient, two flips: up to four launches per use of a weight that is a few hundred KB.  A
+// block moves RT rows x 64 columns through shared memory: both sides are read and written in runs.
+template <typename T>
+__global__ void __launch_bounds__(256) conv_pack_weight_kernel(const T* __restrict__ w, __nv_bfloat16* __restrict__ out, int cout, int cin,
+                                                               int kk, int rows_p, int cols_p, int flip, int rt) {
+  extern __shared__ float cw[];                  // [rt][64][kk]
+  const int r0 = blockIdx.x * rt, c0 = blockIdx.y * 64;
+  const int rows = flip ? cin : cout, cols = flip ? cout : cin;
+  const int n = rt * 64 * kk;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    int r, c, t;                                 // the fastest index is the one that is contiguous in w
+    t = i % kk;
+    if (flip) { r = (i / kk) % rt; c = i / (kk * rt); }
+    else { c = (i / kk) % 64; r = i / (kk * 64); }
+    const int R = r0 + r, C = c0 + c;
+    float v = 0.f;
+    if (R < rows && C < cols) v = static_cast<float>(w[((size_t)(flip ? C : R) * cin + (flip ? R : C)) * kk + t]);
+    cw[(r * 64 + c) * kk + (flip ? kk - 1 - t : t)] = v;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int c = i % 64, t = (i / 64) % kk, r = i / (64 * kk);
+    if (r0 + r < rows_p && c0 + c < cols_p)
+      out[((size_t)(r0 + r) * kk + t) * cols_p + c0 + c] = __float2bfloat16(cw[(r * 64 + c) * kk + t]);
+  }
+}
+
+}  // namespace pnm
+
+extern "C" int pnm_conv_pack_weight(const void* w, int is_bf16, void* out, int cout, int cin, int ksize, int rows_p, int cols_p, int flip,
+                                    void* stream) {
+  const int kk = ksize * ksize;
+  if (cout <= 0 || cin <= 0 || ksize < 1 || ksize > 7 || rows_p < (flip ? cin : cout) || cols_p < (flip ? cout : cin)) return -2;
+  const int rt = kk <= 9 ? 8 : 1;                // 64 columns of an 8-row tile of a 3 x 3 filter: 18 KB
+  const dim3 grid((rows_p + rt - 1) / rt, (cols_p + 63) / 64);
+  const size_t smem = (size_t)rt * 64 * kk * sizeof(float);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
+  if (is_bf16) pnm::conv_pack_weight_kernel<<<grid, 256, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(w), o, cout, cin, kk, rows_p, cols_p, flip, rt);
+  else pnm::conv_pack_weight_kernel<<<grid, 256, smem, st>>>(reinterpret_cast<const float*>(w), o, cout, cin, kk, rows_p, cols_p, flip, rt);
+  return cudaGetLastError() == cudaSuccess ? 0 : -17;
+}

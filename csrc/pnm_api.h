@@ -27,6 +27,11 @@ int pnm_gemm_tn_stacked(const void* A, int lda, const void* B, int ldb, void* C,
 int pnm_gemm_nt_stacked(const void* A, int lda, const void* B, int ldb, float* out, float* colsum, int Mp, int Na, int Nb, int batch,
                         int max_ctas, void* stream);
 
+// w [cout, cin, k, k] (fp32, or bf16 when is_bf16) -> out [rows_p, k*k, cols_p] bf16, zero-padded; rows / columns are output / input
+// channels, with `flip` input / output channels of the mirrored filter.
+int pnm_conv_pack_weight(const void* w, int is_bf16, void* out, int cout, int cin, int ksize, int rows_p, int cols_p, int flip,
+                         void* stream);
+
 // y = LN(x [+ r]) [+ post]; bf16 rows of C channels (C % 8 == 0, C <= 1024), fp32 gamma / beta / statistics.
 int pnm_layernorm_fwd(const void* x, const void* r, const float* gamma, const float* beta, void* y, void* sum_out,
                       float* mean, float* rstd, const void* post, long long M, int C, float eps, void* stream);

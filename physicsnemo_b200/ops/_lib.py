@@ -15,6 +15,8 @@ import subprocess
 import threading
 from pathlib import Path
 
+import torch
+
 _PKG_DIR = Path(__file__).resolve().parents[1]
 _REPO = _PKG_DIR.parent
 _SRC_DIR = _REPO / "csrc"
@@ -119,6 +121,12 @@ def load(required: bool = False):
                 raise RuntimeError(f"sm_100a kernel library unavailable: {exc}") from exc
             return None
     return _lib
+
+
+def stream() -> int:
+    """Handle of the current CUDA stream: ``torch.cuda.current_stream().cuda_stream`` without the stream object that it builds
+    (a few microseconds of every launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def available() -> bool:

@@ -35,6 +35,8 @@ def _lib_conv():
         vp, i, u, d = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint, ctypes.c_double
         lib.pnm_conv2d_nhwc.argtypes = [vp, vp, vp, i, i, i, i, i, i, vp, i, i, i, vp]
         lib.pnm_conv2d_nhwc.restype = i
+        lib.pnm_conv_pack_weight.argtypes = [vp, i, vp, i, i, i, i, i, i, vp]
+        lib.pnm_conv_pack_weight.restype = i
         lib.pnm_conv2d_wgrad_nhwc.argtypes = [vp, vp, vp, vp, i, i, i, i, i, vp, vp, vp, vp, u, d, i, vp]
         lib.pnm_conv2d_wgrad_nhwc.restype = i
         lib._conv_declared = True
@@ -73,6 +75,33 @@ def _pack_weight(weight: torch.Tensor, cin_pad: int | None = None, cout_pad: int
     return w.reshape(cout_pad, -1).to(torch.bfloat16).contiguous()
 
 
+def _pack_kernel(weight: torch.Tensor, rows: int, cols: int, flip: bool) -> torch.Tensor | None:
+    """``weight`` as ``[rows, k*k*cols]`` bf16 in one launch (``flip``: mirrored, input channels first); ``None`` where the
+    kernel does not apply."""
+    if type(weight) not in (torch.Tensor, torch.nn.Parameter) or not weight.is_cuda or not weight.is_contiguous() \
+            or weight.dtype not in (torch.float32, torch.bfloat16):
+        return None
+    cout, cin, k, _ = weight.shape
+    out = torch.empty(rows, k * k * cols, dtype=torch.bfloat16, device=weight.device)
+    err = _lib_conv().pnm_conv_pack_weight(weight.data_ptr(), int(weight.dtype == torch.bfloat16), out.data_ptr(), cout, cin, k, rows, cols,
+                                           int(flip), _lib.stream())
+    if err:
+        raise RuntimeError(f"pnm_conv_pack_weight failed ({err})")
+    _g.launch_count += 1
+    return out
+
+
+def _forward_operand(weight: torch.Tensor, cin_pad: int, cout_pad: int) -> torch.Tensor:
+    w = _pack_kernel(weight, cout_pad, cin_pad, False)
+    return _pack_weight(weight, cin_pad, cout_pad) if w is None else w
+
+
+def _backward_operand(weight: torch.Tensor, cin_pad: int, cout_pad: int) -> torch.Tensor:
+    """Operand of the input gradient: the mirrored filter with the roles of the channels exchanged."""
+    w = _pack_kernel(weight, cin_pad, cout_pad, True)
+    return _pack_weight(weight.detach().flip(2, 3).transpose(0, 1), cout_pad, cin_pad) if w is None else w
+
+
 def _conv_dims(weight: torch.Tensor):
     """Padded channel counts of the kernels for this filter: (cin', cout').
 
@@ -94,11 +123,11 @@ def _launch(x_nhwc: torch.Tensor, w_packed: torch.Tensor, bias, ksize: int, act:
     n, h, w, cin = x_nhwc.shape
     cout = w_packed.shape[0]
     y = torch.empty(n, h, w, cout, dtype=torch.bfloat16, device=x_nhwc.device)
-    b = None if bias is None else bias.detach().float().contiguous()
+    b = None if bias is None else _g._f32(bias.detach())
     if b is not None and b.numel() != cout:
         b = F.pad(b, (0, cout - b.numel()))
     err = _lib_conv().pnm_conv2d_nhwc(x_nhwc.data_ptr(), w_packed.data_ptr(), y.data_ptr(), n, h, w, cin, cout, ksize,
-                                      None if b is None else b.data_ptr(), act, 0, 0, torch.cuda.current_stream().cuda_stream)
+                                      None if b is None else b.data_ptr(), act, 0, 0, _lib.stream())
     if err:
         raise RuntimeError(f"pnm_conv2d_nhwc failed ({err})")
     _g.launch_count += 1
@@ -125,7 +154,7 @@ def wgrad3x3(dy_nhwc: torch.Tensor, x_nhwc: torch.Tensor, want_bias: bool, up_ro
     err = _lib_conv().pnm_conv2d_wgrad_nhwc(
         dy_nhwc.data_ptr(), x_nhwc.data_ptr(), dw.data_ptr(), None if db is None else db.data_ptr(), n, h, w, cin, cout,
         None if up_rows is None else up_rows.data_ptr(), None if down_rows is None else down_rows.data_ptr(), None, None,
-        0, 0.0, 0, torch.cuda.current_stream().cuda_stream)
+        0, 0.0, 0, _lib.stream())
     if err:
         raise RuntimeError(f"pnm_conv2d_wgrad_nhwc failed ({err})")
     _g.launch_count += 1
@@ -143,7 +172,7 @@ class _ConvSame(torch.autograd.Function):
     def forward(ctx, x, weight, bias, act: int):
         cin_p, cout_p = _conv_dims(weight)
         xh = _as_nhwc_bf16(x, cin_p)
-        y = _launch(xh, _pack_weight(weight, cin_p, cout_p), bias, weight.shape[-1], act)
+        y = _launch(xh, _forward_operand(weight, cin_p, cout_p), bias, weight.shape[-1], act)
         if act != 0:
             raise RuntimeError("fused activations are inference-only in conv2d_same; apply the activation separately when training")
         ctx.save_for_backward(xh, weight)
@@ -162,8 +191,7 @@ class _ConvSame(torch.autograd.Function):
         dyh = _as_nhwc_bf16(dy, cout_p)
         dx = dw = db = None
         if ctx.needs_input_grad[0]:
-            wt = weight.detach().flip(2, 3).transpose(0, 1)                           # [Cin, Cout, k, k]
-            dxh = _launch(dyh, _pack_weight(wt, cout_p, cin_p), None, k, 0)
+            dxh = _launch(dyh, _backward_operand(weight, cin_p, cout_p), None, k, 0)
             dx = dxh[..., :cin].permute(0, 3, 1, 2).to(ctx.x_dtype)
         need_w, need_b = ctx.needs_input_grad[1], ctx.has_bias and ctx.needs_input_grad[2]
         if k == 3 and (need_w or need_b):
@@ -197,7 +225,7 @@ def conv2d_same(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
     code = _ACT[act]
     if code and not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
         cin_p, cout_p = _conv_dims(weight)
-        y = _launch(_as_nhwc_bf16(x, cin_p), _pack_weight(weight, cin_p, cout_p), bias, weight.shape[-1], code)
+        y = _launch(_as_nhwc_bf16(x, cin_p), _forward_operand(weight, cin_p, cout_p), bias, weight.shape[-1], code)
         return y[..., :weight.shape[0]].permute(0, 3, 1, 2)
     y = _ConvSame.apply(x, weight, bias, 0)
     if code:

@@ -829,3 +829,18 @@ def test_afno_block_fused_residuals_match_plain_block():
         assert (g1 - g0).norm().item() <= 3e-2 * g0.norm().item()
         for a, b in zip(p1, p0):
             assert (a - b).norm().item() <= 5e-2 * b.norm().item() + 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cout,cin,k,cin_p,cout_p", [(128, 128, 3, 128, 128), (4, 16, 3, 64, 64), (130, 72, 5, 128, 192), (64, 200, 1, 256, 64),
+                                                     (8, 64, 7, 64, 64)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_conv_weight_packing_matches_the_tensor_operations(cout, cin, k, cin_p, cout_p, dtype):
+    """A permutation with zero padding and one rounding: equal, for the forward and for the mirrored backward operand."""
+    from physicsnemo_b200.ops import conv
+
+    w = torch.randn(cout, cin, k, k, generator=torch.Generator().manual_seed(k)).to(dtype)
+    fwd = conv._pack_weight(w, cin_p, cout_p)
+    bwd = conv._pack_weight(w.flip(2, 3).transpose(0, 1), cout_p, cin_p)
+    assert torch.equal(conv._forward_operand(w.cuda(), cin_p, cout_p).cpu(), fwd)
+    assert torch.equal(conv._backward_operand(w.cuda(), cin_p, cout_p).cpu(), bwd)
