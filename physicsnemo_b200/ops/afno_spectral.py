@@ -101,7 +101,7 @@ class _AfnoFilterTcFn(torch.autograd.Function):
     def forward(ctx, tokens, w1, b1, w2, b2, geo: FilterGeometry, lam: float, exchange, add_input=False, residual=None):
         lib = _lib_af()
         dev = tokens.device
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.stream()
         g = geo
         rows, ld, cb2 = g.B * g.H, g.nblk * g.Cb, 2 * g.Cb
         own = slice(g.blk0, g.blk0 + g.nblk)
@@ -146,7 +146,7 @@ class _AfnoFilterTcFn(torch.autograd.Function):
         w1e, w2e, Z, O1, O2 = ctx.saved_tensors
         g, exchange, lam = ctx.geo, ctx.exchange, ctx.lam
         dev = dout.device
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.stream()
         rows, ld, cb2 = g.B * g.H, g.nblk * g.Cb, 2 * g.Cb
         dY2 = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
         dY = torch.empty_like(dY2)
@@ -223,7 +223,7 @@ class _AfnoFilterFn(torch.autograd.Function):
     def forward(ctx, tokens, w1, b1, w2, b2, geo: FilterGeometry, lam: float, exchange):
         lib = _lib_af()
         dev = tokens.device
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.stream()
         g = geo
         rows, ld = g.B * g.H, g.nblk * g.Cb
         Y = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
@@ -255,7 +255,7 @@ class _AfnoFilterFn(torch.autograd.Function):
         w1f, w2f, Z, O1, O2 = ctx.saved_tensors
         g, exchange = ctx.geo, ctx.exchange
         dev = dout.device
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.stream()
         rows, ld = g.B * g.H, g.nblk * g.Cb
         dY2 = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
         dY = torch.empty_like(dY2)
@@ -307,7 +307,7 @@ class TokenChannelExchange:
 
     def transform(self, lib, tokens, Yin, Yout, cols_fn, g: FilterGeometry, kw_in: int, kw_out: int):
         rt = self.rt
-        st = torch.cuda.current_stream().cuda_stream
+        st = _lib.stream()
         n = tokens.numel()
         src_view, src_ptrs = self.regions.region(n // 2, tokens.device)
         dst_view, dst_ptrs = self.regions.region(n // 2, tokens.device)

@@ -69,7 +69,7 @@ def flash_forward(q, k, v, is_causal: bool = False, scale: float | None = None, 
     lse = torch.empty(BH, Sq, dtype=torch.float32, device=q.device)
     err = _lib_fa().pnm_flash_attn_fwd(q3.data_ptr(), k3.data_ptr(), v3.data_ptr(), out.data_ptr(), lse.data_ptr(), BH, Sq, Skv, D,
                                        ldv, scale, int(bool(is_causal)), vt, int(P_IN_TMEM if p_in_tmem is None else p_in_tmem),
-                                       torch.cuda.current_stream().cuda_stream)
+                                       _lib.stream())
     if err:
         raise RuntimeError(f"pnm_flash_attn_fwd failed ({err})")
     _g.launch_count += 1

@@ -54,7 +54,7 @@ class _EDMConditioning(torch.autograd.Function):
         ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         err = _lib_cond().pnm_edm_conditioning(n32.data_ptr(), f32.data_ptr(), ptr(x32), w0c.data_ptr(), ptr(b0c), w1c.data_ptr(), ptr(b1c),
                                                out.data_ptr(), B, C, E, 1 if w0.dtype == torch.float32 else 0,
-                                               torch.cuda.current_stream().cuda_stream)
+                                               _lib.stream())
         if err:
             raise RuntimeError(f"pnm_edm_conditioning failed ({err})")
         _g.launch_count += 1

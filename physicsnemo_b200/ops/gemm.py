@@ -301,7 +301,7 @@ class _MlpChainFn(torch.autograd.Function):
                 w = F.pad(w, (0, 0, 0, (-n_true) % 8))
             b = biases[i]
             if b is not None:
-                b = b.detach().float().contiguous()
+                b = _f32(b)
                 if b.numel() != w.shape[0]:
                     b = F.pad(b, (0, w.shape[0] - b.numel()))
             last = i == n_layers - 1

@@ -42,7 +42,7 @@ def _lib_sm():
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    return _lib.stream()
 
 
 def softmax_rows_(s: torch.Tensor, scale: float, lse: Optional[torch.Tensor] = None) -> torch.Tensor:

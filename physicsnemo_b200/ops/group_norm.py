@@ -85,15 +85,14 @@ class _GroupNormFn(torch.autograd.Function):
         S = _slices(B, C, hw, lay, v)
         lib = _lib_gn()
         dev = x.device
-        gamma = weight.detach().float().contiguous()
-        beta = bias.detach().float().contiguous()
+        gamma, beta = _g._f32(weight), _g._f32(bias)
         y = torch.empty_like(x)                       # preserves the memory format
         mean = torch.empty(B * num_groups, dtype=torch.float32, device=dev)
         rstd = torch.empty_like(mean)
         scratch = torch.empty(lib.pnm_groupnorm_scratch_floats(B, C, num_groups, S), dtype=torch.float32, device=dev)
         err = lib.pnm_groupnorm_fwd(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mean.data_ptr(),
                                     rstd.data_ptr(), scratch.data_ptr(), B, C, hw, num_groups, S, lay, _DT[x.dtype],
-                                    int(silu), float(eps), torch.cuda.current_stream().cuda_stream)
+                                    int(silu), float(eps), _lib.stream())
         if err:
             raise RuntimeError(f"pnm_groupnorm_fwd failed ({err})")
         _g.launch_count += 2
@@ -121,7 +120,7 @@ class _GroupNormFn(torch.autograd.Function):
         scratch = torch.empty(lib.pnm_groupnorm_scratch_floats(B, C, G, S), dtype=torch.float32, device=dev)
         err = lib.pnm_groupnorm_bwd(x.data_ptr(), dy.data_ptr(), gamma.data_ptr(), beta.data_ptr(), mean.data_ptr(),
                                     rstd.data_ptr(), dx.data_ptr(), dgb[0].data_ptr(), dgb[1].data_ptr(), scratch.data_ptr(),
-                                    B, C, hw, G, S, lay, _DT[x.dtype], int(silu), torch.cuda.current_stream().cuda_stream)
+                                    B, C, hw, G, S, lay, _DT[x.dtype], int(silu), _lib.stream())
         if err:
             raise RuntimeError(f"pnm_groupnorm_bwd failed ({err})")
         _g.launch_count += 3
@@ -162,7 +161,7 @@ class _GroupNormShardedFn(torch.autograd.Function):
         err = lib.pnm_groupnorm_fwd_sharded(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mean.data_ptr(),
                                             rstd.data_ptr(), scratch.data_ptr(), B, C, hw, int(hw_global), num_groups, S,
                                             _DT[x.dtype], int(silu), float(eps), *rt.peer_args(rt.next_epoch()),
-                                            counter.data_ptr(), torch.cuda.current_stream().cuda_stream)
+                                            counter.data_ptr(), _lib.stream())
         if err:
             raise RuntimeError(f"pnm_groupnorm_fwd_sharded failed ({err})")
         _g.launch_count += 3
@@ -188,7 +187,7 @@ class _GroupNormShardedFn(torch.autograd.Function):
                                             rstd.data_ptr(), dx.data_ptr(), dgb[0].data_ptr(), dgb[1].data_ptr(),
                                             scratch.data_ptr(), B, C, hw, hw_global, G, S, _DT[x.dtype], int(silu),
                                             *rt.peer_args(rt.next_epoch()), _counter(rt).data_ptr(),
-                                            torch.cuda.current_stream().cuda_stream)
+                                            _lib.stream())
         if err:
             raise RuntimeError(f"pnm_groupnorm_bwd_sharded failed ({err})")
         _g.launch_count += 4

@@ -24,8 +24,8 @@ class _LayerNormFn(torch.autograd.Function):
         y = torch.empty_like(x2d)
         mean = torch.empty((M,), dtype=torch.float32, device=x2d.device)
         rstd = torch.empty((M,), dtype=torch.float32, device=x2d.device)
-        g32 = gamma.detach().float().contiguous()
-        b32 = beta.detach().float().contiguous() if beta is not None else None
+        g32 = _g._f32(gamma)
+        b32 = _g._f32(beta) if beta is not None else None
         code = lib.pnm_layernorm_fwd(x2d.data_ptr(), None, g32.data_ptr(), None if b32 is None else b32.data_ptr(),
                                      y.data_ptr(), None, mean.data_ptr(), rstd.data_ptr(),
                                      None if post is None else post.data_ptr(), M, C, float(eps),

@@ -28,7 +28,7 @@ def _lib_pa():
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    return _lib.stream()
 
 
 def _ptr_array(ptrs: Sequence[int]):

@@ -48,7 +48,7 @@ def _launch_unpatchify(tokens: torch.Tensor, image: torch.Tensor, dims, to_image
     """Run the kernel; False when it declines the shape (nothing was written then)."""
     B, h, w, p0, p1, C = dims
     rc = _lib_pl().pnm_unpatchify_bf16(tokens.data_ptr(), image.data_ptr(), B, h, w, p0, p1, C, int(to_image),
-                                       torch.cuda.current_stream().cuda_stream)
+                                       _lib.stream())
     if rc == -2:
         return False
     _g._check(rc, "pnm_unpatchify_bf16")
@@ -102,7 +102,7 @@ class _SquaredErrorFn(torch.autograd.Function):
         partial = torch.empty(lib.pnm_sq_err_partials(), dtype=torch.float32, device=p.device)
         out = torch.empty(1, dtype=torch.float32, device=p.device)
         rc = lib.pnm_sq_err_sum(p.data_ptr(), t.data_ptr(), p.numel(), _DTYPE_CODE[p.dtype], _DTYPE_CODE[t.dtype], float(scale),
-                                partial.data_ptr(), out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+                                partial.data_ptr(), out.data_ptr(), _lib.stream())
         _g._check(rc, "pnm_sq_err_sum")
         _g.launch_count += 2
         ctx.save_for_backward(p, t)
@@ -116,7 +116,7 @@ class _SquaredErrorFn(torch.autograd.Function):
         grad = torch.empty_like(p)
         rc = _lib_pl().pnm_sq_err_grad(p.data_ptr(), t.data_ptr(), g.data_ptr(), p.numel(), _DTYPE_CODE[p.dtype],
                                        _DTYPE_CODE[t.dtype], 2.0 * ctx.scale, grad.data_ptr(),
-                                       torch.cuda.current_stream().cuda_stream)
+                                       _lib.stream())
         _g._check(rc, "pnm_sq_err_grad")
         _g.launch_count += 1
         return grad, None, None

@@ -75,7 +75,7 @@ class _TokenAttention(torch.autograd.Function):
         out = torch.empty_like(qk)
         lse = torch.empty(P, H, dtype=torch.float32, device=qk.device)
         err = _lib_pa().pnm_pixel_attn_fwd(qk.data_ptr(), tokens.data_ptr(), cu32.data_ptr(), out.data_ptr(), lse.data_ptr(), P, H, Dt,
-                                           _DT[qk.dtype], torch.cuda.current_stream().cuda_stream)
+                                           _DT[qk.dtype], _lib.stream())
         if err:
             raise RuntimeError(f"pnm_pixel_attn_fwd failed ({err})")
         _g.launch_count += 1
@@ -96,7 +96,7 @@ class _TokenAttention(torch.autograd.Function):
                 else torch.empty(blocks, N, Dt, dtype=torch.float32, device=qk.device))
         err = _lib_pa().pnm_pixel_attn_bwd(qk.data_ptr(), tokens.data_ptr(), cu32.data_ptr(), dout.data_ptr(), lse.data_ptr(),
                                            delta.data_ptr(), dqk.data_ptr(), dtok.data_ptr(), P, H, Dt, N, int(atomic), _DT[qk.dtype],
-                                           torch.cuda.current_stream().cuda_stream)
+                                           _lib.stream())
         if err:
             raise RuntimeError(f"pnm_pixel_attn_bwd failed ({err})")
         _g.launch_count += 1
@@ -156,7 +156,7 @@ def counting_sort_and_pack(flat_idx: torch.Tensor, total_pixels: int) -> Tuple[t
     idx = flat_idx.to(torch.int32).contiguous()
     scratch = torch.zeros(2 * total_pixels + 1, dtype=torch.int32, device=idx.device)
     counts, cursor, bad = scratch[:total_pixels], scratch[total_pixels:2 * total_pixels], scratch[2 * total_pixels:]
-    st = torch.cuda.current_stream().cuda_stream
+    st = _lib.stream()
     err = lib.pnm_counting_histogram(idx.data_ptr(), counts.data_ptr(), n, total_pixels, bad.data_ptr(), st)
     if err:
         raise RuntimeError(f"pnm_counting_histogram failed ({err})")

@@ -34,7 +34,7 @@ def _run(x: torch.Tensor, mode: int, scale: float) -> torch.Tensor:
     n, c, h, w = x.shape
     ho, wo = (h // 2, w // 2) if mode == 0 else (2 * h, 2 * w)
     y = torch.empty((n, c, ho, wo), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
-    rc = _fn()(x.data_ptr(), y.data_ptr(), n, h, w, c, mode, float(scale), torch.cuda.current_stream().cuda_stream)
+    rc = _fn()(x.data_ptr(), y.data_ptr(), n, h, w, c, mode, float(scale), _lib.stream())
     _g._check(rc, "pnm_resample2x_nhwc")
     _g.launch_count += 1
     return y
@@ -93,7 +93,7 @@ class _AddScale(torch.autograd.Function):
     @staticmethod
     def forward(ctx, a, b, scale: float):
         out = torch.empty_like(a)
-        rc = _add_scale_fn()(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), float(scale), torch.cuda.current_stream().cuda_stream)
+        rc = _add_scale_fn()(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), float(scale), _lib.stream())
         _g._check(rc, "pnm_add_scale_bf16")
         _g.launch_count += 1
         ctx.scale = float(scale)
@@ -104,7 +104,7 @@ class _AddScale(torch.autograd.Function):
         g = g.contiguous(memory_format=torch.channels_last) if g.dim() == 4 and not g.is_contiguous() else g.contiguous() if not (
             g.is_contiguous() or (g.dim() == 4 and g.is_contiguous(memory_format=torch.channels_last))) else g
         d = torch.empty_like(g)
-        rc = _add_scale_fn()(g.data_ptr(), None, d.data_ptr(), g.numel(), ctx.scale, torch.cuda.current_stream().cuda_stream)
+        rc = _add_scale_fn()(g.data_ptr(), None, d.data_ptr(), g.numel(), ctx.scale, _lib.stream())
         _g._check(rc, "pnm_add_scale_bf16")
         _g.launch_count += 1
         return d, d, None                      # both branches receive the same scaled gradient

@@ -78,7 +78,7 @@ class _ShNorm(torch.autograd.Function):
         y = torch.empty_like(xc)
         err = _lib_sh().pnm_sh_norm_fwd(xc.data_ptr(), y.data_ptr(), a32.data_ptr(), None if b32 is None else b32.data_ptr(),
                                         w32.data_ptr(), m32.data_ptr(), g32.data_ptr(), B, L, M, C, float(eps), int(subtract_mean),
-                                        _DTYPES[x.dtype], torch.cuda.current_stream().cuda_stream)
+                                        _DTYPES[x.dtype], _lib.stream())
         if err:
             raise RuntimeError(f"pnm_sh_norm_fwd failed ({err})")
         _g.launch_count += 1
@@ -101,7 +101,7 @@ class _ShNorm(torch.autograd.Function):
         dbias = torch.empty(grid, C, dtype=torch.float32, device=xc.device)
         err = lib.pnm_sh_norm_bwd(xc.data_ptr(), dy.data_ptr(), dx.data_ptr(), a32.data_ptr(), w32.data_ptr(), m32.data_ptr(),
                                   g32.data_ptr(), daw.data_ptr(), dbias.data_ptr(), B, L, M, C, eps, sub, _DTYPES[xc.dtype], grid,
-                                  torch.cuda.current_stream().cuda_stream)
+                                  _lib.stream())
         if err:
             raise RuntimeError(f"pnm_sh_norm_bwd failed ({err})")
         _g.launch_count += 1

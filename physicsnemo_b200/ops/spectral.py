@@ -38,7 +38,7 @@ def _launch(a, a_p, a_r, a_modes, b, b_r, b_q, b_modes, out, o_p, o_q, o_modes, 
     shp, sa, sb, so = arr(shape, ctypes.c_int), arr(a_modes, ctypes.c_longlong), arr(b_modes, ctypes.c_longlong), arr(o_modes, ctypes.c_longlong)
     ch = arr([a_p, a_r, b_r, b_q, o_p, o_q], ctypes.c_longlong)
     err = _lib_sp().pnm_spectral_contract(a.data_ptr(), b.data_ptr(), out.data_ptr(), nd, shp, sa, sb, so, ch, P, Q, R, int(conj_a), int(conj_b),
-                                          int(accumulate), torch.cuda.current_stream().cuda_stream)
+                                          int(accumulate), _lib.stream())
     if err:
         raise RuntimeError(f"pnm_spectral_contract failed ({err})")
     _g.launch_count += 1
