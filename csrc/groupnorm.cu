@@ -53,9 +53,19 @@ template <> struct Vec<float> {
   }
 };
 
-__device__ __forceinline__ float gn_silu(float z) { return z / (1.f + __expf(-z)); }
+// Sigmoid in fp32.  For bf16 tensors by the two-ulp reciprocal (its error is 2^-16 of a bf16 ulp): the IEEE division costs ten
+// instructions an element and, worse, a slow path whose branch keeps the loads of the next pixels from being issued early.
+// Denominators beyond 2^126 give 0, which is the limit.
+template <typename T>
+__device__ __forceinline__ float gn_sigmoid(float z) {
+  const float d = 1.f + __expf(-z);
+  return sizeof(T) == 2 ? __fdividef(1.f, d) : 1.f / d;
+}
+template <typename T>
+__device__ __forceinline__ float gn_silu(float z) { return sizeof(T) == 2 ? z * gn_sigmoid<T>(z) : z / (1.f + __expf(-z)); }
+template <typename T>
 __device__ __forceinline__ float gn_silu_grad(float z) {
-  const float s = 1.f / (1.f + __expf(-z));
+  const float s = gn_sigmoid<T>(z);
   return s * (1.f + z * (1.f - s));
 }
 
@@ -125,7 +135,7 @@ __global__ void __launch_bounds__(256) gn_apply_cf(const T* __restrict__ x, cons
   for (long long v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
     Vec<T>::load(xi + v * V, f);
 #pragma unroll
-    for (int i = 0; i < V; ++i) { const float z = f[i] * scale + shift; f[i] = kSilu ? gn_silu(z) : z; }
+    for (int i = 0; i < V; ++i) { const float z = f[i] * scale + shift; f[i] = kSilu ? gn_silu<T>(z) : z; }
     Vec<T>::store(yo + v * V, f);
   }
 }
@@ -149,7 +159,7 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cf(const T* __restrict__ x, 
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const float xh = (f[i] - mu) * rs;
-      const float dz = kSilu ? e[i] * gn_silu_grad(xh * ga + be) : e[i];
+      const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga + be) : e[i];
       a += dz * xh; d += dz;
     }
   }
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(256) gn_bwd_apply_cf(const T* __restrict__ x, 
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const float xh = (f[i] - mu) * rs;
-      const float dz = kSilu ? e[i] * gn_silu_grad(xh * ga + be) : e[i];
+      const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga + be) : e[i];
       f[i] = rs * (ga * dz - A - xh * Bq);
     }
     Vec<T>::store(o + v * V, f);
@@ -351,7 +361,7 @@ __global__ void __launch_bounds__(256) gn_apply_cl_sh(const T* __restrict__ x, c
   for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
     Vec<T>::load(x + off + p * sh.C, f);
 #pragma unroll
-    for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu(z) : z; }
+    for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu<T>(z) : z; }
     Vec<T>::store(y + off + p * sh.C, f);
   }
 }
@@ -389,14 +399,14 @@ __global__ void __launch_bounds__(256) gn_bwd_apply_cl_sh(const T* __restrict__ 
     A[i] = gab[g].x * inv_n; Bq[i] = gab[g].y * inv_n;
   }
   const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 2
+#pragma unroll 4
   for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
     Vec<T>::load(x + off + p * sh.C, f);
     Vec<T>::load(dy + off + p * sh.C, e);
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const float xh = (f[i] - mu[i]) * rs[i];
-      const float dz = kSilu ? e[i] * gn_silu_grad(xh * ga[i] + be[i]) : e[i];
+      const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga[i] + be[i]) : e[i];
       f[i] = rs[i] * (ga[i] * dz - A[i] - xh * Bq[i]);
     }
     Vec<T>::store(dx + off + p * sh.C, f);
@@ -430,7 +440,7 @@ __global__ void __launch_bounds__(256) gn_apply_cl(const T* __restrict__ x, cons
   for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
     Vec<T>::load(x + off + p * sh.C, f);
 #pragma unroll
-    for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu(z) : z; }
+    for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu<T>(z) : z; }
     Vec<T>::store(y + off + p * sh.C, f);
   }
 }
@@ -456,14 +466,14 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
       a[i] = d[i] = 0.f;
     }
     const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 2
+#pragma unroll 4
     for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
       Vec<T>::load(x + off + p * sh.C, f);
       Vec<T>::load(dy + off + p * sh.C, e);
 #pragma unroll
       for (int i = 0; i < V; ++i) {
         const float xh = (f[i] - mu[i]) * rs[i];
-        const float dz = kSilu ? e[i] * gn_silu_grad(xh * ga[i] + be[i]) : e[i];
+        const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga[i] + be[i]) : e[i];
         a[i] += dz * xh; d[i] += dz;
       }
     }
@@ -508,14 +518,14 @@ __global__ void __launch_bounds__(256) gn_bwd_apply_cl(const T* __restrict__ x, 
     A[i] = ab.x * inv_n; Bq[i] = ab.y * inv_n;
   }
   const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 2
+#pragma unroll 4
   for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
     Vec<T>::load(x + off + p * sh.C, f);
     Vec<T>::load(dy + off + p * sh.C, e);
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const float xh = (f[i] - mu[i]) * rs[i];
-      const float dz = kSilu ? e[i] * gn_silu_grad(xh * ga[i] + be[i]) : e[i];
+      const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga[i] + be[i]) : e[i];
       f[i] = rs[i] * (ga[i] * dz - A[i] - xh * Bq[i]);
     }
     Vec<T>::store(dx + off + p * sh.C, f);
