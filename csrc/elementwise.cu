@@ -260,7 +260,95 @@ extern "C" int pnm_conv_pack_weight(const void* w, int is_bf16, void* out, int c
   const size_t smem = (size_t)rt * 64 * kk * sizeof(float);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
-  if (is_bf16) pnm::conv_pack_weight_kernel<<<grid, 256, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(w), o, cout, cin, kk, rows_p, cols_p, flip, rt);
-  else pnm::conv_pack_weight_kernel<<<grid, 256, smem, st>>>(reinterpret_cast<const float*>(w), o, cout, cin, kk, rows_p, cols_p, flip, rt);
+  const auto launch = [&](auto* src) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(src)>>;
+    if (kk == 9) pnm::conv_pack_weight_kernel<T, 9><<<grid, 256, smem, st>>>(src, o, cout, cin, kk, rows_p, cols_p, flip, rt);
+    else if (kk == 1) pnm::conv_pack_weight_kernel<T, 1><<<grid, 256, smem, st>>>(src, o, cout, cin, kk, rows_p, cols_p, flip, rt);
+    else pnm::conv_pack_weight_kernel<T, 0><<<grid, 256, smem, st>>>(src, o, cout, cin, kk, rows_p, cols_p, flip, rt);
+  };
+  if (is_bf16) launch(reinterpret_cast<const __nv_bfloat16*>(w));
+  else launch(reinterpret_cast<const float*>(w));
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
+}
+
+// ------------------------------------------------------------------------------------- per-image channel vectors (channels-last)
+namespace pnm {
+
+// y[b, p, c] = x[b, p, c] + v[b, c]: the injection of an embedding into a feature map.  As a broadcast tensor addition on a
+// channels-last map this ran at a quarter of the copy rate, and its gradient (the sum over the pixels) at a tenth.
+__global__ void __launch_bounds__(256) add_channel_kernel(const uint4* __restrict__ x, const uint4* __restrict__ v, uint4* __restrict__ y,
+                                                          long long per_image, int tpp, long long nvec) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
+    const long long b = i / per_image;
+    const uint4 a = x[i], s = __ldg(v + b * tpp + i % tpp);
+    const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, ws[4] = {s.x, s.y, s.z, s.w};
+    uint32_t wo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 p = unpack_bf16x2(wa[k]), q = unpack_bf16x2(ws[k]);
+      wo[k] = pack_bf16x2(p.x + q.x, p.y + q.y);
+    }
+    y[i] = make_uint4(wo[0], wo[1], wo[2], wo[3]);
+  }
+}
+
+// part[b][s][c] = sum of g[b, p, c] over the pixels of slice s; grid (S, B).  A thread owns 8 channels of every ppi-th pixel.
+__global__ void __launch_bounds__(256) channel_sum_kernel(const uint4* __restrict__ g, float* __restrict__ part, long long hw, int C) {
+  __shared__ float stage[256 * 8];
+  const int tpp = C / 8, ppi = 256 / tpp, chunk = threadIdx.x % tpp, lane = threadIdx.x / tpp;
+  const bool active = (int)threadIdx.x < tpp * ppi;
+  const long long per = (hw + gridDim.x - 1) / gridDim.x, p0 = blockIdx.x * per, p1 = p0 + per < hw ? p0 + per : hw;
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (active) {
+    const uint4* base = g + (long long)blockIdx.y * hw * tpp + chunk;
+#pragma unroll 4
+    for (long long p = p0 + lane; p < p1; p += ppi) {
+      const uint4 u = base[p * tpp];
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) { const float2 f = unpack_bf16x2(w[k]); a[2 * k] += f.x; a[2 * k + 1] += f.y; }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) stage[threadIdx.x * 8 + k] = a[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += 256) {
+    float s = 0.f;
+    for (int l = 0; l < ppi; ++l) s += stage[l * C + c];
+    part[((long long)blockIdx.y * gridDim.x + blockIdx.x) * C + c] = s;
+  }
+}
+
+// out[b][c] = sum over the slices, bf16; grid (ceil(C / 32), B), block (32, 8)
+__global__ void __launch_bounds__(256) channel_fold_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int S, int C) {
+  __shared__ float red[8][32];
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  float s = 0.f;
+  if (c < C)
+    for (int k = threadIdx.y; k < S; k += 8) s += part[((long long)blockIdx.y * S + k) * C + c];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < C) {
+    for (int k = 1; k < 8; ++k) s += red[k][threadIdx.x];
+    out[(long long)blockIdx.y * C + c] = __float2bfloat16(s);
+  }
+}
+
+}  // namespace pnm
+
+extern "C" int pnm_add_channel_bf16(const void* x, const void* v, void* y, int B, long long hw, int C, void* stream) {
+  if (B <= 0 || hw <= 0 || C <= 0 || (C & 7)) return -2;
+  const long long nvec = (long long)B * hw * (C / 8), blocks = (nvec + 255) / 256;
+  pnm::add_channel_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(
+      (const uint4*)x, (const uint4*)v, (uint4*)y, hw * (C / 8), C / 8, nvec);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// part: at least B * slices * C floats
+extern "C" int pnm_channel_sum_bf16(const void* g, void* out, float* part, int B, long long hw, int C, int slices, void* stream) {
+  if (B <= 0 || B > 65535 || hw <= 0 || C <= 0 || (C & 7) || C > 2048 || slices <= 0) return -2;
+  cudaStream_t st = (cudaStream_t)stream;
+  pnm::channel_sum_kernel<<<dim3(slices, B), 256, 0, st>>>((const uint4*)g, part, hw, C);
+  pnm::channel_fold_kernel<<<dim3((C + 31) / 32, B), dim3(32, 8), 0, st>>>(part, (__nv_bfloat16*)out, slices, C);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -27,6 +27,10 @@ int pnm_gemm_tn_stacked(const void* A, int lda, const void* B, int ldb, void* C,
 int pnm_gemm_nt_stacked(const void* A, int lda, const void* B, int ldb, float* out, float* colsum, int Mp, int Na, int Nb, int batch,
                         int max_ctas, void* stream);
 
+// Channels-last bf16 maps [B, hw, C], C % 8 == 0: y = x + v[b, c]; out[b, c] = sum over the pixels (fp32 partials in `part`,
+// B * slices * C floats; C <= 2048).
+int pnm_add_channel_bf16(const void* x, const void* v, void* y, int B, long long hw, int C, void* stream);
+int pnm_channel_sum_bf16(const void* g, void* out, float* part, int B, long long hw, int C, int slices, void* stream);
 // w [cout, cin, k, k] (fp32, or bf16 when is_bf16) -> out [rows_p, k*k, cols_p] bf16, zero-padded; rows / columns are output / input
 // channels, with `flip` input / output channels of the mirrored filter.
 int pnm_conv_pack_weight(const void* w, int is_bf16, void* out, int cout, int cin, int ksize, int rows_p, int cols_p, int flip,

@@ -76,7 +76,7 @@ class UNetBlock(torch.nn.Module):
             scale, shift = cond.chunk(2, dim=1)
             h = silu(torch.addcmul(shift, self.norm1(h), scale + 1))
         else:
-            h = self.norm1(h + cond)
+            h = self.norm1(_resample.add_channel(h, cond))
         h = self.conv1(torch.nn.functional.dropout(h, p=self.dropout, training=self.training))
         # residual join and rescaling in one pass (one kernel forward, one shared by both branches backward)
         h = _resample.add_scale(h, x if self.skip is None else self.skip(x), self.skip_scale)

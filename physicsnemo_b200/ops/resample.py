@@ -117,3 +117,52 @@ def add_scale(a: torch.Tensor, b: torch.Tensor, scale: float) -> torch.Tensor:
             and a.numel() % 8 == 0 and _same_dense_layout(a, b) and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and _lib.available()):
         return _AddScale.apply(a, b, scale)
     return (a + b) * scale
+
+
+def _channel_lib():
+    lib = _lib.load(required=True)
+    if not getattr(lib, "_channel_declared", False):
+        c = ctypes
+        vp, i, l = c.c_void_p, c.c_int, c.c_longlong
+        lib.pnm_add_channel_bf16.argtypes = [vp, vp, vp, i, l, i, vp]
+        lib.pnm_channel_sum_bf16.argtypes = [vp, vp, vp, i, l, i, i, vp]
+        lib.pnm_add_channel_bf16.restype = lib.pnm_channel_sum_bf16.restype = i
+        lib._channel_declared = True
+    return lib
+
+
+class _AddChannel(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, v):
+        b, c, h, w = x.shape
+        y = torch.empty_like(x)
+        rc = _channel_lib().pnm_add_channel_bf16(x.data_ptr(), v.data_ptr(), y.data_ptr(), b, h * w, c, _lib.stream())
+        _g._check(rc, "pnm_add_channel_bf16")
+        _g.launch_count += 1
+        return y
+
+    @staticmethod
+    def backward(ctx, g):
+        dv = None
+        if ctx.needs_input_grad[1]:
+            g = g.contiguous(memory_format=torch.channels_last)
+            b, c, h, w = g.shape
+            # two CTAs per SM, at least eight passes of a CTA's pixels each
+            slices = max(1, min(2 * 148 // b, h * w // (8 * max(1, 2048 // c))))
+            dv = torch.empty(b, c, 1, 1, dtype=torch.bfloat16, device=g.device)
+            part = torch.empty(b * slices * c, dtype=torch.float32, device=g.device)
+            rc = _channel_lib().pnm_channel_sum_bf16(g.data_ptr(), dv.data_ptr(), part.data_ptr(), b, h * w, c, slices, _lib.stream())
+            _g._check(rc, "pnm_channel_sum_bf16")
+            _g.launch_count += 2
+        return g, dv
+
+
+def add_channel(x: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
+    """``x + v`` for a feature map ``x [B, C, H, W]`` and channel vectors ``v [B, C, 1, 1]``; own kernels (the gradient of ``v``
+    is one reduction over the pixels) for channels-last bf16 maps, the PyTorch expression otherwise."""
+    if (type(x) is torch.Tensor and type(v) is torch.Tensor and x.is_cuda and v.is_cuda and x.dtype == v.dtype == torch.bfloat16
+            and x.dim() == 4 and x.numel() > 0 and v.shape == (*x.shape[:2], 1, 1) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048
+            and x.shape[0] <= 65535 and x.is_contiguous(memory_format=torch.channels_last) and v.is_contiguous()
+            and x.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0 and _lib.available()):
+        return _AddChannel.apply(x, v)
+    return x + v
