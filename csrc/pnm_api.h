@@ -297,6 +297,12 @@ int pnm_afno_cols_dft(const void* Y, void* E, const void* mask, const int* geom,
 int pnm_afno_rows_c2r_add(const void* X, void* out, const void* add0, const void* add1, const int* geom, long long Tp, int kweight,
                           void* stream);
 int pnm_afno_cols_idft(const void* E, void* Yout, const int* geom, int Mp, float lambda, void* stream);
+// Block weights w [2, nb, cb, cb], biases b [2, nb, cb] (fp32) of both layers -> real matrices e [nblk, 2 cb (out), 2 cb (in)] bf16 and
+// biases be [nblk, 2 cb] of the blocks blk0 .. blk0 + nblk - 1; the gradients of all blocks back.
+int pnm_afno_expand_weights(const float* w1, const float* b1, const float* w2, const float* b2, void* e1, float* be1, void* e2,
+                            float* be2, int nb, int blk0, int nblk, int cb, void* stream);
+int pnm_afno_fold_grads(const float* de1, const float* dbe1, const float* de2, const float* dbe2, float* dw1, float* db1, float* dw2,
+                        float* db2, int nb, int cb, void* stream);
 
 // out = (a + b) * scale over n bf16 elements (n % 8 == 0; b may be null)
 int pnm_add_scale_bf16(const void* a, const void* b, void* out, long long n, float scale, void* stream);

@@ -32,8 +32,10 @@ def _lib_af():
         lib.pnm_afno_cols_bwd.argtypes = [vp] * 11 + [i, vp, vp]
         lib.pnm_afno_cols_dft.argtypes = [vp, vp, vp, vp, i, f, vp]
         lib.pnm_afno_cols_idft.argtypes = [vp, vp, vp, i, f, vp]
+        lib.pnm_afno_expand_weights.argtypes = [vp] * 8 + [i, i, i, i, vp]
+        lib.pnm_afno_fold_grads.argtypes = [vp] * 8 + [i, i, vp]
         for n in ("pnm_afno_rows_r2c", "pnm_afno_rows_c2r", "pnm_afno_rows_c2r_add", "pnm_afno_cols_fwd", "pnm_afno_cols_bwd", "pnm_afno_cols_dft",
-                  "pnm_afno_cols_idft"):
+                  "pnm_afno_cols_idft", "pnm_afno_expand_weights", "pnm_afno_fold_grads"):
             getattr(lib, n).restype = i
         lib._afno_declared = True
     return lib
@@ -92,6 +94,22 @@ def _fold_weight_grad(dwe: torch.Tensor, cb: int) -> torch.Tensor:
     return torch.stack([(a + d).transpose(1, 2), (c - b).transpose(1, 2)])
 
 
+def _expand_parameters(w1, b1, w2, b2, g):
+    """``(w1e, b1e, w2e, b2e)`` of the blocks this rank owns: bf16 matrices and fp32 biases, one launch for fp32 parameters."""
+    if not all(t.dtype == torch.float32 and t.is_contiguous() for t in (w1, b1, w2, b2)):
+        own = slice(g.blk0, g.blk0 + g.nblk)
+        be = [torch.cat([b.detach()[0, own], b.detach()[1, own]], dim=1).float().contiguous() for b in (b1, b2)]
+        return _expand_weight(w1.detach()[:, own]), be[0], _expand_weight(w2.detach()[:, own]), be[1]
+    cb2 = 2 * g.Cb
+    e = torch.empty(2, g.nblk, cb2, cb2, dtype=torch.bfloat16, device=w1.device)
+    be = torch.empty(2, g.nblk, cb2, dtype=torch.float32, device=w1.device)
+    rc = _lib_af().pnm_afno_expand_weights(w1.data_ptr(), b1.data_ptr(), w2.data_ptr(), b2.data_ptr(), e[0].data_ptr(), be[0].data_ptr(),
+                                           e[1].data_ptr(), be[1].data_ptr(), g.nb, g.blk0, g.nblk, g.Cb, _lib.stream())
+    _g._check(rc, "pnm_afno_expand_weights")
+    _g.launch_count += 1
+    return e[0], be[0], e[1], be[1]
+
+
 class _AfnoFilterTcFn(torch.autograd.Function):
     """The filter with its block MLP on the tensor cores: Fourier kernels write / read the ``[real | imag]`` bf16
     expansion of the spectrum, the two complex layers are ``gemm_tn`` calls with bias / ReLU epilogues, their backward
@@ -104,16 +122,13 @@ class _AfnoFilterTcFn(torch.autograd.Function):
         st = _lib.stream()
         g = geo
         rows, ld, cb2 = g.B * g.H, g.nblk * g.Cb, 2 * g.Cb
-        own = slice(g.blk0, g.blk0 + g.nblk)
         Y = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
         Y2 = torch.empty_like(Y)
         Z = torch.empty(g.nblk, g.Mp, cb2, dtype=torch.bfloat16, device=dev)
         if g.Mp > g.Mb:
             Z[:, g.Mb:].zero_()                                   # rows that pad a block to the GEMM's M tile
         O1, O2 = torch.empty_like(Z), torch.empty_like(Z)
-        w1e, w2e = _expand_weight(w1.detach()[:, own]), _expand_weight(w2.detach()[:, own])
-        b1e = torch.cat([b1.detach()[0, own], b1.detach()[1, own]], dim=1).float().contiguous()
-        b2e = torch.cat([b2.detach()[0, own], b2.detach()[1, own]], dim=1).float().contiguous()
+        w1e, b1e, w2e, b2e = _expand_parameters(w1, b1, w2, b2, g)
 
         def cols():
             _g._check(lib.pnm_afno_cols_dft(Y.data_ptr(), Z.data_ptr(), None, g.arr, g.Mp, 0.0, st), "pnm_afno_cols_dft")
@@ -183,6 +198,15 @@ class _AfnoFilterTcFn(torch.autograd.Function):
         _g.launch_count += 4
         dt = ctx.dtypes
         own = slice(g.blk0, g.blk0 + g.nblk)
+
+        if g.nblk == g.nb and all(t == torch.float32 for t in dt):
+            dws = torch.empty(2, 2, g.nb, g.Cb, g.Cb, dtype=torch.float32, device=dev)
+            dbs = torch.empty(2, 2, g.nb, g.Cb, dtype=torch.float32, device=dev)
+            rc = lib.pnm_afno_fold_grads(dw1e.data_ptr(), db1e.data_ptr(), dw2e.data_ptr(), db2e.data_ptr(), dws[0].data_ptr(),
+                                         dbs[0].data_ptr(), dws[1].data_ptr(), dbs[1].data_ptr(), g.nb, g.Cb, st)
+            _g._check(rc, "pnm_afno_fold_grads")
+            _g.launch_count += 1
+            return dx, dws[0], dbs[0], dws[1], dbs[1], None, None, None, None, (d if ctx.has_residual else None)
 
         def scatter(part, shape, dtype):
             if g.nblk == g.nb:                       # this rank owns every block: nothing to embed

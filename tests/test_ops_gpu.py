@@ -844,3 +844,47 @@ def test_conv_weight_packing_matches_the_tensor_operations(cout, cin, k, cin_p, 
     bwd = conv._pack_weight(w.flip(2, 3).transpose(0, 1), cout_p, cin_p)
     assert torch.equal(conv._forward_operand(w.cuda(), cin_p, cout_p).cpu(), fwd)
     assert torch.equal(conv._backward_operand(w.cuda(), cin_p, cout_p).cpu(), bwd)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,cb,blk0,nblk", [(1, 8, 0, 1), (8, 96, 0, 8), (8, 96, 6, 2), (3, 40, 0, 3), (4, 128, 2, 1)])
+def test_afno_parameter_kernels_match_the_tensor_operations(nb, cb, blk0, nblk):
+    """A permutation, a sign and one rounding: equal; the folded gradients are the same fp32 sums."""
+    from types import SimpleNamespace
+
+    from physicsnemo_b200.ops import afno_spectral as af
+
+    gen = torch.Generator().manual_seed(cb)
+    w, b = [[torch.randn(2, nb, *s, generator=gen).cuda() for _ in range(2)] for s in ((cb, cb), (cb,))]
+    g = SimpleNamespace(nb=nb, Cb=cb, blk0=blk0, nblk=nblk)
+    own = slice(blk0, blk0 + nblk)
+    got = af._expand_parameters(w[0], b[0], w[1], b[1], g)
+    for k in range(2):
+        assert torch.equal(got[2 * k], af._expand_weight(w[k][:, own]))
+        assert torch.equal(got[2 * k + 1], torch.cat([b[k][0, own], b[k][1, own]], dim=1))
+    if nblk == nb:
+        de, dbe = [[torch.randn(nb, *s, generator=gen).cuda() for _ in range(2)] for s in ((2 * cb, 2 * cb), (2 * cb,))]
+        dw, db = torch.empty(2, 2, nb, cb, cb, device="cuda"), torch.empty(2, 2, nb, cb, device="cuda")
+        rc = af._lib_af().pnm_afno_fold_grads(de[0].data_ptr(), dbe[0].data_ptr(), de[1].data_ptr(), dbe[1].data_ptr(), dw[0].data_ptr(),
+                                              db[0].data_ptr(), dw[1].data_ptr(), db[1].data_ptr(), nb, cb, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        for k in range(2):
+            assert torch.equal(dw[k], af._fold_weight_grad(de[k], cb))
+            assert torch.equal(db[k], torch.stack([dbe[k][:, :cb], dbe[k][:, cb:]]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,c,h,w", [(1, 8, 1, 1), (2, 24, 5, 7), (3, 128, 33, 64), (1, 2048, 9, 3), (2, 512, 64, 64)])
+def test_channel_vector_addition(b, c, h, w):
+    from physicsnemo_b200.ops import resample
+
+    gen = torch.Generator().manual_seed(c)
+    x = torch.randn(b, c, h, w, generator=gen).bfloat16().cuda().contiguous(memory_format=torch.channels_last).requires_grad_()
+    v = torch.randn(b, c, 1, 1, generator=gen).bfloat16().cuda().requires_grad_()
+    g = torch.randn(b, c, h, w, generator=gen).bfloat16().cuda()
+    y = resample.add_channel(x, v)
+    y.backward(g)
+    assert torch.equal(y, x.detach() + v.detach()) and torch.equal(x.grad, g)
+    ref = g.double().sum((2, 3), keepdim=True)
+    # fp32 sums of h * w values of size one, then one bf16 rounding of the result
+    assert float((v.grad.double() - ref).abs().max()) <= 2 ** -8 * float(ref.abs().max()) + 1e-5 * (h * w) ** 0.5
