@@ -114,7 +114,7 @@ class _Mlp3LnFn(torch.autograd.Function):
         m, dev = z1.shape[0], z1.device
         dy = dy.contiguous()
         lib = _lib_mlp()
-        # dW3, dW2, their biases, db1 and the blocks of dW1 in one zeroed buffer
+        # dW3, dW2, their biases, db1 and the blocks of dW1 of the plain sources in one zeroed buffer
         sizes = [WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 3 + [WIDTH * WIDTH] * n
         acc = torch.zeros(sum(sizes), dtype=torch.float32, device=dev).split(sizes)
         dw3, dw2 = acc[0].view(WIDTH, WIDTH), acc[1].view(WIDTH, WIDTH)
@@ -154,13 +154,15 @@ class _Mlp3LnFn(torch.autograd.Function):
                                                  pairs.stride(0), rows, WIDTH, _g._stream())
                 _g._check(code, "pnm_segment_sum_split")
                 _g.launch_count += 1
+            # every sum against the table in one product; the two halves of a sum are added afterwards
+            both = torch.zeros(pairs.shape[1] * (WIDTH + 1), dtype=torch.float32, device=dev)
+            part = both[:pairs.shape[1] * WIDTH].view(-1, WIDTH)
+            _g.gemm_nt(pairs, src, out=part, colsum_out=None if summed_bias else both[part.numel():])
+            blocks = part.view(len(js), 2, WIDTH, WIDTH).sum(1)
             for k, j in enumerate(js):
-                for h in (2 * k, 2 * k + 1):
-                    hl = pairs[:, h * WIDTH:(h + 1) * WIDTH]
-                    if summed_bias:
-                        _g.gemm_nt(hl, src, out=dw1[j])
-                    else:
-                        _g.gemm_nt(hl, src, out=dw1[j], colsum_out=db1)
+                dw1[j] = blocks[k]
+            if not summed_bias:
+                db1 = both[part.numel():].view(len(js), 2, WIDTH)[0].sum(0)
                 summed_bias = True
             if any(need[j] for j in js):
                 wt = torch.cat([w1t[j * WIDTH:(j + 1) * WIDTH] for j in js for _ in range(2)], 1)
