@@ -245,15 +245,34 @@ __device__ __forceinline__ void cl_fold_slices(const float2* part, float2* out, 
   if (threadIdx.x == 0) counter[b] = 0;
 }
 
+// Sums a[i], q[i] over the threads that share a channel, into sums[c] = (sum a, sum q): the values of all threads are laid out in
+// `stage` (2 x 256 x V floats) and every channel is added up by one thread, in a fixed order.  (Shared-memory atomics serialise on
+// the pixels of a channel.  512 x 512, 256 and 128 channels together: 99 -> 80 us.  The backward statistics keep theirs: there the
+// larger staging cost more than it gave, 222 against 260 us.)
+template <int V>
+__device__ __forceinline__ void cl_channel_sums(const CLThread& t, const float* a, const float* q, float* stage, float2* sums, int C) {
+  float* sa = stage + threadIdx.x * V;
+  float* sq = stage + blockDim.x * V + threadIdx.x * V;
+#pragma unroll
+  for (int i = 0; i < V; ++i) { sa[i] = t.active ? a[i] : 0.f; sq[i] = t.active ? q[i] : 0.f; }
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {
+    float x = 0.f, y = 0.f;
+    for (int l = 0; l < t.ppi; ++l) { x += stage[l * C + c]; y += stage[blockDim.x * V + l * C + c]; }
+    sums[c] = make_float2(x, y);
+  }
+  __syncthreads();
+}
+constexpr size_t cl_stats_smem(int V, int C) { return (2 * 256 * (size_t)V + 2 * (size_t)C) * sizeof(float); }
+
 // part[b][s][g] = (sum x, sum x^2) of slice s; gsum[b][g] = their sum over the slices (written by the last CTA of item b)
 template <typename T>
 __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, float2* __restrict__ part, float2* __restrict__ gsum,
                                                     GNShape sh) {
   constexpr int V = Vec<T>::N;
-  extern __shared__ float smem[];                        // [C][2]
+  extern __shared__ float smem[];                        // staging of cl_channel_sums, then [C] sums
   const int s = blockIdx.x, b = blockIdx.y;
-  for (int i = threadIdx.x; i < 2 * sh.C; i += blockDim.x) smem[i] = 0.f;
-  __syncthreads();
+  float2* sums = reinterpret_cast<float2*>(smem + 2 * 256 * V);
   const CLThread t = cl_thread<V>(sh, s);
   float a[V], q[V], f[V];
 #pragma unroll
@@ -266,13 +285,11 @@ __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, floa
 #pragma unroll
       for (int i = 0; i < V; ++i) { a[i] += f[i]; q[i] += f[i] * f[i]; }
     }
-#pragma unroll
-    for (int i = 0; i < V; ++i) { atomicAdd(&smem[2 * (t.c0 + i)], a[i]); atomicAdd(&smem[2 * (t.c0 + i) + 1], q[i]); }
   }
-  __syncthreads();
+  cl_channel_sums<V>(t, a, q, smem, sums, sh.C);
   for (int g = threadIdx.x; g < sh.G; g += blockDim.x) {
     float a2 = 0.f, q2 = 0.f;
-    for (int k = 0; k < sh.cpg; ++k) { a2 += smem[2 * (g * sh.cpg + k)]; q2 += smem[2 * (g * sh.cpg + k) + 1]; }
+    for (int k = 0; k < sh.cpg; ++k) { a2 += sums[g * sh.cpg + k].x; q2 += sums[g * sh.cpg + k].y; }
     part[((long long)b * sh.S + s) * sh.G + g] = make_float2(a2, q2);
   }
   cl_fold_slices(part, gsum, g_gn_fwd_counter, sh, b);
@@ -568,7 +585,7 @@ int gn_forward(const void* x, const float* gamma, const float* beta, void* y, fl
   } else {
     const dim3 grid(sh.S, sh.B);
     float2* gsum = partial + (long long)sh.B * sh.S * sh.G;
-    gn_stats_cl<T><<<grid, 256, 2 * sh.C * sizeof(float), st>>>(xi, partial, gsum, sh);
+    gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, sh);
     if (act) gn_apply_cl<T, true><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gsum, gamma, beta, yo, mean, rstd, sh, eps);
     else gn_apply_cl<T, false><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gsum, gamma, beta, yo, mean, rstd, sh, eps);
   }
@@ -612,7 +629,7 @@ int gn_forward_sh(const void* x, const float* gamma, const float* beta, void* y,
   T* yo = static_cast<T*>(y);
   const dim3 grid(sh.S, sh.B);
   float2* gsum = partial + (long long)sh.B * sh.S * sh.G;
-  gn_stats_cl<T><<<grid, 256, 2 * sh.C * sizeof(float), st>>>(xi, partial, gsum, sh);
+  gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, sh);
   gn_publish_moments<<<sh.B, 256, 0, st>>>(gsum, sh, peer, counter);
   if (act) gn_apply_cl_sh<T, true><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gamma, beta, yo, mean, rstd, sh, eps, count_global, peer, err);
   else gn_apply_cl_sh<T, false><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gamma, beta, yo, mean, rstd, sh, eps, count_global, peer, err);
@@ -642,7 +659,7 @@ static bool gn_supported(const GNShape& sh, int layout, int dtype) {
   const int V = dtype == 0 ? 8 : 4;
   if (sh.B <= 0 || sh.C <= 0 || sh.G <= 0 || sh.C % sh.G || sh.S <= 0 || sh.HW <= 0) return false;
   if (layout == 0) return sh.HW % V == 0 && (long long)sh.B * sh.C <= 65535;
-  return sh.C % V == 0 && sh.C / V <= 256 && sh.B <= 65535 && 2 * sh.C * sizeof(float) <= 48 * 1024;
+  return sh.C % V == 0 && sh.C / V <= 256 && sh.B <= 65535 && cl_stats_smem(V, sh.C) <= 48 * 1024;
 }
 
 }  // namespace pnm
