@@ -259,8 +259,8 @@ __device__ __forceinline__ float ex2_poly(float x) {
 }
 // GELU in its tanh form (|gelu_tanh - gelu_erf| < 1e-3, below bf16 resolution for O(1) values).
 __device__ __forceinline__ float gelu_f(float x) {
-  float u = x * (0.7978845608f + 0.0356774081f * x * x);
-  return 0.5f * x * (1.f + tanh_fast(u));
+  const float u = x * (0.7978845608f + 0.0356774081f * x * x), h = 0.5f * x;
+  return fmaf(h, tanh_fast(u), h);
 }
 __device__ __forceinline__ float gelu_grad_f(float x) {
   float x2 = x * x;
@@ -269,7 +269,10 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
   float du = 0.7978845608f + 0.1070322243f * x2;
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
 }
-__device__ __forceinline__ float silu_f(float x) { return x * (0.5f + 0.5f * tanh_fast(0.5f * x)); }
+__device__ __forceinline__ float silu_f(float x) {
+  const float h = 0.5f * x;
+  return fmaf(h, tanh_fast(h), h);
+}
 __device__ __forceinline__ float silu_grad_f(float x) {
   float s = 0.5f + 0.5f * tanh_fast(0.5f * x);
   return s * (1.f + x * (1.f - s));

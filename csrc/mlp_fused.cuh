@@ -4,9 +4,11 @@
 //   h2 = act(h1 W2^T + b2)
 //   y  = LayerNorm(h2 W3^T + b3) * gamma + beta (+ post)
 //
-// What bounds it: memory.  An edge row needs its own 256 bytes, two gathered node rows (mostly from L2) and 256 bytes of
-// result; run layer by layer the same chain moves fifteen such rows through HBM.  Here everything between the sources and
-// the result stays on the SM:
+// An edge row needs its own 256 bytes, two gathered node rows (mostly from L2) and 256 bytes of result; run layer by layer the
+// same chain moves fifteen such rows through HBM.  Here everything between the sources and the result stays on the SM, and what
+// is left is the latency of a tile's chain (product, epilogue, product, epilogue, product, normalisation):
+// 1.5 M rows from three sources take 0.56 ms (0.66 ms with the pre-activations kept), one source 0.34 ms, where the rows'
+// own traffic is worth 0.2 ms.  A MeshGraphNet step on 250 k nodes / 1.4 M edges, forward: 1.26 -> 0.70 ms.
 //   * W1, W2, W3 (96 + 32 + 32 KB in bf16 for three sources) are loaded once per persistent CTA and stay in shared memory;
 //   * gathered rows arrive by TMA gather4 (four indexed rows of 128 bytes per instruction, written in the same 128-byte
 //     swizzle as a plain tile), so no gathered copy of the node features exists;
@@ -361,8 +363,10 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
         for (int j = 0; j < 4; ++j) {
           const float4 b = vb[j], ga = vb[j + kMlpW / 4], be = vb[j + kMlpW / 2];
           const float2 r0 = unpack_bf16x2(res.w[2 * j]), r1 = unpack_bf16x2(res.w[2 * j + 1]);   // zeros without a residual
-          p[2 * j] = pack_bf16x2((v[4 * j] + b.x - mean) * rstd * ga.x + be.x + r0.x, (v[4 * j + 1] + b.y - mean) * rstd * ga.y + be.y + r0.y);
-          p[2 * j + 1] = pack_bf16x2((v[4 * j + 2] + b.z - mean) * rstd * ga.z + be.z + r1.x, (v[4 * j + 3] + b.w - mean) * rstd * ga.w + be.w + r1.y);
+          const float h0 = (v[4 * j] + b.x - mean) * rstd, h1 = (v[4 * j + 1] + b.y - mean) * rstd, h2 = (v[4 * j + 2] + b.z - mean) * rstd,
+                      h3 = (v[4 * j + 3] + b.w - mean) * rstd;
+          p[2 * j] = pack_bf16x2(fmaf(h0, ga.x, be.x) + r0.x, fmaf(h1, ga.y, be.y) + r0.y);
+          p[2 * j + 1] = pack_bf16x2(fmaf(h2, ga.z, be.z) + r1.x, fmaf(h3, ga.w, be.w) + r1.y);
         }
         if (live) stg32(g.y + row * g.ld_y + col + c * 16, p);
         res = next;
