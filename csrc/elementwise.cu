@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "pnm_api.h"
@@ -224,13 +225,16 @@ namespace pnm {
 // with `flip`, input channels of the mirrored filter (the operand of the input gradient).  Tensor operations take a padded,
 // permuted copy, a cast and, for the gradient, two flips: up to four launches per use of a weight that is a few hundred KB.  A
 // block moves RT rows x 64 columns through shared memory: both sides are read and written in runs.
-template <typename T>
+// KK = 0: any filter size; 1 and 9 are compiled in (the index arithmetic is most of the kernel's instructions).
+template <typename T, int KK>
 __global__ void __launch_bounds__(256) conv_pack_weight_kernel(const T* __restrict__ w, __nv_bfloat16* __restrict__ out, int cout, int cin,
-                                                               int kk, int rows_p, int cols_p, int flip, int rt) {
+                                                               int kk_any, int rows_p, int cols_p, int flip, int rt_any) {
   extern __shared__ float cw[];                  // [rt][64][kk]
+  const int kk = KK ? KK : kk_any, rt = KK ? 8 : rt_any;
   const int r0 = blockIdx.x * rt, c0 = blockIdx.y * 64;
   const int rows = flip ? cin : cout, cols = flip ? cout : cin;
   const int n = rt * 64 * kk;
+#pragma unroll 6
   for (int i = threadIdx.x; i < n; i += 256) {
     int r, c, t;                                 // the fastest index is the one that is contiguous in w
     t = i % kk;
@@ -275,7 +279,8 @@ extern "C" int pnm_conv_pack_weight(const void* w, int is_bf16, void* out, int c
 namespace pnm {
 
 // y[b, p, c] = x[b, p, c] + v[b, c]: the injection of an embedding into a feature map.  As a broadcast tensor addition on a
-// channels-last map this ran at a quarter of the copy rate, and its gradient (the sum over the pixels) at a tenth.
+// channels-last map this ran at a quarter of the copy rate, and its gradient (the sum over the pixels) at a tenth: 512 x 512 x 128
+// 79 -> 22 us and 182 -> 32 us.
 __global__ void __launch_bounds__(256) add_channel_kernel(const uint4* __restrict__ x, const uint4* __restrict__ v, uint4* __restrict__ y,
                                                           long long per_image, int tpp, long long nvec) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {

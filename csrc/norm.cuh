@@ -16,14 +16,13 @@ constexpr int kLnMaxVec = 4;  // supports C up to 32 lanes * 8 elems * 4 = 1024
 // the kernel is bound by instruction issue, not by memory (ncu: warps stall "not selected" / on the shuffle chains while
 // DRAM is ~50 % busy); two rows per warp halve the instructions per row.  This form is for the fused residual add; without
 // `r` the streaming kernel below runs.
-template <int VEC, bool HAS_R, int LPR = 32>
+template <int VEC, int LPR>
 __global__ void __launch_bounds__(kLnWarps * 32, VEC == 1 ? 3 : 2)
-layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ r_in,
+layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ r,
                      const float* __restrict__ gamma, const float* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                      __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                      const __nv_bfloat16* __restrict__ post, long long M, int C, float eps) {
   constexpr int RW = 32 / LPR;                            // rows per warp and step
-  const __nv_bfloat16* r = HAS_R ? r_in : nullptr;      // without the second input its ring of registers disappears
   const int lane = threadIdx.x & 31, l = lane % LPR, sub = lane / LPR;
   const long long first = ((long long)blockIdx.x * kLnWarps + (threadIdx.x >> 5)) * RW + sub;
   const long long stride = (long long)gridDim.x * kLnWarps * RW;
@@ -46,7 +45,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
       const int c = (v * LPR + l) * 8;
       const bool live = row < M && c < C;
       nx[slot][v] = live ? *reinterpret_cast<const uint4*>(x + row * C + c) : make_uint4(0u, 0u, 0u, 0u);
-      if (HAS_R) nr[slot][v] = live ? *reinterpret_cast<const uint4*>(r + row * C + c) : make_uint4(0u, 0u, 0u, 0u);
+      nr[slot][v] = live ? *reinterpret_cast<const uint4*>(r + row * C + c) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
 #pragma unroll
@@ -62,7 +61,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
       float s = 0.f;
       uint4 cx[VEC], cr[VEC];
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) { cx[v] = nx[d][v]; if (HAS_R) cr[v] = nr[d][v]; }
+      for (int v = 0; v < VEC; ++v) { cx[v] = nx[d][v]; cr[v] = nr[d][v]; }
       fetch(d, row + D * stride);
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
@@ -70,19 +69,17 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
         if (c < C) {
           const uint4 u = cx[v];
           const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-          uint32_t rw[4] = {0, 0, 0, 0};
-          if (HAS_R) {
-            const uint4 ur = cr[v];
-            rw[0] = ur.x; rw[1] = ur.y; rw[2] = ur.z; rw[3] = ur.w;
-          }
+          const uint4 ur = cr[v];
+          const uint32_t rw[4] = {ur.x, ur.y, ur.z, ur.w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             float2 f = unpack_bf16x2(w[j]);
-            if (HAS_R) { float2 fr = unpack_bf16x2(rw[j]); f.x += fr.x; f.y += fr.y; }
+            const float2 fr = unpack_bf16x2(rw[j]);
+            f.x += fr.x; f.y += fr.y;
             val[v][2 * j] = f.x; val[v][2 * j + 1] = f.y;
             s += f.x + f.y;
           }
-          if (HAS_R && sum_out && in) {
+          if (sum_out && in) {
             uint4 o;
             o.x = pack_bf16x2(val[v][0], val[v][1]); o.y = pack_bf16x2(val[v][2], val[v][3]);
             o.z = pack_bf16x2(val[v][4], val[v][5]); o.w = pack_bf16x2(val[v][6], val[v][7]);
@@ -489,7 +486,7 @@ inline int launch_layernorm_fwd(const void* x, const void* r, const float* gamma
   const long long resident = (long long)num_sms * (C <= 128 ? 3 : 2);
   int grid = (int)(want < resident * 2 ? want : resident * 2);
   if (grid < 1) grid = 1;
-#define PNM_LN_FWD(V, L) layernorm_fwd_kernel<V, true, L><<<grid, kLnWarps * 32, 0, st>>>(X, R, gamma, beta, Y, S, mean, rstd, P, M, C, eps)
+#define PNM_LN_FWD(V, L) layernorm_fwd_kernel<V, L><<<grid, kLnWarps * 32, 0, st>>>(X, R, gamma, beta, Y, S, mean, rstd, P, M, C, eps)
   if (C <= 128) { PNM_LN_FWD(1, 16); }
   else if (C <= 256) { PNM_LN_FWD(2, 16); }
   else if (C <= 512) { PNM_LN_FWD(2, 32); }
