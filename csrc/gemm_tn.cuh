@@ -116,7 +116,7 @@ struct GemmCfg {
   static constexpr int EPI = BN / 16;         // epilogue warps: 4 lane quarters x (BN / 64) column blocks
   static constexpr int THREADS = 64 + 32 * EPI;
   // staging buffers of a warp: the auxiliary tile of the next block is prefetched while this one is worked on (128 columns: two
-  // ahead); two outputs alternate.  256 columns without either leave the shared memory to the operand stages.
+  // ahead); two outputs alternate.  256 columns without an auxiliary tile leave the shared memory to the operand stages.
   static constexpr int NBUF = BN == 256 ? (MODE == MODE_PLAIN ? 1 : 2) : (MODE == MODE_AUX ? 3 : 2);
   static constexpr int STAGE_BYTES = kBM * kBK * 2 + BN * kBK * 2;
   static constexpr int STAGING = EPI * NBUF * kChunkBytes;
