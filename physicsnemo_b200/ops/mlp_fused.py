@@ -110,7 +110,8 @@ class _Mlp3LnFn(torch.autograd.Function):
     def backward(ctx, dy):
         segs, post = ctx.segs, ctx.post
         n = len(segs)
-        srcs, (w1, w2, w3, gamma, z1, z2, x3, mean, rstd) = ctx.saved_tensors[:n], ctx.saved_tensors[n:]
+        saved = ctx.saved_tensors                            # read once: activation checkpointing allows no second time
+        srcs, (w1, w2, w3, gamma, z1, z2, x3, mean, rstd) = saved[:n], saved[n:]
         m, dev = z1.shape[0], z1.device
         dy = dy.contiguous()
         lib = _lib_mlp()

@@ -73,3 +73,31 @@ def test_mlp3_ln_takes_the_same_calls_as_the_layered_path():
                 y = m(x)
             assert _rel(y.cpu(), m.double()(x.double()).detach().cpu()) < 1e-2
             m.float()
+
+
+@pytest.mark.gpu
+def test_mlp3_ln_under_activation_checkpointing():
+    """Checkpointing recomputes the forward and unpacks every saved tensor once: same gradients as without."""
+    from torch.utils.checkpoint import checkpoint
+
+    from physicsnemo_b200.nn.module.gnn_layers.graph_types import Graph
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_edge_block import MeshEdgeBlock
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_node_block import MeshNodeBlock
+
+    torch.manual_seed(0)
+    edge, node = MeshEdgeBlock(W, W, W, W, 2).cuda(), MeshNodeBlock("mean", W, W, W, W, 2).cuda()
+    graph = Graph(torch.randint(0, 301, (2, 1500)).cuda(), num_nodes=301)
+    e, v = torch.randn(1500, W, device="cuda").bfloat16(), torch.randn(301, W, device="cuda").bfloat16()
+    grads = []
+    for wrap in (lambda f, *a: f(*a), lambda f, *a: checkpoint(f, *a, use_reentrant=False)):
+        leaves = [e.clone().requires_grad_(), v.clone().requires_grad_()]
+        params = [*edge.parameters(), *node.parameters()]
+        for p in params:
+            p.grad = None
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            out = wrap(lambda a, b: node(*edge(a, b, graph), graph), *leaves)
+        torch.autograd.backward(out, [torch.ones_like(t) for t in out])
+        grads.append([t.grad.clone() for t in (*leaves, *params)])
+    for a, b in zip(*grads):
+        # the same kernels on the same values; only the order of fp32 atomic additions differs
+        assert _rel(a, b.double()) < 1e-4
