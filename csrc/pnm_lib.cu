@@ -115,12 +115,16 @@ int pnm_gemm_tn(const void* A, int lda, const void* A2, int lda2, const void* A3
     if (Z) return pnm::launch_gemm_tn_pair<256, pnm::MODE_Z>(c, g_num_sms, g_err_ptr, st);
     return pnm::launch_gemm_tn_pair<256, pnm::MODE_PLAIN>(c, g_num_sms, g_err_ptr, st);
   }
-  // An auxiliary operand: 256-column tiles read A once per 256 columns of the result; with fewer of them than SMs, 128-column
-  // tiles use more SMs (GELU', 256 -> 512: 73 row tiles as 128 columns 18.4 us, 74 as 256 columns 14.2 us; 1 M rows, 256 -> 1024:
-  // 1.40 and 0.99 ms).  Two outputs: 128-column tiles, whose eight warps have two staging buffers and six operand stages (40 000 rows,
-  // GELU, 256 -> 1024: 44 us against 52 us with 256 columns, 1 M rows 1.03 against 1.21 ms).
-  const bool wide = N > 128 && (long long)((M + 127) / 128) * ((N + 255) / 256) >= g_num_sms;
-  if (AUX) return wide && act != pnm::ACT_SOFTMAX64 ? pnm::launch_gemm_tn<256, pnm::MODE_AUX>(c, g_num_sms, g_err_ptr, st)
+  // An auxiliary operand with arithmetic on it (GELU', SiLU', softmax backward): 256-column tiles, whose sixteen epilogue warps hide
+  // it and which read A once per 256 columns (1 M rows: GELU' 256 -> 1024 1.40 -> 0.99 ms, SiLU' 256 -> 512 0.76 -> 0.51 ms, softmax
+  // backward 512 -> 512 1.28 -> 0.83 ms); with fewer of them than SMs, 128-column tiles use more SMs (GELU' 256 -> 512: 73 row tiles
+  // as 128 columns 18.4 us, 74 as 256 columns 14.2 us).  A plain addition or a mask gains nothing (1 M rows, 256 -> 512: 0.49 ms
+  // either way; 512 -> 512 0.76 against 0.84 ms) and stays on 128 columns, as do two outputs (40 000 rows, GELU, 256 -> 1024: 44
+  // against 52 us).
+  const bool arithmetic = aux_mode == pnm::AUX_DGELU || aux_mode == pnm::AUX_DSILU || aux_mode == pnm::AUX_DSOFTMAX;
+  const bool wide = arithmetic && act != pnm::ACT_SOFTMAX64 && N > 128 &&
+                    (long long)((M + 127) / 128) * ((N + 255) / 256) >= g_num_sms;
+  if (AUX) return wide ? pnm::launch_gemm_tn<256, pnm::MODE_AUX>(c, g_num_sms, g_err_ptr, st)
                        : pnm::launch_gemm_tn<128, pnm::MODE_AUX>(c, g_num_sms, g_err_ptr, st);
   if (Z) return pnm::launch_gemm_tn<128, pnm::MODE_Z>(c, g_num_sms, g_err_ptr, st);
   if (bn == 0) {
