@@ -65,7 +65,8 @@ segment_sum_split_kernel(const __nv_bfloat16* __restrict__ in, const int* __rest
     for (int j = 0; j < 4; ++j) {
       hi[j] = pack_bf16x2(acc[2 * j], acc[2 * j + 1]);
       const float2 f = unpack_bf16x2(hi[j]);
-      lo[j] = pack_bf16x2(acc[2 * j] - f.x, acc[2 * j + 1] - f.y);
+      // a sum that is not finite in bf16 stays what it is: inf - inf must not make it NaN
+      lo[j] = pack_bf16x2(fabsf(f.x) < 3.4e38f ? acc[2 * j] - f.x : 0.f, fabsf(f.y) < 3.4e38f ? acc[2 * j + 1] - f.y : 0.f);
     }
     __nv_bfloat16* dst = out + n * ldo + c;
     *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);

@@ -128,7 +128,8 @@ class _Mlp3LnFn(torch.autograd.Function):
                                      dx3.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), norm[2 * WIDTH:].data_ptr(), m, WIDTH,
                                      _g._stream())
         _g._check(code, "pnm_layernorm_bwd")
-        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), _w_t(w3).data_ptr(), _w_t(w2).data_ptr(), ctx.act,
+        w3t, w2t = _w_t(w3), _w_t(w2)                        # held: the second look-up may empty the cache
+        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), w3t.data_ptr(), w2t.data_ptr(), ctx.act,
                                 g1.data_ptr(), dw3.data_ptr(), dw2.data_ptr(), db3.data_ptr(), db2.data_ptr(), m, _g._stream())
         _g._check(code, "pnm_mlp3_bwd")
         _g.launch_count += 3

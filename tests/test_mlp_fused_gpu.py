@@ -101,3 +101,25 @@ def test_mlp3_ln_under_activation_checkpointing():
     for a, b in zip(*grads):
         # the same kernels on the same values; only the order of fp32 atomic additions differs
         assert _rel(a, b.double()) < 1e-4
+
+
+@pytest.mark.gpu
+def test_split_segment_sums_keep_the_fp32_sum_and_its_infinities():
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+    from physicsnemo_b200.ops import gemm as G
+
+    x = torch.randn(500, W, device="cuda").bfloat16()
+    index = torch.arange(500, device="cuda") % 7                       # segments 7, 8 and 9 are empty
+    x[0, :4] = torch.tensor([float("inf"), -float("inf"), float("nan"), 3.3e38], device="cuda").bfloat16()
+    x[7, 3] = 3.3e38                                                   # finite rows whose sum is not
+    seg = ops.SegmentIndex(index, 10)
+    out = torch.empty(10, 2 * W, dtype=torch.bfloat16, device="cuda")
+    rc = mf._lib_mlp().pnm_segment_sum_split(x.data_ptr(), seg.perm.data_ptr(), seg.offsets.data_ptr(), out.data_ptr(), 2 * W, 10, W, G._stream())
+    assert rc == 0
+    got = out[:, :W].double() + out[:, W:].double()
+    ref = torch.zeros(10, W, device="cuda", dtype=torch.float64).index_add_(0, index, x.double())
+    assert torch.isposinf(got[0, 0]) and torch.isneginf(got[0, 1]) and torch.isnan(got[0, 2]) and torch.isposinf(got[0, 3])
+    got[0, :4] = ref[0, :4] = 0
+    # two bf16 parts carry 16 bits of the sum
+    assert float((got - ref).abs().max()) <= 2 ** -16 * float(ref.abs().max()) + 1e-5
