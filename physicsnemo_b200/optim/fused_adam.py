@@ -236,6 +236,9 @@ class FusedAdam(Optimizer):
                                          hyper.data_ptr() if hyper is not None else None)
                 if err:
                     raise RuntimeError(f"pnm_adam_multi failed with CUDA error {err}")
+                # the kernel writes through raw pointers: whatever is derived from a parameter (its bf16 copies, what autograd
+                # saved) sees a change by the version counter alone
+                torch.autograd.graph.increment_version(fused)
                 self.kernel_launches += 1
                 _g.launch_count += 1
         return loss

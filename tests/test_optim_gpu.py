@@ -91,3 +91,30 @@ def test_fused_adam_capturable_resume_keeps_step_count():
         b.grad = g.clone()
         ref.step()
     assert torch.allclose(a2, b, atol=1e-5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("width,layers", [(128, 2), (256, 1)])       # one kernel for the whole MLP; layer by layer
+def test_fused_adam_step_reaches_the_next_forward(width, layers):
+    """The MLPs work on bf16 copies of their matrices: a step must be seen by the next forward and by its backward."""
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_graph_mlp import MeshGraphMLP
+
+    m = MeshGraphMLP(width, width, width, layers, torch.nn.SiLU()).cuda()
+    opt = FusedAdam(m.parameters(), lr=5e-2)
+    x = torch.randn(300, width, device="cuda").bfloat16()
+    for step in range(3):
+        leaf = x.clone().requires_grad_()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = m(leaf)
+        opt.zero_grad()
+        y.backward(x)
+        twin = MeshGraphMLP(width, width, width, layers, torch.nn.SiLU()).double().cuda()
+        twin.load_state_dict(m.state_dict())
+        ref_leaf = x.double().requires_grad_()
+        ref = twin(ref_leaf)
+        ref.backward(x.double())
+        # bf16 products against 64 bits; the step moves every weight by about half its spread
+        assert (y.double() - ref).norm() < 1.5e-2 * ref.norm(), step
+        assert (leaf.grad.double() - ref_leaf.grad).norm() < 3e-2 * ref_leaf.grad.norm(), step
+        versions = [p._version for p in m.parameters()]
+        opt.step()
+        assert all(p._version > v for p, v in zip(m.parameters(), versions))
