@@ -248,27 +248,51 @@ def fused_path_enabled(x: torch.Tensor) -> bool:
 
 
 _wcache: dict = {}
+_captured: dict = {}         # id -> weak reference of every parameter that a captured graph reads
 
 
 def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     """bf16 (optionally transposed) copy of a parameter, cached until the parameter changes.
 
     An entry belongs to ONE tensor object (the parameter itself, or the one that ``w`` is a view of), held by a weak reference:
-    a later parameter may get the id, the address and the version of one that is gone."""
+    a later parameter may get the id, the address and the version of one that is gone.
+
+    Under stream capture the conversion goes into the graph, whose replays then read the parameter as it is at that time.  What
+    else a graph does to a parameter (the optimizer step of a captured training step) leaves no trace in its version, so from then
+    on nothing is kept of that parameter."""
     if w.dtype == torch.bfloat16 and not transpose:
         return w.detach()
     owner = w if w._base is None else w._base
+    if w.is_cuda and torch.cuda.is_current_stream_capturing():
+        _captured[id(owner)] = _weak(owner, _captured, id(owner))
+        return _to_bf16(w, transpose)
+    ref = _captured.get(id(owner))
+    if ref is not None and ref() is owner:
+        return _to_bf16(w, transpose)
     key = (id(owner), transpose)
     ver = (w._version, w.data_ptr(), tuple(w.shape), w.stride())
     hit = _wcache.get(key)
     if hit is not None and hit[2]() is owner and hit[0] == ver:
         return hit[1]
-    src = w.detach()
-    val = (src.t() if transpose else src).to(torch.bfloat16).contiguous()
+    val = _to_bf16(w, transpose)
     if len(_wcache) > 4096:
         _wcache.clear()
     _wcache[key] = (ver, val, weakref.ref(owner))
     return val
+
+
+def _to_bf16(w: torch.Tensor, transpose: bool) -> torch.Tensor:
+    src = w.detach()
+    return (src.t() if transpose else src).to(torch.bfloat16).contiguous()
+
+
+def _weak(owner: torch.Tensor, table: dict, key) -> weakref.ref:
+    """Weak reference to ``owner`` that takes ``table[key]`` away when ``owner`` goes (unless another tensor has that key by then)."""
+    def gone(ref):
+        held = table.get(key)
+        if (held[2] if isinstance(held, tuple) else held) is ref:
+            table.pop(key, None)
+    return weakref.ref(owner, gone)
 
 
 def _pad_cols(t: torch.Tensor, mult: int = 8) -> torch.Tensor:

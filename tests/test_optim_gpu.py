@@ -118,3 +118,36 @@ def test_fused_adam_step_reaches_the_next_forward(width, layers):
         versions = [p._version for p in m.parameters()]
         opt.step()
         assert all(p._version > v for p, v in zip(m.parameters(), versions))
+
+
+def test_captured_step_trains_the_matrices_it_reads():
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.utils.capture import GraphedStep
+
+    w = torch.nn.Parameter(torch.randn(64, 128, device="cuda") / 128 ** 0.5)
+    opt = FusedAdam([w], lr=5e-2, capturable=True)
+    x = torch.randn(256, 128, device="cuda").bfloat16().requires_grad_()
+    before = torch.empty_like(w)
+
+    def step(t):
+        t.grad = w.grad = None
+        before.copy_(w.detach())
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = ops.linear(t, w)
+        y.square().mean().backward()
+        opt.step()
+        return y.detach(), t.grad
+
+    step(x)
+    graphed = GraphedStep(step, [x], warmup=1)
+    for k in range(3):
+        y, dx = graphed()
+        ref = x.detach().double() @ before.double().t()
+        gref = (2 / ref.numel()) * ref @ before.double()
+        assert (y.double() - ref).norm() < 1e-2 * ref.norm(), k
+        assert (dx.double() - gref).norm() < 2e-2 * gref.norm(), k
+        # a forward between replays: the graph changed the parameter, and its version does not say so
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            now = ops.linear(x.detach(), w)
+        ref = x.detach().double() @ w.detach().double().t()
+        assert (now.double() - ref).norm() < 1e-2 * ref.norm(), k
