@@ -269,7 +269,8 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     ref = _captured.get(id(owner))
     if ref is not None and ref() is owner:
         return _to_bf16(w, transpose)
-    key = (id(owner), transpose)
+    # views of one tensor (the parts of a stacked matrix, say) have entries of their own
+    key = (id(owner), transpose) if owner is w else (id(owner), transpose, w.data_ptr(), tuple(w.shape), w.stride())
     ver = (w._version, w.data_ptr(), tuple(w.shape), w.stride())
     hit = _wcache.get(key)
     if hit is not None and hit[2]() is owner and hit[0] == ver:

@@ -22,3 +22,14 @@ def test_views_of_one_parameter_share_its_life():
     first = G._bf16_weight(a.reshape(4, 8))
     assert G._bf16_weight(a.reshape(4, 8)) is first and first.shape == (4, 8)
     assert G._bf16_weight(a.reshape(8, 4)).shape == (8, 4)
+
+
+def test_views_used_in_turn_keep_their_copies():
+    p = torch.nn.Parameter(torch.randn(3 * 8, 8))
+    views = [*p.chunk(3), p[:8].t(), p]
+    first = [G._bf16_weight(v) for v in views]
+    assert all(G._bf16_weight(v) is f for v, f in zip(views, first))
+    assert all(torch.equal(f, v.detach().bfloat16()) for v, f in zip(views, first))
+    with torch.no_grad():
+        p.mul_(2)
+    assert all(torch.equal(G._bf16_weight(v), 2 * f) for v, f in zip(views, first))
