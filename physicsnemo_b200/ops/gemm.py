@@ -255,7 +255,7 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     """bf16 (optionally transposed) copy of a parameter, cached until the parameter changes.
 
     An entry belongs to ONE tensor object (the parameter itself, or the one that ``w`` is a view of), held by a weak reference:
-    a later parameter may get the id, the address and the version of one that is gone.
+    a later parameter may get the id, the address and the version of one that is gone.  It goes with that object.
 
     Under stream capture the conversion goes into the graph, whose replays then read the parameter as it is at that time.  What
     else a graph does to a parameter (the optimizer step of a captured training step) leaves no trace in its version, so from then
@@ -278,7 +278,7 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     val = _to_bf16(w, transpose)
     if len(_wcache) > 4096:
         _wcache.clear()
-    _wcache[key] = (ver, val, weakref.ref(owner))
+    _wcache[key] = (ver, val, _weak(owner, _wcache, key))
     return val
 
 

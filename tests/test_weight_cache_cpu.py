@@ -1,4 +1,6 @@
 """The cached bf16 copy of a parameter belongs to that parameter alone."""
+import gc
+
 import torch
 
 from physicsnemo_b200.ops import gemm as G
@@ -33,3 +35,14 @@ def test_views_used_in_turn_keep_their_copies():
     with torch.no_grad():
         p.mul_(2)
     assert all(torch.equal(G._bf16_weight(v), 2 * f) for v, f in zip(views, first))
+
+
+def test_copies_go_with_their_parameter():
+    gc.collect()
+    before = set(G._wcache)
+    p = torch.nn.Parameter(torch.randn(8, 8))
+    G._bf16_weight(p), G._bf16_weight(p, transpose=True), G._bf16_weight(p[:4])
+    assert len(set(G._wcache) - before) == 3
+    del p
+    gc.collect()
+    assert set(G._wcache) <= before
