@@ -262,15 +262,21 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     on nothing is kept of that parameter."""
     if w.dtype == torch.bfloat16 and not transpose:
         return w.detach()
-    owner = w if w._base is None else w._base
-    if w.is_cuda and torch.cuda.is_current_stream_capturing():
+    base = w._base
+    owner = w if base is None else base
+    stream = _stream() if w.is_cuda else 0
+    if stream and torch.cuda.is_current_stream_capturing():          # the default stream (0) cannot be captured
         _captured[id(owner)] = _weak(owner, _captured, id(owner))
         return _to_bf16(w, transpose)
-    ref = _captured.get(id(owner))
-    if ref is not None and ref() is owner:
-        return _to_bf16(w, transpose)
-    # views of one tensor (the parts of a stacked matrix, say) have entries of their own
-    key = (id(owner), transpose) if owner is w else (id(owner), transpose, w.data_ptr(), tuple(w.shape), w.stride())
+    if _captured:
+        ref = _captured.get(id(owner))
+        if ref is not None and ref() is owner:
+            return _to_bf16(w, transpose)
+    # Each stream has copies of its own: one that another stream was asked to make need not be there yet.  So do the views of one
+    # tensor (the parts of a stacked matrix, say).
+    key = (id(owner), transpose, stream) if stream else (id(owner), transpose)
+    if base is not None:
+        key += (w.storage_offset(), tuple(w.shape), w.stride())
     ver = (w._version, w.data_ptr(), tuple(w.shape), w.stride())
     hit = _wcache.get(key)
     if hit is not None and hit[2]() is owner and hit[0] == ver:

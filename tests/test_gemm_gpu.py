@@ -223,3 +223,21 @@ def test_gemm_tn_cta_pair_tiles(M, N, K, mode):
     _close(out, ref)
     assert (out.float() - single.float()).abs().max().item() <= 2e-2 * ref.abs().max().item()
     assert ops.device_error() == 0
+
+
+def test_weight_copy_of_another_stream_is_not_used_before_it_is_made():
+    w = torch.nn.Parameter(torch.randn(256, 128, device="cuda"))
+    ref = w.detach().bfloat16()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(100_000_000)                   # about 50 ms: the conversion below waits behind it
+        first = G._bf16_weight(w)
+    with torch.cuda.stream(other):
+        got = G._bf16_weight(w).clone()
+        other.synchronize()
+        assert torch.equal(got, ref) and G._bf16_weight(w) is not first
+    with torch.cuda.stream(busy):
+        assert G._bf16_weight(w) is first
+    torch.cuda.synchronize()
+    assert torch.equal(first, ref)
