@@ -144,10 +144,8 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
     for (int ph = 0; ph < phases; ++ph) {
       const bool second = ph & 1;
       // first phase: dx3 from TMA; second: g2 from the group's warps
-      // (every phase of `ready` is waited for in turn: the parity of the last tile's second phase looks like this tile's)
-      const bool ok = second ? mbar_wait(&ready[grp], 0, abort_flag, g.err, ERR_WAIT_AUX) &&
-                                   mbar_wait(&ready[grp], 1, abort_flag, g.err, ERR_WAIT_AUX)
-                             : mbar_wait(&dfull[grp], (ph >> 1) & 1, abort_flag, g.err, ERR_WAIT_AUX);
+      bool ok = second ? mbar_wait(&ready[grp], 1, abort_flag, g.err, ERR_WAIT_AUX)
+                       : mbar_wait(&dfull[grp], (ph >> 1) & 1, abort_flag, g.err, ERR_WAIT_AUX);
       if (!__all_sync(0xffffffffu, ok)) break;
       float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 16
@@ -155,6 +153,13 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         const uint2 v = *reinterpret_cast<const uint2*>(x + r * 128 + ((u ^ (r & 7)) << 4) + low);
         const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y);
         t[0] += a.x; t[1] += a.y; t[2] += b.x; t[3] += b.y;
+      }
+      // Every phase of `ready` is seen in turn, and this warp arrives on `done` only after it has seen the one before: without that
+      // arrival the group cannot complete the next.  (Waited for after the arrival, a phase could be over and the next of the same
+      // parity be awaited, which itself needs this warp.)  The products wait for the same phase, so nothing is delayed.
+      if (!second) {
+        ok = mbar_wait(&ready[grp], 0, abort_flag, g.err, ERR_WAIT_AUX);
+        if (!__all_sync(0xffffffffu, ok)) break;
       }
       __syncwarp();
       if (lane == 0) {

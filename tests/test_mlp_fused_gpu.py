@@ -123,3 +123,30 @@ def test_split_segment_sums_keep_the_fp32_sum_and_its_infinities():
     got[0, :4] = ref[0, :4] = 0
     # two bf16 parts carry 16 bits of the sum
     assert float((got - ref).abs().max()) <= 2 ** -16 * float(ref.abs().max()) + 1e-5
+
+
+@pytest.mark.gpu
+def test_mlp3_backward_beside_other_work():
+    """Many tiles per CTA while other kernels share the SMs and the memory, so that the roles of a CTA run at other speeds: every
+    pass gives the sums of the first, and no wait runs out."""
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    rows = 148 * 128 * 9 + 65
+    x, up = (torch.randn(rows, W, device="cuda").bfloat16() for _ in range(2))
+    p = [t.cuda().requires_grad_() for t in (*(torch.randn(W, W) / W ** 0.5 for _ in range(3)), *(0.1 * torch.randn(W) for _ in range(3)),
+                                             1 + 0.1 * torch.randn(W), 0.1 * torch.randn(W))]
+    big = torch.randn(1 << 26, device="cuda")
+    side, first = torch.cuda.Stream(), None
+    for k in range(25):
+        with torch.cuda.stream(side):
+            for _ in range(k % 4):
+                big.mul_(1.0)
+        leaf = x.clone().requires_grad_()
+        grads = torch.autograd.grad(mf.mlp3_ln([leaf], [None], p[:3], p[3:6], 2, p[6], p[7], 1e-5, 0), [leaf, *p], up)
+        first = first or grads
+        assert torch.equal(grads[0], first[0])
+        # sums over rows: the same addends, another order of the fp32 additions of the CTAs
+        assert all(_rel(a, b.double()) < 1e-5 for a, b in zip(grads[1:], first[1:]))
+    torch.cuda.synchronize()
+    assert ops.device_error() == 0
