@@ -140,6 +140,7 @@ layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
 // worth 60 % of the HBM rate); a ring of bulk copies holds 190 KB whatever the registers do.  One producer warp, eight
 // consumer warps; a stage is a run of whole rows, i.e. ONE contiguous copy per tensor (rows are C * 2 bytes, a multiple of 16).
 constexpr int kLnStreamThreads = (kLnWarps + 1) * 32;
+constexpr int kLnFoldBytes = kLnWarps * 2 * 264 * 4;   // column sums of the warps of a backward CTA
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
@@ -270,7 +271,9 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
   constexpr int RW = 32 / LPR;                   // rows per warp and step (two for C <= 128: half a warp would idle)
   extern __shared__ __align__(128) uint8_t ln_smem[];
   const uint32_t tile_bytes = uint32_t(stage_rows) * C * 2, stage_bytes = tile_bytes * (dres ? 3 : 2);
-  uint64_t* full = reinterpret_cast<uint64_t*>(ln_smem + size_t(stages) * stage_bytes);
+  // the barriers and the flag lie behind the ring AND behind the fold, which is the larger of the two for C <= 32
+  const size_t ring_bytes = size_t(stages) * stage_bytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ln_smem + (ring_bytes > kLnFoldBytes ? ring_bytes : kLnFoldBytes));
   uint64_t* empty = full + stages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + stages);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane % LPR, sub = lane / LPR;
@@ -384,7 +387,7 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
   // consumers (after a wait that ran out the results are void, but copies may still land: the ring is not touched then)
   __syncthreads();
   if (*abort_flag) return;
-  float* red = reinterpret_cast<float*>(ln_smem);   // [warps][2][264]
+  float* red = reinterpret_cast<float*>(ln_smem);   // kLnFoldBytes: [warps][2][264]
   constexpr int COLS = LPR * 8;                     // columns one vector slot covers
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
@@ -447,9 +450,8 @@ inline LnStream ln_stream_plan(long long M, int C, int tensors, int least_rows, 
   p.stages = budget / stage < 2 ? 2 : (budget / stage > 8 ? 8 : budget / stage);
   const long long tiles = (M + rows - 1) / rows, cap = (long long)num_sms * per_sm;
   p.grid = int(tiles < cap ? tiles : cap);
-  p.smem = p.stages * stage + p.stages * 16 + 16;
-  const int fold = kLnWarps * 2 * 264 * 4;       // the backward folds its warps in the ring
-  if (p.smem < fold) p.smem = fold;
+  const int ring = p.stages * stage;             // the backward folds its warps in the ring's place
+  p.smem = (ring > kLnFoldBytes ? ring : kLnFoldBytes) + p.stages * 16 + 16;
   return p;
 }
 template <typename K>

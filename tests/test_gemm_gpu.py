@@ -132,6 +132,37 @@ def test_layernorm(C):
     _close(b.grad, br.grad, tol=2e-2)
 
 
+def _layernorm_against_64_bits(M, C, post=False, residual=False):
+    """One forward and backward; bf16 results carry one rounding (2^-9 at most, 1.7e-3 in the 2-norm), the column sums are fp32."""
+    x, r, dy, dr = (_rand(M, C) for _ in range(4))
+    w, b = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda")
+    got = [t.clone().requires_grad_(True) for t in (x, r, w, b)]
+    ref = [t.double().requires_grad_(True) for t in (x, r, w, b)]
+    y = ops.layer_norm(got[0], got[2], got[3], post=got[1] if post else None, return_residual=residual)
+    yr = torch.nn.functional.layer_norm(ref[0], (C,), ref[2], ref[3]) + (ref[1] if post else 0)
+    if residual:
+        y, alias = y
+        torch.autograd.backward([y, alias], [dy, dr])
+        torch.autograd.backward([yr, ref[0] * 1], [dy.double(), dr.double()])
+    else:
+        y.backward(dy)
+        yr.backward(dy.double())
+    rel = lambda a, e: float((a.double() - e).norm() / e.norm())  # noqa: E731
+    assert rel(y.detach(), yr.detach()) < 4e-3 and rel(got[0].grad, ref[0].grad) < 4e-3
+    assert rel(got[2].grad, ref[2].grad) < 2e-5 and rel(got[3].grad, ref[3].grad) < 2e-5
+    if post:
+        assert torch.equal(got[1].grad, dy)
+
+
+@pytest.mark.parametrize("M", [1, 1531, 60001])
+@pytest.mark.parametrize("C", [8, 16, 24, 32, 40])
+def test_layernorm_narrow_rows(M, C):
+    """Rows so short that the fold of the column sums is larger than the ring of row tiles."""
+    for _ in range(5):
+        _layernorm_against_64_bits(M, C)
+    assert ops.device_error() == 0
+
+
 def test_mlp_chain_matches_torch():
     M = 2050
     x = _rand(M, 6).requires_grad_(True)
