@@ -86,6 +86,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Bounded wait that never raises the abort flag: lets a copy in flight land before the CTA leaves.  `parity` is that of the phase
+// that the copy completes and must be the barrier's last: any wait for the other parity is over at once.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, parity)) {
+    if (globaltimer_ns() - t0 > kWaitBudgetNs) break;
+  }
+}
+// The same for a ring of which `issued` stages were filled so far, one after the other.
+__device__ __forceinline__ void ring_drain(uint64_t* full, uint32_t stages, uint32_t issued) {
+  for (uint32_t i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_drain(&full[i % stages], (i / stages) & 1);
+}
+// After a wait that ran out: time for products in flight (a microsecond each) to retire before their TMEM is freed.
+__device__ __forceinline__ void abort_settle() {
+  const unsigned long long t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < 200000ull) {}
+}
+
 // --------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

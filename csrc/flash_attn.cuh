@@ -57,14 +57,6 @@ __host__ __device__ constexpr int flash_kv_stages() { return D == 64 ? 4 : 2; } 
 template <int D>
 constexpr int flash_smem_bytes() { return 1024 + (1 + 2 * flash_kv_stages<D>()) * (128 * D * 2) + 2 * (128 * 128 * 2) + kFaBarBytes; }
 
-// Bounded wait that never raises the abort flag: used to let copies in flight land before an aborted CTA leaves.
-__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
-  const unsigned long long t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (globaltimer_ns() - t0 > kWaitBudgetNs) break;
-  }
-}
-
 template <int D, bool VT, bool PTM>
 __global__ void __launch_bounds__(kFaThreads, 1) flash_fwd_kernel(const __grid_constant__ FlashArgs g) {
   static_assert(D == 64 || D == 128, "head dimension 64 or 128");

@@ -264,11 +264,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tma_load_2d(sb, &tmB, &full[s], k, nt * BN + (g.batch_m_tiles ? (mt / g.batch_m_tiles) * g.N : 0));
         }
       }
-      if (!ok) {
-        // give copies already in flight a bounded chance to land before the CTA leaves
-        for (int s = 0; s < STAGES; ++s)
-          for (int i = 0; i < (1 << 14) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
-      }
+      ring_drain(full, STAGES, it);
+      if (!ok) abort_settle();                   // the loads of a stage that was only begun complete no phase
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer

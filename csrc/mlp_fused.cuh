@@ -183,10 +183,10 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
         if (!ok) break;
       }
     }
-    // copies still in flight land before the CTA leaves (bounded)
-    if (!ok)
-      for (int s = 0; s < Cfg::SLOTS; ++s)
-        for (int i = 0; i < (1 << 14) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
+    if (lane == 0) {                             // copies land before the CTA leaves, also after a wait that ran out
+      mbar_drain(wfull, 0);
+      ring_drain(full, Cfg::SLOTS, it);
+    }
   } else if (warp == 1) {
     // -------------------------------------------------------------------------------- MMA issuer of both groups
     // One thread polls: a layer whose operand is in place goes first, then the next source chunk.  (An issuer per group would
@@ -376,6 +376,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
+    if (*abort_flag) abort_settle();
     tc_fence_after();
     tmem_dealloc(tmem, kMlpTmemCols);
   }

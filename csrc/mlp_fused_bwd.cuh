@@ -176,6 +176,8 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
   } else if (warp == 3) {
     // ------------------------------------------------------------------------------------------------ dx3 tiles
     if (lane == 0) {
+      uint32_t issued[2] = {0, 0};
+#pragma unroll 1
       for (int n = 0; n < mine; ++n) {
         const int grp = n & 1, k = n >> 1;       // k-th tile of the group
         if (k && !mbar_wait(&dfree[grp], (k - 1) & 1, abort_flag, g.err, ERR_WAIT_EMPTY)) break;
@@ -184,7 +186,10 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         mbar_expect_tx(&dfull[grp], 2 * kMlpChunk);
         tma_load_2d(dst, &tmD, &dfull[grp], 0, m0);
         tma_load_2d(dst + kMlpChunk, &tmD, &dfull[grp], 64, m0);
+        ++issued[grp];
       }
+      for (int grp = 0; grp < 2; ++grp)          // copies land before the CTA leaves, also after a wait that ran out
+        if (issued[grp]) mbar_drain(&dfull[grp], (issued[grp] - 1) & 1);
     }
   } else {
     // ------------------------------------------------- two threads per row of a tile, columns [64 half, 64 half + 64)
@@ -301,6 +306,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
+    if (*abort_flag) abort_settle();
     tc_fence_after();
     tmem_dealloc(tmem, kMlpTmemCols);
   }

@@ -169,7 +169,7 @@ layernorm_fwd_stream_kernel(const __nv_bfloat16* __restrict__ x, const float* __
   if (warp == kLnWarps) {
     if (lane == 0) {
       int s = 0;
-      uint32_t ph = 1;
+      uint32_t ph = 1, issued = 0;
       for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         if (!mbar_wait(&empty[s], ph, abort_flag, err, ERR_WAIT_EMPTY)) break;
         const long long row = t * stage_rows;
@@ -178,7 +178,9 @@ layernorm_fwd_stream_kernel(const __nv_bfloat16* __restrict__ x, const float* __
         bulk_load(ln_smem + size_t(s) * stage_bytes, x + row * C, bytes, &full[s]);
         if (post) bulk_load(ln_smem + size_t(s) * stage_bytes + tile_bytes, post + row * C, bytes, &full[s]);
         if (++s == stages) { s = 0; ph ^= 1; }
+        ++issued;
       }
+      ring_drain(full, stages, issued);          // copies land before the CTA leaves, also after a wait that ran out
     }
     return;
   }
@@ -292,7 +294,7 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
   if (warp == kLnWarps) {
     if (lane == 0) {
       int s = 0;
-      uint32_t ph = 1;
+      uint32_t ph = 1, issued = 0;
       for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
         if (!mbar_wait(&empty[s], ph, abort_flag, err, ERR_WAIT_EMPTY)) break;
         const long long row = t * stage_rows;
@@ -303,7 +305,9 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
         bulk_load(st + tile_bytes, dy + row * C, bytes, &full[s]);
         if (dres) bulk_load(st + 2 * tile_bytes, dres + row * C, bytes, &full[s]);
         if (++s == stages) { s = 0; ph ^= 1; }
+        ++issued;
       }
+      ring_drain(full, stages, issued);          // copies land before the CTA leaves, also after a wait that ran out
     }
   } else {
     float gam[VEC][8];
@@ -384,7 +388,7 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
     }
   }
   // fold the warps of this CTA, one vector slot at a time, in the ring's memory: every copy into it has been waited for by all
-  // consumers (after a wait that ran out the results are void, but copies may still land: the ring is not touched then)
+  // consumers (after a wait that ran out the results are void)
   __syncthreads();
   if (*abort_flag) return;
   float* red = reinterpret_cast<float*>(ln_smem);   // kLnFoldBytes: [warps][2][264]
