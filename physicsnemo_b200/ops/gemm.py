@@ -18,6 +18,7 @@ from typing import Optional, Sequence
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -34,6 +35,13 @@ def _ptr(t: Optional[torch.Tensor]):
 
 def _stream():
     return _lib.stream()
+
+
+def call_is_observed() -> bool:
+    """Whether forward-mode differentiation, a function transform or a trace is under way.  A call that needs no gradient may skip
+    its autograd function only without them: a bare launch would drop the tangent, and a trace would hold nothing but the
+    allocation of its result."""
+    return forward_ad._current_level >= 0 or torch._C._is_tracing() or torch._C._are_functorch_transforms_active()
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:

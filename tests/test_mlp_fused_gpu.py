@@ -150,3 +150,19 @@ def test_mlp3_backward_beside_other_work():
         assert all(_rel(a, b.double()) < 1e-5 for a, b in zip(grads[1:], first[1:]))
     torch.cuda.synchronize()
     assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+def test_mlp3_ln_without_gradients_keeps_forward_mode_and_tracing_honest():
+    from torch.autograd import forward_ad
+
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_graph_mlp import MeshGraphMLP
+
+    m = MeshGraphMLP(W, W, W, 2, torch.nn.SiLU()).cuda().requires_grad_(False)
+    x, other = (torch.randn(300, W, device="cuda").bfloat16() for _ in range(2))
+    with torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False), torch.no_grad():
+        want = m(other)
+        traced = torch.jit.trace(lambda a: m(a), (x,), check_trace=False)
+        assert torch.equal(traced(other), want)
+        with forward_ad.dual_level(), pytest.raises((NotImplementedError, RuntimeError)):
+            m(forward_ad.make_dual(x, other))
