@@ -91,32 +91,6 @@ gather_rows_scaled_kernel(const __nv_bfloat16* __restrict__ in, int ldi, const i
   }
 }
 
-// out[e,:] = base[e,:] + in[idx[e],:] (* scale[idx[e]]): the two gradients of rows that were both passed on and aggregated, in
-// one pass (a gather into a buffer and an addition move two more rows per edge)
-__global__ void __launch_bounds__(256)
-gather_rows_add_kernel(const __nv_bfloat16* __restrict__ in, int ldi, const int* __restrict__ idx, const float* __restrict__ scale,
-                       const __nv_bfloat16* __restrict__ base, long long ldb, __nv_bfloat16* __restrict__ out, long long ldo, long long E,
-                       int C) {
-  const int cpr = C >> 3;
-  const long long total = E * cpr;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const long long e = t / cpr;
-    const int c = int(t - e * cpr) << 3;
-    const long long src = (long long)__ldg(idx + e);
-    const float s = scale ? __ldg(scale + src) : 1.f;
-    const uint4 v = *reinterpret_cast<const uint4*>(in + src * ldi + c);
-    const uint4 b = *reinterpret_cast<const uint4*>(base + e * ldb + c);
-    const uint32_t vi[4] = {v.x, v.y, v.z, v.w}, bi[4] = {b.x, b.y, b.z, b.w};
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 x = unpack_bf16x2(vi[j]), y = unpack_bf16x2(bi[j]);
-      w[j] = pack_bf16x2(y.x + x.x * s, y.y + x.y * s);
-    }
-    *reinterpret_cast<uint4*>(out + e * ldo + c) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
-
 inline int grid_for(long long work_items, int threads, int num_sms) {
   long long want = (work_items + threads - 1) / threads;
   long long cap = (long long)num_sms * 16;
@@ -133,15 +107,6 @@ inline int launch_gather_rows(const void* in, int ldi, const int* idx, const flo
     gather_rows_scaled_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)in, ldi, idx, scale, (__nv_bfloat16*)out, ldo, E, C);
   else
     gather_rows_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)in, ldi, idx, (__nv_bfloat16*)out, ldo, E, C);
-  return cudaGetLastError() == cudaSuccess ? 0 : -41;
-}
-
-inline int launch_gather_rows_add(const void* in, int ldi, const int* idx, const float* scale, const void* base, long long ldb, void* out,
-                                  long long ldo, long long E, int C, int num_sms, cudaStream_t st) {
-  if (C % 8 || ldi % 8 || ldo % 8 || ldb % 8 || !idx || !base) return -40;
-  if (E <= 0) return 0;
-  gather_rows_add_kernel<<<grid_for(E * (C >> 3), 256, num_sms), 256, 0, st>>>(
-      (const __nv_bfloat16*)in, ldi, idx, scale, (const __nv_bfloat16*)base, ldb, (__nv_bfloat16*)out, ldo, E, C);
   return cudaGetLastError() == cudaSuccess ? 0 : -41;
 }
 

@@ -63,9 +63,6 @@ int pnm_segment_sum_split(const void* in, const int* perm, const int* offsets, v
 // out[e,:] = in[idx[e],:] (* scale[idx[e]]); bf16 rows, int32 indices (idx may be null = identity).
 int pnm_gather_rows(const void* in, int ldi, const int* idx, const float* scale, void* out, int ldo, long long E,
                     int C, void* stream);
-// out[e,:] = base[e,:] + in[idx[e],:] (* scale[idx[e]]).
-int pnm_gather_rows_add(const void* in, int ldi, const int* idx, const float* scale, const void* base, long long ldb, void* out,
-                        long long ldo, long long E, int C, void* stream);
 // out[n,:] (+)= sum over k in [offsets[n], offsets[n+1]) of in[perm[k],:]; mode 1 divides by the count.
 int pnm_segment_sum(const void* in, int ldi, const int* perm, const int* offsets, void* out, int ldo, long long N,
                     int C, int accumulate, int mode, void* stream);

@@ -343,12 +343,6 @@ int pnm_gather_rows(const void* in, int ldi, const int* idx, const float* scale,
   return pnm::launch_gather_rows(in, ldi, idx, scale, out, ldo, E, C, g_num_sms, reinterpret_cast<cudaStream_t>(stream));
 }
 
-int pnm_gather_rows_add(const void* in, int ldi, const int* idx, const float* scale, const void* base, long long ldb, void* out, long long ldo,
-                        long long E, int C, void* stream) {
-  if (ensure_init()) return -1;
-  return pnm::launch_gather_rows_add(in, ldi, idx, scale, base, ldb, out, ldo, E, C, g_num_sms, reinterpret_cast<cudaStream_t>(stream));
-}
-
 int pnm_segment_sum(const void* in, int ldi, const int* perm, const int* offsets, void* out, int ldo, long long N,
                     int C, int accumulate, int mode, void* stream) {
   if (ensure_init()) return -1;

@@ -4,7 +4,6 @@ import torch.nn as nn
 from torch import Tensor
 
 from .... import ops
-from .graph_types import segments
 from .mesh_graph_mlp import MeshGraphMLP
 from .utils import aggregate, aggregate_and_concat
 
@@ -24,7 +23,7 @@ class MeshNodeBlock(nn.Module):
 
     def forward(self, efeat: Tensor, nfeat: Tensor, graph):
         if ops.fused_path_enabled(efeat) and efeat.dtype == torch.bfloat16 and nfeat.dtype == torch.bfloat16:
-            agg, efeat = ops.segment_reduce(efeat, segments(graph, "dst", nfeat.shape[0]), self.aggregation, return_rows=True)
+            agg = aggregate(efeat, nfeat.shape[0], graph, self.aggregation)
             return efeat, self.node_mlp((agg, nfeat), post=nfeat)
         cat_feat = aggregate_and_concat(efeat, nfeat, graph, self.aggregation)
         return efeat, self.node_mlp(cat_feat, post=nfeat)

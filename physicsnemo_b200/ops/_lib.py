@@ -86,7 +86,6 @@ def _declare(lib):
         "pnm_gemm_nt_stacked": ([vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp], i32),
         "pnm_layernorm_fwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, vp], i32),
         "pnm_gather_rows": ([vp, i32, vp, vp, vp, i32, i64, i32, vp], i32),
-        "pnm_gather_rows_add": ([vp, i32, vp, vp, vp, i64, vp, i64, i64, i32, vp], i32),
         "pnm_segment_sum": ([vp, i32, vp, vp, vp, i32, i64, i32, i32, i32, vp], i32),
         "pnm_layernorm_bwd_scratch_floats": ([i64, i32], i64),
         "pnm_layernorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, vp], i32),

@@ -81,33 +81,15 @@ class _GatherFn(torch.autograd.Function):
 
 
 class _SegmentFn(torch.autograd.Function):
-    """With ``rows`` the input is handed on as a second output, and the backward adds the two gradients while it gathers."""
-
     @staticmethod
-    def forward(ctx, x, seg, mean, rows):
+    def forward(ctx, x, seg, mean):
         ctx.seg, ctx.mean = seg, mean
-        ctx.set_materialize_grads(False)
-        out = _segment_raw(_ok(x), seg, mean)
-        return (out, x.view_as(x)) if rows else out
+        return _segment_raw(_ok(x), seg, mean)
 
     @staticmethod
-    def backward(ctx, g, passed=None):
+    def backward(ctx, g):
         seg = ctx.seg
-        if g is None:
-            return passed, None, None, None
-        scale = seg.inv_count if ctx.mean else None
-        g = _ok(g)
-        if passed is None:
-            return _gather_raw(g, seg.index32, scale), None, None, None
-        passed = _ok(passed)
-        lib = _lib.load(required=True)
-        E, C = passed.shape
-        out = torch.empty((E, C), dtype=torch.bfloat16, device=g.device)
-        code = lib.pnm_gather_rows_add(g.data_ptr(), g.stride(0), seg.index32.data_ptr(), None if scale is None else scale.data_ptr(),
-                                       passed.data_ptr(), passed.stride(0), out.data_ptr(), out.stride(0), E, C, _g._stream())
-        _g._check(code, "pnm_gather_rows_add")
-        _g.launch_count += 1
-        return out, None, None, None
+        return _gather_raw(_ok(g), seg.index32, seg.inv_count if ctx.mean else None), None, None
 
 
 def _fused(x: torch.Tensor) -> bool:
@@ -121,19 +103,14 @@ def gather_rows(x: torch.Tensor, seg: SegmentIndex) -> torch.Tensor:
     return x[seg.index]
 
 
-def segment_reduce(x: torch.Tensor, seg: SegmentIndex, reduce: str = "sum", return_rows: bool = False):
-    """Sum (or mean) of the rows of ``x`` that share a segment id; result has ``seg.num_segments`` rows.
-
-    ``return_rows=True`` returns ``(sums, x')`` where ``x'`` is ``x`` routed through the same autograd node: a caller that
-    passes the rows on gets the sum of their two gradients from one kernel instead of a gather and an addition."""
+def segment_reduce(x: torch.Tensor, seg: SegmentIndex, reduce: str = "sum") -> torch.Tensor:
+    """Sum (or mean) of the rows of ``x`` that share a segment id; result has ``seg.num_segments`` rows."""
     if reduce not in ("sum", "mean"):
         raise ValueError(f"unsupported reduction {reduce}")
     if _fused(x):
-        if return_rows and not (torch.is_grad_enabled() and x.requires_grad):
-            return _SegmentFn.apply(x, seg, reduce == "mean", False), x
-        return _SegmentFn.apply(x, seg, reduce == "mean", return_rows)
+        return _SegmentFn.apply(x, seg, reduce == "mean")
     out = torch.zeros((seg.num_segments, x.shape[1]), dtype=x.dtype, device=x.device)
     out.index_add_(0, seg.index, x)
     if reduce == "mean":
         out = out * seg.inv_count.to(out.dtype).unsqueeze(1)
-    return (out, x) if return_rows else out
+    return out

@@ -82,3 +82,34 @@ def test_meshgraphnet_fused_matches_fp32():
     bad = [(n, _rel(p.grad, q.grad)) for (n, p), (_, q) in zip(model.named_parameters(), ref.named_parameters())
            if _rel(p.grad, q.grad) > 0.25]
     assert not bad, bad
+
+
+def _node_block(edges, nodes, aggregation="sum"):
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_node_block import MeshNodeBlock
+
+    block = MeshNodeBlock(aggregation, 128, 128, 128, 128, 2).cuda()
+    return block, Graph(torch.randint(0, nodes, (2, edges)).cuda(), num_nodes=nodes)
+
+
+def test_node_block_hands_on_the_edge_rows_themselves():
+    block, graph = _node_block(700, 90)
+    leaf = torch.randn(700, 128, device="cuda").bfloat16().requires_grad_()
+    v = torch.randn(90, 128, device="cuda").bfloat16()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        rows = leaf * 1
+        back, _ = block(rows, v, graph)
+    assert back is rows
+    back.mul_(2)                                             # in place, under grad
+    rows.sum().backward()
+    assert torch.equal(leaf.grad, torch.full_like(leaf, 2))
+
+
+@pytest.mark.parametrize("aggregation", ["sum", "mean"])
+def test_node_block_trains_on_a_graph_without_edges(aggregation):
+    block, graph = _node_block(0, 90, aggregation)
+    e = torch.zeros(0, 128, device="cuda").bfloat16().requires_grad_()
+    v = torch.randn(90, 128, device="cuda").bfloat16().requires_grad_()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        out = block(e * 1, v, graph)
+    torch.autograd.backward(out, [torch.ones_like(t) for t in out])
+    assert e.grad.shape == (0, 128) and torch.isfinite(v.grad).all() and v.grad.abs().sum() > 0
