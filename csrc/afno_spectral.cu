@@ -792,11 +792,9 @@ static int af_check(const AfGeom& g) {
 }
 
 template <typename K>
-static int af_smem_attr(K kernel, size_t bytes, unsigned long long& mask) {
+static int af_smem_attr(K* kernel, size_t bytes, DeviceMask& mask) {
   if (bytes > 220 * 1024) return -2;
-  if (first_use_on_device(mask) && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
-    return -4;
-  return 0;
+  return allow_smem(kernel, 220 * 1024, mask) ? 0 : -4;
 }
 
 }  // namespace pnm
@@ -818,7 +816,7 @@ int pnm_afno_rows_r2c(const void* const* tokens, void* Y, const int* geom, long 
     const pnm::RowPlan rp = pnm::row_plan(g.KX, g.Cb);
     const size_t smem2 = sizeof(float) * (2 * (size_t)(g.W / 2) * g.Cb + 2 * (size_t)(g.W / 2 - 1) * rp.pad);
     if (smem2 <= 220 * 1024) {
-      static unsigned long long mask2 = 0;
+      static pnm::DeviceMask mask2{0};
       if (int rc = pnm::af_smem_attr(pnm::afno_rows_r2c_v2_kernel, smem2, mask2)) return rc;
       pnm::afno_rows_r2c_v2_kernel<<<dim3(g.B * g.H, g.nblk), rp.threads, smem2, (cudaStream_t)stream>>>(
           pnm::make_tok(tokens), (float2*)Y, g, kweight, p, wait, err, rp.groups, rp.passes);
@@ -826,7 +824,7 @@ int pnm_afno_rows_r2c(const void* const* tokens, void* Y, const int* geom, long 
     }
   }
   const size_t smem = sizeof(float) * ((size_t)g.W * g.Cb + 2 * g.W);
-  static unsigned long long mask = 0;
+  static pnm::DeviceMask mask{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_rows_r2c_kernel, smem, mask)) return rc;
   pnm::afno_rows_r2c_kernel<<<dim3(g.B * g.H, g.nblk), 2 * g.Cb, smem, (cudaStream_t)stream>>>(pnm::make_tok(tokens), (float2*)Y, g,
                                                                                               kweight, p, wait, err);
@@ -845,7 +843,7 @@ int pnm_afno_rows_c2r(const void* X, const void* const* tokens, const int* geom,
     const pnm::RowPlan rp = pnm::row_plan(g.W / 2 + 1, g.Cb);
     const size_t smem2 = sizeof(float2) * ((size_t)g.KX * g.Cb + (size_t)g.KX * rp.pad) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
     if (smem2 <= 220 * 1024) {
-      static unsigned long long mask2 = 0;
+      static pnm::DeviceMask mask2{0};
       if (int rc = pnm::af_smem_attr(pnm::afno_rows_c2r_v2_kernel, smem2, mask2)) return rc;
       pnm::afno_rows_c2r_v2_kernel<<<dim3(g.B * g.H, g.nblk), rp.threads, smem2, (cudaStream_t)stream>>>(
           (const float2*)X, pnm::make_tok(tokens), g, kweight, p, signal, (unsigned int*)counter, rp.groups, rp.passes, nullptr,
@@ -854,7 +852,7 @@ int pnm_afno_rows_c2r(const void* X, const void* const* tokens, const int* geom,
     }
   }
   const size_t smem = sizeof(float2) * ((size_t)g.KX * g.Cb + g.W) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
-  static unsigned long long mask = 0;
+  static pnm::DeviceMask mask{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_rows_c2r_kernel, smem, mask)) return rc;
   pnm::afno_rows_c2r_kernel<<<dim3(g.B * g.H, g.nblk), 2 * g.Cb, smem, (cudaStream_t)stream>>>((const float2*)X, pnm::make_tok(tokens),
                                                                                               g, kweight, p, signal,
@@ -872,7 +870,7 @@ int pnm_afno_rows_c2r_add(const void* X, void* out, const void* add0, const void
   const pnm::RowPlan rp = pnm::row_plan(g.W / 2 + 1, g.Cb);
   const size_t smem2 = sizeof(float2) * ((size_t)g.KX * g.Cb + (size_t)g.KX * rp.pad) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
   if (smem2 > 220 * 1024) return -2;
-  static unsigned long long mask2 = 0;
+  static pnm::DeviceMask mask2{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_rows_c2r_v2_kernel, smem2, mask2)) return rc;
   const void* ptrs[8] = {out, out, out, out, out, out, out, out};
   pnm::afno_rows_c2r_v2_kernel<<<dim3(g.B * g.H, g.nblk), rp.threads, smem2, (cudaStream_t)stream>>>(
@@ -888,7 +886,7 @@ int pnm_afno_cols_fwd(const void* Y, void* Yout, void* Zs, void* O1s, void* O2s,
   pnm::AfGeom g{geom[0], geom[1], geom[2], geom[3], geom[4], geom[5], geom[6], geom[7], 1, geom[8], geom[9]};
   if (pnm::af_check(g) || nb < g.blk0 + g.nblk) return -2;
   const size_t smem = sizeof(float2) * (2 * (size_t)g.H * g.Cb + g.H);
-  static unsigned long long mask = 0;
+  static pnm::DeviceMask mask{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_cols_fwd_kernel, smem, mask)) return rc;
   pnm::AfWeights wt{w1, b1, w2, b2, nb};
   pnm::afno_cols_fwd_kernel<<<dim3(g.B * g.KX, g.nblk), 2 * g.Cb, smem, (cudaStream_t)stream>>>(
@@ -902,7 +900,7 @@ int pnm_afno_cols_bwd(const void* dYout, void* dY, const void* Zs, const void* O
   pnm::AfGeom g{geom[0], geom[1], geom[2], geom[3], geom[4], geom[5], geom[6], geom[7], 1, geom[8], geom[9]};
   if (pnm::af_check(g) || nb < g.blk0 + g.nblk) return -2;
   const size_t smem = sizeof(float2) * (3 * (size_t)g.H * g.Cb + g.H);
-  static unsigned long long mask = 0;
+  static pnm::DeviceMask mask{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_cols_bwd_kernel, smem, mask)) return rc;
   pnm::AfWeights wt{w1, nullptr, w2, nullptr, nb};
   pnm::AfGrads gd{dw1, db1, dw2, db2};
@@ -917,7 +915,7 @@ int pnm_afno_cols_dft(const void* Y, void* E, const void* mask, const int* geom,
   if (pnm::af_check(g) || Mp < g.B * g.KX * g.H) return -2;
   const int chunks = (g.Cb % 16 == 0 && g.Cb >= 64) ? 2 : 1;
   const size_t smem = sizeof(float2) * (2 * (size_t)g.H * (g.Cb / chunks) + g.H1 * g.H1 + g.H + g.H2 * g.H2);
-  static unsigned long long mask_bits = 0;
+  static pnm::DeviceMask mask_bits{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_cols_dft_v2_kernel, smem, mask_bits)) return rc;
   pnm::afno_cols_dft_v2_kernel<<<dim3(g.B * g.KX, g.nblk * chunks), 256, smem, (cudaStream_t)stream>>>(
       (const float2*)Y, (__nv_bfloat16*)E, (const __nv_bfloat16*)mask, g, lambda, chunks, Mp);
@@ -929,7 +927,7 @@ int pnm_afno_cols_idft(const void* E, void* Yout, const int* geom, int Mp, float
   if (pnm::af_check(g) || Mp < g.B * g.KX * g.H) return -2;
   const int chunks = (g.Cb % 16 == 0 && g.Cb >= 64) ? 2 : 1;
   const size_t smem = sizeof(float2) * (2 * (size_t)g.H * (g.Cb / chunks) + g.H1 * g.H1 + g.H + g.H2 * g.H2);
-  static unsigned long long mask_bits = 0;
+  static pnm::DeviceMask mask_bits{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_cols_idft_v2_kernel, smem, mask_bits)) return rc;
   pnm::afno_cols_idft_v2_kernel<<<dim3(g.B * g.KX, g.nblk * chunks), 256, smem, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)E, (float2*)Yout, g, lambda, chunks, Mp);

@@ -290,11 +290,8 @@ inline int launch_gemm_nt(const NtCall& c, int num_sms, int* err_word, cudaStrea
   splits = (kblocks + per - 1) / per;
   g.out = c.out; g.ldo = c.ldo; g.colsum = c.colsum; g.err = err_word;
   g.batch = nprob; g.batch_rows = M / nprob; g.splits = splits; g.out_stride = c.out_stride;
-  static unsigned long long attr_mask = 0;
-  if (first_use_on_device(attr_mask)) {
-    if (cudaFuncSetAttribute(gemm_nt_kernel<BNB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-      return -22;
-  }
+  static DeviceMask smem_set{0};
+  if (!allow_smem(gemm_nt_kernel<BNB>, Cfg::SMEM, smem_set)) return -22;
   gemm_nt_kernel<BNB><<<tiles * splits * nprob, kNtThreads, Cfg::SMEM, stream>>>(tA, tB, tB3, tUp, tDown, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -23;
 }

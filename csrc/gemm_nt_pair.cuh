@@ -251,11 +251,8 @@ inline int launch_gemm_nt_pair(const NtCall& c, int num_sms, int* err_word, cuda
   splits = (kblocks + per - 1) / per;
   g.out = c.out; g.ldo = c.ldo; g.colsum = c.colsum; g.err = err_word;
   g.batch = 1; g.batch_rows = M; g.splits = splits; g.out_stride = 0;
-  static unsigned long long attr_mask = 0;
-  if (first_use_on_device(attr_mask)) {
-    if (cudaFuncSetAttribute(gemm_nt_pair_kernel<BNB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-      return -22;
-  }
+  static DeviceMask smem_set{0};
+  if (!allow_smem(gemm_nt_pair_kernel<BNB>, Cfg::SMEM, smem_set)) return -22;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * tiles * splits);
   cfg.blockDim = dim3(kNtThreads);

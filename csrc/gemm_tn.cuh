@@ -703,12 +703,8 @@ inline int launch_gemm_tn(const GemmCall& c, int num_sms, int* err_word, cudaStr
     g.num_m_tiles = c.img_n * g.tiles_x * g.tiles_y;
     g.M = g.num_m_tiles * kBM;            // every row of a tile is "in range"; the copy engine clips at image edges
   }
-  static unsigned long long attr_mask = 0;   // one bit per device: the attribute belongs to the device's context
-  if (first_use_on_device(attr_mask)) {
-    if (cudaFuncSetAttribute(gemm_tn_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) !=
-        cudaSuccess)
-      return -16;
-  }
+  static DeviceMask smem_set{0};
+  if (!allow_smem(gemm_tn_kernel<BN, MODE>, Cfg::SMEM, smem_set)) return -16;
   if (split) {                                // 256-row tiles of 128 columns
     g.num_m_tiles = (g.num_m_tiles + 1) / 2;
     g.num_n_tiles = (c.N + 127) / 128;

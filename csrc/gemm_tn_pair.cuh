@@ -453,11 +453,8 @@ inline int launch_gemm_tn_pair(const GemmCall& c, int num_sms, int* err_word, cu
   if (!c.conv) { tA2 = tA; tA3 = tA; }
   g.num_m_tiles = (tiles128 + 1) / 2;
   g.num_n_tiles = (c.N + BN - 1) / BN;
-  static unsigned long long attr_mask = 0;
-  if (first_use_on_device(attr_mask)) {
-    if (cudaFuncSetAttribute(gemm_tn_pair_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-      return -16;
-  }
+  static DeviceMask smem_set{0};
+  if (!allow_smem(gemm_tn_pair_kernel<BN, MODE>, Cfg::SMEM, smem_set)) return -16;
   const int tiles = g.num_m_tiles * g.num_n_tiles;
   int clusters = num_sms / 2;
   if (clusters > tiles) clusters = tiles;

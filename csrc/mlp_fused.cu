@@ -8,10 +8,8 @@ namespace pnm {
 template <int NSRC, int ACT, bool SAVE>
 static int launch_mlp3(const CUtensorMap* tm, const CUtensorMap* tw, const MlpArgs& g, int grid, cudaStream_t st) {
   using Cfg = MlpCfg<NSRC>;
-  static unsigned long long attr_mask = 0;
-  if (first_use_on_device(attr_mask) &&
-      cudaFuncSetAttribute(mlp3_ln_kernel<NSRC, ACT, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-    return -16;
+  static DeviceMask smem_set{0};
+  if (!allow_smem(mlp3_ln_kernel<NSRC, ACT, SAVE>, Cfg::SMEM, smem_set)) return -16;
   mlp3_ln_kernel<NSRC, ACT, SAVE><<<grid, kMlpThreads, Cfg::SMEM, st>>>(tm[0], tm[1], tm[2], tw[0], tw[1], tw[2], g);
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
 }
@@ -31,10 +29,8 @@ static int launch_mlp3_act(const CUtensorMap* tm, const CUtensorMap* tw, const M
 
 template <int ACT>
 static int launch_mlp3_bwd(const CUtensorMap& td, const CUtensorMap& t3, const CUtensorMap& t2, const MlpBwdArgs& g, int grid, cudaStream_t st) {
-  static unsigned long long attr_mask = 0;
-  if (first_use_on_device(attr_mask) &&
-      cudaFuncSetAttribute(mlp3_bwd_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlpBwdSmem) != cudaSuccess)
-    return -16;
+  static DeviceMask smem_set{0};
+  if (!allow_smem(mlp3_bwd_kernel<ACT>, kMlpBwdSmem, smem_set)) return -16;
   mlp3_bwd_kernel<ACT><<<grid, kMlpThreads, kMlpBwdSmem, st>>>(td, t3, t2, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
 }

@@ -458,16 +458,13 @@ inline LnStream ln_stream_plan(long long M, int C, int tensors, int least_rows, 
   p.smem = (ring > kLnFoldBytes ? ring : kLnFoldBytes) + p.stages * 16 + 16;
   return p;
 }
-template <typename K>
-inline bool ln_stream_attr(K* kernel, unsigned long long& mask) {
-  return !first_use_on_device(mask) || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024) == cudaSuccess;
-}
+constexpr int kLnSmemMax = 225 * 1024;
 
 template <int VEC, int LPR>
 inline int launch_ln_fwd_stream(const __nv_bfloat16* x, const float* gamma, const float* beta, __nv_bfloat16* y, float* mean, float* rstd,
                                 const __nv_bfloat16* post, long long M, int C, float eps, int num_sms, int* err, cudaStream_t st) {
-  static unsigned long long mask = 0;
-  if (!ln_stream_attr(layernorm_fwd_stream_kernel<VEC, LPR>, mask)) return -31;
+  static DeviceMask smem_set{0};
+  if (!allow_smem(layernorm_fwd_stream_kernel<VEC, LPR>, kLnSmemMax, smem_set)) return -31;
   const LnStream p = ln_stream_plan(M, C, post ? 2 : 1, kLnWarps * (32 / LPR), VEC <= 2 ? 3 : 2, num_sms);
   layernorm_fwd_stream_kernel<VEC, LPR><<<p.grid, kLnStreamThreads, p.smem, st>>>(x, gamma, beta, y, mean, rstd, post, M, C, eps, p.rows,
                                                                                   p.stages, err);
@@ -513,8 +510,8 @@ template <int VEC, int LPR>
 inline int launch_ln_bwd_stream(const __nv_bfloat16* dy, const __nv_bfloat16* x, const float* gamma, const float* mean, const float* rstd,
                                 const __nv_bfloat16* dres, __nv_bfloat16* dx, float* scratch, long long M, int C, const LnStream& p, int* err,
                                 cudaStream_t st) {
-  static unsigned long long mask = 0;
-  if (!ln_stream_attr(layernorm_bwd_stream_kernel<VEC, LPR>, mask)) return -33;
+  static DeviceMask smem_set{0};
+  if (!allow_smem(layernorm_bwd_stream_kernel<VEC, LPR>, kLnSmemMax, smem_set)) return -33;
   layernorm_bwd_stream_kernel<VEC, LPR><<<p.grid, kLnStreamThreads, p.smem, st>>>(dy, x, gamma, mean, rstd, dres, dx, scratch, M, C, p.rows,
                                                                              p.stages, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -33;

@@ -404,10 +404,8 @@ int pnm_pa_tokens_fwd(const void* const* srcs, int world, int use_flags, long lo
   int* err = pnm::error_word_ptr();
   if (!err) return -1;
   const size_t smem = pnm::pa_fwd_smem(D, Cout);
-  static unsigned long long mask = 0;
-  if (pnm::first_use_on_device(mask) &&
-      cudaFuncSetAttribute(pnm::pa_tokens_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
-    return -4;
+  static pnm::DeviceMask smem_set{0};
+  if (!pnm::allow_smem(pnm::pa_tokens_fwd_kernel, 160 * 1024, smem_set)) return -4;
   if (smem > 160 * 1024) return -2;
   pnm::PeerArgs p{};
   if (use_flags) p = pnm::make_peer_args(bases, rank, world, epoch, capacity_floats, budget_s, epoch_base);
@@ -427,10 +425,8 @@ int pnm_pa_tokens_bwd(const void* const* srcs, int world, int use_flags, const f
   if (!err) return -1;
   const size_t smem = pnm::pa_bwd_smem(D, Cout);
   if (smem > 226 * 1024) return -2;
-  static unsigned long long mask = 0;
-  if (pnm::first_use_on_device(mask) &&
-      cudaFuncSetAttribute(pnm::pa_tokens_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess)
-    return -4;
+  static pnm::DeviceMask smem_set{0};
+  if (!pnm::allow_smem(pnm::pa_tokens_bwd_kernel, 226 * 1024, smem_set)) return -4;
   pnm::PeerArgs p{};
   if (use_flags) p = pnm::make_peer_args(bases, rank, world, epoch, capacity_floats, budget_s, epoch_base);
   pnm::pa_tokens_bwd_kernel<<<H, pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(pnm::make_src(srcs, world, use_flags), Wqkv, Wo,

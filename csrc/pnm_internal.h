@@ -1,5 +1,6 @@
 // Declarations shared by the translation units of the kernel library (not part of the C ABI).
 #pragma once
+#include <atomic>
 #include "peer.cuh"
 
 namespace pnm {
@@ -12,13 +13,17 @@ int num_sms();                 // SM count of the current device
 PeerArgs make_peer_args(const void* const* bases, int rank, int world, unsigned int epoch, long long capacity_floats,
                         double budget_s, const void* epoch_base);
 
-// Set-once-per-device bookkeeping for cudaFuncSetAttribute calls: returns true when `mask` did not yet carry the
-// bit of the current device (and sets it).
-inline bool first_use_on_device(unsigned long long& mask) {
-  const int dev = current_device();
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (mask & bit) return false;
-  mask |= bit;
+// Which devices a kernel's attributes have been set on, one bit each (they belong to the device's context).
+using DeviceMask = std::atomic<unsigned long long>;
+
+// Allows `kernel` `bytes` of dynamic shared memory on the current device, once per device and kernel.  The bit follows the
+// attribute: a thread that sees it may launch, and threads that make the first call together all set it.
+template <typename K>
+inline bool allow_smem(K* kernel, size_t bytes, DeviceMask& done) {
+  const unsigned long long bit = 1ull << (current_device() & 63);
+  if (done.load(std::memory_order_acquire) & bit) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) return false;
+  done.fetch_or(bit, std::memory_order_release);
   return true;
 }
 
