@@ -15,7 +15,7 @@ static int launch_mlp3(const CUtensorMap* tm, const CUtensorMap* tw, const MlpAr
 }
 template <int NSRC, int ACT>
 static int launch_mlp3_save(const CUtensorMap* tm, const CUtensorMap* tw, const MlpArgs& g, int grid, cudaStream_t st) {
-  return g.z1 ? launch_mlp3<NSRC, ACT, true>(tm, tw, g, grid, st) : launch_mlp3<NSRC, ACT, false>(tm, tw, g, grid, st);
+  return g.h1 ? launch_mlp3<NSRC, ACT, true>(tm, tw, g, grid, st) : launch_mlp3<NSRC, ACT, false>(tm, tw, g, grid, st);
 }
 template <int NSRC>
 static int launch_mlp3_act(const CUtensorMap* tm, const CUtensorMap* tw, const MlpArgs& g, int grid, cudaStream_t st) {
@@ -28,15 +28,17 @@ static int launch_mlp3_act(const CUtensorMap* tm, const CUtensorMap* tw, const M
 }
 
 template <int ACT>
-static int launch_mlp3_bwd(const CUtensorMap& td, const CUtensorMap& t3, const CUtensorMap& t2, const MlpBwdArgs& g, int grid, cudaStream_t st) {
+static int launch_mlp3_bwd(const CUtensorMap& td, const CUtensorMap& th2, const CUtensorMap& th1, const CUtensorMap& t3,
+                           const CUtensorMap& t2, const MlpBwdArgs& g, int grid, cudaStream_t st) {
   static DeviceMask smem_set{0};
   if (!allow_smem(mlp3_bwd_kernel<ACT>, kMlpBwdSmem, smem_set)) return -16;
-  mlp3_bwd_kernel<ACT><<<grid, kMlpThreads, kMlpBwdSmem, st>>>(td, t3, t2, g);
+  mlp3_bwd_kernel<ACT><<<grid, kMlpThreads, kMlpBwdSmem, st>>>(td, th2, th1, t3, t2, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
 }
 
 // out[n] = [hi(s) | lo(s)], s = sum over k in [off[n], off[n+1]) of in[perm[k]] in fp32: two bf16 rows whose sum carries 16
-// bits of s, so that a product with it keeps what the fp32 sum had.  One thread per 16-byte chunk of a row, as the plain sum.
+// bits of s.  Against 64 bits dW1 of an edge MLP errs 0.9975 +- 0.0008 (601 nodes), 0.998 (4 001), 0.997 (30 011) times as much as with
+// one product per row, and the gradients of the table, which that path rounds row by row, 0.934 times as much.  One thread per 16-byte chunk of a row, as the plain sum.
 __global__ void __launch_bounds__(256)
 segment_sum_split_kernel(const __nv_bfloat16* __restrict__ in, const int* __restrict__ perm, const int* __restrict__ offsets,
                          __nv_bfloat16* __restrict__ out, long long ldo, long long N, int C) {
@@ -72,8 +74,8 @@ segment_sum_split_kernel(const __nv_bfloat16* __restrict__ in, const int* __rest
 
 }  // namespace pnm
 
-extern "C" int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, const void* W3t, const void* W2t, int act, void* g1, float* dW3,
-                            float* dW2, float* db3, float* db2, long long M, void* stream) {
+extern "C" int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, const void* h2, const void* h1, const void* W3t, const void* W2t,
+                            int act, void* g1, float* dW3, float* dW2, float* db3, float* db2, long long M, void* stream) {
   using namespace pnm;
   int* err = error_word_ptr();
   if (!err) return -1;
@@ -81,8 +83,10 @@ extern "C" int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, con
   if (((reinterpret_cast<uintptr_t>(z2) | reinterpret_cast<uintptr_t>(z1) | reinterpret_cast<uintptr_t>(g1)) & 31) ||
       ((reinterpret_cast<uintptr_t>(dW3) | reinterpret_cast<uintptr_t>(dW2)) & 15))
     return -3;
-  CUtensorMap td, t3, t2;
+  CUtensorMap td, th2, th1, t3, t2;
   if (make_tmap_2d_b16(&td, dx3, M, kMlpW, kMlpW, kMlpRows, 64)) return -9;
+  if (make_tmap_2d_b16(&th2, h2, M, kMlpW, kMlpW, kMlpRows, 64)) return -12;
+  if (make_tmap_2d_b16(&th1, h1, M, kMlpW, kMlpW, kMlpRows, 64)) return -13;
   if (make_tmap_2d_b16(&t3, W3t, kMlpW, kMlpW, kMlpW, kMlpW, 64)) return -10;
   if (make_tmap_2d_b16(&t2, W2t, kMlpW, kMlpW, kMlpW, kMlpW, 64)) return -11;
   MlpBwdArgs g{};
@@ -94,9 +98,9 @@ extern "C" int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, con
   const int grid = int(tiles < sms ? tiles : sms);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   switch (act) {
-    case MLP_SILU: return launch_mlp3_bwd<MLP_SILU>(td, t3, t2, g, grid, st);
-    case MLP_RELU: return launch_mlp3_bwd<MLP_RELU>(td, t3, t2, g, grid, st);
-    case MLP_GELU: return launch_mlp3_bwd<MLP_GELU>(td, t3, t2, g, grid, st);
+    case MLP_SILU: return launch_mlp3_bwd<MLP_SILU>(td, th2, th1, t3, t2, g, grid, st);
+    case MLP_RELU: return launch_mlp3_bwd<MLP_RELU>(td, th2, th1, t3, t2, g, grid, st);
+    case MLP_GELU: return launch_mlp3_bwd<MLP_GELU>(td, th2, th1, t3, t2, g, grid, st);
   }
   return -7;
 }
@@ -115,15 +119,16 @@ extern "C" int pnm_segment_sum_split(const void* in, const int* perm, const int*
 extern "C" int pnm_mlp3_ln_fwd(int nsrc, const void* const* src, const long long* rows, const int* ld, const int* const* idx, const void* W1,
                                const void* W2, const void* W3, const float* b1, const float* b2, const float* b3, const float* gamma,
                                const float* beta, float eps, int act, const void* post, long long ld_post, void* y, long long ld_y, void* z1,
-                               void* z2, void* x3, float* mean, float* rstd, long long M, void* stream) {
+                               void* z2, void* h1, void* h2, void* x3, float* mean, float* rstd, long long M, void* stream) {
   using namespace pnm;
   int* err = error_word_ptr();
   if (!err) return -1;
   if (nsrc < 1 || nsrc > 3 || M <= 0 || M > 0x7fffff00LL || !gamma || !y) return -2;
-  const bool save = z1 != nullptr;
-  if (save && (!z2 || !x3 || !mean || !rstd)) return -5;
+  const bool save = h1 != nullptr;
+  if (save && (!h1 || !h2 || !x3 || !mean || !rstd || (act != MLP_RELU && (!z1 || !z2)))) return -5;
   const uintptr_t sectors = reinterpret_cast<uintptr_t>(post) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z1) |
-                            reinterpret_cast<uintptr_t>(z2) | reinterpret_cast<uintptr_t>(x3) | uintptr_t((post ? ld_post : 0) * 2) |
+                            reinterpret_cast<uintptr_t>(z2) | reinterpret_cast<uintptr_t>(h1) | reinterpret_cast<uintptr_t>(h2) |
+                            reinterpret_cast<uintptr_t>(x3) | uintptr_t((post ? ld_post : 0) * 2) |
                             uintptr_t(ld_y * 2);
   if (sectors & 31) return -3;                   // rows are read and written as 32-byte vectors
   const uintptr_t vec = reinterpret_cast<uintptr_t>(b1) | reinterpret_cast<uintptr_t>(b2) | reinterpret_cast<uintptr_t>(b3) |
@@ -144,6 +149,7 @@ extern "C" int pnm_mlp3_ln_fwd(int nsrc, const void* const* src, const long long
   g.post = reinterpret_cast<const __nv_bfloat16*>(post); g.ld_post = ld_post;
   g.y = reinterpret_cast<__nv_bfloat16*>(y); g.ld_y = ld_y;
   g.z1 = reinterpret_cast<__nv_bfloat16*>(z1); g.z2 = reinterpret_cast<__nv_bfloat16*>(z2); g.x3 = reinterpret_cast<__nv_bfloat16*>(x3);
+  g.h1 = reinterpret_cast<__nv_bfloat16*>(h1); g.h2 = reinterpret_cast<__nv_bfloat16*>(h2);
   g.mean = mean; g.rstd = rstd; g.eps = eps; g.act = act; g.err = err;
   const long long tiles = (M + kMlpRows - 1) / kMlpRows;
   const int sms = num_sms();

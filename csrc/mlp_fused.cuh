@@ -7,8 +7,8 @@
 // An edge row needs its own 256 bytes, two gathered node rows (mostly from L2) and 256 bytes of result; run layer by layer the
 // same chain moves fifteen such rows through HBM.  Here everything between the sources and the result stays on the SM, and what
 // is left is the latency of a tile's chain (product, epilogue, product, epilogue, product, normalisation):
-// 1.5 M rows from three sources take 0.56 ms (0.66 ms with the pre-activations kept), one source 0.34 ms, where the rows'
-// own traffic is worth 0.2 ms.  A MeshGraphNet step on 250 k nodes / 1.4 M edges, forward: 1.26 -> 0.70 ms.
+// 1.4 M rows from three sources take 0.53 ms, where the rows' own traffic is worth 0.15 ms; with what the backward needs (five more
+// rows each, 0.33 ms) 0.73 ms.  A MeshGraphNet step on 250 k nodes / 1.4 M edges, forward: 1.26 -> 0.70 ms.
 //   * W1, W2, W3 (96 + 32 + 32 KB in bf16 for three sources) are loaded once per persistent CTA and stay in shared memory;
 //   * gathered rows arrive by TMA gather4 (four indexed rows of 128 bytes per instruction, written in the same 128-byte
 //     swizzle as a plain tile), so no gathered copy of the node features exists;
@@ -30,7 +30,7 @@ constexpr int kMlpW = 128;                       // width of every layer
 constexpr int kMlpRows = 128;                    // rows of a tile
 constexpr int kMlpChunk = kMlpRows * 128;        // 128 rows x 64 bf16
 constexpr int kMlpThreads = 640;                 // producer, MMA warp, 2 idle warps, 2 x 8 epilogue warps
-constexpr int kMlpTmemCols = 512;                // per group of 256: accumulator 128, packed A operand 64, row statistics 4
+constexpr int kMlpTmemCols = 512;                // per group of 256: accumulator 128, packed A operand 64, row statistics 8
 
 enum { MLP_SILU = 2, MLP_RELU = 3, MLP_GELU = 1 };   // same codes as the GEMM epilogues
 
@@ -40,7 +40,10 @@ struct MlpArgs {
   const float *b1, *b2, *b3, *gamma, *beta;
   const __nv_bfloat16* post; long long ld_post;
   __nv_bfloat16* y; long long ld_y;
-  __nv_bfloat16 *z1, *z2, *x3;                   // kept for the backward (contiguous [M, 128]) or null
+  // kept for the backward or null: pre-activations (whole tiles, see z_offset), their activations and the rows before the LayerNorm
+  // (contiguous [M, 128]), the moments of the rounded rows.  ReLU keeps no pre-activations: the signs of the activations are all
+  // that its derivative needs.
+  __nv_bfloat16 *z1, *z2, *h1, *h2, *x3;
   float *mean, *rstd;
   float eps;
   int act;
@@ -96,6 +99,14 @@ template <int ACT>
 __device__ __forceinline__ float mlp_act(float x) {
   return ACT == MLP_SILU ? silu_f(x) : ACT == MLP_GELU ? gelu_f(x) : fmaxf(x, 0.f);
 }
+
+// Pre-activations lie as the threads hold them: vector c (16 columns) of lane l of a warp at (warp's block) + (32 c + l) * 16, so that a
+// warp's 32-byte vectors are 1 KB in one piece, here and in the backward.  (With a row of its own per lane every access touches 32
+// lines; the busiest unit of the kernel that keeps its rows is the one that handles those, at 61 %.)
+__device__ __forceinline__ long long z_offset(long long tile, int q, int half, int lane) {
+  return (((tile * 4 + q) * 2 + half) * 4 * 32 + lane) * 16;
+}
+constexpr int kZStep = 32 * 16;                  // elements from one vector of a thread to its next
 
 template <int NSRC>
 struct MlpCfg {
@@ -271,7 +282,8 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
 #pragma unroll 1
       for (int layer = 0; layer < 2; ++layer) {
         const float* bias = vec + layer * kMlpW + col;
-        __nv_bfloat16* z = layer ? g.z2 : g.z1;
+        __nv_bfloat16* z = (layer ? g.z2 : g.z1) + z_offset(tile, q, half, lane);
+        __nv_bfloat16* h = (layer ? g.h2 : g.h1) + row * kMlpW + col;
         ok = mbar_wait(&accfull[grp], uses & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         ++uses;
@@ -285,19 +297,35 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
           float* x = v[c & 1];
           add_vec16(x, bias + c * 16);
           uint32_t p[8];
-          if (SAVE) {
+          if (SAVE && ACT != MLP_RELU) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) p[j] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
-            if (live) stg32(z + row * kMlpW + col + c * 16, p);
+            stg32(z + c * kZStep, p);            // rows past M too: the buffer holds whole tiles
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) p[j] = pack_bf16x2(mlp_act<ACT>(x[2 * j]), mlp_act<ACT>(x[2 * j + 1]));
           tmem_st8(aop + c * 8, p);
+          if (SAVE && ACT == MLP_RELU && live) stg32(h + c * 16, p);
         }
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&aready[grp]);
+        if (SAVE && ACT != MLP_RELU) {
+          // The weight gradient's operand is this product's: recomputed from the rounded pre-activation it would be rounded twice (dW2
+          // against 64 bits 0.0054 instead of 0.0049).  Read back and stored while the product runs (814 -> 778 us at 1.4 M rows; not
+          // with ReLU, which stores nothing else: 631 -> 650 us).
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            float p[16];
+            tmem_ld16(aop + c * 16, p);
+            tmem_ld_wait();
+            if (live) {
+              stg32(h + c * 32, reinterpret_cast<const uint32_t*>(p));
+              stg32(h + c * 32 + 16, reinterpret_cast<const uint32_t*>(p) + 8);
+            }
+          }
+        }
       }
       if (ok) {
         ok = mbar_wait(&accfull[grp], uses & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL);
@@ -306,7 +334,8 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
       ++uses;
       tc_fence_after();
       // moments of this half about its first element (a value of the row: no cancellation against a large mean)
-      float pivot = 0.f, sum = 0.f, sq = 0.f;
+      // (and, for the backward, those of the rounded rows that it will read: moments of other values would cost it precision)
+      float pivot = 0.f, sum = 0.f, sq = 0.f, sum_k = 0.f, sq_k = 0.f;
       if (ok) {
         float v[2][16];
         tmem_ld16(acc, v[0]);
@@ -316,20 +345,28 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
           if (c < 3) tmem_ld16(acc + (c + 1) * 16, v[(c + 1) & 1]);
           float* x = v[c & 1];
           add_vec16(x, vec + 2 * kMlpW + col + c * 16);
+          if (c == 0) pivot = x[0];
           if (SAVE) {
             uint32_t p[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) p[j] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
+            for (int j = 0; j < 8; ++j) {
+              p[j] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
+              const float2 k = unpack_bf16x2(p[j]);
+              const float d0 = k.x - pivot, d1 = k.y - pivot;
+              sum_k += d0 + d1;
+              sq_k = fmaf(d0, d0, fmaf(d1, d1, sq_k));
+            }
             if (live) stg32(g.x3 + row * kMlpW + col + c * 16, p);
           }
-          if (c == 0) pivot = x[0];
 #pragma unroll
           for (int j = 0; j < 16; ++j) { const float d = x[j] - pivot; sum += d; sq += d * d; }
         }
       }
       const float shift = sum * (1.f / 64), mean_h = pivot + shift, dev_h = fmaxf(sq - sum * shift, 0.f);
+      const float shift_k = sum_k * (1.f / 64), mean_k = pivot + shift_k, dev_k = fmaxf(sq_k - sum_k * shift_k, 0.f);
       if (ok) {
         tmem_st2(stat + 2 * half, mean_h, dev_h);
+        if (SAVE) tmem_st2(stat + 4 + 2 * half, mean_k, dev_k);
         tmem_st_wait();
       }
       Vec32 res = {};
@@ -344,7 +381,14 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
       const float2 other = tmem_ld2(stat + 2 * (half ^ 1));
       const float mean = 0.5f * (mean_h + other.x), gap = mean_h - other.x;
       const float rstd = rsqrtf((dev_h + other.y + 32.f * gap * gap) * (1.f / kMlpW) + g.eps);
-      if (SAVE && live && half == 0) { g.mean[row] = mean; g.rstd[row] = rstd; }
+      if (SAVE) {
+        const float2 other_k = tmem_ld2(stat + 4 + 2 * (half ^ 1));
+        const float gap_k = mean_k - other_k.x;
+        if (live && half == 0) {
+          g.mean[row] = 0.5f * (mean_k + other_k.x);
+          g.rstd[row] = rsqrtf((dev_k + other_k.y + 32.f * gap_k * gap_k) * (1.f / kMlpW) + g.eps);
+        }
+      }
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         float v[16];

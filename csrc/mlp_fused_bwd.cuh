@@ -5,14 +5,14 @@
 //   g1 = (g2 W2) * act'(z1)       dW2 += g2^T act(z1),  db2 += g2
 //
 // Layer by layer these are two data-gradient and two weight-gradient products that move ten 256-byte rows per row of M; here
-// a row tile is read once (dx3, z2, z1) and only g1 is written: four rows (1.5 M rows: 0.55 ms; the rows are worth 0.23 ms, the
-// rest is the chain of two products and three passes over a tile).  (The LayerNorm backward before it stays a kernel
+// a row tile is read once (dx3, z2, act(z2), z1, act(z1)) and only g1 is written: six rows
+// (1.7 M rows: 0.47 ms, the rows are worth 0.39 ms; with the activations recomputed from z in the same threads 0.62 ms).  (The LayerNorm backward before it stays a kernel
 // of its own: its column sums are free when a warp works along a row, but cost eight instructions per element when, as here,
 // a thread owns a row; with it inside, this kernel was bound by instruction issue at 1.41 ms for 1.5 M rows.)
-// dx3 arrives by TMA; g2 overwrites it.  A gradient tile lies in shared memory once, in the 128-byte-swizzled layout that
+// dx3 and act(z2) arrive by TMA; g2 overwrites dx3 and act(z1) takes the place of act(z2).  A gradient tile lies in shared memory once, in the 128-byte-swizzled layout that
 // tcgen05 reads both ways: as the K-major A operand of the data gradient and, with the row index as the reduction, as the
-// MN-major A operand of the weight gradient; the activations that the weight gradient needs are recomputed from z.  Both
-// weight gradients accumulate in TMEM over all tiles of a persistent CTA and are added to memory once at its end.
+// MN-major A operand of the weight gradient.  (The activations are the forward's own operands: recomputed from the rounded z
+// they would be rounded twice.)  Both weight gradients accumulate in TMEM over all tiles of a persistent CTA and are added to memory once at its end.
 // Two tiles are in flight, one per group of eight warps (two threads per row); ONE thread issues all products, since products
 // that accumulate into the same TMEM columns are only ordered within a thread.  A further warp per group sums the columns
 // of the gradient tile while the tensor cores read it.
@@ -23,7 +23,7 @@ namespace pnm {
 
 struct MlpBwdArgs {
   long long M;
-  const __nv_bfloat16 *z2, *z1;                  // contiguous [M, 128]
+  const __nv_bfloat16 *z2, *z1;                  // whole tiles (z_offset); ReLU: the activations, contiguous [M, 128]
   __nv_bfloat16* g1;                             // [M, 128]
   float *dW3, *dW2, *db3, *db2;                  // added to
   int* err;
@@ -43,24 +43,18 @@ __device__ __forceinline__ void tile_put16(uint8_t* tile, int r, int c, const ui
   *reinterpret_cast<uint4*>(row + (((u + 1) ^ (r & 7)) << 4)) = make_uint4(p[4], p[5], p[6], p[7]);
 }
 
-// Makes the compiler forget where a vector came from: without it the tanh of act(z) is kept for act'(z) across the wait between
-// them, 64 more live registers than there are.
-__device__ __forceinline__ void forget(Vec32& v) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) asm volatile("" : "+r"(v.w[j]));
-}
-
 template <int ACT>
 __global__ void __launch_bounds__(kMlpThreads, 1)
-mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmW3t, const __grid_constant__ CUtensorMap tmW2t,
-                const MlpBwdArgs g) {
+mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmH2, const __grid_constant__ CUtensorMap tmH1,
+                const __grid_constant__ CUtensorMap tmW3t, const __grid_constant__ CUtensorMap tmW2t, const MlpBwdArgs g) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* wts = smem_raw;
   uint8_t* tiles_smem = wts + 4 * kMlpChunk;     // per group: gradient tile (2 chunks), activation tile (2 chunks)
   uint64_t* wfull = reinterpret_cast<uint64_t*>(tiles_smem + 8 * kMlpChunk);
-  uint64_t* dfull = wfull + 1;                   // [2] dx3 of a tile has arrived
-  uint64_t* dfree = dfull + 2;                   // [2] the gradient tile was read for the last time
-  uint64_t* ready = dfree + 2;                   // [2] the activation tile (second phase: and g2) is written, the accumulator was read
+  uint64_t* dfull = wfull + 1;                   // [2] dx3 and act(z2) of a tile have arrived
+  uint64_t* hfull = dfull + 2;                   // [2] act(z1) has arrived
+  uint64_t* dfree = hfull + 2;                   // [2] both tiles were read for the last time
+  uint64_t* ready = dfree + 2;                   // [2] the accumulator was read (second phase: and g2 is written)
   uint64_t* done = ready + 2;                    // [2] the phase's products and column sums are finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -71,7 +65,9 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
 
   if (threadIdx.x == 0) {
     mbar_init(wfull, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&dfull[i], 1); mbar_init(&dfree[i], 2); mbar_init(&ready[i], 8); mbar_init(&done[i], 2); }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&dfull[i], 1); mbar_init(&hfull[i], 1); mbar_init(&dfree[i], 2); mbar_init(&ready[i], 8); mbar_init(&done[i], 2);
+    }
     *abort_flag = 0;
     mbar_fence_init();
     if (smem_u32(smem_raw) & 1023) { atomicCAS(g.err, 0, ERR_BAD_ARG); *abort_flag = 1; }
@@ -101,7 +97,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         for (int grp = 0; grp < 2; ++grp) {
           const int layer = at[grp] & 1;
           if (!left[grp] || !mbar_try_wait(&ready[grp], layer)) continue;
-          if (layer == 0 && !mbar_try_wait(&dfull[grp], (at[grp] >> 1) & 1)) continue;
+          if (!mbar_try_wait(layer ? &hfull[grp] : &dfull[grp], (at[grp] >> 1) & 1)) continue;
           any = true;
           tc_fence_after();
           const uint32_t xs = smem_u32(tiles_smem + grp * 4 * kMlpChunk), ws = smem_u32(wts + layer * 2 * kMlpChunk);
@@ -135,12 +131,14 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
       }
     }
   } else if (warp <= 2) {
-    // ------------------------------------------------------------- column sums of group warp - 1: lane l owns four columns
+    // ------------------------------- column sums of group warp - 1: lane l owns four columns; between them the load of act(z1)
     const int grp = warp - 1;
     const uint8_t* x = tiles_smem + grp * 4 * kMlpChunk + (lane >> 4) * kMlpChunk;
     const int u = (lane & 15) >> 1, low = (lane & 1) * 8;
     float s[2][4] = {};
+    uint32_t issued = 0;
     const int phases = 2 * (grp == 0 ? (mine + 1) / 2 : mine / 2);
+    uint8_t* ht = tiles_smem + (grp * 4 + 2) * kMlpChunk;
     for (int ph = 0; ph < phases; ++ph) {
       const bool second = ph & 1;
       // first phase: dx3 from TMA; second: g2 from the group's warps
@@ -154,27 +152,33 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y);
         t[0] += a.x; t[1] += a.y; t[2] += b.x; t[3] += b.y;
       }
-      // Every phase of `ready` is seen in turn, and this warp arrives on `done` only after it has seen the one before: without that
-      // arrival the group cannot complete the next.  (Waited for after the arrival, a phase could be over and the next of the same
-      // parity be awaited, which itself needs this warp.)  The products wait for the same phase, so nothing is delayed.
-      if (!second) {
-        ok = mbar_wait(&ready[grp], 0, abort_flag, g.err, ERR_WAIT_AUX);
-        if (!__all_sync(0xffffffffu, ok)) break;
-      }
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&done[grp]);
         if (second) mbar_arrive(&dfree[grp]);
       }
+      // Every phase of `done` is awaited here; each needs this warp's own arrival, so none is missed.  `ready` has completed its phase of
+      // the same number by then and cannot complete the one after the next without `done`: no wait here can meet a phase of the same
+      // parity two further on, however slow this warp is.
+      ok = mbar_wait(&done[grp], ph & 1, abort_flag, g.err, ERR_WAIT_AUX);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!second && lane == 0) {                // act(z2) was read by the first phase's products: act(z1) takes its place
+        const int m0 = (int(blockIdx.x) + (ph + grp) * int(gridDim.x)) * kMlpRows;      // tile ph / 2 of the group
+        mbar_expect_tx(&hfull[grp], 2 * kMlpChunk);
+        tma_load_2d(ht, &tmH1, &hfull[grp], 0, m0);
+        tma_load_2d(ht + kMlpChunk, &tmH1, &hfull[grp], 64, m0);
+        ++issued;
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) { s[0][i] += second ? 0.f : t[i]; s[1][i] += second ? t[i] : 0.f; }
     }
+    if (issued) mbar_drain(&hfull[grp], (issued - 1) & 1);
     const int col = (lane >> 4) * 64 + u * 8 + (lane & 1) * 4;
     if (phases)
 #pragma unroll
       for (int i = 0; i < 4; ++i) { atomicAdd(g.db3 + col + i, s[0][i]); atomicAdd(g.db2 + col + i, s[1][i]); }
   } else if (warp == 3) {
-    // ------------------------------------------------------------------------------------------------ dx3 tiles
+    // --------------------------------------------------------------------------------------- dx3 and act(z2) tiles
     if (lane == 0) {
       uint32_t issued[2] = {0, 0};
 #pragma unroll 1
@@ -183,9 +187,11 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         if (k && !mbar_wait(&dfree[grp], (k - 1) & 1, abort_flag, g.err, ERR_WAIT_EMPTY)) break;
         uint8_t* dst = tiles_smem + grp * 4 * kMlpChunk;
         const int m0 = (int(blockIdx.x) + n * int(gridDim.x)) * kMlpRows;
-        mbar_expect_tx(&dfull[grp], 2 * kMlpChunk);
-        tma_load_2d(dst, &tmD, &dfull[grp], 0, m0);
-        tma_load_2d(dst + kMlpChunk, &tmD, &dfull[grp], 64, m0);
+        mbar_expect_tx(&dfull[grp], 4 * kMlpChunk);
+        for (int c = 0; c < 2; ++c) {
+          tma_load_2d(dst + c * kMlpChunk, &tmD, &dfull[grp], 64 * c, m0);
+          tma_load_2d(dst + (2 + c) * kMlpChunk, &tmH2, &dfull[grp], 64 * c, m0);
+        }
         ++issued[grp];
       }
       for (int grp = 0; grp < 2; ++grp)          // copies land before the CTA leaves, also after a wait that ran out
@@ -197,36 +203,26 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
     const uint32_t lanes = uint32_t(q * 32) << 16;
     const uint32_t acc = tmem + grp * 128 + lanes + col;
     uint8_t* gt = tiles_smem + grp * 4 * kMlpChunk;
-    uint8_t* ht = gt + 2 * kMlpChunk;
     uint32_t phase = 0;
     bool ok = true;
-    auto offset = [&](int n) {                   // rows past M repeat the last one: their dx3 is zero and their g1 not stored
-      const long long row = ((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + r;
-      return (row < g.M ? row : g.M - 1) * kMlpW + col;
+    constexpr int step = ACT == MLP_RELU ? 16 : kZStep;
+    auto offset = [&](int n) {                   // rows past M: their dx3 is zero and their g1 not stored
+      const long long tile = (long long)blockIdx.x + (long long)n * gridDim.x, row = tile * kMlpRows + r;
+      return ACT == MLP_RELU ? (row < g.M ? row : g.M - 1) * kMlpW + col : z_offset(tile, q, half, lane);
     };
     Vec32 z[4];
     if (grp < mine) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) z[c] = ldg32(g.z2 + offset(grp) + c * 16);
+      for (int c = 0; c < 4; ++c) z[c] = ldg32(g.z2 + offset(grp) + c * step);
     }
     for (int n = grp; n < mine; n += 2) {
       const bool live = ((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + r < g.M;
       const long long o = offset(n);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {              // act(z2): the other operand of dW3
-        uint32_t p[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 zv = unpack_bf16x2(z[c].w[j]);
-          p[j] = pack_bf16x2(mlp_act<ACT>(zv.x), mlp_act<ACT>(zv.y));
-        }
-        tile_put16(ht, r, half * 4 + c, p);
-      }
-      fence_async_smem();
-      tc_fence_before();
+      __nv_bfloat16* g1 = g.g1 + (((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + r) * kMlpW + col;
+      tc_fence_before();                         // the accumulator was read: the last tile's g1 is on its way
       __syncwarp();
       if (lane == 0) mbar_arrive(&ready[grp]);
-      // ---- g2 = (dx3 W3) act'(z2), then act(z1); each vector of z1 is requested where one of z2 is used up
+      // ---- g2 = (dx3 W3) act'(z2); each vector of z1 is requested where one of z2 is used up
       ok = mbar_wait(&done[grp], phase & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL) && ok;
       ++phase;
       tc_fence_after();
@@ -235,7 +231,6 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         float v[16];
         tmem_ld16(acc + c * 16, v);
         tmem_ld_wait();
-        forget(z[c]);
         uint32_t p[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -243,17 +238,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
           p[j] = pack_bf16x2(v[2 * j] * mlp_dact<ACT>(zv.x), v[2 * j + 1] * mlp_dact<ACT>(zv.y));
         }
         tile_put16(gt, r, half * 4 + c, p);
-        z[c] = ldg32(g.z1 + o + c * 16);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t p[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 zv = unpack_bf16x2(z[c].w[j]);
-          p[j] = pack_bf16x2(mlp_act<ACT>(zv.x), mlp_act<ACT>(zv.y));
-        }
-        tile_put16(ht, r, half * 4 + c, p);
+        z[c] = ldg32(g.z1 + o + c * step);
       }
       fence_async_smem();
       tc_fence_before();
@@ -269,15 +254,14 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
         float v[16];
         tmem_ld16(acc + c * 16, v);
         tmem_ld_wait();
-        forget(z[c]);
         uint32_t p[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float2 zv = unpack_bf16x2(z[c].w[j]);
           p[j] = pack_bf16x2(v[2 * j] * mlp_dact<ACT>(zv.x), v[2 * j + 1] * mlp_dact<ACT>(zv.y));
         }
-        if (live) stg32(g.g1 + o + c * 16, p);
-        z[c] = ldg32(g.z2 + on + c * 16);
+        if (live) stg32(g1 + c * 16, p);
+        z[c] = ldg32(g.z2 + on + c * step);
       }
     }
     // A wait that ran out leaves wrong values behind (the error word says so); the loop ends all the same, since every later

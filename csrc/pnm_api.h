@@ -45,17 +45,18 @@ int pnm_layernorm_bwd(const void* dy, const void* x, const float* gamma, const f
                       void* stream);
 
 // y = LN(act(act([src0 | src1 | src2] W1^T + b1) W2^T + b2) W3^T + b3) [+ post], every layer 128 wide, bf16 tables and weights,
-// fp32 vectors; row m of source j is src[j][idx[j] ? idx[j][m] : m].  act: 1 GELU, 2 SiLU, 3 ReLU.  z1 / z2 / x3 (the
-// pre-activations, [M, 128]) and mean / rstd are kept for the backward when z1 is given.  Tables that are written or added
+// fp32 vectors; row m of source j is src[j][idx[j] ? idx[j][m] : m].  act: 1 GELU, 2 SiLU, 3 ReLU.  When h1 is given,
+// the backward's needs are kept: the pre-activations z1 / z2 (whole tiles of 128 rows, in an order of the kernel's own; not with ReLU),
+// h1 / h2 = act(z1), act(z2), the rows x3 before the LayerNorm ([M, 128] each) and mean / rstd of the bf16 rows x3.  Tables that are written or added
 // start on 32-byte boundaries, row by row.
 int pnm_mlp3_ln_fwd(int nsrc, const void* const* src, const long long* rows, const int* ld, const int* const* idx, const void* W1,
                     const void* W2, const void* W3, const float* b1, const float* b2, const float* b3, const float* gamma,
                     const float* beta, float eps, int act, const void* post, long long ld_post, void* y, long long ld_y, void* z1,
-                    void* z2, void* x3, float* mean, float* rstd, long long M, void* stream);
-// Its backward from dx3 = d loss / d (third pre-activation) down to g1 = d loss / d z1, [M, 128] each; W3t / W2t: transposed
+                    void* z2, void* h1, void* h2, void* x3, float* mean, float* rstd, long long M, void* stream);
+// Its backward (ReLU: h2, h1 also stand for z2, z1) from dx3 = d loss / d (third pre-activation) down to g1 = d loss / d z1, [M, 128] each; W3t / W2t: transposed
 // bf16 weights; the fp32 gradients are added to.
-int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, const void* W3t, const void* W2t, int act, void* g1, float* dW3,
-                 float* dW2, float* db3, float* db2, long long M, void* stream);
+int pnm_mlp3_bwd(const void* dx3, const void* z2, const void* z1, const void* h2, const void* h1, const void* W3t, const void* W2t, int act,
+                 void* g1, float* dW3, float* dW2, float* db3, float* db2, long long M, void* stream);
 // out[n] = [hi | lo], hi + lo = fp32 sum of the contiguous [., C] rows in[perm[k]], k in [offsets[n], offsets[n+1]).
 int pnm_segment_sum_split(const void* in, const int* perm, const int* offsets, void* out, long long ldo, long long N, int C,
                           void* stream);

@@ -17,6 +17,7 @@ from . import gemm as _g
 from . import graph as _graph
 
 WIDTH = 128
+ROWS = 128                                                   # rows of a tile of the kernel
 _ACTS = (_g.ACT_GELU, _g.ACT_SILU, _g.ACT_RELU)
 
 
@@ -26,8 +27,8 @@ def _lib_mlp():
         c = ctypes
         vp, i, l, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
         lib.pnm_mlp3_ln_fwd.argtypes = [i, c.POINTER(vp), c.POINTER(l), c.POINTER(i), c.POINTER(vp), vp, vp, vp, vp, vp, vp, vp, vp, f, i,
-                                        vp, l, vp, l, vp, vp, vp, vp, vp, l, vp]
-        lib.pnm_mlp3_bwd.argtypes = [vp, vp, vp, vp, vp, i, vp, vp, vp, vp, vp, l, vp]
+                                        vp, l, vp, l, vp, vp, vp, vp, vp, vp, vp, l, vp]
+        lib.pnm_mlp3_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, i, vp, vp, vp, vp, vp, l, vp]
         lib.pnm_segment_sum_split.argtypes = [vp, vp, vp, vp, l, l, i, vp]
         lib.pnm_mlp3_ln_fwd.restype = lib.pnm_mlp3_bwd.restype = lib.pnm_segment_sum_split.restype = i
         lib._mlp3_declared = True
@@ -74,16 +75,20 @@ def _forward(srcs, segs, weights, biases, act, gamma, beta, eps, post, save: boo
     w16 = [_g._bf16_weight(w) for w in weights]
     vecs = [_vec(t) for t in (*biases, gamma, beta)]
     y = torch.empty((m, WIDTH), dtype=torch.bfloat16, device=dev)
-    kept = ()
-    if save:
+    kept, given = (), [None] * 7
+    if save:                                                 # h1, h2, x3, mean, rstd; z1 and z2 (whole tiles) but for ReLU
         kept = (*torch.empty((3, m, WIDTH), dtype=torch.bfloat16, device=dev).unbind(0),
                 *torch.empty((2, m), dtype=torch.float32, device=dev).unbind(0))
+        if act != _g.ACT_RELU:
+            kept += torch.empty((2, -(-m // ROWS), ROWS * WIDTH), dtype=torch.bfloat16, device=dev).unbind(0)
+        h1, h2, x3, mean, rstd, *z = [t.data_ptr() for t in kept]
+        given = [*(z or (None, None)), h1, h2, x3, mean, rstd]
     vp = ctypes.c_void_p
     code = lib.pnm_mlp3_ln_fwd(
         n, (vp * n)(*[t.data_ptr() for t in srcs]), (ctypes.c_longlong * n)(*[t.shape[0] for t in srcs]),
         (ctypes.c_int * n)(*[t.stride(0) for t in srcs]), (vp * n)(*[None if s is None else s.index32.data_ptr() for s in segs]),
         *[w.data_ptr() for w in w16], *[_g._ptr(v) for v in vecs], float(eps), act, _g._ptr(post), 0 if post is None else post.stride(0),
-        y.data_ptr(), WIDTH, *([t.data_ptr() for t in kept] if save else [None] * 5), m, _g._stream())
+        y.data_ptr(), WIDTH, *given, m, _g._stream())
     _g._check(code, "pnm_mlp3_ln_fwd")
     _g.launch_count += 1
     return y, kept
@@ -115,8 +120,9 @@ class _Mlp3LnFn(torch.autograd.Function):
         segs, post = ctx.segs, ctx.post
         n = len(segs)
         saved = ctx.saved_tensors                            # read once: activation checkpointing allows no second time
-        srcs, (w1, w2, w3, gamma, z1, z2, x3, mean, rstd) = saved[:n], saved[n:]
-        m, dev = z1.shape[0], z1.device
+        srcs, (w1, w2, w3, gamma, h1, h2, x3, mean, rstd, *z) = saved[:n], saved[n:]
+        z1, z2 = z or (h1, h2)
+        m, dev = x3.shape[0], x3.device
         dy = dy.contiguous()
         lib = _lib_mlp()
         # dW3, dW2, their biases, db1 and the blocks of dW1 of the plain sources in one zeroed buffer
@@ -133,8 +139,8 @@ class _Mlp3LnFn(torch.autograd.Function):
                                      _g._stream())
         _g._check(code, "pnm_layernorm_bwd")
         w3t, w2t = _w_t(w3), _w_t(w2)                        # held: the second look-up may empty the cache
-        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), w3t.data_ptr(), w2t.data_ptr(), ctx.act,
-                                g1.data_ptr(), dw3.data_ptr(), dw2.data_ptr(), db3.data_ptr(), db2.data_ptr(), m, _g._stream())
+        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), h2.data_ptr(), h1.data_ptr(), w3t.data_ptr(), w2t.data_ptr(),
+                                ctx.act, g1.data_ptr(), dw3.data_ptr(), dw2.data_ptr(), db3.data_ptr(), db2.data_ptr(), m, _g._stream())
         _g._check(code, "pnm_mlp3_bwd")
         _g.launch_count += 3
         need = ctx.needs_input_grad[5:]

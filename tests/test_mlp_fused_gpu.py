@@ -166,3 +166,44 @@ def test_mlp3_ln_without_gradients_keeps_forward_mode_and_tracing_honest():
         assert torch.equal(traced(other), want)
         with forward_ad.dual_level(), pytest.raises((NotImplementedError, RuntimeError)):
             m(forward_ad.make_dual(x, other))
+
+
+@pytest.mark.gpu
+def test_mlp3_keeps_the_moments_of_the_rows_that_the_backward_reads():
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    x = torch.randn(5000, W, device="cuda").bfloat16()
+    p = [torch.randn(W, W, device="cuda") / W ** 0.5 for _ in range(3)] + [0.1 * torch.randn(W, device="cuda") for _ in range(5)]
+    _, (h1, h2, x3, mean, rstd, *_) = mf._forward([x], [None], p[:3], p[3:6], 2, p[6], p[7], 1e-5, None, True)
+    ref = x3.double()
+    # fp32 moments of exactly these values
+    assert float((mean.double() - ref.mean(1)).abs().max()) < 1e-6 * float(ref.abs().max())
+    assert float((rstd.double() / torch.rsqrt(ref.var(1, unbiased=False) + 1e-5) - 1).abs().max()) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", [1, 2, 3])
+def test_mlp3_weight_gradients_are_as_exact_as_layer_by_layer(act):
+    """The operands of the weight gradients are those of the forward products, rounded once: the error against 64 bits is that of the
+    layered path (16 384 entries a matrix and four draws: the ratio scatters by half a per cent; operands rounded twice give 1.08)."""
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    err = {"one": [0.0] * 3, "layered": [0.0] * 3}
+    for draw in range(4):
+        x, up = (torch.randn(6001, W, device="cuda").bfloat16() for _ in range(2))
+        p = [torch.randn(W, W, device="cuda") / W ** 0.5 for _ in range(3)] + [0.1 * torch.randn(W, device="cuda") for _ in range(3)]
+        p += [1 + 0.1 * torch.randn(W, device="cuda"), 0.1 * torch.randn(W, device="cuda")]
+        q = [t.double().requires_grad_() for t in p]
+        h = ACTS[act](F.linear(ACTS[act](F.linear(x.double(), q[0], q[3])), q[1], q[4]))
+        ref = torch.autograd.grad(F.layer_norm(F.linear(h, q[2], q[5]), (W,), q[6], q[7]), q[:3], up.double())
+        for name in err:
+            w = [t.clone().requires_grad_() for t in p]
+            if name == "one":
+                y = mf.mlp3_ln([x], [None], w[:3], w[3:6], act, w[6], w[7], 1e-5, None)
+            else:
+                y = ops.layer_norm(ops.mlp_chain(x, w[:3], w[3:6], [act, act, 0]), w[6], w[7])
+            for k, (g, r) in enumerate(zip(torch.autograd.grad(y, w[:3], up), ref)):
+                err[name][k] += _rel(g, r)
+    for one, layered in zip(err["one"], err["layered"]):
+        assert one < 1.03 * layered
