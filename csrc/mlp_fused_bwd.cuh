@@ -31,9 +31,10 @@ struct MlpBwdArgs {
 
 constexpr int kMlpBwdSmem = 12 * kMlpChunk + 256;
 
+// v act'(z); ReLU selects, so that an infinite v beside a negative z is 0 and not NaN
 template <int ACT>
-__device__ __forceinline__ float mlp_dact(float z) {
-  return ACT == MLP_SILU ? silu_grad_f(z) : ACT == MLP_GELU ? gelu_grad_f(z) : (z > 0.f ? 1.f : 0.f);
+__device__ __forceinline__ float mlp_dact(float v, float z) {
+  return ACT == MLP_SILU ? v * silu_grad_f(z) : ACT == MLP_GELU ? v * gelu_grad_f(z) : (z > 0.f ? v : 0.f);
 }
 // 16 packed columns [16 c, 16 c + 16) of tile row r -> the swizzled tile of two 64-column chunks
 __device__ __forceinline__ void tile_put16(uint8_t* tile, int r, int c, const uint32_t* p) {
@@ -235,7 +236,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float2 zv = unpack_bf16x2(z[c].w[j]);
-          p[j] = pack_bf16x2(v[2 * j] * mlp_dact<ACT>(zv.x), v[2 * j + 1] * mlp_dact<ACT>(zv.y));
+          p[j] = pack_bf16x2(mlp_dact<ACT>(v[2 * j], zv.x), mlp_dact<ACT>(v[2 * j + 1], zv.y));
         }
         tile_put16(gt, r, half * 4 + c, p);
         z[c] = ldg32(g.z1 + o + c * step);
@@ -258,7 +259,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float2 zv = unpack_bf16x2(z[c].w[j]);
-          p[j] = pack_bf16x2(v[2 * j] * mlp_dact<ACT>(zv.x), v[2 * j + 1] * mlp_dact<ACT>(zv.y));
+          p[j] = pack_bf16x2(mlp_dact<ACT>(v[2 * j], zv.x), mlp_dact<ACT>(v[2 * j + 1], zv.y));
         }
         if (live) stg32(g1 + c * 16, p);
         z[c] = ldg32(g.z2 + on + c * step);

@@ -207,3 +207,25 @@ def test_mlp3_weight_gradients_are_as_exact_as_layer_by_layer(act):
                 err[name][k] += _rel(g, r)
     for one, layered in zip(err["one"], err["layered"]):
         assert one < 1.03 * layered
+
+
+@pytest.mark.gpu
+def test_relu_backward_drops_infinities_of_inactive_units():
+    """As layer by layer: the derivative selects.  Positive matrices make every unit's gradient infinite; one unit is active."""
+    from physicsnemo_b200.ops import gemm as G
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    m, dev = 200, "cuda"
+    dx3 = torch.full((m, W), 3e38, device=dev).bfloat16()
+    h2, h1 = torch.zeros(m, W, device=dev).bfloat16(), torch.zeros(m, W, device=dev).bfloat16()
+    h2[:, 5] = h1[:, 7] = 1.0
+    w = torch.ones(W, W, device=dev).bfloat16()
+    g1 = torch.empty(m, W, dtype=torch.bfloat16, device=dev)
+    dw, db = torch.zeros(2, W, W, device=dev), torch.zeros(2, W, device=dev)
+    rc = mf._lib_mlp().pnm_mlp3_bwd(dx3.data_ptr(), h2.data_ptr(), h1.data_ptr(), h2.data_ptr(), h1.data_ptr(), w.data_ptr(), w.data_ptr(),
+                                    G.ACT_RELU, g1.data_ptr(), dw[0].data_ptr(), dw[1].data_ptr(), db[0].data_ptr(), db[1].data_ptr(), m,
+                                    G._stream())
+    assert rc == 0
+    want = torch.zeros(m, W, device=dev)
+    want[:, 7] = float("inf")
+    assert torch.equal(g1.float(), want)
