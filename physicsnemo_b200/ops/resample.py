@@ -144,7 +144,9 @@ class _AddChannel(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dv = None
-        if ctx.needs_input_grad[1]:
+        if ctx.needs_input_grad[1] and torch.is_grad_enabled():          # a graph of the gradient is wanted (create_graph)
+            dv = g.sum((2, 3), keepdim=True)
+        elif ctx.needs_input_grad[1]:
             g = g.contiguous(memory_format=torch.channels_last)
             b, c, h, w = g.shape
             # two CTAs per SM, at least eight passes of a CTA's pixels each
@@ -159,8 +161,9 @@ class _AddChannel(torch.autograd.Function):
 
 def add_channel(x: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     """``x + v`` for a feature map ``x [B, C, H, W]`` and channel vectors ``v [B, C, 1, 1]``; own kernels (the gradient of ``v``
-    is one reduction over the pixels) for channels-last bf16 maps, the PyTorch expression otherwise."""
-    if (type(x) is torch.Tensor and type(v) is torch.Tensor and x.is_cuda and v.is_cuda and x.dtype == v.dtype == torch.bfloat16
+    is one reduction over the pixels) for channels-last bf16 maps, the PyTorch expression otherwise (and in forward mode, under a
+    function transform and while tracing, where it has what a kernel has not)."""
+    if (not _g.call_is_observed() and type(x) is torch.Tensor and type(v) is torch.Tensor and x.is_cuda and v.is_cuda and x.dtype == v.dtype == torch.bfloat16
             and x.dim() == 4 and x.numel() > 0 and v.shape == (*x.shape[:2], 1, 1) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048
             and x.shape[0] <= 65535 and x.is_contiguous(memory_format=torch.channels_last) and v.is_contiguous()
             and x.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0 and _lib.available()):

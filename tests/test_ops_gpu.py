@@ -888,3 +888,26 @@ def test_channel_vector_addition(b, c, h, w):
     ref = g.double().sum((2, 3), keepdim=True)
     # fp32 sums of h * w values of size one, then one bf16 rounding of the result
     assert float((v.grad.double() - ref).abs().max()) <= 2 ** -8 * float(ref.abs().max()) + 1e-5 * (h * w) ** 0.5
+
+
+@pytest.mark.gpu
+def test_channel_vector_addition_keeps_what_the_tensor_expression_has():
+    """Gradients of gradients, forward mode, function transforms and traces, as ``x + v``."""
+    from torch.autograd import forward_ad
+
+    from physicsnemo_b200.ops import resample
+
+    x, w = (torch.randn(2, 64, 8, 8, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last).requires_grad_() for _ in range(2))
+    v, t = (torch.randn(2, 64, 1, 1, device="cuda").bfloat16().requires_grad_() for _ in range(2))
+    second = []
+    for add in (resample.add_channel, torch.add):
+        first, = torch.autograd.grad((add(x, v) * w).sum(), v, create_graph=True)
+        second.append(torch.autograd.grad(first.float().square().sum(), w)[0])
+    assert torch.equal(*second) and second[0].abs().sum() > 0
+    x, v, t = x.detach(), v.detach(), t.detach()
+    with forward_ad.dual_level():
+        y = resample.add_channel(x, forward_ad.make_dual(v, t))
+        assert torch.equal(forward_ad.unpack_dual(y).tangent, t.expand_as(x))
+    assert torch.equal(torch.func.vmap(lambda a: resample.add_channel(x, a))(torch.stack([v, t])), torch.stack([x + v, x + t]))
+    traced = torch.jit.trace(resample.add_channel, (x, t), check_trace=False)
+    assert torch.equal(traced(x, v), x + v)
