@@ -262,8 +262,9 @@ layernorm_fwd_stream_kernel(const __nv_bfloat16* __restrict__ x, const float* __
 
 // dx = rstd * (g*dy - mean_c(g*dy) - xhat * mean_c(g*dy*xhat)) (+ dres); partial dgamma / dbeta rows go to
 // scratch[blockIdx.x][2][C], so that the column sums stay in registers until a CTA is done.
-// Measured (copy = 6.65 TB/s): 1 M x 256 forward 0.213 -> 0.191 ms (0.81 of copy), backward 0.420 -> 0.396 ms (0.78);
-// 1.4 M x 128 forward 0.177 -> 0.159 ms, backward 0.507 -> 0.293 ms (two rows per warp); 32 400 x 768 27.2 -> 25.7 us, 56.1 -> 49.9 us.
+// Measured against one row per warp from registers: 1 M x 256 forward 0.213 -> 0.191 ms (0.82 of 6544 GB/s), backward with a residual
+// gradient 0.420 -> 0.339 ms (0.92); 1.4 M x 128 forward 0.177 -> 0.159 ms, backward 0.507 -> 0.259 ms (two rows per warp);
+// 32 400 x 768 27.2 -> 25.7 us, 56.1 -> 54.2 us.
 template <int VEC, int LPR>
 __global__ void __launch_bounds__(kLnStreamThreads, VEC == 1 ? 3 : (VEC == 2 ? 2 : 1))
 layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
@@ -441,21 +442,26 @@ layernorm_bwd_finalize_kernel(const float* __restrict__ scratch, int nblocks, in
 }
 
 // Rows of a stage, stages and CTAs per SM of the streaming kernels: stages of about 16 KB per tensor (more rows where they are
-// short), `per_sm` rings that together fill the shared memory; with few rows in all, the smallest stage that still gives every
-// warp a row, so that the rows spread over more SMs.
+// short) of which two fit a ring, `per_sm` rings that together fill the shared memory; with few rows in all, the smallest stage that
+// still gives every warp a row, so that the rows spread over more SMs.  (Three tensors of 16 KB, twice, fill half the shared memory: a
+// third of the CTAs then ran as a second wave.  1 M x 256 backward with a residual gradient 398 -> 339 us, 0.92 of the copy rate;
+// 1.4 M x 128 296 -> 259 us; 100 003 x 256 64 -> 50 us.)
 struct LnStream { int rows, stages, grid, smem; };
 inline LnStream ln_stream_plan(long long M, int C, int tensors, int least_rows, int per_sm, int num_sms) {
   LnStream p;
-  int rows = (16384 / (2 * C)) / least_rows * least_rows;
+  const int budget = 220 * 1024 / per_sm - 256, fits = budget / (4 * C * tensors);      // rows of each of two stages
+  int rows = 16384 / (2 * C);
+  if (rows > fits) rows = fits;
   if (rows > 256) rows = 256;
+  rows = rows / least_rows * least_rows;
   if (rows < least_rows || M < (long long)num_sms * per_sm * rows) rows = least_rows;
-  const int stage = rows * C * 2 * tensors, budget = 220 * 1024 / per_sm - 256;
+  const int stage = rows * C * 2 * tensors;
   p.rows = rows;
-  p.stages = budget / stage < 2 ? 2 : (budget / stage > 8 ? 8 : budget / stage);
-  const long long tiles = (M + rows - 1) / rows, cap = (long long)num_sms * per_sm;
-  p.grid = int(tiles < cap ? tiles : cap);
+  p.stages = budget / stage > 8 ? 8 : budget / stage;
   const int ring = p.stages * stage;             // the backward folds its warps in the ring's place
   p.smem = (ring > kLnFoldBytes ? ring : kLnFoldBytes) + p.stages * 16 + 16;
+  const long long tiles = (M + rows - 1) / rows, cap = (long long)num_sms * per_sm;
+  p.grid = int(tiles < cap ? tiles : cap);
   return p;
 }
 constexpr int kLnSmemMax = 225 * 1024;
@@ -503,7 +509,10 @@ inline int launch_layernorm_fwd(const void* x, const void* r, const float* gamma
 inline int ln_bwd_rows(int C) { return C <= 128 ? 2 * kLnWarps : kLnWarps; }
 inline int ln_bwd_per_sm(int C) { return C <= 256 ? 3 : (C <= 512 ? 2 : 1); }
 inline int layernorm_bwd_grid(long long M, int num_sms, int C) {
-  return M > 0 ? ln_stream_plan(M, C, 2, ln_bwd_rows(C), ln_bwd_per_sm(C), num_sms).grid : 1;
+  if (M <= 0) return 1;
+  const int a = ln_stream_plan(M, C, 2, ln_bwd_rows(C), ln_bwd_per_sm(C), num_sms).grid;
+  const int b = ln_stream_plan(M, C, 3, ln_bwd_rows(C), ln_bwd_per_sm(C), num_sms).grid;
+  return a > b ? a : b;
 }
 
 template <int VEC, int LPR>

@@ -1,4 +1,4 @@
-"""The once-per-device kernel attributes of the launchers, on the host with a stand-in for the CUDA call."""
+"""Host side of the launchers: the once-per-device kernel attributes (with a stand-in for the CUDA call) and the LayerNorm plan."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -49,12 +49,48 @@ int main() {
 """
 
 
-@pytest.mark.skipif(not Path(NVCC).exists(), reason="no nvcc")
-def test_no_thread_launches_before_the_attribute_is_set(tmp_path):
-    src = tmp_path / "first_use.cu"
-    src.write_text(PROGRAM)
-    exe = tmp_path / "first_use"
+PLAN = r"""
+#include <cstdio>
+#include "norm.cuh"
+using namespace pnm;
+int main() {
+  const int sms = 148;
+  for (int C = 8; C <= 1024; C += 8)
+    for (long long M : {1LL, 7LL, 100LL, 3551LL, 10656LL, 14207LL, 14208LL, 60001LL, 113663LL, 113664LL, 1000000LL, 3000000LL})
+      for (int tensors = 1; tensors <= 3; ++tensors)
+        for (int backward = 0; backward < 2; ++backward) {
+          if (tensors == (backward ? 1 : 3)) continue;
+          const int least = backward ? ln_bwd_rows(C) : kLnWarps * (C <= 256 ? 2 : 1);
+          const int per_sm = backward ? ln_bwd_per_sm(C) : (C <= 512 ? 3 : 2);
+          const LnStream p = ln_stream_plan(M, C, tensors, least, per_sm, sms);
+          const long long ring = 1LL * p.stages * p.rows * C * 2 * tensors;
+          const bool ok = p.rows >= least && p.rows % least == 0 && p.stages >= 2 && p.stages <= 8 && p.grid >= 1 &&
+                          p.smem >= ring + 16 * p.stages + 8 && (!backward || p.smem >= kLnFoldBytes + 16 * p.stages + 8) &&
+                          p.smem <= kLnSmemMax && 1LL * per_sm * (p.smem + 1024) <= 228 * 1024 &&   // all CTAs of the grid are resident
+                          p.grid <= sms * per_sm && (!backward || p.grid <= layernorm_bwd_grid(M, sms, C));
+          if (!ok) return printf("C %d M %lld tensors %d backward %d: rows %d stages %d grid %d smem %d\\n", C, M, tensors, backward, p.rows,
+                                 p.stages, p.grid, p.smem), 1;
+        }
+  return 0;
+}
+"""
+
+
+def _run(tmp_path, program):
+    src, exe = tmp_path / "program.cu", tmp_path / "program"
+    src.write_text(program)
     built = subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(CSRC), "-Xcompiler", "-pthread",
                             "-o", str(exe), str(src)], capture_output=True, text=True)
     assert built.returncode == 0, built.stderr[-2000:]
-    assert subprocess.run([str(exe)], timeout=60).returncode == 0
+    done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0, done.stdout
+
+
+@pytest.mark.skipif(not Path(NVCC).exists(), reason="no nvcc")
+def test_no_thread_launches_before_the_attribute_is_set(tmp_path):
+    _run(tmp_path, PROGRAM)
+
+
+@pytest.mark.skipif(not Path(NVCC).exists(), reason="no nvcc")
+def test_layernorm_plans_fit_the_sm(tmp_path):
+    _run(tmp_path, PLAN)
