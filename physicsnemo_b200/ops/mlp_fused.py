@@ -125,17 +125,16 @@ class _Mlp3LnFn(torch.autograd.Function):
         m, dev = x3.shape[0], x3.device
         dy = dy.contiguous()
         lib = _lib_mlp()
-        # dW3, dW2, their biases, db1 and the blocks of dW1 of the plain sources in one zeroed buffer
-        sizes = [WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 3 + [WIDTH * WIDTH] * n
-        acc = torch.zeros(sum(sizes), dtype=torch.float32, device=dev).split(sizes)
-        dw3, dw2 = acc[0].view(WIDTH, WIDTH), acc[1].view(WIDTH, WIDTH)
-        db3, db2, db1 = acc[2:5]
+        # all gradients of parameters in one zeroed buffer, and nothing else: it lives as long as they do
+        sizes = [n * WIDTH * WIDTH, WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 5
+        dw1, dw2, dw3, db1, db2, db3, dgamma, dbeta = torch.zeros(sum(sizes), dtype=torch.float32, device=dev).split(sizes)
+        dw1, dw2, dw3 = dw1.view(WIDTH, -1), dw2.view(WIDTH, WIDTH), dw3.view(WIDTH, WIDTH)
+        block = [dw1[:, j * WIDTH:(j + 1) * WIDTH] for j in range(n)]            # of source j
         rows = torch.empty((2, m, WIDTH), dtype=torch.bfloat16, device=dev)
         dx3, g1 = rows[0], rows[1]
-        norm = torch.empty(2 * WIDTH + lib.pnm_layernorm_bwd_scratch_floats(m, WIDTH), dtype=torch.float32, device=dev)
-        dgamma, dbeta = norm[:WIDTH], norm[WIDTH:2 * WIDTH]
+        scratch = torch.empty(lib.pnm_layernorm_bwd_scratch_floats(m, WIDTH), dtype=torch.float32, device=dev)
         code = lib.pnm_layernorm_bwd(dy.data_ptr(), x3.data_ptr(), _vec(gamma).data_ptr(), mean.data_ptr(), rstd.data_ptr(), None,
-                                     dx3.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), norm[2 * WIDTH:].data_ptr(), m, WIDTH,
+                                     dx3.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), scratch.data_ptr(), m, WIDTH,
                                      _g._stream())
         _g._check(code, "pnm_layernorm_bwd")
         w3t, w2t = _w_t(w3), _w_t(w2)                        # held: the second look-up may empty the cache
@@ -146,14 +145,13 @@ class _Mlp3LnFn(torch.autograd.Function):
         need = ctx.needs_input_grad[5:]
         w1t = _w_t(w1)                                       # [128 n, 128]: rows j * 128 .. belong to source j
         dsrc = [None] * n
-        dw1 = [acc[5 + j].view(WIDTH, WIDTH) for j in range(n)]
         summed_bias = False
         for j in range(n):
             if segs[j] is None:
                 if need[j]:
                     own = {"aux": dy, "aux_mode": _g.AUX_ADD} if post == j else {}
                     dsrc[j] = _g.gemm_tn(g1, w1t[j * WIDTH:(j + 1) * WIDTH], **own)
-                _g.gemm_nt(g1, srcs[j], out=dw1[j], colsum_out=None if summed_bias else db1)
+                _g.gemm_nt(g1, srcs[j], out=block[j], colsum_out=None if summed_bias else db1)
                 summed_bias = True
         # An indexed source: sum g1 over the rows that read a table row FIRST (the products are linear), then one small product
         # per table instead of one per row of M.  The fp32 sums go into the products as a bf16 pair (hi + lo).
@@ -170,16 +168,16 @@ class _Mlp3LnFn(torch.autograd.Function):
             both = torch.zeros(pairs.shape[1] * (WIDTH + 1), dtype=torch.float32, device=dev)
             part = both[:pairs.shape[1] * WIDTH].view(-1, WIDTH)
             _g.gemm_nt(pairs, src, out=part, colsum_out=None if summed_bias else both[part.numel():])
-            blocks = part.view(len(js), 2, WIDTH, WIDTH).sum(1)
+            halves = part.view(len(js), 2, WIDTH, WIDTH)
             for k, j in enumerate(js):
-                dw1[j] = blocks[k]
+                torch.add(halves[k, 0], halves[k, 1], out=block[j])
             if not summed_bias:
                 db1 = both[part.numel():].view(len(js), 2, WIDTH)[0].sum(0)
                 summed_bias = True
             if any(need[j] for j in js):
                 wt = torch.cat([w1t[j * WIDTH:(j + 1) * WIDTH] for j in js for _ in range(2)], 1)
                 dsrc[js[0]] = _g.gemm_tn(pairs, wt)
-        grads = [torch.cat(dw1, 1) if n > 1 else dw1[0], dw2, dw3, db1, db2, db3, dgamma, dbeta]
+        grads = [dw1, dw2, dw3, db1, db2, db3, dgamma, dbeta]
         grads = [None if dt is None else (t if t.dtype == dt else t.to(dt)) for t, dt in zip(grads, ctx.dtypes)]
         return (None, None, None, None, None, *dsrc, *grads)
 

@@ -229,3 +229,17 @@ def test_relu_backward_drops_infinities_of_inactive_units():
     want = torch.zeros(m, W, device=dev)
     want[:, 7] = float("inf")
     assert torch.equal(g1.float(), want)
+
+
+@pytest.mark.gpu
+def test_mlp3_gradients_hold_no_other_memory():
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    e, v = torch.randn(5000, W, device="cuda").bfloat16(), torch.randn(700, W, device="cuda").bfloat16()
+    seg = ops.SegmentIndex(torch.randint(0, 700, (5000,), device="cuda"), 700)
+    p = [torch.randn(W, k, device="cuda") / W for k in (3 * W, W, W)] + [torch.randn(W, device="cuda") for _ in range(5)]
+    p = [t.requires_grad_() for t in p]
+    mf.mlp3_ln([e, v, v], [None, seg, seg], p[:3], p[3:6], 2, p[6], p[7], 1e-5, 0).float().square().sum().backward()
+    held = {t.grad.untyped_storage().data_ptr(): t.grad.untyped_storage().nbytes() for t in p}
+    assert sum(held.values()) == sum(t.grad.numel() * 4 for t in p)
