@@ -56,12 +56,18 @@ def _check(code: int, what: str):
         raise RuntimeError(f"{what} failed with code {code}")
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t``, or a copy of it where it does not start on a 16-byte boundary (a slice of a flat buffer, say): the kernels move vectors
+    of that size, and ``contiguous()`` leaves such a tensor where it is."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
-    """2-D view whose last dim is contiguous and whose row stride is a multiple of 8."""
+    """2-D view whose last dim is contiguous, whose row stride is a multiple of 8 and that starts on a 16-byte boundary."""
     assert t.dim() == 2
-    if t.stride(1) != 1 or t.stride(0) % 8 != 0 or t.data_ptr() % 16 != 0:
+    if t.stride(1) != 1 or t.stride(0) % 8 != 0:
         t = t.contiguous()
-    return t
+    return _aligned(t)
 
 
 def gemm_tn(

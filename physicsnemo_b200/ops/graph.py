@@ -64,9 +64,9 @@ def _segment_raw(x: torch.Tensor, seg: SegmentIndex, mean: bool = False, out: Op
 
 
 def _ok(x: torch.Tensor) -> torch.Tensor:
-    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+    if x.stride(1) != 1 or x.stride(0) % 8:
         x = x.contiguous()
-    return x
+    return _g._aligned(x)
 
 
 class _GatherFn(torch.autograd.Function):

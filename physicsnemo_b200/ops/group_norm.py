@@ -79,6 +79,7 @@ class _GroupNormFn(torch.autograd.Function):
         if lay is None:
             x = x.contiguous()
             lay = 0
+        x = _g._aligned(x)
         B, C = x.shape[:2]
         hw = x.numel() // (B * C)
         v = 8 if x.dtype == torch.bfloat16 else 4
@@ -113,6 +114,7 @@ class _GroupNormFn(torch.autograd.Function):
             dy = dy.contiguous(memory_format=torch.channels_last if x.dim() == 4 else torch.channels_last_3d)
         if dy.dtype != x.dtype:
             dy = dy.to(x.dtype)
+        dy = _g._aligned(dy)
         lib = _lib_gn()
         dev = x.device
         dx = torch.empty_like(x)

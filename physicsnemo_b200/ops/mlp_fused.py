@@ -123,7 +123,7 @@ class _Mlp3LnFn(torch.autograd.Function):
         srcs, (w1, w2, w3, gamma, h1, h2, x3, mean, rstd, *z) = saved[:n], saved[n:]
         z1, z2 = z or (h1, h2)
         m, dev = x3.shape[0], x3.device
-        dy = dy.contiguous()
+        dy = _g._aligned(dy.contiguous())
         lib = _lib_mlp()
         # all gradients of parameters in one zeroed buffer, and nothing else: it lives as long as they do
         sizes = [n * WIDTH * WIDTH, WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 5

@@ -46,9 +46,9 @@ class _LayerNormFn(torch.autograd.Function):
         lib = _lib.load(required=True)
         x2d, g32, mean, rstd = ctx.saved_tensors
         if dalias is not None:
-            dalias = dalias.contiguous()
+            dalias = _g._aligned(dalias.contiguous())
         M, C = x2d.shape
-        dy = dy.contiguous()
+        dy = _g._aligned(dy.contiguous())
         dx = torch.empty_like(x2d)
         dgamma = torch.empty((C,), dtype=torch.float32, device=x2d.device)
         dbeta = torch.empty((C,), dtype=torch.float32, device=x2d.device)
@@ -79,13 +79,13 @@ def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     x2 = x.reshape(-1, C)
     if x2.dtype != torch.bfloat16:
         x2 = x2.to(torch.bfloat16)
-    x2 = x2.contiguous()
+    x2 = _g._aligned(x2.contiguous())
     p2 = None
     if post is not None:
         p2 = post.reshape(-1, C)
         if p2.dtype != torch.bfloat16:
             p2 = p2.to(torch.bfloat16)
-        p2 = p2.contiguous()
+        p2 = _g._aligned(p2.contiguous())
     if return_residual:
         y, alias = _LayerNormFn.apply(x2, weight, bias, eps, p2, True)
         return y.reshape(x.shape), alias.reshape(x.shape)

@@ -103,6 +103,7 @@ class _AddScale(torch.autograd.Function):
     def backward(ctx, g):
         g = g.contiguous(memory_format=torch.channels_last) if g.dim() == 4 and not g.is_contiguous() else g.contiguous() if not (
             g.is_contiguous() or (g.dim() == 4 and g.is_contiguous(memory_format=torch.channels_last))) else g
+        g = _g._aligned(g)
         d = torch.empty_like(g)
         rc = _add_scale_fn()(g.data_ptr(), None, d.data_ptr(), g.numel(), ctx.scale, _lib.stream())
         _g._check(rc, "pnm_add_scale_bf16")
@@ -147,7 +148,7 @@ class _AddChannel(torch.autograd.Function):
         if ctx.needs_input_grad[1] and torch.is_grad_enabled():          # a graph of the gradient is wanted (create_graph)
             dv = g.sum((2, 3), keepdim=True)
         elif ctx.needs_input_grad[1]:
-            g = g.contiguous(memory_format=torch.channels_last)
+            g = _g._aligned(g.contiguous(memory_format=torch.channels_last))
             b, c, h, w = g.shape
             # two CTAs per SM, at least eight passes of a CTA's pixels each
             slices = max(1, min(2 * 148 // b, h * w // (8 * max(1, 2048 // c))))

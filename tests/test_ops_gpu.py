@@ -911,3 +911,50 @@ def test_channel_vector_addition_keeps_what_the_tensor_expression_has():
     assert torch.equal(torch.func.vmap(lambda a: resample.add_channel(x, a))(torch.stack([v, t])), torch.stack([x + v, x + t]))
     traced = torch.jit.trace(resample.add_channel, (x, t), check_trace=False)
     assert torch.equal(traced(x, v), x + v)
+
+
+def _odd(t):
+    """A copy of ``t`` (same strides) that starts one element behind a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:]
+    out = flat.as_strided(t.size(), t.stride(), flat.storage_offset())
+    out.copy_(t)
+    assert out.data_ptr() % 16 and out.stride() == t.stride()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", ["layer_norm", "layer_norm_post", "layer_norm_residual", "group_norm", "add_channel", "gather", "segment_sum",
+                                "mlp3", "linear"])
+def test_tensors_that_start_off_a_vector_boundary(op):
+    """Inputs and incoming gradients that are slices of a flat buffer give what aligned ones give."""
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import group_norm, mlp_fused, resample
+
+    rn = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    p = [torch.randn(128, 128, device="cuda") / 12 for _ in range(3)] + [torch.randn(128, device="cuda") for _ in range(5)]
+    rows, image, seg = rn(700, 128), rn(2, 128, 16, 16).contiguous(memory_format=torch.channels_last), None
+    if op in ("gather", "segment_sum"):
+        seg = ops.SegmentIndex(torch.randint(0, 700 if op == "gather" else 90, (700,), device="cuda"), 700 if op == "gather" else 90)
+    fn, args = {
+        "layer_norm": (lambda x: ops.layer_norm(x, p[6], p[7]), [rows]),
+        "layer_norm_post": (lambda x, r: ops.layer_norm(x, p[6], p[7], post=r), [rows, rn(700, 128)]),
+        "layer_norm_residual": (lambda x: ops.layer_norm(x, p[6], p[7], return_residual=True), [rows]),
+        "group_norm": (lambda x: group_norm.group_norm(x, 32, p[6], p[7], 1e-5, silu=True), [image]),
+        "add_channel": (resample.add_channel, [image, rn(2, 128, 1, 1)]),
+        "gather": (lambda x: ops.gather_rows(x, seg), [rows]),
+        "segment_sum": (lambda x: ops.segment_reduce(x, seg), [rows]),
+        "mlp3": (lambda x: mlp_fused.mlp3_ln([x], [None], p[:3], p[3:6], 2, p[6], p[7], 1e-5, 0), [rows]),
+        "linear": (lambda x: ops.linear(x, p[0], p[3]), [rows]),
+    }[op]
+    results = []
+    for place in (lambda t: t, _odd):
+        leaves = [(t if op == "mlp3" else place(t)).detach().requires_grad_() for t in args]       # that kernel's callers check its sources
+        out = fn(*leaves)
+        outs = list(out) if isinstance(out, tuple) else [out]
+        gen = torch.Generator("cuda").manual_seed(1)
+        torch.autograd.backward(outs, [place(torch.empty_like(t).copy_(torch.randn(t.shape, generator=gen, device="cuda"))) for t in outs])
+        results.append([*outs, *[t.grad for t in leaves]])
+    for a, b in zip(*results):
+        # GroupNorm's backward adds channel sums by fp32 atomics in any order (1e-6 of the sums): one bf16 value in some hundred may
+        # round the other way, 2^-9 of it each
+        assert torch.equal(a, b) or (op == "group_norm" and float((a.double() - b.double()).norm()) < 5e-4 * float(b.double().norm()))
