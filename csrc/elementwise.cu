@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "pnm_api.h"
+#include "pnm_internal.h"
 
 namespace pnm {
 
@@ -344,7 +345,9 @@ __global__ void __launch_bounds__(256) channel_fold_kernel(const float* __restri
 extern "C" int pnm_add_channel_bf16(const void* x, const void* v, void* y, int B, long long hw, int C, void* stream) {
   if (B <= 0 || hw <= 0 || C <= 0 || (C & 7)) return -2;
   const long long nvec = (long long)B * hw * (C / 8), blocks = (nvec + 255) / 256;
-  pnm::add_channel_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(
+  const long long most = (long long)pnm::num_sms() * 16;
+  if (most <= 0) return -1;
+  pnm::add_channel_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, (cudaStream_t)stream>>>(
       (const uint4*)x, (const uint4*)v, (uint4*)y, hw * (C / 8), C / 8, nvec);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

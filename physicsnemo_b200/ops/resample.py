@@ -151,7 +151,7 @@ class _AddChannel(torch.autograd.Function):
             g = _g._aligned(g.contiguous(memory_format=torch.channels_last))
             b, c, h, w = g.shape
             # two CTAs per SM, at least eight passes of a CTA's pixels each
-            slices = max(1, min(2 * 148 // b, h * w // (8 * max(1, 2048 // c))))
+            slices = max(1, min(2 * _channel_lib().pnm_num_sms() // b, h * w // (8 * max(1, 2048 // c))))
             dv = torch.empty(b, c, 1, 1, dtype=torch.bfloat16, device=g.device)
             part = torch.empty(b * slices * c, dtype=torch.float32, device=g.device)
             rc = _channel_lib().pnm_channel_sum_bf16(g.data_ptr(), dv.data_ptr(), part.data_ptr(), b, h * w, c, slices, _lib.stream())
