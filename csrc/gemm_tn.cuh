@@ -116,8 +116,10 @@ struct GemmCfg {
   static constexpr int EPI = BN / 16;         // epilogue warps: 4 lane quarters x (BN / 64) column blocks
   static constexpr int THREADS = 64 + 32 * EPI;
   // staging buffers of a warp: the auxiliary tile of the next block is prefetched while this one is worked on (128 columns: two
-  // ahead); two outputs alternate.  256 columns without an auxiliary tile leave the shared memory to the operand stages.
-  static constexpr int NBUF = BN == 256 ? (MODE == MODE_PLAIN ? 1 : 2) : (MODE == MODE_AUX ? 3 : 2);
+  // ahead); two outputs (128 columns only) alternate.  256 columns without an auxiliary tile leave the shared memory to the operand
+  // stages.
+  static_assert(BN == 128 || MODE != MODE_Z, "two outputs: 128-column tiles");
+  static constexpr int NBUF = BN == 256 ? (MODE == MODE_AUX ? 2 : 1) : (MODE == MODE_AUX ? 3 : 2);
   static constexpr int STAGE_BYTES = kBM * kBK * 2 + BN * kBK * 2;
   static constexpr int STAGING = EPI * NBUF * kChunkBytes;
   static constexpr int BUDGET = 232448 - 1024 /*align*/ - 512 /*barriers*/;
@@ -404,11 +406,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             float x[16], a[16];
             load16(k, x);
             stage_read16(arow, lane, k, a);
-            switch (g.aux_mode) {
-              case AUX_ADD:
-#pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] += a[j];
-                break;
+            switch (g.aux_mode) {                // the modes that come here: those with arithmetic
               case AUX_DGELU:
 #pragma unroll
                 for (int j = 0; j < 16; ++j) x[j] *= gelu_grad_f(a[j]);
@@ -416,10 +414,6 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               case AUX_DSILU:
 #pragma unroll
                 for (int j = 0; j < 16; ++j) x[j] *= silu_grad_f(a[j]);
-                break;
-              case AUX_DRELU:
-#pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] = a[j] > 0.f ? x[j] : 0.f;
                 break;
               case AUX_DSOFTMAX:
 #pragma unroll

@@ -27,10 +27,10 @@
 
 namespace pnm {
 
-// Two staging buffers per epilogue warp in every mode: a third buffer for the auxiliary operand costs a stage and
-// measured slower on K = 3072 (132 vs 124 us) and no faster on K = 768.
 constexpr int kPairThreads = 320;
 
+// Two staging buffers per epilogue warp in every mode: a third buffer for the auxiliary operand costs a stage and
+// measured slower on K = 3072 (132 vs 124 us) and no faster on K = 768.
 template <int BN, int MODE>
 struct PairCfg {
   static constexpr int NBUF = 2;
