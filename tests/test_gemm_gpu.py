@@ -272,3 +272,43 @@ def test_weight_copy_of_another_stream_is_not_used_before_it_is_made():
         assert G._bf16_weight(w) is first
     torch.cuda.synchronize()
     assert torch.equal(first, ref)
+
+
+@pytest.mark.parametrize("N", [256, 384, 448, 1000, 136])
+@pytest.mark.parametrize("aux_mode", [G.AUX_DGELU, G.AUX_DSILU, G.AUX_DSOFTMAX])
+@pytest.mark.parametrize("form", ["plain", "bias, scale before", "bias, scale after", "two sources, activation"])
+def test_gemm_tn_wide_aux_tiles(aux_mode, N, form):
+    """256-column tiles with an auxiliary operand need a tile per SM (157 row tiles here): ragged rows, a last tile of 128, 192, 232 or
+    136 columns, and all that the epilogue does before and after the operand."""
+    if aux_mode == G.AUX_DSOFTMAX:
+        N = N // 64 * 64
+    M, K1, K2 = 20001, 128, 64
+    a, a2, b = _rand(M, K1), _rand(M, K2), _rand(N, K1 + K2, scale=0.2)
+    aux = torch.softmax(torch.randn(M, N // 64, 64, device="cuda"), -1).reshape(M, N).bfloat16() if aux_mode == G.AUX_DSOFTMAX else _rand(M, N)
+    kw = {"aux": aux, "aux_mode": aux_mode}
+    if form == "two sources, activation":
+        kw |= {"a2": a2, "act": G.ACT_SILU}
+    else:
+        a = torch.cat([a, a2], 1)
+        kw["scale_post"] = form != "bias, scale before"
+        if form != "plain":
+            kw |= {"bias": torch.randn(N, device="cuda"), "scale": torch.rand(N, device="cuda") + 0.5}
+        else:
+            kw["scale"] = torch.ones(N, device="cuda")           # keeps the deep shapes off the CTA-pair kernel
+    grp = torch.zeros(N // 64, device="cuda") if aux_mode == G.AUX_DSOFTMAX and form == "bias, scale after" else None
+    out = ops.gemm_tn(a, b, group_out=grp, **kw)
+    ref, z = ops.gemm_tn_reference(a, b, **kw)
+    _close(out, ref, tol=3e-2)
+    if grp is not None:
+        y, p = z.reshape(M, -1, 64), aux.float().reshape(M, -1, 64)
+        ds = p * (y - (y * p).sum(-1, keepdim=True))
+        _close(grp, (ds * torch.log(p.clamp_min(1e-30)) * (p > 0)).double().sum((0, 2)), tol=5e-2)
+    assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("form", [{}, {"post": True}, {"residual": True}, {"post": True, "residual": True}])
+@pytest.mark.parametrize("C", [8, 128, 200, 256, 512, 768, 1024])
+def test_layernorm_rings_that_wrap(C, form):
+    """Rows enough that every CTA uses every stage of its ring again, with a last tile that is not full."""
+    _layernorm_against_64_bits(120001 if C <= 256 else 60001, C, **form)
+    assert ops.device_error() == 0

@@ -243,3 +243,71 @@ def test_mlp3_gradients_hold_no_other_memory():
     mf.mlp3_ln([e, v, v], [None, seg, seg], p[:3], p[3:6], 2, p[6], p[7], 1e-5, 0).float().square().sum().backward()
     held = {t.grad.untyped_storage().data_ptr(): t.grad.untyped_storage().nbytes() for t in p}
     assert sum(held.values()) == sum(t.grad.numel() * 4 for t in p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["two tables", "indexed only", "one indexed, no biases", "table twice and once"])
+def test_mlp3_ln_sources_and_missing_vectors(form):
+    """Sources by index and row by row in every mixture, without biases and shift, against 64 bits."""
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    rows, gen = 9001, torch.Generator().manual_seed(3)
+    rn = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    tables = [rn(rows, W).bfloat16(), rn(700, W).bfloat16(), rn(311, W).bfloat16()]
+    index = [None, torch.randint(0, 700, (rows,), generator=gen), torch.randint(0, 311, (rows,), generator=gen)]
+    use, vectors = {"two tables": ([(0, 0), (1, 1), (2, 2)], True), "indexed only": ([(1, 1), (2, 2)], True),
+                    "one indexed, no biases": ([(1, 1)], False), "table twice and once": ([(2, 2), (0, 0), (2, 2)], True)}[form]
+    n = len(use)
+    params = [rn(W, W * n) / (W * n) ** 0.5, rn(W, W) / W ** 0.5, rn(W, W) / W ** 0.5, 1 + 0.1 * rn(W)]
+    params += [0.1 * rn(W) for _ in range(4)] if vectors else []
+    up = rn(rows, W).bfloat16()
+    ref_t, ref_p = [t.double().requires_grad_() for t in tables], [t.double().requires_grad_() for t in params]
+    w1, w2, w3, ga, b1, b2, b3, be = [*ref_p, None, None, None, None][:8]
+    x = torch.cat([ref_t[t] if index[i] is None else ref_t[t][index[i]] for t, i in use], 1)
+    ref = F.layer_norm(F.linear(F.gelu(F.linear(F.gelu(F.linear(x, w1, b1)), w2, b2)), w3, b3), (W,), ga, be)
+    ref.backward(up.double())
+    got_t, got_p = [t.cuda().requires_grad_() for t in tables], [t.cuda().requires_grad_() for t in params]
+    w1, w2, w3, ga, b1, b2, b3, be = [*got_p, None, None, None, None][:8]
+    seg = [None if i is None else ops.SegmentIndex(i.cuda(), tables[k].shape[0]) for k, i in enumerate(index)]
+    srcs, segs = [got_t[t] for t, _ in use], [seg[i] for _, i in use]
+    assert mf.supported(srcs, segs, [w1, w2, w3], [b1, b2, b3], [1, 1, 0], ga, be, None)
+    out = mf.mlp3_ln(srcs, segs, [w1, w2, w3], [b1, b2, b3], 1, ga, be, 1e-5, None)
+    out.backward(up.cuda())
+    # as in the test of the three usual forms
+    assert _rel(out.detach().cpu(), ref.detach()) < 8e-3
+    for a, b in zip((*got_t, *got_p), (*ref_t, *ref_p)):
+        assert (a.grad is None) == (b.grad is None) and (b.grad is None or _rel(a.grad.cpu(), b.grad) < 0.02)
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("aggregation", ["sum", "mean"])
+@pytest.mark.parametrize("checkpointed", [False, True])
+def test_message_passing_step_against_64_bits(aggregation, checkpointed):
+    from torch.utils.checkpoint import checkpoint
+
+    from physicsnemo_b200.nn.module.gnn_layers.graph_types import Graph
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_edge_block import MeshEdgeBlock
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_node_block import MeshNodeBlock
+
+    edge, node = MeshEdgeBlock(W, W, W, W, 2).cuda(), MeshNodeBlock(aggregation, W, W, W, W, 2).cuda()
+    index = torch.randint(0, 301, (2, 1500)).cuda()
+    e, v = torch.randn(1500, W, device="cuda").bfloat16(), torch.randn(301, W, device="cuda").bfloat16()
+    ups = [torch.randn(1500, W, device="cuda").bfloat16(), torch.randn(301, W, device="cuda").bfloat16()]
+    results = []
+    for exact in (False, True):
+        if exact:
+            edge, node = edge.double(), node.double()
+        for p in (*edge.parameters(), *node.parameters()):
+            p.grad = None
+        graph = Graph(index, num_nodes=301)
+        leaves = [(t.double() if exact else t.clone()).requires_grad_() for t in (e, v)]
+        step = lambda a, b: node(*edge(a, b, graph), graph)  # noqa: E731
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=not exact):
+            out = checkpoint(step, *leaves, use_reentrant=False) if checkpointed and not exact else step(*leaves)
+        torch.autograd.backward(out, [t.to(o.dtype) for t, o in zip(ups, out)])
+        results.append([t.detach().clone() for t in out] + [t.grad.clone() for t in leaves] + [p.grad.clone() for p in (*edge.parameters(), *node.parameters())])
+    for k, (a, b) in enumerate(zip(*results)):
+        # outputs: four bf16 roundings; gradients: 0.8 % at this size with 128 entries in a bias
+        assert _rel(a, b.double()) < (8e-3 if k < 2 else 0.02)
