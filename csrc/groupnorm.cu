@@ -55,7 +55,8 @@ template <> struct Vec<float> {
 
 // Sigmoid in fp32.  For bf16 tensors by the two-ulp reciprocal (its error is 2^-16 of a bf16 ulp): the IEEE division costs ten
 // instructions an element and, worse, a slow path whose branch keeps the loads of the next pixels from being issued early.
-// Denominators beyond 2^126 give 0, which is the limit.
+// Denominators beyond 2^126 give 0, which is the limit.  Errors against 64 bits with either form, five shapes, six draws: results and
+// input gradients the same to eight digits (1.678e-3 and 1.659e-3 at 1 x 256 x 256 x 256), parameter gradients 1e-7 to 5e-7 both.
 template <typename T>
 __device__ __forceinline__ float gn_sigmoid(float z) {
   const float d = 1.f + __expf(-z);

@@ -263,8 +263,8 @@ layernorm_fwd_stream_kernel(const __nv_bfloat16* __restrict__ x, const float* __
 // dx = rstd * (g*dy - mean_c(g*dy) - xhat * mean_c(g*dy*xhat)) (+ dres); partial dgamma / dbeta rows go to
 // scratch[blockIdx.x][2][C], so that the column sums stay in registers until a CTA is done.
 // Measured against one row per warp from registers: 1 M x 256 forward 0.213 -> 0.191 ms (0.82 of 6544 GB/s), backward with a residual
-// gradient 0.420 -> 0.339 ms (0.92); 1.4 M x 128 forward 0.177 -> 0.159 ms, backward 0.507 -> 0.259 ms (two rows per warp);
-// 32 400 x 768 27.2 -> 25.7 us, 56.1 -> 54.2 us.
+// gradient 0.420 -> 0.336 ms (0.93); 1.4 M x 128 forward 0.177 -> 0.159 ms, backward 0.507 -> 0.256 ms (two rows per warp);
+// 32 400 x 768 27.2 -> 25.6 us, 56.1 -> 50.3 us.
 template <int VEC, int LPR>
 __global__ void __launch_bounds__(kLnStreamThreads, VEC == 1 ? 3 : (VEC == 2 ? 2 : 1))
 layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma,
