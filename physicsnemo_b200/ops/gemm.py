@@ -262,7 +262,13 @@ def fused_path_enabled(x: torch.Tensor) -> bool:
 
 
 _wcache: dict = {}
-_captured: dict = {}         # id -> weak reference of every parameter that a captured graph reads
+_captured: dict = {}         # id -> weak reference of every parameter that a captured graph reads or writes
+
+
+def keep_no_copies(params) -> None:
+    """From now on no bf16 copies of these parameters are kept: a captured graph changes them in ways that no version shows."""
+    for p in params:
+        _captured[id(p)] = _weak(p, _captured, id(p))
 
 
 def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
@@ -280,7 +286,7 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     owner = w if base is None else base
     stream = _stream() if w.is_cuda else 0
     if stream and torch.cuda.is_current_stream_capturing():          # the default stream (0) cannot be captured
-        _captured[id(owner)] = _weak(owner, _captured, id(owner))
+        keep_no_copies([owner])
         return _to_bf16(w, transpose)
     if _captured:
         ref = _captured.get(id(owner))

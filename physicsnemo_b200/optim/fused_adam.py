@@ -239,6 +239,8 @@ class FusedAdam(Optimizer):
                 # the kernel writes through raw pointers: whatever is derived from a parameter (its bf16 copies, what autograd
                 # saved) sees a change by the version counter alone
                 torch.autograd.graph.increment_version(fused)
+                if torch.cuda.is_current_stream_capturing():
+                    _g.keep_no_copies(fused)              # replays of the graph write without this line
                 self.kernel_launches += 1
                 _g.launch_count += 1
         return loss

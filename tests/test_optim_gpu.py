@@ -151,3 +151,29 @@ def test_captured_step_trains_the_matrices_it_reads():
             now = ops.linear(x.detach(), w)
         ref = x.detach().double() @ w.detach().double().t()
         assert (now.double() - ref).norm() < 1e-2 * ref.norm(), k
+
+
+def test_captured_optimizer_step_reaches_eager_forwards():
+    """The step alone in a graph, forward and backward launched from the host."""
+    from physicsnemo_b200 import ops
+
+    w = torch.nn.Parameter(torch.randn(64, 128, device="cuda") / 128 ** 0.5)
+    w.grad = torch.randn_like(w)
+    opt = FusedAdam([w], lr=5e-2, capturable=True)
+    x = torch.randn(256, 128, device="cuda").bfloat16()
+
+    def agrees():
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            y = ops.linear(x, w)
+        ref = x.double() @ w.detach().double().t()
+        return float((y.double() - ref).norm()) < 1e-2 * float(ref.norm())
+
+    assert agrees()
+    opt.step()
+    assert agrees()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        opt.step()
+    for _ in range(3):
+        graph.replay()
+        assert agrees()
