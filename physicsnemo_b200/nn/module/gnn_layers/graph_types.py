@@ -56,7 +56,8 @@ def edge_index_of(graph) -> torch.Tensor:
 
 
 def segments(graph, which: str, num_nodes: int) -> SegmentIndex:
-    """Cached ``SegmentIndex`` of the edges by ``"src"`` or ``"dst"`` node."""
+    """``SegmentIndex`` of the edges by ``"src"`` or ``"dst"`` node, cached on the graph while its edges are what they were: an entry
+    goes by the version of the index (edges may be rewritten in place) and holds it (another index may get its address)."""
     cache = getattr(graph, "_pnm_cache", None)
     if cache is None:
         cache = {}
@@ -65,7 +66,10 @@ def segments(graph, which: str, num_nodes: int) -> SegmentIndex:
         except Exception:  # objects that refuse new attributes: no caching
             pass
     ei = edge_index_of(graph)
-    key = (which, num_nodes, ei.data_ptr(), ei.shape[1], str(ei.device))
-    if key not in cache:
-        cache[key] = SegmentIndex(ei[0 if which == "src" else 1], num_nodes)
-    return cache[key]
+    key = (which, num_nodes, ei.data_ptr(), ei.shape[1], ei.device, -1 if ei.is_inference() else ei._version)
+    hit = cache.get(key)
+    if hit is None:
+        if len(cache) >= 16:
+            cache.clear()
+        hit = cache[key] = (SegmentIndex(ei[0 if which == "src" else 1], num_nodes), ei)
+    return hit[0]

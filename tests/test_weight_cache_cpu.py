@@ -46,3 +46,18 @@ def test_copies_go_with_their_parameter():
     del p
     gc.collect()
     assert set(G._wcache) <= before
+
+
+def test_edge_orders_follow_the_edges():
+    """The sorted orders that a graph keeps are those of its edges now: after a change in place and for an index at an old address."""
+    from physicsnemo_b200.nn.module.gnn_layers.graph_types import Graph, segments
+
+    graph = Graph(torch.tensor([[0, 1, 2], [2, 2, 0]], dtype=torch.int32), num_nodes=3)
+    first = segments(graph, "dst", 3)
+    assert segments(graph, "dst", 3) is first and first.counts.tolist() == [1, 0, 2]
+    graph.edge_index[1] = torch.tensor([1, 1, 1])
+    assert segments(graph, "dst", 3).counts.tolist() == [0, 3, 0]
+    for k in range(40):                              # replaced again and again: nothing may be recognised by its address
+        graph.edge_index = torch.full((2, 3), k % 3, dtype=torch.int32)
+        assert segments(graph, "dst", 3).counts.tolist() == [3 * (k % 3 == n) for n in range(3)]
+    assert len(graph._pnm_cache) <= 16
