@@ -122,10 +122,14 @@ def load(required: bool = False):
     return _lib
 
 
+# absent from CPU builds of torch, where nothing is launched
+_raw_stream, _current_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream() -> int:
     """Handle of the current CUDA stream: ``torch.cuda.current_stream().cuda_stream`` without the stream object that it builds
     (a few microseconds of every launch)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return _raw_stream(_current_device())
 
 
 def available() -> bool:

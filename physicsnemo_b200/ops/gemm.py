@@ -67,7 +67,7 @@ def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
     assert t.dim() == 2
     if t.stride(1) != 1 or t.stride(0) % 8 != 0:
         t = t.contiguous()
-    return _aligned(t)
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def gemm_tn(
@@ -284,7 +284,7 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
         return w.detach()
     base = w._base
     owner = w if base is None else base
-    stream = _stream() if w.is_cuda else 0
+    stream = _lib.stream() if w.is_cuda else 0
     if stream and torch.cuda.is_current_stream_capturing():          # the default stream (0) cannot be captured
         keep_no_copies([owner])
         return _to_bf16(w, transpose)
@@ -297,7 +297,7 @@ def _bf16_weight(w: torch.Tensor, transpose: bool = False) -> torch.Tensor:
     key = (id(owner), transpose, stream) if stream else (id(owner), transpose)
     if base is not None:
         key += (w.storage_offset(), tuple(w.shape), w.stride())
-    ver = (w._version, w.data_ptr(), tuple(w.shape), w.stride())
+    ver = (w._version, w.data_ptr(), w.shape, w.stride())
     hit = _wcache.get(key)
     if hit is not None and hit[2]() is owner and hit[0] == ver:
         return hit[1]
