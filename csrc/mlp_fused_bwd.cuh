@@ -5,14 +5,15 @@
 //   g1 = (g2 W2) * act'(z1)       dW2 += g2^T act(z1),  db2 += g2
 //
 // Layer by layer these are two data-gradient and two weight-gradient products that move ten 256-byte rows per row of M; here
-// a row tile is read once (dx3, z2, act(z2), z1, act(z1)) and only g1 is written: six rows
-// (1.7 M rows: 0.47 ms, the rows are worth 0.39 ms; with the activations recomputed from z in the same threads 0.62 ms).  (The LayerNorm backward before it stays a kernel
-// of its own: its column sums are free when a warp works along a row, but cost eight instructions per element when, as here,
-// a thread owns a row; with it inside, this kernel was bound by instruction issue at 1.41 ms for 1.5 M rows.)
-// dx3 and act(z2) arrive by TMA; g2 overwrites dx3 and act(z1) takes the place of act(z2).  A gradient tile lies in shared memory once, in the 128-byte-swizzled layout that
-// tcgen05 reads both ways: as the K-major A operand of the data gradient and, with the row index as the reduction, as the
-// MN-major A operand of the weight gradient.  (The activations are the forward's own operands: recomputed from the rounded z
-// they would be rounded twice.)  Both weight gradients accumulate in TMEM over all tiles of a persistent CTA and are added to memory once at its end.
+// a row tile is read once (dx3, z2, act(z2), z1, act(z1)) and only g1 is written: six rows (1.7 M rows: 0.47 ms, the rows are
+// worth 0.39 ms; with the activations recomputed from z in the same threads 0.62 ms).  (The LayerNorm backward before it stays a
+// kernel of its own: its column sums are free when a warp works along a row, but cost eight instructions per element when, as
+// here, a thread owns a row; with it inside, this kernel was bound by instruction issue at 1.41 ms for 1.5 M rows.)
+// dx3 and act(z2) arrive by TMA; g2 overwrites dx3 and act(z1) takes the place of act(z2).  A gradient tile lies in shared memory
+// once, in the 128-byte-swizzled layout that tcgen05 reads both ways: as the K-major A operand of the data gradient and, with the
+// row index as the reduction, as the MN-major A operand of the weight gradient.  (The activations are the forward's own operands:
+// recomputed from the rounded z they would be rounded twice.)  Both weight gradients accumulate in TMEM over all tiles of a
+// persistent CTA and are added to memory once at its end.
 // Two tiles are in flight, one per group of eight warps (two threads per row); ONE thread issues all products, since products
 // that accumulate into the same TMEM columns are only ordered within a thread.  A further warp per group sums the columns
 // of the gradient tile while the tensor cores read it.
