@@ -32,7 +32,7 @@ static int launch_mlp3_bwd(const CUtensorMap& td, const CUtensorMap& th2, const 
                            const CUtensorMap& t2, const MlpBwdArgs& g, int grid, cudaStream_t st) {
   static DeviceMask smem_set{0};
   if (!allow_smem(mlp3_bwd_kernel<ACT>, kMlpBwdSmem, smem_set)) return -16;
-  mlp3_bwd_kernel<ACT><<<grid, kMlpThreads, kMlpBwdSmem, st>>>(td, th2, th1, t3, t2, g);
+  mlp3_bwd_kernel<ACT><<<grid, kMlpBwdThreads, kMlpBwdSmem, st>>>(td, th2, th1, t3, t2, g);
   return cudaGetLastError() == cudaSuccess ? 0 : -17;
 }
 
@@ -139,7 +139,10 @@ extern "C" int pnm_mlp3_ln_fwd(int nsrc, const void* const* src, const long long
   for (int j = 0; j < nsrc; ++j) {
     if (rows[j] <= 0 || (!idx[j] && rows[j] < M)) return -2;
     g.idx[j] = idx[j];
-    if (make_tmap_2d_b16(&tm[j], src[j], idx[j] ? rows[j] : M, kMlpW, ld[j], idx[j] ? 1 : kMlpRows, 64)) return -10 - j;
+    g.src[j] = reinterpret_cast<const __nv_bfloat16*>(src[j]); g.ld_src[j] = ld[j];
+    if ((reinterpret_cast<uintptr_t>(src[j]) & 15) || (ld[j] & 7)) return -10 - j;
+    if (idx[j]) tm[j] = CUtensorMap{};           // rows are copied one by one
+    else if (make_tmap_2d_b16(&tm[j], src[j], M, kMlpW, ld[j], kMlpRows, 64)) return -10 - j;
   }
   for (int j = nsrc; j < 3; ++j) { tm[j] = tm[0]; g.idx[j] = nullptr; }
   if (make_tmap_2d_b16(&tw[0], W1, kMlpW, nsrc * kMlpW, nsrc * kMlpW, kMlpW, 64)) return -13;

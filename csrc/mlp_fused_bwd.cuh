@@ -30,6 +30,7 @@ struct MlpBwdArgs {
   int* err;
 };
 
+constexpr int kMlpBwdThreads = 640;              // issuer, 2 warps of column sums, producer, 2 x 8 warps of the tiles
 constexpr int kMlpBwdSmem = 12 * kMlpChunk + 256;
 
 // v act'(z); ReLU selects, so that an infinite v beside a negative z is 0 and not NaN
@@ -46,7 +47,7 @@ __device__ __forceinline__ void tile_put16(uint8_t* tile, int r, int c, const ui
 }
 
 template <int ACT>
-__global__ void __launch_bounds__(kMlpThreads, 1)
+__global__ void __launch_bounds__(kMlpBwdThreads, 1)
 mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmH2, const __grid_constant__ CUtensorMap tmH1,
                 const __grid_constant__ CUtensorMap tmW3t, const __grid_constant__ CUtensorMap tmW2t, const MlpBwdArgs g) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
