@@ -28,26 +28,30 @@ from ..layer_norm import get_layer_norm_class
 from .utils import concat_efeat, concat_efeat_hetero, edge_sources, sum_efeat
 
 
+def _param(mod: nn.Module, name: str):
+    """``getattr(mod, name)`` with the plain parameter looked up first (a module's own attribute look-up costs a microsecond)."""
+    p = mod._parameters.get(name)
+    return getattr(mod, name) if p is None else p
+
+
 def _layers(model: nn.Sequential):
     """``(weights, biases, activation codes, LayerNorm or None)`` of Linear/act…/[LayerNorm]; ``None`` for another structure."""
-    mods = list(model)
-    norm = mods[-1] if isinstance(mods[-1], nn.LayerNorm) else None
-    body = mods[:-1] if norm is not None else mods
+    body = list(model._modules.values())
+    norm = body.pop() if isinstance(body[-1], nn.LayerNorm) else None
     weights, biases, acts = [], [], []
-    i = 0
-    while i < len(body):
-        if not isinstance(body[i], nn.Linear):
+    open_layer = False                                       # a Linear that no activation has followed yet
+    for m in body:
+        if isinstance(m, nn.Linear):
+            weights.append(_param(m, "weight"))
+            biases.append(_param(m, "bias"))
+            acts.append(0)
+            open_layer = True
+            continue
+        code = activation_code(m) if open_layer else None
+        if not code:
             return None
-        code = 0
-        if i + 1 < len(body) and not isinstance(body[i + 1], nn.Linear):
-            code = activation_code(body[i + 1])
-            if code is None:
-                return None
-            i += 1
-        weights.append(body[i - (1 if code else 0)].weight)
-        biases.append(body[i - (1 if code else 0)].bias)
-        acts.append(code)
-        i += 1
+        acts[-1] = code
+        open_layer = False
     return weights, biases, acts, norm
 
 

@@ -3,7 +3,9 @@
 The library is plain C ABI (see ``csrc/pnm_api.h``) bound through ``ctypes``: every
 call passes raw device pointers and the current CUDA stream.  ``build()`` compiles the
 single translation unit ``csrc/pnm_lib.cu`` with
-``nvcc -gencode arch=compute_100a,code=sm_100a`` (cross-compiles without a GPU).
+``nvcc -gencode arch=compute_100a,code=sm_100a`` (cross-compiles without a GPU), and the CPython
+extension ``_pnm_host.so`` from ``csrc/host_calls.cpp``: the host side of the hottest calls
+(operand checks, allocation, launch), without ctypes.
 On a machine with a CUDA device a missing library is an error, never a silent
 fallback.
 """
@@ -22,8 +24,10 @@ _REPO = _PKG_DIR.parent
 _SRC_DIR = _REPO / "csrc"
 _LIB_DIR = _PKG_DIR / "lib"
 _LIB_PATH = _LIB_DIR / "libpnm_b200.so"
+_HOST_PATH = _LIB_DIR / "_pnm_host.so"
 _lock = threading.Lock()
 _lib = None
+_host = None
 _load_error: str | None = None
 
 NVCC_FLAGS = [
@@ -44,7 +48,33 @@ def needs_build() -> bool:
     if not _LIB_PATH.exists():
         return True
     built = _LIB_PATH.stat().st_mtime
-    return any(s.stat().st_mtime > built for s in _sources())
+    return any(s.stat().st_mtime > built for s in _sources()) or _host_needs_build()
+
+
+def _host_needs_build() -> bool:
+    if torch.version.cuda is None:                           # nothing is launched without CUDA
+        return False
+    return not _HOST_PATH.exists() or any(p.stat().st_mtime > _HOST_PATH.stat().st_mtime
+                                          for p in (_SRC_DIR / "host_calls.cpp", _SRC_DIR / "pnm_api.h"))
+
+
+def _build_host() -> None:
+    import sysconfig
+
+    top = Path(torch.__file__).resolve().parent
+    cuda = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    include = [top / "include", top / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
+    tmp_out = _LIB_DIR / f"._pnm_host.{os.getpid()}.so.tmp"
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{p}" for p in include], f"-I{_SRC_DIR}", "-o", str(tmp_out), str(_SRC_DIR / "host_calls.cpp"), f"-L{top / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-L{_LIB_DIR}", f"-l:{_LIB_PATH.name}",
+           "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{top / 'lib'}"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        if tmp_out.exists():
+            tmp_out.unlink()
+        raise RuntimeError(f"{cmd[0]} failed:\n{proc.stdout}\n{proc.stderr}")
+    os.replace(tmp_out, _HOST_PATH)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -68,6 +98,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     os.replace(tmp_out, _LIB_PATH)
     if verbose:
         print(proc.stderr)
+    if torch.version.cuda is not None:
+        _build_host()
     return _LIB_PATH
 
 
@@ -120,6 +152,24 @@ def load(required: bool = False):
                 raise RuntimeError(f"sm_100a kernel library unavailable: {exc}") from exc
             return None
     return _lib
+
+
+def host():
+    """The extension with the host side of the hottest calls (an error where it is missing: there is no second path)."""
+    global _host
+    if _host is None:
+        import importlib.util
+
+        load(required=True)
+        with _lock:
+            if _host is None:
+                if not _HOST_PATH.exists():
+                    raise RuntimeError(f"{_HOST_PATH} not built; run `python -c 'import __graft_entry__ as g; g.build()'`")
+                spec = importlib.util.spec_from_file_location("_pnm_host", _HOST_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                _host = module
+    return _host
 
 
 # absent from CPU builds of torch, where nothing is launched

@@ -371,8 +371,8 @@ def afno_filter(tokens: torch.Tensor, w1, b1, w2, b2, geo: FilterGeometry, spars
     if fn is _AfnoFilterTcFn and exchange is None and (add_input or residual is not None):
         if residual is not None and (residual.dtype != torch.bfloat16 or residual.shape != tokens.shape):
             raise ValueError("residual must be a bf16 tensor of the tokens' shape")
-        return fn.apply(tokens, w1, b1, w2, b2, geo, float(sparsity_threshold), None, add_input, residual)
-    out = fn.apply(tokens, w1, b1, w2, b2, geo, float(sparsity_threshold), exchange)
+        return _g.apply_function(fn, tokens, w1, b1, w2, b2, geo, float(sparsity_threshold), None, add_input, residual)
+    out = _g.apply_function(fn, tokens, w1, b1, w2, b2, geo, float(sparsity_threshold), exchange)
     if add_input:
         out = out + tokens
     return out if residual is None else out + residual

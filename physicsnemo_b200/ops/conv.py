@@ -81,12 +81,7 @@ def _pack_kernel(weight: torch.Tensor, rows: int, cols: int, flip: bool) -> torc
     if type(weight) not in (torch.Tensor, torch.nn.Parameter) or not weight.is_cuda or not weight.is_contiguous() \
             or weight.dtype not in (torch.float32, torch.bfloat16):
         return None
-    cout, cin, k, _ = weight.shape
-    out = torch.empty(rows, k * k * cols, dtype=torch.bfloat16, device=weight.device)
-    err = _lib_conv().pnm_conv_pack_weight(weight.data_ptr(), int(weight.dtype == torch.bfloat16), out.data_ptr(), cout, cin, k, rows, cols,
-                                           int(flip), _lib.stream())
-    if err:
-        raise RuntimeError(f"pnm_conv_pack_weight failed ({err})")
+    out = _lib.host().conv_pack_weight(weight, rows, cols, flip)
     _g.launch_count += 1
     return out
 
@@ -120,16 +115,11 @@ def _cout_bwd(weight: torch.Tensor) -> int:
 
 
 def _launch(x_nhwc: torch.Tensor, w_packed: torch.Tensor, bias, ksize: int, act: int) -> torch.Tensor:
-    n, h, w, cin = x_nhwc.shape
     cout = w_packed.shape[0]
-    y = torch.empty(n, h, w, cout, dtype=torch.bfloat16, device=x_nhwc.device)
     b = None if bias is None else _g._f32(bias.detach())
     if b is not None and b.numel() != cout:
         b = F.pad(b, (0, cout - b.numel()))
-    err = _lib_conv().pnm_conv2d_nhwc(x_nhwc.data_ptr(), w_packed.data_ptr(), y.data_ptr(), n, h, w, cin, cout, ksize,
-                                      None if b is None else b.data_ptr(), act, 0, 0, _lib.stream())
-    if err:
-        raise RuntimeError(f"pnm_conv2d_nhwc failed ({err})")
+    y = _lib.host().conv2d_nhwc(x_nhwc, w_packed, b, ksize, act)
     _g.launch_count += 1
     return y
 
@@ -227,7 +217,7 @@ def conv2d_same(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
         cin_p, cout_p = _conv_dims(weight)
         y = _launch(_as_nhwc_bf16(x, cin_p), _forward_operand(weight, cin_p, cout_p), bias, weight.shape[-1], code)
         return y[..., :weight.shape[0]].permute(0, 3, 1, 2)
-    y = _ConvSame.apply(x, weight, bias, 0)
+    y = _g.apply_function(_ConvSame, x, weight, bias, 0)
     if code:
         y = {1: F.gelu, 2: F.silu, 3: F.relu}[code](y)
     return y

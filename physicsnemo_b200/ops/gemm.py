@@ -44,6 +44,27 @@ def call_is_observed() -> bool:
     return forward_ad._current_level >= 0 or torch._C._is_tracing() or torch._C._are_functorch_transforms_active()
 
 
+class _NoContext:
+    """Stands for an autograd function's context where no backward will follow."""
+
+    needs_input_grad = (False,) * 64
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def apply_function(fn, *args):
+    """``fn.apply(*args)``; without gradients ``fn.forward`` alone, whose launches cost less than the function object around them
+    (about 12 us a call).  For functions whose results are tensors of their own (or views of such)."""
+    if torch.is_grad_enabled():
+        for a in args:
+            if isinstance(a, torch.Tensor) and a.requires_grad:
+                return fn.apply(*args)
+    if call_is_observed():
+        return fn.apply(*args)
+    return fn.forward(_NoContext(), *args)
+
+
 def _f32(t: torch.Tensor) -> torch.Tensor:
     """fp32 contiguous values of a parameter vector, for a launch (no autograd): the parameter itself where it is that already."""
     if t.dtype == torch.float32 and t.is_contiguous():
@@ -59,14 +80,6 @@ def _check(code: int, what: str):
 def _aligned(t: torch.Tensor) -> torch.Tensor:
     """``t``, or a copy of it where it does not start on a 16-byte boundary (a slice of a flat buffer, say): the kernels move vectors
     of that size, and ``contiguous()`` leaves such a tensor where it is."""
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
-def _rowmajor2d(t: torch.Tensor) -> torch.Tensor:
-    """2-D view whose last dim is contiguous, whose row stride is a multiple of 8 and that starts on a 16-byte boundary."""
-    assert t.dim() == 2
-    if t.stride(1) != 1 or t.stride(0) % 8 != 0:
-        t = t.contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
@@ -95,44 +108,9 @@ def gemm_tn(
     pre-activation.  Returns ``out`` or ``(out, z)``.
     """
     global launch_count
-    lib = _lib.load(required=True)
-    a = _rowmajor2d(a)
-    b = _rowmajor2d(b)
-    M, K1 = a.shape
-    N, K = b.shape
-    K2 = K
-    if a2 is not None:
-        a2 = _rowmajor2d(a2)
-        K2 = K1 + a2.shape[1]
-        if a3 is not None:
-            a3 = _rowmajor2d(a3)
-            assert a3.shape[0] == M and K2 + a3.shape[1] == K
-        else:
-            assert a2.shape[0] == M and K2 == K
-    else:
-        assert K1 == K, f"A has K={K1} but B has K={K}"
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    z = torch.empty((M, N), dtype=torch.bfloat16, device=a.device) if z_out else None
-    if aux is not None:
-        aux = _rowmajor2d(aux)
-        assert aux.shape == (M, N) and aux.dtype == torch.bfloat16
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous()
-    if scale is not None:
-        assert scale.dtype == torch.float32 and scale.numel() == N and scale.is_contiguous()
-    code = lib.pnm_gemm_tn(
-        _ptr(a), a.stride(0), _ptr(a2), 0 if a2 is None else a2.stride(0), _ptr(a3), 0 if a3 is None else a3.stride(0),
-        _ptr(b), b.stride(0),
-        _ptr(out), out.stride(0), _ptr(z), 0 if z is None else z.stride(0),
-        _ptr(aux), 0 if aux is None else aux.stride(0),
-        M, N, K, K1, K2, _ptr(bias), _ptr(scale), _ptr(group_out), act, aux_mode, int(scale_post), bn, max_ctas,
-        _stream(),
-    )
-    _check(code, "pnm_gemm_tn")
+    res = _lib.host().gemm_tn(a, b, bias, scale, act, aux, aux_mode, a2, a3, z_out, out, group_out, scale_post, bn, max_ctas)
     launch_count += 1
-    return (out, z) if z_out else out
+    return res
 
 
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, *, colsum: bool = False, out: Optional[torch.Tensor] = None,
@@ -142,22 +120,9 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, *, colsum: bool = False, out: Opti
     ``out`` / ``colsum_out`` accumulate when given (they must hold valid fp32 data).
     """
     global launch_count
-    lib = _lib.load(required=True)
-    a = _rowmajor2d(a)
-    b = _rowmajor2d(b)
-    M, Na = a.shape
-    Nb = b.shape[1]
-    assert b.shape[0] == M
-    if out is None:
-        out = torch.zeros((Na, Nb), dtype=torch.float32, device=a.device)
-    cs = None
-    if colsum or colsum_out is not None:
-        cs = colsum_out if colsum_out is not None else torch.zeros((Na,), dtype=torch.float32, device=a.device)
-    code = lib.pnm_gemm_nt(_ptr(a), a.stride(0), _ptr(b), b.stride(0), _ptr(out), out.stride(0), _ptr(cs),
-                           M, Na, Nb, max_ctas, _stream())
-    _check(code, "pnm_gemm_nt")
+    res = _lib.host().gemm_nt(a, b, colsum, out, colsum_out, max_ctas)
     launch_count += 1
-    return (out, cs) if cs is not None else out
+    return res
 
 
 # ------------------------------------------------------------------ oracles
@@ -497,7 +462,7 @@ def mlp_chain(x, weights: Sequence[torch.Tensor], biases: Sequence[Optional[torc
         any(t.requires_grad for t in xs) or any(w.requires_grad for w in weights)
         or (residual is not None and residual.requires_grad)
     )
-    y = _MlpChainFn.apply(r2, tuple(acts), n, need_z, len(x2s), *x2s, *weights, *biases)
+    y = apply_function(_MlpChainFn, r2, tuple(acts), n, need_z, len(x2s), *x2s, *weights, *biases)
     return y.reshape(*shp[:-1], y.shape[-1])
 
 

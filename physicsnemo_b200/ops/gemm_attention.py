@@ -118,7 +118,7 @@ class _GemmAttention(torch.autograd.Function):
 def gemm_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None) -> torch.Tensor:
     """``softmax(scale · q kᵀ) v`` for ``[..., S, D]`` tensors on the library's GEMM and softmax kernels (bf16 compute)."""
     scale = float(scale) if scale is not None else 1.0 / math.sqrt(q.shape[-1])
-    return _GemmAttention.apply(q, k, v, scale)
+    return G.apply_function(_GemmAttention, q, k, v, scale)
 
 
 # ------------------------------------------------------------------------------------------------- sequence sharded

@@ -39,26 +39,14 @@ class SegmentIndex:
 
 def _gather_raw(x: torch.Tensor, idx32: torch.Tensor, scale: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    lib = _lib.load(required=True)
-    E, C = idx32.numel(), x.shape[1]
-    if out is None:
-        out = torch.empty((E, C), dtype=torch.bfloat16, device=x.device)
-    code = lib.pnm_gather_rows(x.data_ptr(), x.stride(0), idx32.data_ptr(), None if scale is None else scale.data_ptr(),
-                               out.data_ptr(), out.stride(0), E, C, _g._stream())
-    _g._check(code, "pnm_gather_rows")
+    out = _lib.host().gather_rows(x, idx32, scale, out)
     _g.launch_count += 1
     return out
 
 
 def _segment_raw(x: torch.Tensor, seg: SegmentIndex, mean: bool = False, out: Optional[torch.Tensor] = None,
                  accumulate: bool = False) -> torch.Tensor:
-    lib = _lib.load(required=True)
-    C = x.shape[1]
-    if out is None:
-        out = torch.empty((seg.num_segments, C), dtype=torch.bfloat16, device=x.device)
-    code = lib.pnm_segment_sum(x.data_ptr(), x.stride(0), seg.perm.data_ptr(), seg.offsets.data_ptr(), out.data_ptr(),
-                               out.stride(0), seg.num_segments, C, int(accumulate), int(mean), _g._stream())
-    _g._check(code, "pnm_segment_sum")
+    out = _lib.host().segment_sum(x, seg.perm, seg.offsets, seg.num_segments, accumulate, mean, out)
     _g.launch_count += 1
     return out
 
@@ -99,7 +87,7 @@ def _fused(x: torch.Tensor) -> bool:
 def gather_rows(x: torch.Tensor, seg: SegmentIndex) -> torch.Tensor:
     """``x[seg.index]`` (differentiable; backward is the sorted segment sum)."""
     if _fused(x):
-        return _GatherFn.apply(x, seg)
+        return _g.apply_function(_GatherFn, x, seg)
     return x[seg.index]
 
 
@@ -108,7 +96,7 @@ def segment_reduce(x: torch.Tensor, seg: SegmentIndex, reduce: str = "sum") -> t
     if reduce not in ("sum", "mean"):
         raise ValueError(f"unsupported reduction {reduce}")
     if _fused(x):
-        return _SegmentFn.apply(x, seg, reduce == "mean")
+        return _g.apply_function(_SegmentFn, x, seg, reduce == "mean")
     out = torch.zeros((seg.num_segments, x.shape[1]), dtype=x.dtype, device=x.device)
     out.index_add_(0, seg.index, x)
     if reduce == "mean":

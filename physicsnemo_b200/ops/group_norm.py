@@ -84,18 +84,9 @@ class _GroupNormFn(torch.autograd.Function):
         hw = x.numel() // (B * C)
         v = 8 if x.dtype == torch.bfloat16 else 4
         S = _slices(B, C, hw, lay, v)
-        lib = _lib_gn()
-        dev = x.device
         gamma, beta = _g._f32(weight), _g._f32(bias)
-        y = torch.empty_like(x)                       # preserves the memory format
-        mean = torch.empty(B * num_groups, dtype=torch.float32, device=dev)
-        rstd = torch.empty_like(mean)
-        scratch = torch.empty(lib.pnm_groupnorm_scratch_floats(B, C, num_groups, S), dtype=torch.float32, device=dev)
-        err = lib.pnm_groupnorm_fwd(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mean.data_ptr(),
-                                    rstd.data_ptr(), scratch.data_ptr(), B, C, hw, num_groups, S, lay, _DT[x.dtype],
-                                    int(silu), float(eps), _lib.stream())
-        if err:
-            raise RuntimeError(f"pnm_groupnorm_fwd failed ({err})")
+        # y has x's memory format
+        y, mean, rstd = _lib.host().groupnorm_fwd(x, gamma, beta, num_groups, S, lay, _DT[x.dtype], silu, eps)
         _g.launch_count += 2
         ctx.save_for_backward(x, gamma, beta, mean, rstd)
         ctx.cfg = (num_groups, S, lay, bool(silu), weight.dtype, bias.dtype)
@@ -132,7 +123,7 @@ class _GroupNormFn(torch.autograd.Function):
 def group_norm(x: torch.Tensor, num_groups: int, weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5,
                silu: bool = False) -> torch.Tensor:
     """``silu(group_norm(x))`` (or plain ``group_norm``) on the CUDA kernels; ``supported(x, G)`` must hold."""
-    return _GroupNormFn.apply(x, weight, bias, int(num_groups), float(eps), bool(silu))
+    return _g.apply_function(_GroupNormFn, x, weight, bias, int(num_groups), float(eps), bool(silu))
 
 
 class _GroupNormShardedFn(torch.autograd.Function):

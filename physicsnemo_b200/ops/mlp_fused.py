@@ -25,38 +25,33 @@ def _lib_mlp():
     lib = _lib.load(required=True)
     if not getattr(lib, "_mlp3_declared", False):
         c = ctypes
-        vp, i, l, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
-        lib.pnm_mlp3_ln_fwd.argtypes = [i, c.POINTER(vp), c.POINTER(l), c.POINTER(i), c.POINTER(vp), vp, vp, vp, vp, vp, vp, vp, vp, f, i,
-                                        vp, l, vp, l, vp, vp, vp, vp, vp, vp, vp, l, vp]
+        vp, i, l = c.c_void_p, c.c_int, c.c_longlong
         lib.pnm_mlp3_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, i, vp, vp, vp, vp, vp, l, vp]
         lib.pnm_segment_sum_split.argtypes = [vp, vp, vp, vp, l, l, i, vp]
-        lib.pnm_mlp3_ln_fwd.restype = lib.pnm_mlp3_bwd.restype = lib.pnm_segment_sum_split.restype = i
+        lib.pnm_mlp3_bwd.restype = lib.pnm_segment_sum_split.restype = i
         lib._mlp3_declared = True
     return lib
-
-
-def _row_table(t: torch.Tensor) -> bool:
-    """A bf16 table of 128 columns whose rows start on 32-byte boundaries (the kernel moves whole sectors)."""
-    return (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[1] == WIDTH
-            and t.shape[0] > 0 and t.stride(1) == 1 and t.stride(0) >= WIDTH and t.stride(0) % 16 == 0 and t.data_ptr() % 32 == 0)
 
 
 def supported(srcs: Sequence[torch.Tensor], segs: Sequence, weights, biases, acts, gamma, beta, post: Optional[int]) -> bool:
     """Three 128-wide layers with the same activation after the first two and a 128-wide affine LayerNorm, on aligned
     bf16 tables of one device."""
-    if not 1 <= len(srcs) <= 3 or len(weights) != 3 or list(acts) != [acts[0], acts[0], _g.ACT_NONE] or acts[0] not in _ACTS:
+    if not 1 <= len(srcs) <= 3 or len(weights) != 3 or len(acts) != 3 or acts[0] not in _ACTS or acts[1] != acts[0] or acts[2] != _g.ACT_NONE:
         return False
-    if any(tuple(w.shape) != (WIDTH, k) for w, k in zip(weights, (WIDTH * len(srcs), WIDTH, WIDTH))):
+    # bf16 tables of 128 columns whose rows start on 32-byte boundaries; parameters of the right shapes on the same device
+    if not _lib.host().mlp3_operands_ok(srcs, weights, biases, gamma, beta):
         return False
-    if gamma is None or gamma.numel() != WIDTH or not all(_row_table(t) for t in srcs):
-        return False
-    rows = {s.num_items if s is not None else t.shape[0] for t, s in zip(srcs, segs)}
-    if len(rows) != 1 or 0 in rows or any(s is not None and s.num_segments != t.shape[0] for t, s in zip(srcs, segs)):
-        return False
-    if post is not None and segs[post] is not None:
-        return False
-    params = [*weights, *[b for b in biases if b is not None], gamma] + ([beta] if beta is not None else [])
-    return all(type(p) in (torch.Tensor, torch.nn.Parameter) and p.device == srcs[0].device for p in params)
+    rows = None
+    for t, s in zip(srcs, segs):
+        n = t.shape[0]
+        if s is not None:
+            if s.num_segments != n:
+                return False
+            n = s.num_items
+        if n == 0 or (rows is not None and rows != n):
+            return False
+        rows = n
+    return post is None or segs[post] is None
 
 
 def _vec(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -68,30 +63,12 @@ def _vec(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
 
 
 def _forward(srcs, segs, weights, biases, act, gamma, beta, eps, post, save: bool):
-    lib = _lib_mlp()
-    n = len(srcs)
     m = segs[0].num_items if segs[0] is not None else srcs[0].shape[0]
-    dev = srcs[0].device
-    w16 = [_g._bf16_weight(w) for w in weights]
-    vecs = [_vec(t) for t in (*biases, gamma, beta)]
-    y = torch.empty((m, WIDTH), dtype=torch.bfloat16, device=dev)
-    kept, given = (), [None] * 7
-    if save:                                                 # h1, h2, x3, mean, rstd; z1 and z2 (whole tiles) but for ReLU
-        kept = (*torch.empty((3, m, WIDTH), dtype=torch.bfloat16, device=dev).unbind(0),
-                *torch.empty((2, m), dtype=torch.float32, device=dev).unbind(0))
-        if act != _g.ACT_RELU:
-            kept += torch.empty((2, -(-m // ROWS), ROWS * WIDTH), dtype=torch.bfloat16, device=dev).unbind(0)
-        h1, h2, x3, mean, rstd, *z = [t.data_ptr() for t in kept]
-        given = [*(z or (None, None)), h1, h2, x3, mean, rstd]
-    vp = ctypes.c_void_p
-    code = lib.pnm_mlp3_ln_fwd(
-        n, (vp * n)(*[t.data_ptr() for t in srcs]), (ctypes.c_longlong * n)(*[t.shape[0] for t in srcs]),
-        (ctypes.c_int * n)(*[t.stride(0) for t in srcs]), (vp * n)(*[None if s is None else s.index32.data_ptr() for s in segs]),
-        *[w.data_ptr() for w in w16], *[_g._ptr(v) for v in vecs], float(eps), act, _g._ptr(post), 0 if post is None else post.stride(0),
-        y.data_ptr(), WIDTH, *given, m, _g._stream())
-    _g._check(code, "pnm_mlp3_ln_fwd")
+    # kept: h1, h2, x3, mean, rstd; z1 and z2 (whole tiles) but for ReLU
+    res = _lib.host().mlp3_fwd(srcs, [None if s is None else s.index32 for s in segs], [_g._bf16_weight(w) for w in weights],
+                               (*biases, gamma, beta), eps, act, post, m, save)
     _g.launch_count += 1
-    return y, kept
+    return (res[0], res[1:]) if save else (res, ())
 
 
 def _w_t(w: torch.Tensor) -> torch.Tensor:

@@ -19,18 +19,8 @@ from . import gemm as _g
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x2d, gamma, beta, eps, post=None, alias_out=False):
-        lib = _lib.load(required=True)
-        M, C = x2d.shape
-        y = torch.empty_like(x2d)
-        mean = torch.empty((M,), dtype=torch.float32, device=x2d.device)
-        rstd = torch.empty((M,), dtype=torch.float32, device=x2d.device)
         g32 = _g._f32(gamma)
-        b32 = _g._f32(beta) if beta is not None else None
-        code = lib.pnm_layernorm_fwd(x2d.data_ptr(), None, g32.data_ptr(), None if b32 is None else b32.data_ptr(),
-                                     y.data_ptr(), None, mean.data_ptr(), rstd.data_ptr(),
-                                     None if post is None else post.data_ptr(), M, C, float(eps),
-                                     _g._stream())
-        _g._check(code, "pnm_layernorm_fwd")
+        y, mean, rstd = _lib.host().layernorm_fwd(x2d, g32, _g._f32(beta) if beta is not None else None, eps, post)
         _g.launch_count += 1
         ctx.save_for_backward(x2d, g32, mean, rstd)
         ctx.has_beta = beta is not None
@@ -87,6 +77,6 @@ def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
             p2 = p2.to(torch.bfloat16)
         p2 = _g._aligned(p2.contiguous())
     if return_residual:
-        y, alias = _LayerNormFn.apply(x2, weight, bias, eps, p2, True)
+        y, alias = _g.apply_function(_LayerNormFn, x2, weight, bias, eps, p2, True)
         return y.reshape(x.shape), alias.reshape(x.shape)
-    return _LayerNormFn.apply(x2, weight, bias, eps, p2).reshape(x.shape)
+    return _g.apply_function(_LayerNormFn, x2, weight, bias, eps, p2).reshape(x.shape)

@@ -42,26 +42,14 @@ def supported(H: int, D: int, slices: int, C: int, params: Sequence[torch.Tensor
 
 def prepare_fwd(Wx, bx, Wfx, Ws, bs, temp, H: int, D: int):
     """``(Wc bf16 [H*S, C], bc [H*S], inv_t [H*S], Wfx bf16, Wback bf16 [C, H*S + H*D])``."""
-    C = Wx.shape[1]
-    dev = Wx.device
-    HS, inner = H * S, H * D
-    Wc = torch.empty(HS, C, dtype=torch.bfloat16, device=dev)
-    bc = torch.empty(HS, dtype=torch.float32, device=dev)
-    inv_t = torch.empty(HS, dtype=torch.float32, device=dev)
-    Wfx16 = torch.empty(inner, C, dtype=torch.bfloat16, device=dev)
-    Wback = torch.empty(C, HS + inner, dtype=torch.bfloat16, device=dev)
-    err = _lib_pa().pnm_pa_prepare_fwd(Wx.data_ptr(), bx.data_ptr(), Wfx.data_ptr(), Ws.data_ptr(), bs.data_ptr(),
-                                       temp.data_ptr(), Wc.data_ptr(), bc.data_ptr(), inv_t.data_ptr(), Wfx16.data_ptr(),
-                                       Wback.data_ptr(), H, D, C, _st())
-    _g._check(err, "pnm_pa_prepare_fwd")
+    res = _lib.host().pa_prepare_fwd(Wx, bx, Wfx, Ws, bs, temp, H, D)
     _g.launch_count += 1
-    return Wc, bc, inv_t, Wfx16, Wback
+    return res
 
 
-def new_saved(H: int, D: int, Cout: int, dev) -> List[torch.Tensor]:
-    f = dict(dtype=torch.float32, device=dev)
-    return [torch.empty(H, S, D, **f), torch.empty(H, S, **f), torch.empty(H, S, D, **f), torch.empty(H, S, D, **f),
-            torch.empty(H, S, D, **f), torch.empty(H, S, S, **f), torch.empty(H, S, D, **f), torch.empty(Cout, H * S, **f)]
+def new_saved(H: int, D: int, Cout: int, like: torch.Tensor) -> List[torch.Tensor]:
+    t = (H, S, D)
+    return _lib.host().empties(like, False, t, (H, S), t, t, t, (H, S, S), t, (Cout, H * S))
 
 
 def tokens_fwd(src_ptrs: Sequence[int], norm_off: int, ld_tok: int, Wqkv, Wo, H: int, D: int, peer: Optional[tuple] = None):
@@ -70,9 +58,8 @@ def tokens_fwd(src_ptrs: Sequence[int], norm_off: int, ld_tok: int, Wqkv, Wo, H:
     ``peer``: ``PeerRuntime.peer_args(epoch)`` when the sources are peers' buffers whose flags must be awaited.
     """
     Cout = Wo.shape[0]
-    dev = Wo.device
-    saved = new_saved(H, D, Cout, dev)
-    wcomb16 = torch.empty(Cout, H * S, dtype=torch.bfloat16, device=dev)
+    saved = new_saved(H, D, Cout, Wo)
+    wcomb16 = torch.empty(Cout, H * S, dtype=torch.bfloat16, device=Wo.device)
     world = len(src_ptrs)
     use_flags = int(peer is not None)
     bases, rank, _w, epoch, cap, budget, ebase = peer if peer is not None else (None, 0, 1, 0, 0, 1.0, None)

@@ -137,7 +137,8 @@ def physics_attention_irregular(mod, x: torch.Tensor, residual: torch.Tensor | N
             if rb.dtype != torch.bfloat16:
                 rb = rb.to(torch.bfloat16)
             rb = rb.contiguous()
-        out = _PhysAttnFn.apply(
+        out = G.apply_function(
+            _PhysAttnFn,
             xb.contiguous(), rb, mod.heads, mod.dim_head, mod.slice_num, exchange,
             mod.in_project_x.weight, mod.in_project_x.bias, mod.in_project_fx.weight, mod.in_project_fx.bias,
             mod.in_project_slice.weight, mod.in_project_slice.bias, mod.temperature, mod.qkv_project.weight,

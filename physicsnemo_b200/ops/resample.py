@@ -63,14 +63,14 @@ class _Up2x(torch.autograd.Function):
 def down2x(x: torch.Tensor) -> torch.Tensor:
     """2 × 2 mean (``F.avg_pool2d(x, 2)``)."""
     if supported(x) and x.shape[2] % 2 == 0 and x.shape[3] % 2 == 0:
-        return _Down2x.apply(x)
+        return _g.apply_function(_Down2x, x)
     return F.avg_pool2d(x, 2)
 
 
 def up2x(x: torch.Tensor) -> torch.Tensor:
     """2 × 2 replication (``F.interpolate(x, scale_factor=2, mode="nearest")``)."""
     if supported(x):
-        return _Up2x.apply(x)
+        return _g.apply_function(_Up2x, x)
     return F.interpolate(x, scale_factor=2, mode="nearest")
 
 
@@ -116,7 +116,7 @@ def add_scale(a: torch.Tensor, b: torch.Tensor, scale: float) -> torch.Tensor:
     same dense layout; the PyTorch expression otherwise."""
     if (type(a) is torch.Tensor and type(b) is torch.Tensor and a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
             and a.numel() % 8 == 0 and _same_dense_layout(a, b) and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and _lib.available()):
-        return _AddScale.apply(a, b, scale)
+        return _g.apply_function(_AddScale, a, b, scale)
     return (a + b) * scale
 
 
@@ -168,5 +168,5 @@ def add_channel(x: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
             and x.dim() == 4 and x.numel() > 0 and v.shape == (*x.shape[:2], 1, 1) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048
             and x.shape[0] <= 65535 and x.is_contiguous(memory_format=torch.channels_last) and v.is_contiguous()
             and x.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0 and _lib.available()):
-        return _AddChannel.apply(x, v)
+        return _g.apply_function(_AddChannel, x, v)
     return x + v
