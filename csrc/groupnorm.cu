@@ -266,6 +266,22 @@ __device__ __forceinline__ void cl_channel_sums(const CLThread& t, const float* 
 }
 constexpr size_t cl_stats_smem(int V, int C) { return (2 * 256 * (size_t)V + 2 * (size_t)C) * sizeof(float); }
 
+// Pixels whose loads are issued together.  Forward and backward of 512 x 512 bf16 pixels with one, two, three, four pixels ahead: 256
+// channels 113, 113, 103, 105 and 276, 229, 188, 190 us, 128 channels 72, 71, 65, 65 and 169, 141, 116, 117 us; fp32 (half as many
+// channels a thread, 128 channels, 256 x 256) 37, 37, 40, 41 and 54, 53, 52, 62 us.
+template <typename T>
+constexpr int kClAhead = sizeof(T) == 2 ? 3 : 2;
+// the vectors of pixels pix, pix + ppi, .., zeros past the end of the slice
+template <typename T>
+__device__ __forceinline__ void cl_load_ahead(const T* x, const CLThread& t, long long pix, int C, uint4* raw) {
+#pragma unroll
+  for (int k = 0; k < kClAhead<T>; ++k) {
+    const long long q = pix + k * t.ppi;
+    raw[k] = make_uint4(0, 0, 0, 0);
+    if (q < t.p1) raw[k] = *reinterpret_cast<const uint4*>(x + q * C);
+  }
+}
+
 // part[b][s][g] = (sum x, sum x^2) of slice s; gsum[b][g] = their sum over the slices (written by the last CTA of item b)
 template <typename T>
 __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, float2* __restrict__ part, float2* __restrict__ gsum,
@@ -280,11 +296,15 @@ __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, floa
   for (int i = 0; i < V; ++i) a[i] = q[i] = 0.f;
   if (t.active) {
     const T* base = x + (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 4
-    for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
-      Vec<T>::load(base + p * sh.C, f);
+    for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
+      uint4 raw[kClAhead<T>];
+      cl_load_ahead(base, t, pix, sh.C, raw);
 #pragma unroll
-      for (int i = 0; i < V; ++i) { a[i] += f[i]; q[i] += f[i] * f[i]; }
+      for (int k = 0; k < kClAhead<T>; ++k) {
+        Vec<T>::load(reinterpret_cast<const T*>(&raw[k]), f);
+#pragma unroll
+        for (int i = 0; i < V; ++i) { a[i] += f[i]; q[i] += f[i] * f[i]; }
+      }
     }
   }
   cl_channel_sums<V>(t, a, q, smem, sums, sh.C);
@@ -454,16 +474,51 @@ __global__ void __launch_bounds__(256) gn_apply_cl(const T* __restrict__ x, cons
     shift[i] = beta[c] - m.x * scale[i];
   }
   const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 4
-  for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
-    Vec<T>::load(x + off + p * sh.C, f);
+  for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
+    uint4 raw[kClAhead<T>];
+    cl_load_ahead(x + off, t, pix, sh.C, raw);
 #pragma unroll
-    for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu<T>(z) : z; }
-    Vec<T>::store(y + off + p * sh.C, f);
+    for (int k = 0; k < kClAhead<T>; ++k) {
+      Vec<T>::load(reinterpret_cast<const T*>(&raw[k]), f);
+#pragma unroll
+      for (int i = 0; i < V; ++i) { const float z = f[i] * scale[i] + shift[i]; f[i] = kSilu ? gn_silu<T>(z) : z; }
+      const long long q = pix + k * t.ppi;
+      if (q < t.p1) Vec<T>::store(y + off + q * sh.C, f);
+    }
   }
 }
 
-template <typename T, bool kSilu>
+// What a thread of the channels-last backward keeps of its V channels.  The group's values once per half of them (MU = 2: groups of a
+// multiple of V / 2 channels, as 32 groups of 128 and more channels are) or per channel (MU = V): with six values per channel the
+// registers left none for loads in flight.  bf16 rows are only centred and rstd goes into the channel's factor (two multiplications
+// less an element; results and errors against 64 bits the same to seven digits); fp32 rows are normalised first, as before.
+template <typename T, int MU>
+struct CLBwd {
+  static constexpr int V = Vec<T>::N;
+  static constexpr bool kCentred = sizeof(T) == 2;
+  float mu[MU], rs[MU], ga[V], be[V];
+  __device__ __forceinline__ CLBwd(const CLThread& t, const GNShape& sh, int b, const float* mean, const float* rstd, const float* gamma,
+                                   const float* beta) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = t.c0 + i, g = b * sh.G + c / sh.cpg;
+      mu[i * MU / V] = mean[g]; rs[i * MU / V] = rstd[g];
+      ga[i] = kCentred ? rstd[g] * gamma[c] : gamma[c];
+      be[i] = beta[c];
+    }
+  }
+  // x - mean, times rstd where rows are normalised; dz from it
+  __device__ __forceinline__ float row(float x, int i) const {
+    const float c = x - mu[i * MU / V];
+    return kCentred ? c : c * rs[i * MU / V];
+  }
+  template <bool kSilu>
+  __device__ __forceinline__ float dz(float xr, float dy, int i) const {
+    return kSilu ? dy * gn_silu_grad<T>(xr * ga[i] + be[i]) : dy;
+  }
+};
+
+template <typename T, bool kSilu, int MU>
 __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, const T* __restrict__ dy,
                                                         const float* __restrict__ gamma, const float* __restrict__ beta,
                                                         const float* __restrict__ mean, const float* __restrict__ rstd,
@@ -476,27 +531,32 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
   __syncthreads();
   const CLThread t = cl_thread<V>(sh, s);
   if (t.active) {
-    float mu[V], rs[V], ga[V], be[V], a[V], d[V], f[V], e[V];
+    const CLBwd<T, MU> w(t, sh, b, mean, rstd, gamma, beta);
+    float a[V], d[V];
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int c = t.c0 + i, g = c / sh.cpg;
-      mu[i] = mean[b * sh.G + g]; rs[i] = rstd[b * sh.G + g]; ga[i] = gamma[c]; be[i] = beta[c];
-      a[i] = d[i] = 0.f;
-    }
+    for (int i = 0; i < V; ++i) a[i] = d[i] = 0.f;
     const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 4
-    for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
-      Vec<T>::load(x + off + p * sh.C, f);
-      Vec<T>::load(dy + off + p * sh.C, e);
+    for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
+      uint4 rx[kClAhead<T>], ry[kClAhead<T>];
+      cl_load_ahead(x + off, t, pix, sh.C, rx);
+      cl_load_ahead(dy + off, t, pix, sh.C, ry);         // a zero dy adds nothing
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const float xh = (f[i] - mu[i]) * rs[i];
-        const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga[i] + be[i]) : e[i];
-        a[i] += dz * xh; d[i] += dz;
+      for (int k = 0; k < kClAhead<T>; ++k) {
+        float f[V], e[V];
+        Vec<T>::load(reinterpret_cast<const T*>(&rx[k]), f);
+        Vec<T>::load(reinterpret_cast<const T*>(&ry[k]), e);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
+          a[i] += dz * xr; d[i] += dz;
+        }
       }
     }
 #pragma unroll
-    for (int i = 0; i < V; ++i) { atomicAdd(&smem[2 * (t.c0 + i)], a[i]); atomicAdd(&smem[2 * (t.c0 + i) + 1], d[i]); }
+    for (int i = 0; i < V; ++i) {
+      atomicAdd(&smem[2 * (t.c0 + i)], w.kCentred ? a[i] * w.rs[i * MU / V] : a[i]);
+      atomicAdd(&smem[2 * (t.c0 + i) + 1], d[i]);
+    }
   }
   __syncthreads();
   // parameter gradients: every slice adds its channel sums (dgamma / dbeta are zeroed by the caller)
@@ -517,7 +577,7 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
   cl_fold_slices(part, group_ab, g_gn_bwd_counter, sh, b);
 }
 
-template <typename T, bool kSilu>
+template <typename T, bool kSilu, int MU>
 __global__ void __launch_bounds__(256) gn_bwd_apply_cl(const T* __restrict__ x, const T* __restrict__ dy,
                                                         const float* __restrict__ gamma, const float* __restrict__ beta,
                                                         const float* __restrict__ mean, const float* __restrict__ rstd,
@@ -527,26 +587,34 @@ __global__ void __launch_bounds__(256) gn_bwd_apply_cl(const T* __restrict__ x, 
   const CLThread t = cl_thread<V>(sh, s);
   if (!t.active) return;
   const float inv_n = 1.f / ((float)sh.cpg * (float)sh.HW);
-  float mu[V], rs[V], ga[V], be[V], A[V], Bq[V], f[V], e[V];
+  const CLBwd<T, MU> w(t, sh, b, mean, rstd, gamma, beta);
+  float A[MU], Bq[MU];
 #pragma unroll
   for (int i = 0; i < V; ++i) {
-    const int c = t.c0 + i, g = c / sh.cpg;
-    mu[i] = mean[b * sh.G + g]; rs[i] = rstd[b * sh.G + g]; ga[i] = gamma[c]; be[i] = beta[c];
-    const float2 ab = group_ab[b * sh.G + g];
-    A[i] = ab.x * inv_n; Bq[i] = ab.y * inv_n;
+    const float2 ab = group_ab[b * sh.G + (t.c0 + i) / sh.cpg];
+    const float rs = w.rs[i * MU / V];
+    A[i * MU / V] = w.kCentred ? rs * (ab.x * inv_n) : ab.x * inv_n;
+    Bq[i * MU / V] = w.kCentred ? rs * (rs * (ab.y * inv_n)) : ab.y * inv_n;
   }
   const long long off = (long long)b * sh.HW * sh.C + t.c0;
-#pragma unroll 4
-  for (long long p = t.p0 + t.lane_pix; p < t.p1; p += t.ppi) {
-    Vec<T>::load(x + off + p * sh.C, f);
-    Vec<T>::load(dy + off + p * sh.C, e);
+  for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
+    uint4 rx[kClAhead<T>], ry[kClAhead<T>];
+    cl_load_ahead(x + off, t, pix, sh.C, rx);
+    cl_load_ahead(dy + off, t, pix, sh.C, ry);
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const float xh = (f[i] - mu[i]) * rs[i];
-      const float dz = kSilu ? e[i] * gn_silu_grad<T>(xh * ga[i] + be[i]) : e[i];
-      f[i] = rs[i] * (ga[i] * dz - A[i] - xh * Bq[i]);
+    for (int k = 0; k < kClAhead<T>; ++k) {
+      float f[V], e[V];
+      Vec<T>::load(reinterpret_cast<const T*>(&rx[k]), f);
+      Vec<T>::load(reinterpret_cast<const T*>(&ry[k]), e);
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
+        const float g = w.ga[i] * dz - A[i * MU / V] - xr * Bq[i * MU / V];
+        f[i] = w.kCentred ? g : w.rs[i * MU / V] * g;
+      }
+      const long long q = pix + k * t.ppi;
+      if (q < t.p1) Vec<T>::store(dx + off + q * sh.C, f);
     }
-    Vec<T>::store(dx + off + p * sh.C, f);
   }
 }
 
@@ -593,6 +661,21 @@ int gn_forward(const void* x, const float* gamma, const float* beta, void* y, fl
   return (int)cudaGetLastError();
 }
 
+template <typename T, int MU>
+void launch_bwd_stats_cl(dim3 grid, size_t sm, cudaStream_t st, int act, const T* x, const T* dy, const float* gamma, const float* beta,
+                         const float* mean, const float* rstd, float2* pc, float2* ab, float* dgamma, float* dbeta, const GNShape& sh) {
+  if (act) gn_bwd_stats_cl<T, true, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+  else gn_bwd_stats_cl<T, false, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+}
+template <typename T, int MU>
+void launch_bwd_apply_cl(dim3 grid, cudaStream_t st, int act, const T* x, const T* dy, const float* gamma, const float* beta, const float* mean,
+                         const float* rstd, const float2* ab, T* dx, const GNShape& sh) {
+  if (act) gn_bwd_apply_cl<T, true, MU><<<grid, 256, 0, st>>>(x, dy, gamma, beta, mean, rstd, ab, dx, sh);
+  else gn_bwd_apply_cl<T, false, MU><<<grid, 256, 0, st>>>(x, dy, gamma, beta, mean, rstd, ab, dx, sh);
+}
+template <typename T>
+bool cl_half_groups(const GNShape& sh) { return sh.cpg % (Vec<T>::N / 2) == 0; }   // CLBwd with MU = 2
+
 template <typename T>
 int gn_backward(const void* x, const void* dy, const float* gamma, const float* beta, const float* mean, const float* rstd,
                 void* dx, float* dgamma, float* dbeta, float* scratch, GNShape sh, int layout, int act, cudaStream_t st) {
@@ -608,15 +691,15 @@ int gn_backward(const void* x, const void* dy, const float* gamma, const float* 
     else gn_bwd_stats_cf<T, false><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, pc, sh);
     gn_bwd_reduce<<<sh.B, 256, 2 * sh.G * sizeof(float), st>>>(pc, gamma, ab, dgamma, dbeta, sh);
   } else {
-    if (act) gn_bwd_stats_cl<T, true><<<grid, 256, sm, st>>>(xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
-    else gn_bwd_stats_cl<T, false><<<grid, 256, sm, st>>>(xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+    if (cl_half_groups<T>(sh)) launch_bwd_stats_cl<T, 2>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+    else launch_bwd_stats_cl<T, Vec<T>::N>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
   }
   if (layout == 0) {
     if (act) gn_bwd_apply_cf<T, true><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, ab, o, sh);
     else gn_bwd_apply_cf<T, false><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, ab, o, sh);
   } else {
-    if (act) gn_bwd_apply_cl<T, true><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, ab, o, sh);
-    else gn_bwd_apply_cl<T, false><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, ab, o, sh);
+    if (cl_half_groups<T>(sh)) launch_bwd_apply_cl<T, 2>(grid, st, act, xi, di, gamma, beta, mean, rstd, ab, o, sh);
+    else launch_bwd_apply_cl<T, Vec<T>::N>(grid, st, act, xi, di, gamma, beta, mean, rstd, ab, o, sh);
   }
   return (int)cudaGetLastError();
 }
@@ -648,8 +731,8 @@ int gn_backward_sh(const void* x, const void* dy, const float* gamma, const floa
   T* o = static_cast<T*>(dx);
   const dim3 grid(sh.S, sh.B);
   const size_t sm = 2 * sh.C * sizeof(float);
-  if (act) gn_bwd_stats_cl<T, true><<<grid, 256, sm, st>>>(xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
-  else gn_bwd_stats_cl<T, false><<<grid, 256, sm, st>>>(xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+  if (cl_half_groups<T>(sh)) launch_bwd_stats_cl<T, 2>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+  else launch_bwd_stats_cl<T, Vec<T>::N>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
   gn_publish_ab<<<sh.B, 256, 0, st>>>(ab, sh, peer, counter);
   if (act) gn_bwd_apply_cl_sh<T, true><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, di, gamma, beta, mean, rstd, o, sh, count_global, peer, err);
   else gn_bwd_apply_cl_sh<T, false><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, di, gamma, beta, mean, rstd, o, sh, count_global, peer, err);
