@@ -99,8 +99,8 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
 #pragma unroll
         for (int grp = 0; grp < 2; ++grp) {
           const int layer = at[grp] & 1;
-          if (!left[grp] || !mbar_try_wait(&ready[grp], layer)) continue;
-          if (!mbar_try_wait(layer ? &hfull[grp] : &dfull[grp], (at[grp] >> 1) & 1)) continue;
+          if (!left[grp] || !mbar_test(&ready[grp], layer)) continue;
+          if (!mbar_test(layer ? &hfull[grp] : &dfull[grp], (at[grp] >> 1) & 1)) continue;
           any = true;
           tc_fence_after();
           const uint32_t xs = smem_u32(tiles_smem + grp * 4 * kMlpChunk), ws = smem_u32(wts + layer * 2 * kMlpChunk);
@@ -219,9 +219,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
       for (int c = 0; c < 4; ++c) z[c] = ldg32(g.z2 + offset(grp) + c * step);
     }
     for (int n = grp; n < mine; n += 2) {
-      const bool live = ((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + r < g.M;
       const long long o = offset(n);
-      __nv_bfloat16* g1 = g.g1 + (((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + r) * kMlpW + col;
       tc_fence_before();                         // the accumulator was read: the last tile's g1 is on its way
       __syncwarp();
       if (lane == 0) mbar_arrive(&ready[grp]);
@@ -252,20 +250,21 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
       ok = mbar_wait(&done[grp], phase & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL) && ok;
       ++phase;
       tc_fence_after();
+      uint32_t out[32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float v[16];
         tmem_ld16(acc + c * 16, v);
         tmem_ld_wait();
-        uint32_t p[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float2 zv = unpack_bf16x2(z[c].w[j]);
-          p[j] = pack_bf16x2(mlp_dact<ACT>(v[2 * j], zv.x), mlp_dact<ACT>(v[2 * j + 1], zv.y));
+          out[8 * c + j] = pack_bf16x2(mlp_dact<ACT>(v[2 * j], zv.x), mlp_dact<ACT>(v[2 * j + 1], zv.y));
         }
-        if (live) stg32(g1 + c * 16, p);
         z[c] = ldg32(g.z2 + on + c * step);
       }
+      // through the columns of the accumulator that this thread has just read: eight lines an access instead of 32 rows
+      store_rows(acc, out, g.g1 + col, kMlpW, ((long long)blockIdx.x + (long long)n * gridDim.x) * kMlpRows + q * 32, g.M, lane);
     }
     // A wait that ran out leaves wrong values behind (the error word says so); the loop ends all the same, since every later
     // wait gives up at once.  Otherwise every product of the CTA has been waited for by the warps that used its result, so the
