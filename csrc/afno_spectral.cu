@@ -41,6 +41,7 @@ struct AfGeom {
 };
 
 __device__ __forceinline__ const __nv_bfloat16* token_addr(const TokenPtrs& tp, const AfGeom& g, long long t, int c) {
+  if (t < g.Tp) return tp.p[0] + t * g.C + c;    // without the 64-bit division (hundreds of instructions with it per CTA's thread)
   const int owner = int(t / g.Tp);
   return tp.p[owner] + (t - owner * g.Tp) * g.C + c;
 }
@@ -195,6 +196,38 @@ static RowPlan row_plan(int n_items, int cb) {
   return p;
 }
 
+// tw[r][k] = (cos, sin)(2 pi (((r + first) k) mod W) / W), r < rows, k < pad.  Only W values occur: they are computed once, in `base` (W float2),
+// and looked up.  (Every entry by itself, with its integer divisions, cost more: 2 x 90 x 180 tokens of 768
+// channels, with divisions also out of the loops over samples and the spectrum read by 16-byte vectors, to the spectrum 135 -> 117 us, back 131 -> 99, with
+// addends 154 -> 116.)  All threads of the CTA; ends with a barrier.
+__device__ __forceinline__ void row_twiddles(float2* tw, float2* base, int rows, int first, int pad, int W) {
+  for (int m = threadIdx.x; m < W; m += blockDim.x) {
+    float sn, cs;
+    sincospif(2.f * m / W, &sn, &cs);
+    base[m] = make_float2(cs, sn);
+  }
+  __syncthreads();
+  const float inv = 1.f / W;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int r = threadIdx.x >> 5; r < rows; r += warps)
+    for (int k = lane; k < pad; k += 32) {
+      const int x = (r + first) * k;             // below 2^24 for every row that fits the shared memory
+      int m = x - int(float(x) * inv) * W;
+      m += m < 0 ? W : m >= W ? -W : 0;
+      tw[r * pad + k] = base[m];
+    }
+  __syncthreads();
+}
+// (row, column) of the items i = threadIdx.x, + blockDim.x, .. of a table with `cols` columns, without a division per item
+struct ItemWalk {
+  int row, col, drow, dcol, cols;
+  __device__ __forceinline__ explicit ItemWalk(int c) : row(threadIdx.x / c), col(threadIdx.x % c), drow(blockDim.x / c), dcol(blockDim.x % c), cols(c) {}
+  __device__ __forceinline__ void next() {
+    row += drow; col += dcol;
+    if (col >= cols) { col -= cols; ++row; }
+  }
+};
+
 __global__ void __launch_bounds__(512)
 afno_rows_r2c_v2_kernel(TokenPtrs tok, float2* __restrict__ Y, AfGeom g, int kweight, PeerArgs peer, int wait, int* err, int groups,
                         int passes) {
@@ -207,20 +240,15 @@ afno_rows_r2c_v2_kernel(TokenPtrs tok, float2* __restrict__ Y, AfGeom g, int kwe
   float* x0 = xo + (size_t)nfold * g.Cb;             // [Cb]   sample w = 0
   float* xh = x0 + g.Cb;                             // [Cb]   sample w = W/2
   float2* tw2 = reinterpret_cast<float2*>(xh + g.Cb);   // [nfold][pad]: (cos, sin)(2 pi ((k w) mod W) / W), w = row + 1
-  const int row = blockIdx.x, j = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  const int row = blockIdx.x, j = blockIdx.y, tid = threadIdx.x;
   bool ok = true;
   if (wait) ok = peer_small_wait(peer, peer_epoch(peer), err, &sh_ok);
-  for (int i = tid; i < nfold * pad; i += nt) {
-    const int w = i / pad + 1, k = i % pad;
-    float sn, cs;
-    sincospif(2.f * ((k * w) % g.W) / g.W, &sn, &cs);
-    tw2[i] = make_float2(cs, sn);
-  }
+  row_twiddles(tw2, reinterpret_cast<float2*>(xe), nfold, 1, pad, g.W);   // the row comes to where the W values were
   const int c0 = (g.blk0 + j) * g.Cb;
   const int vec = g.Cb >> 3;
   const float nanv = __int_as_float(0x7fc00000);
-  for (int i = tid; i < (Wh + 1) * vec; i += nt) {
-    const int w = i / vec, v = i % vec;
+  for (ItemWalk it(vec); it.row <= Wh; it.next()) {
+    const int w = it.row, v = it.col;
     float f[8], h[8];
     const bool pair = w > 0 && w < Wh;
     if (ok) {
@@ -290,20 +318,26 @@ afno_rows_c2r_v2_kernel(const float2* __restrict__ X, TokenPtrs tok, AfGeom g, i
   float2* xs = reinterpret_cast<float2*>(sm);                     // [KX][Cb] spectrum, weighted
   float2* twT = xs + (size_t)g.KX * g.Cb;                         // [KX][pad]
   __nv_bfloat16* ys = reinterpret_cast<__nv_bfloat16*>(twT + (size_t)g.KX * pad);   // [W][Cb]
-  const int row = blockIdx.x, j = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
+  const int row = blockIdx.x, j = blockIdx.y, tid = threadIdx.x;
   const int ldx = g.nblk * g.Cb;
-  for (int i = tid; i < g.KX * pad; i += nt) {
-    const int kx = i / pad, w = i % pad;
-    float sn, cs;
-    sincospif(2.f * ((kx * w) % g.W) / g.W, &sn, &cs);
-    twT[i] = make_float2(cs, sn);
+  {
+    ItemWalk it(CP);
+    while (it.row < g.KX) {                      // two channels at a time, four loads in flight
+      float4 v[4];
+      int at[4];
+      float s[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k, it.next()) {
+        at[k] = it.row < g.KX ? it.row * CP + it.col : -1;
+        s[k] = (kweight && it.row > 0) ? 2.f : 1.f;
+        if (at[k] >= 0) v[k] = *reinterpret_cast<const float4*>(X + ((size_t)row * g.KX + it.row) * ldx + j * g.Cb + 2 * it.col);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (at[k] >= 0) reinterpret_cast<float4*>(xs)[at[k]] = make_float4(v[k].x * s[k], v[k].y * s[k], v[k].z * s[k], v[k].w * s[k]);
+    }
   }
-  for (int i = tid; i < g.KX * g.Cb; i += nt) {
-    const int kx = i / g.Cb, c = i % g.Cb;
-    const float2 v = X[((size_t)row * g.KX + kx) * ldx + j * g.Cb + c];
-    const float s = (kweight && kx > 0) ? 2.f : 1.f;
-    xs[i] = make_float2(v.x * s, v.y * s);
-  }
+  row_twiddles(twT, reinterpret_cast<float2*>(ys), g.KX, 0, pad, g.W);
   __syncthreads();
   const int cp = tid % CP, wg = tid / CP;
   if (wg < groups) {
@@ -341,8 +375,8 @@ afno_rows_c2r_v2_kernel(const float2* __restrict__ X, TokenPtrs tok, AfGeom g, i
   __syncthreads();
   const int c0 = (g.blk0 + j) * g.Cb;
   const int vec = g.Cb >> 3;
-  for (int i = tid; i < g.W * vec; i += nt) {
-    const int w = i / vec, v = i % vec;
+  for (ItemWalk it(vec); it.row < g.W; it.next()) {
+    const int w = it.row, v = it.col;
     uint4 u = *reinterpret_cast<const uint4*>(ys + w * g.Cb + v * 8);
     if (add0) {
       // residual terms of the surrounding block (local [T, C] token layout), summed in fp32 and rounded once
