@@ -266,9 +266,8 @@ __device__ __forceinline__ void cl_channel_sums(const CLThread& t, const float* 
 }
 constexpr size_t cl_stats_smem(int V, int C) { return (2 * 256 * (size_t)V + 2 * (size_t)C) * sizeof(float); }
 
-// Pixels whose loads are issued together.  Forward and backward of 512 x 512 bf16 pixels with one, two, three, four pixels ahead: 256
-// channels 113, 113, 103, 105 and 276, 229, 188, 190 us, 128 channels 72, 71, 65, 65 and 169, 141, 116, 117 us; fp32 (half as many
-// channels a thread, 128 channels, 256 x 256) 37, 37, 40, 41 and 54, 53, 52, 62 us.
+// Pixels whose loads the forward issues together: 512 x 512 bf16 pixels with one, two, three, four pixels, 256 channels 113, 113, 103, 105 us,
+// 128 channels 72, 71, 65, 65 us; fp32 (half as many channels a thread, 128 channels, 256 x 256) 37, 37, 40, 41 us.
 template <typename T>
 constexpr int kClAhead = sizeof(T) == 2 ? 3 : 2;
 // the vectors of pixels pix, pix + ppi, .., zeros past the end of the slice
@@ -518,6 +517,31 @@ struct CLBwd {
   }
 };
 
+// f(pixel, vector of x, vector of dy) for every pixel of the thread; the next pixel's loads are under way meanwhile.  (Two or three pixels at a
+// time, with or without the next ones under way, need 80 to 128 registers and leave too few warps: 256 / 128 channels of 512 x 512 pixels,
+// 2 x 256 x 128 x 128, 183 / 112 / 48 us as here, 207 / 128 / 54 and 179 / 111 / 56 us so, 213 / 128 / 57 three at a time without.)
+template <typename T, typename F>
+__device__ __forceinline__ void cl_bwd_pixels(const T* x, const T* dy, const CLThread& t, int C, F&& f) {
+  uint4 rx[2], ry[2];
+  auto load = [&](long long q, int h) {
+    if (q < t.p1) {
+      rx[h] = *reinterpret_cast<const uint4*>(x + q * C);
+      ry[h] = *reinterpret_cast<const uint4*>(dy + q * C);
+    }
+  };
+  long long pix = t.p0 + t.lane_pix;
+  load(pix, 0);
+  while (pix < t.p1) {
+    load(pix + t.ppi, 1);
+    f(pix, rx[0], ry[0]);
+    pix += t.ppi;
+    if (pix >= t.p1) break;
+    load(pix + t.ppi, 0);
+    f(pix, rx[1], ry[1]);
+    pix += t.ppi;
+  }
+}
+
 template <typename T, bool kSilu, int MU>
 __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, const T* __restrict__ dy,
                                                         const float* __restrict__ gamma, const float* __restrict__ beta,
@@ -536,22 +560,16 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
 #pragma unroll
     for (int i = 0; i < V; ++i) a[i] = d[i] = 0.f;
     const long long off = (long long)b * sh.HW * sh.C + t.c0;
-    for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
-      uint4 rx[kClAhead<T>], ry[kClAhead<T>];
-      cl_load_ahead(x + off, t, pix, sh.C, rx);
-      cl_load_ahead(dy + off, t, pix, sh.C, ry);         // a zero dy adds nothing
+    cl_bwd_pixels<T>(x + off, dy + off, t, sh.C, [&](long long, const uint4& rx, const uint4& ry) {
+      float f[V], e[V];
+      Vec<T>::load(reinterpret_cast<const T*>(&rx), f);
+      Vec<T>::load(reinterpret_cast<const T*>(&ry), e);
 #pragma unroll
-      for (int k = 0; k < kClAhead<T>; ++k) {
-        float f[V], e[V];
-        Vec<T>::load(reinterpret_cast<const T*>(&rx[k]), f);
-        Vec<T>::load(reinterpret_cast<const T*>(&ry[k]), e);
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
-          a[i] += dz * xr; d[i] += dz;
-        }
+      for (int i = 0; i < V; ++i) {
+        const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
+        a[i] += dz * xr; d[i] += dz;
       }
-    }
+    });
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       atomicAdd(&smem[2 * (t.c0 + i)], w.kCentred ? a[i] * w.rs[i * MU / V] : a[i]);
@@ -597,25 +615,18 @@ __global__ void __launch_bounds__(256) gn_bwd_apply_cl(const T* __restrict__ x, 
     Bq[i * MU / V] = w.kCentred ? rs * (rs * (ab.y * inv_n)) : ab.y * inv_n;
   }
   const long long off = (long long)b * sh.HW * sh.C + t.c0;
-  for (long long pix = t.p0 + t.lane_pix; pix < t.p1; pix += kClAhead<T> * t.ppi) {
-    uint4 rx[kClAhead<T>], ry[kClAhead<T>];
-    cl_load_ahead(x + off, t, pix, sh.C, rx);
-    cl_load_ahead(dy + off, t, pix, sh.C, ry);
+  cl_bwd_pixels<T>(x + off, dy + off, t, sh.C, [&](long long pix, const uint4& rx, const uint4& ry) {
+    float f[V], e[V];
+    Vec<T>::load(reinterpret_cast<const T*>(&rx), f);
+    Vec<T>::load(reinterpret_cast<const T*>(&ry), e);
 #pragma unroll
-    for (int k = 0; k < kClAhead<T>; ++k) {
-      float f[V], e[V];
-      Vec<T>::load(reinterpret_cast<const T*>(&rx[k]), f);
-      Vec<T>::load(reinterpret_cast<const T*>(&ry[k]), e);
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
-        const float g = w.ga[i] * dz - A[i * MU / V] - xr * Bq[i * MU / V];
-        f[i] = w.kCentred ? g : w.rs[i * MU / V] * g;
-      }
-      const long long q = pix + k * t.ppi;
-      if (q < t.p1) Vec<T>::store(dx + off + q * sh.C, f);
+    for (int i = 0; i < V; ++i) {
+      const float xr = w.row(f[i], i), dz = w.template dz<kSilu>(xr, e[i], i);
+      const float g = w.ga[i] * dz - A[i * MU / V] - xr * Bq[i * MU / V];
+      f[i] = w.kCentred ? g : w.rs[i * MU / V] * g;
     }
-  }
+    Vec<T>::store(dx + off + pix * sh.C, f);
+  });
 }
 
 // per batch item: channel sums over slices, group sums A = sum gamma * dbeta_c, B = sum gamma * dgamma_c, and the
