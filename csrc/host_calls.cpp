@@ -1,8 +1,10 @@
 // Host side of the hottest calls as a CPython extension: checks of the operands, allocation of the results and the launch.
 //
 // A small call (a roll-out step of a mesh network, a block on a few thousand points) is bound by its host side: in Python one launch
-// took 15 to 25 us (attributes of every tensor, torch.empty, the foreign-function call with up to 40 arguments).  The
-// functions do what the Python code did, argument by argument; gradients, dispatch and weight copies stay in Python.
+// took 15 to 50 us (attributes of every tensor, torch.empty, the foreign-function call with up to 40 arguments).  The
+// functions do what the Python code did, argument by argument; gradients, dispatch and weight copies stay in Python.  Together with calls
+// that skip the autograd function where no gradient is wanted: a message-passing step of 1 885 nodes (three launches) 151 -> 77 us, a Transolver
+// block of 4 096 points (eleven) 372 -> 227 us, an AFNO block (twelve) 314 -> 227 us, a U-Net block with attention 613 -> 416 us.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
