@@ -33,10 +33,6 @@ def _lib_conv():
     lib = _lib.load(required=True)
     if not getattr(lib, "_conv_declared", False):
         vp, i, u, d = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint, ctypes.c_double
-        lib.pnm_conv2d_nhwc.argtypes = [vp, vp, vp, i, i, i, i, i, i, vp, i, i, i, vp]
-        lib.pnm_conv2d_nhwc.restype = i
-        lib.pnm_conv_pack_weight.argtypes = [vp, i, vp, i, i, i, i, i, i, vp]
-        lib.pnm_conv_pack_weight.restype = i
         lib.pnm_conv2d_wgrad_nhwc.argtypes = [vp, vp, vp, vp, i, i, i, i, i, vp, vp, vp, vp, u, d, i, vp]
         lib.pnm_conv2d_wgrad_nhwc.restype = i
         lib._conv_declared = True

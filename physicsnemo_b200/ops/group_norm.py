@@ -25,9 +25,8 @@ def _lib_gn():
         vp, i, ll, f = c.c_void_p, c.c_int, c.c_longlong, c.c_float
         lib.pnm_groupnorm_scratch_floats.argtypes = [i, i, i, i]
         lib.pnm_groupnorm_scratch_floats.restype = ll
-        lib.pnm_groupnorm_fwd.argtypes = [vp] * 7 + [i, i, ll, i, i, i, i, i, f, vp]
         lib.pnm_groupnorm_bwd.argtypes = [vp] * 10 + [i, i, ll, i, i, i, i, i, vp]
-        lib.pnm_groupnorm_fwd.restype = lib.pnm_groupnorm_bwd.restype = i
+        lib.pnm_groupnorm_bwd.restype = i
         u, d = c.c_uint, c.c_double
         peer = [vp, i, i, u, ll, d, vp, vp, vp]   # bases, rank, world, epoch, capacity, budget_s, epoch_base, counter, stream
         lib.pnm_groupnorm_fwd_sharded.argtypes = [vp] * 7 + [i, i, ll, ll, i, i, i, i, f] + peer

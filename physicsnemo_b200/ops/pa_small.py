@@ -17,11 +17,10 @@ def _lib_pa():
     if not getattr(lib, "_pasmall_declared", False):
         c = ctypes
         vp, i, u, ll, f, d = c.c_void_p, c.c_int, c.c_uint, c.c_longlong, c.c_float, c.c_double
-        lib.pnm_pa_prepare_fwd.argtypes = [vp] * 11 + [i, i, i, vp]
         lib.pnm_pa_tokens_fwd.argtypes = [vp, i, i, ll, i, vp, vp, vp, vp, i, i, i, f, vp, i, u, ll, d, vp, vp]
         lib.pnm_pa_tokens_bwd.argtypes = [vp, i, i, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, vp, i, u, ll, d, vp, vp]
         lib.pnm_pa_prepare_bwd.argtypes = [vp] * 12 + [i, i, i, vp]
-        for n in ("pnm_pa_prepare_fwd", "pnm_pa_tokens_fwd", "pnm_pa_tokens_bwd", "pnm_pa_prepare_bwd"):
+        for n in ("pnm_pa_tokens_fwd", "pnm_pa_tokens_bwd", "pnm_pa_prepare_bwd"):
             getattr(lib, n).restype = i
         lib._pasmall_declared = True
     return lib
