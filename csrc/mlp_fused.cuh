@@ -17,7 +17,8 @@
 //   * the same two threads normalise the row (mean and squared deviations of each half, merged through two TMEM columns) and add `post`;
 // * * rows pass through TMEM on their way to and from global memory, so that an access covers eight lines and not 32 rows (tmem_ld_rows):
 //     with a row per thread the unit that handles lines was busy 4 000 cycles of a tile, and 10 000 where rows are kept.  Kept
-//     activations are read from the A operand itself: W2 and W3 are put in its column order once.
+//     activations go through the accumulator's columns that their thread has just read, before the next product overwrites them: the
+//     A operand keeps the order of the columns, so that every product adds its terms in the order of the plain matrix products.
 // * Three row tiles of 128 are in flight: one per group of eight epilogue warps, and a third accumulator takes the next tile's first
 // product, so that neither its source rows nor its product are waited for (both took 13 000 of a tile's 26 000 cycles).
 // The products are issued by two threads: an issue costs about 75 cycles, and the operands of one thread for all did not fit its registers.
@@ -100,21 +101,6 @@ __device__ __forceinline__ void tmem_ld32_turned(uint32_t taddr, uint32_t* w) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) w[8 * ((i >> 1) & 3) + 2 * (i >> 3) + (i & 1)] = __float_as_uint(r[i]);
 }
-// The same turn on a weight matrix: 8-byte pieces 4 a + b and 4 b + a of a row of 64 columns (K) change places, in the swizzled tile.
-__device__ __forceinline__ void turn_weight_row(uint8_t* chunk, int r) {
-  uint8_t* row = chunk + r * 128;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = a + 1; b < 4; ++b) {
-      const int x = 4 * a + b, y = 4 * b + a;
-      uint2* p = reinterpret_cast<uint2*>(row + (((x >> 1) ^ (r & 7)) << 4) + (x & 1) * 8);
-      uint2* q = reinterpret_cast<uint2*>(row + (((y >> 1) ^ (r & 7)) << 4) + (y & 1) * 8);
-      const uint2 t = *p;
-      *p = *q;
-      *q = t;
-    }
-}
 // 16 rows from lane `taddr` on, 32 columns: a = row t / 4, b = row t / 4 + 8
 __device__ __forceinline__ void tmem_ld_rows(uint32_t taddr, uint32_t* a, uint32_t* b) {
   asm volatile(
@@ -131,12 +117,16 @@ __device__ __forceinline__ void tmem_st_rows(uint32_t taddr, const uint32_t* a, 
       "r"(a[6]), "r"(a[7]), "r"(b[6]), "r"(b[7])
       : "memory");
 }
-// 32 turned words of each of the warp's rows from row0 on -> global memory (row stride ld, in elements), rows past M left out
-__device__ __forceinline__ void store_turned(uint32_t taddr, __nv_bfloat16* dst, long long ld, long long row0, long long M, int lane) {
-  uint32_t v[4][8];
+// Registers of a warp -> the vectors of the turn, and those of the rows from row0 on -> global memory (row stride ld, in elements), rows
+// past M left out
+__device__ __forceinline__ void turn_rows(uint32_t taddr, const uint32_t* w, uint32_t (*v)[8]) {
+  tmem_st32_turned(taddr, w);
+  tmem_st_wait();
   tmem_ld_rows(taddr, v[0], v[1]);
   tmem_ld_rows(taddr + (16u << 16), v[2], v[3]);
   tmem_ld_wait();
+}
+__device__ __forceinline__ void store_turned(const uint32_t (*v)[8], __nv_bfloat16* dst, long long ld, long long row0, long long M, int lane) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const long long r = row0 + 8 * i + (lane >> 2);
@@ -145,14 +135,19 @@ __device__ __forceinline__ void store_turned(uint32_t taddr, __nv_bfloat16* dst,
 }
 __device__ __forceinline__ void store_rows(uint32_t taddr, const uint32_t* w, __nv_bfloat16* dst, long long ld, long long row0, long long M,
                                            int lane) {
-  tmem_st32_turned(taddr, w);
-  tmem_st_wait();
-  store_turned(taddr, dst, ld, row0, M, lane);
+  uint32_t v[4][8];
+  turn_rows(taddr, w, v);
+  store_turned(v, dst, ld, row0, M, lane);
 }
-__device__ __forceinline__ void tmem_st_pair(uint32_t taddr, uint32_t a, uint32_t b) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
+// 8 registers of bf16 pairs -> 32 lanes x 8 columns
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
-__device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b) { tmem_st_pair(taddr, __float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)) : "memory");
+}
 __device__ __forceinline__ float2 tmem_ld2(uint32_t taddr) {
   uint32_t a, b;
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(taddr) : "memory");
@@ -214,8 +209,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
   uint64_t* full = reinterpret_cast<uint64_t*>(vec + 5 * kMlpW);
   uint64_t* empty = full + Cfg::STAGES;
   uint64_t* wfull = empty + Cfg::STAGES;
-  uint64_t* turned = wfull + 1;                  // W2 and W3 are in the column order of the A operand
-  uint64_t* first = turned + 1;                  // [3] an accumulator holds a finished first product
+  uint64_t* first = wfull + 1;                   // [3] an accumulator holds a finished first product
   uint64_t* accfree = first + 3;                 // [3] its tile is finished
   uint64_t* accfull = accfree + 3;               // [2] the group's second or third product is finished
   uint64_t* aready = accfull + 2;                // [2] the accumulator was read, the packed A operand is in place
@@ -230,7 +224,6 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full[s], kMlpProducers); mbar_init(&empty[s], 1); }
     mbar_init(wfull, 1);
-    mbar_init(turned, 16);
     for (int i = 0; i < 3; ++i) { mbar_init(&first[i], 1); mbar_init(&accfree[i], 8); }
     for (int i = 0; i < 2; ++i) { mbar_init(&accfull[i], 1); mbar_init(&aready[i], 8); }
     *abort_flag = 0;
@@ -367,7 +360,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
         const uint32_t wlo = desc_lo(smem_u32(wts + KB * kMlpChunk));
         unsigned long long t0 = 0;
         uint32_t spins = 0;
-        bool ok = mbar_wait(turned, 0, abort_flag, g.err, ERR_WAIT_FULL);
+        bool ok = mbar_wait(wfull, 0, abort_flag, g.err, ERR_WAIT_FULL);
         while (ok && left) {
           bool any = false;
 #pragma unroll
@@ -407,12 +400,6 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
     const uint32_t base = tmem + (uint32_t(q * 32) << 16);
     // the moments of a half row lie in its own part of the A operand, whose last reader is the third product
     const uint32_t aop = base + 3 * kMlpW + grp * 64 + half * 32, other_aop = base + 3 * kMlpW + grp * 64 + (half ^ 1) * 32;
-    // one of 512 rows of 64 columns of W2 and W3 each (also where nothing is kept: the order of the sums is the same then)
-    const int t = threadIdx.x - 32 * kMlpHelpers;
-    if (mbar_wait(wfull, 0, abort_flag, g.err, ERR_WAIT_FULL)) turn_weight_row(wts + (KB + (t >> 7)) * kMlpChunk, t & 127);
-    fence_async_smem();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(turned);
     uint32_t n = 0, uses = 0, a = 0, turn = 0;   // n = 3 turn + a
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++n, turn += a == 2, a = a == 2 ? 0 : a + 1) {
       if ((n & 1) != uint32_t(grp)) continue;
@@ -429,6 +416,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
         uses += layer;
         tc_fence_after();
+        uint32_t act[32];
         float v[2][16];                          // two steps of 16 columns: one is read from TMEM while the other is worked on
         tmem_ld16(acc, v[0]);
 #pragma unroll
@@ -444,17 +432,18 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
             stg32(z + c * kZStep, p);            // rows past M too: the buffer holds whole tiles
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j)            // words 8 c + 2 j, 8 c + 2 j + 1 in their turned place
-            tmem_st_pair(aop + 8 * j + 2 * c, pack_bf16x2(mlp_act<ACT>(x[4 * j]), mlp_act<ACT>(x[4 * j + 1])),
-                         pack_bf16x2(mlp_act<ACT>(x[4 * j + 2]), mlp_act<ACT>(x[4 * j + 3])));
+          for (int j = 0; j < 8; ++j) act[8 * c + j] = pack_bf16x2(mlp_act<ACT>(x[2 * j]), mlp_act<ACT>(x[2 * j + 1]));
+          tmem_st8(aop + 8 * c, act + 8 * c);
         }
-        tmem_st_wait();
+        // The weight gradient's operand is this product's: recomputed from the rounded pre-activation it would be rounded twice (dW2
+        // against 64 bits 0.0054 instead of 0.0049).  Stored while the product runs.
+        uint32_t rows[4][8];
+        if (SAVE) turn_rows(acc, act, rows);
+        else tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&aready[grp]);
-        // The weight gradient's operand is this product's: recomputed from the rounded pre-activation it would be rounded twice (dW2
-        // against 64 bits 0.0054 instead of 0.0049).  Read back and stored while the product runs.
-        if (SAVE) store_turned(aop, h, kMlpW, row0, g.M, lane);
+        if (SAVE) store_turned(rows, h, kMlpW, row0, g.M, lane);
       }
       Vec32 res[4] = {};
       auto load_post = [&]() {

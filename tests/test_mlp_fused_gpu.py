@@ -311,3 +311,23 @@ def test_message_passing_step_against_64_bits(aggregation, checkpointed):
     for k, (a, b) in enumerate(zip(*results)):
         # outputs: four bf16 roundings; gradients: 0.8 % at this size with 128 entries in a bias
         assert _rel(a, b.double()) < (8e-3 if k < 2 else 0.02)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", [1, 2, 3])
+@pytest.mark.parametrize("rows", [77, 3 * 148 * 128 + 5])
+def test_mlp3_products_add_their_terms_in_the_order_of_the_plain_product(rows, act):
+    """Bit for bit what the layered products give from the same operands: no column of an operand changes its place in a sum."""
+    from physicsnemo_b200.ops import gemm as G
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    x = torch.randn(rows, W, device="cuda").bfloat16()
+    w = [(torch.randn(W, W, device="cuda") / W ** 0.5).bfloat16() for _ in range(3)]
+    b = [0.1 * torch.randn(W, device="cuda") for _ in range(3)]
+    gamma, beta = 1 + 0.1 * torch.randn(W, device="cuda"), 0.1 * torch.randn(W, device="cuda")
+    y, (h1, h2, x3, *_) = mf._forward([x], [None], w, b, act, gamma, beta, 1e-5, None, True)
+    assert torch.equal(h1, G.gemm_tn(x, w[0], bias=b[0], act=act))
+    assert torch.equal(h2, G.gemm_tn(h1, w[1], bias=b[1], act=act))
+    assert torch.equal(x3, G.gemm_tn(h2, w[2], bias=b[2]))
+    plain, _ = mf._forward([x], [None], w, b, act, gamma, beta, 1e-5, None, False)
+    assert torch.equal(y, plain)
