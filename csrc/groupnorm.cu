@@ -215,9 +215,12 @@ __device__ __forceinline__ CLThread cl_thread(const GNShape& sh, int s) {
   return t;
 }
 
-// One counter per batch item (zero between launches: the CTA that folds resets it).  Forward and backward keep apart.
-__device__ unsigned int g_gn_fwd_counter[65536];
-__device__ unsigned int g_gn_bwd_counter[65536];
+// One counter per batch item, in the call's own scratch behind the folded sums: calls on other streams have theirs.  Zeroed on the
+// call's stream before the statistics kernel.
+static unsigned int* cl_counters(float2* folded, const GNShape& sh) { return reinterpret_cast<unsigned int*>(folded + (long long)sh.B * sh.G); }
+static cudaError_t cl_zero_counters(float2* folded, const GNShape& sh, cudaStream_t st) {
+  return cudaMemsetAsync(cl_counters(folded, sh), 0, sh.B * sizeof(unsigned int), st);
+}
 
 // Called by every CTA of the (S, B) grid after it wrote its group partials part[b][s][0..G): the CTA that arrives last at
 // the batch item's counter sums part[b][0..S)[g] in a fixed order (one warp per group, lanes over slices, shuffle tree)
@@ -243,7 +246,6 @@ __device__ __forceinline__ void cl_fold_slices(const float2* part, float2* out, 
     for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); q += __shfl_xor_sync(0xffffffffu, q, o); }
     if (lane == 0) out[b * sh.G + g] = make_float2(a, q);
   }
-  if (threadIdx.x == 0) counter[b] = 0;
 }
 
 // Sums a[i], q[i] over the threads that share a channel, into sums[c] = (sum a, sum q): the values of all threads are laid out in
@@ -284,7 +286,7 @@ __device__ __forceinline__ void cl_load_ahead(const T* x, const CLThread& t, lon
 // part[b][s][g] = (sum x, sum x^2) of slice s; gsum[b][g] = their sum over the slices (written by the last CTA of item b)
 template <typename T>
 __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, float2* __restrict__ part, float2* __restrict__ gsum,
-                                                    GNShape sh) {
+                                                    unsigned int* __restrict__ counter, GNShape sh) {
   constexpr int V = Vec<T>::N;
   extern __shared__ float smem[];                        // staging of cl_channel_sums, then [C] sums
   const int s = blockIdx.x, b = blockIdx.y;
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(256) gn_stats_cl(const T* __restrict__ x, floa
     for (int k = 0; k < sh.cpg; ++k) { a2 += sums[g * sh.cpg + k].x; q2 += sums[g * sh.cpg + k].y; }
     part[((long long)b * sh.S + s) * sh.G + g] = make_float2(a2, q2);
   }
-  cl_fold_slices(part, gsum, g_gn_fwd_counter, sh, b);
+  cl_fold_slices(part, gsum, counter, sh, b);
 }
 
 // fills smem mom[g] = (mean, rstd) for all groups of batch item b from the folded sums
@@ -547,7 +549,8 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
                                                         const float* __restrict__ gamma, const float* __restrict__ beta,
                                                         const float* __restrict__ mean, const float* __restrict__ rstd,
                                                         float2* __restrict__ part, float2* __restrict__ group_ab,
-                                                        float* __restrict__ dgamma, float* __restrict__ dbeta, GNShape sh) {
+                                                        float* __restrict__ dgamma, float* __restrict__ dbeta,
+                                                        unsigned int* __restrict__ counter, GNShape sh) {
   constexpr int V = Vec<T>::N;
   extern __shared__ float smem[];                        // [C][2]
   const int s = blockIdx.x, b = blockIdx.y;
@@ -592,7 +595,7 @@ __global__ void __launch_bounds__(256) gn_bwd_stats_cl(const T* __restrict__ x, 
     }
     part[((long long)b * sh.S + s) * sh.G + g] = make_float2(A, Bq);
   }
-  cl_fold_slices(part, group_ab, g_gn_bwd_counter, sh, b);
+  cl_fold_slices(part, group_ab, counter, sh, b);
 }
 
 template <typename T, bool kSilu, int MU>
@@ -665,7 +668,8 @@ int gn_forward(const void* x, const float* gamma, const float* beta, void* y, fl
   } else {
     const dim3 grid(sh.S, sh.B);
     float2* gsum = partial + (long long)sh.B * sh.S * sh.G;
-    gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, sh);
+    if (const cudaError_t e = cl_zero_counters(gsum, sh, st)) return (int)e;
+    gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, cl_counters(gsum, sh), sh);
     if (act) gn_apply_cl<T, true><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gsum, gamma, beta, yo, mean, rstd, sh, eps);
     else gn_apply_cl<T, false><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gsum, gamma, beta, yo, mean, rstd, sh, eps);
   }
@@ -675,8 +679,8 @@ int gn_forward(const void* x, const float* gamma, const float* beta, void* y, fl
 template <typename T, int MU>
 void launch_bwd_stats_cl(dim3 grid, size_t sm, cudaStream_t st, int act, const T* x, const T* dy, const float* gamma, const float* beta,
                          const float* mean, const float* rstd, float2* pc, float2* ab, float* dgamma, float* dbeta, const GNShape& sh) {
-  if (act) gn_bwd_stats_cl<T, true, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
-  else gn_bwd_stats_cl<T, false, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
+  if (act) gn_bwd_stats_cl<T, true, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, cl_counters(ab, sh), sh);
+  else gn_bwd_stats_cl<T, false, MU><<<grid, 256, sm, st>>>(x, dy, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, cl_counters(ab, sh), sh);
 }
 template <typename T, int MU>
 void launch_bwd_apply_cl(dim3 grid, cudaStream_t st, int act, const T* x, const T* dy, const float* gamma, const float* beta, const float* mean,
@@ -702,6 +706,7 @@ int gn_backward(const void* x, const void* dy, const float* gamma, const float* 
     else gn_bwd_stats_cf<T, false><<<grid, 256, 0, st>>>(xi, di, gamma, beta, mean, rstd, pc, sh);
     gn_bwd_reduce<<<sh.B, 256, 2 * sh.G * sizeof(float), st>>>(pc, gamma, ab, dgamma, dbeta, sh);
   } else {
+    if (const cudaError_t e = cl_zero_counters(ab, sh, st)) return (int)e;
     if (cl_half_groups<T>(sh)) launch_bwd_stats_cl<T, 2>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
     else launch_bwd_stats_cl<T, Vec<T>::N>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
   }
@@ -724,7 +729,8 @@ int gn_forward_sh(const void* x, const float* gamma, const float* beta, void* y,
   T* yo = static_cast<T*>(y);
   const dim3 grid(sh.S, sh.B);
   float2* gsum = partial + (long long)sh.B * sh.S * sh.G;
-  gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, sh);
+  if (const cudaError_t e = cl_zero_counters(gsum, sh, st)) return (int)e;
+  gn_stats_cl<T><<<grid, 256, cl_stats_smem(Vec<T>::N, sh.C), st>>>(xi, partial, gsum, cl_counters(gsum, sh), sh);
   gn_publish_moments<<<sh.B, 256, 0, st>>>(gsum, sh, peer, counter);
   if (act) gn_apply_cl_sh<T, true><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gamma, beta, yo, mean, rstd, sh, eps, count_global, peer, err);
   else gn_apply_cl_sh<T, false><<<grid, 256, sh.G * sizeof(float2), st>>>(xi, gamma, beta, yo, mean, rstd, sh, eps, count_global, peer, err);
@@ -742,6 +748,7 @@ int gn_backward_sh(const void* x, const void* dy, const float* gamma, const floa
   T* o = static_cast<T*>(dx);
   const dim3 grid(sh.S, sh.B);
   const size_t sm = 2 * sh.C * sizeof(float);
+  if (const cudaError_t e = cl_zero_counters(ab, sh, st)) return (int)e;
   if (cl_half_groups<T>(sh)) launch_bwd_stats_cl<T, 2>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
   else launch_bwd_stats_cl<T, Vec<T>::N>(grid, sm, st, act, xi, di, gamma, beta, mean, rstd, pc, ab, dgamma, dbeta, sh);
   gn_publish_ab<<<sh.B, 256, 0, st>>>(ab, sh, peer, counter);
@@ -761,8 +768,8 @@ static bool gn_supported(const GNShape& sh, int layout, int dtype) {
 
 extern "C" {
 
-// floats of scratch needed by forward / backward for a given slice count
-long long pnm_groupnorm_scratch_floats(int B, int C, int G, int S) { return 2LL * B * S * C + 2LL * B * G; }
+// floats of scratch needed by forward / backward for a given slice count: partials, folded sums, counters
+long long pnm_groupnorm_scratch_floats(int B, int C, int G, int S) { return 2LL * B * S * C + 2LL * B * G + B; }
 
 // dtype: 0 bf16, 1 fp32.  layout: 0 channels-first, 1 channels-last.  act: 0 none, 1 SiLU.  Returns -1 if the shape is
 // outside what the kernels cover (the caller then uses another path), else the CUDA error code.

@@ -73,3 +73,45 @@ def test_group_norm_channels_last_edges(batch, channels, side, groups, dtype):
     tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-6       # one rounding of the result (2^-9), or sums of a few thousand fp32 terms
     for a, b in ((out, y), *((d.grad, r.grad) for d, r in zip(dev, ref))):
         assert float((a.detach().cpu().double() - b.detach()).norm() / b.detach().norm()) < tol
+
+
+@pytest.mark.skipif(not _lib._HOST_PATH.exists(), reason="the kernel library is not built")
+@pytest.mark.parametrize("batch,channels,groups,slices", [(1, 8, 1, 1), (3, 96, 32, 7), (2, 256, 256, 600)])
+def test_group_norm_scratch_holds_the_counters_of_the_call(batch, channels, groups, slices):
+    from physicsnemo_b200.ops import group_norm as gn
+
+    # partials of every slice, folded sums, one counter per batch item (the last also where a group has a single channel)
+    assert gn._lib_gn().pnm_groupnorm_scratch_floats(batch, channels, groups, slices) >= 2 * batch * slices * groups + 2 * batch * groups + batch
+
+
+@pytest.mark.gpu
+def test_group_norm_channels_last_on_two_streams():
+    """Calls of different slice counts side by side give what they give one after the other."""
+    from physicsnemo_b200.ops import group_norm as gn
+
+    shapes = [(2, 128, 96, 32), (2, 64, 40, 32)]             # batch, channels, side, groups
+    args = [(torch.randn(b, c, s, s, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last), g,
+             torch.randn(c, device="cuda"), torch.randn(c, device="cuda")) for b, c, s, g in shapes]
+    ups = [torch.randn_like(a[0]) for a in args]
+
+    def step(k):
+        x, g, ga, be = args[k]
+        leaves = [t.clone().requires_grad_() for t in (x, ga, be)]
+        y = gn.group_norm(leaves[0], g, *leaves[1:], 1e-5, silu=True)
+        return [y.detach(), *torch.autograd.grad(y, leaves, ups[k])]
+
+    serial = [step(k) for k in range(2)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    beside = [[], []]
+    for _ in range(60):
+        for k, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                beside[k].append(step(k))
+    torch.cuda.synchronize()
+    for want, runs in zip(serial, beside):
+        for got in runs:
+            assert torch.equal(got[0], want[0])              # moments are folded in a fixed order
+            # the backward adds a channel's pixels with fp32 atomics: a rounding of bf16 (2^-9) at most, parameter gradients in fp32
+            assert float((got[1].double() - want[1].double()).norm() / want[1].double().norm()) < 2.0 ** -9
+            assert all(float((a - b).norm() / b.norm()) < 1e-5 for a, b in zip(got[2:], want[2:]))
