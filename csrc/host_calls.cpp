@@ -50,13 +50,21 @@ void need_args(Py_ssize_t got, Py_ssize_t want) {
   if (got != want) throw torch::TypeError("expected " + std::to_string(want) + " arguments, got " + std::to_string(got));
 }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
-// the launch without the interpreter's lock, as a foreign-function call has it
+// without the interpreter's lock while it lives; an exception that leaves the scope has the lock again
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  Unlocked() = default;
+  Unlocked(const Unlocked&) = delete;
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// the launch without the lock, as a foreign-function call has it (the pointers that `f` reads may throw: a tensor without storage)
 template <typename F>
 void launch(const char* name, F&& f) {
   int code;
-  Py_BEGIN_ALLOW_THREADS
-  code = f();
-  Py_END_ALLOW_THREADS
+  {
+    const Unlocked unlocked;
+    code = f();
+  }
   if (code != 0) throw std::runtime_error(std::string(name) + " failed with code " + std::to_string(code));
 }
 uintptr_t address(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); }

@@ -53,6 +53,24 @@ def test_host_calls_refuse_bad_operands():
 
 
 @pytest.mark.gpu
+def test_host_calls_raise_for_tensors_without_storage():
+    """The pointer is read where the interpreter's lock is released: its error arrives as an exception all the same."""
+    host, idx = _lib.host(), torch.zeros(4, dtype=torch.int32, device="cuda")
+    raised = []
+
+    def inner(x):                                                        # x: a wrapper of vmap
+        for call in (lambda: host.gather_rows(x, idx, None, None), lambda: host.gemm_nt(x, x, False, None, None, 0),
+                     lambda: host.segment_sum(x, idx, idx, 3, False, False, None)):
+            with pytest.raises(RuntimeError, match="storage"):
+                call()
+            raised.append(call)
+        return x
+
+    torch.vmap(inner)(torch.randn(2, 3, 8, device="cuda").bfloat16())
+    assert len(raised) == 3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("batch,channels,side,groups,dtype", [(1, 128, 5, 32, torch.bfloat16),     # slices of fewer pixels than are loaded ahead
                                                              (2, 96, 33, 32, torch.bfloat16),     # three channels a group: values per channel
                                                              (1, 24, 7, 3, torch.bfloat16), (2, 64, 37, 32, torch.float32),
