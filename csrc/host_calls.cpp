@@ -5,12 +5,16 @@
 // functions do what the Python code did, argument by argument; gradients, dispatch and weight copies stay in Python.  Together with calls
 // that skip the autograd function where no gradient is wanted: a message-passing step of 1 885 nodes (three launches) 151 -> 77 us, a Transolver
 // block of 4 096 points (eleven) 372 -> 227 us, an AFNO block (twelve) 314 -> 227 us, a U-Net block with attention 613 -> 416 us.
+// As there, the interpreter's lock is released not only for the launch but also where memory is allocated or copied (an allocation may wait
+// for the device): every function reads its arguments, works in an `Unlocked` scope and wraps its results.
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
+
+#include <vector>
 
 #include "pnm_api.h"
 
@@ -41,10 +45,13 @@ bool truth(PyObject* o) {
   if (v < 0) throw python_error();
   return v != 0;
 }
+// what the Python code asserted
+struct Refused : torch::PyTorchError {
+  using PyTorchError::PyTorchError;
+  PyObject* python_type() override { return PyExc_AssertionError; }
+};
 void require(bool ok, const char* what) {
-  if (ok) return;
-  PyErr_SetString(PyExc_AssertionError, what);
-  throw python_error();
+  if (!ok) throw Refused(what);
 }
 void need_args(Py_ssize_t got, Py_ssize_t want) {
   if (got != want) throw torch::TypeError("expected " + std::to_string(want) + " arguments, got " + std::to_string(got));
@@ -57,14 +64,7 @@ struct Unlocked {
   Unlocked(const Unlocked&) = delete;
   ~Unlocked() { PyEval_RestoreThread(state); }
 };
-// the launch without the lock, as a foreign-function call has it (the pointers that `f` reads may throw: a tensor without storage)
-template <typename F>
-void launch(const char* name, F&& f) {
-  int code;
-  {
-    const Unlocked unlocked;
-    code = f();
-  }
+void check(const char* name, int code) {
   if (code != 0) throw std::runtime_error(std::string(name) + " failed with code " + std::to_string(code));
 }
 uintptr_t address(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); }
@@ -100,41 +100,42 @@ PyObject* tuple_of(std::initializer_list<const Tensor*> tensors) {
 PyObject* gemm_tn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 15);
-  const Tensor a = rowmajor2d(tensor(args[0])), b = rowmajor2d(tensor(args[1]));
-  const Tensor bias = optional(args[2]), scale = optional(args[3]);
-  Tensor aux = optional(args[5]), a2 = optional(args[7]), a3 = optional(args[8]), out = optional(args[10]);
-  const Tensor group_out = optional(args[11]);
-  const int64_t M = a.size(0), K1 = a.size(1), N = b.size(0), K = b.size(1);
-  int64_t K2 = K;
-  if (a2.defined()) {
-    a2 = rowmajor2d(a2);
-    K2 = K1 + a2.size(1);
-    if (a3.defined()) {
-      a3 = rowmajor2d(a3);
-      require(a3.size(0) == M && K2 + a3.size(1) == K, "the column blocks of A do not match B");
-    } else {
-      require(a2.size(0) == M && K2 == K, "the column blocks of A do not match B");
-    }
-  } else {
-    require(K1 == K, "A and B have different numbers of columns");
-  }
-  require(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "operands must be bf16");
-  if (!out.defined()) out = empty({M, N}, at::kBFloat16, a);
-  const Tensor z = truth(args[9]) ? empty({M, N}, at::kBFloat16, a) : Tensor();
-  if (aux.defined()) {
-    aux = rowmajor2d(aux);
-    require(aux.size(0) == M && aux.size(1) == N && aux.scalar_type() == at::kBFloat16, "the auxiliary operand must be bf16 [M, N]");
-  }
-  for (const Tensor* v : {&bias, &scale})
-    if (v->defined()) require(v->scalar_type() == at::kFloat && v->numel() == N && v->is_contiguous(), "vectors must be contiguous fp32 [N]");
+  Tensor a = tensor(args[0]), b = tensor(args[1]), aux = optional(args[5]), a2 = optional(args[7]), a3 = optional(args[8]), out = optional(args[10]), z;
+  const Tensor bias = optional(args[2]), scale = optional(args[3]), group_out = optional(args[11]);
   const int act = int(integer(args[4])), aux_mode = int(integer(args[6])), post = truth(args[12]), bn = int(integer(args[13])),
             cap = int(integer(args[14]));
-  auto ld = [](const Tensor& t) { return t.defined() ? int(t.stride(0)) : 0; };
-  void* st = stream();
-  launch("pnm_gemm_tn", [&] {
-    return pnm_gemm_tn(ptr(a), ld(a), ptr(a2), ld(a2), ptr(a3), ld(a3), ptr(b), ld(b), ptr(out), ld(out), ptr(z), ld(z), ptr(aux), ld(aux), int(M),
-                       int(N), int(K), int(K1), int(K2), fptr(bias), fptr(scale), fptr(group_out), act, aux_mode, post, bn, cap, st);
-  });
+  const bool want_z = truth(args[9]);
+  {
+    const Unlocked unlocked;
+    a = rowmajor2d(a); b = rowmajor2d(b);
+    const int64_t M = a.size(0), K1 = a.size(1), N = b.size(0), K = b.size(1);
+    int64_t K2 = K;
+    if (a2.defined()) {
+      a2 = rowmajor2d(a2);
+      K2 = K1 + a2.size(1);
+      if (a3.defined()) {
+        a3 = rowmajor2d(a3);
+        require(a3.size(0) == M && K2 + a3.size(1) == K, "the column blocks of A do not match B");
+      } else {
+        require(a2.size(0) == M && K2 == K, "the column blocks of A do not match B");
+      }
+    } else {
+      require(K1 == K, "A and B have different numbers of columns");
+    }
+    require(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "operands must be bf16");
+    if (!out.defined()) out = empty({M, N}, at::kBFloat16, a);
+    if (want_z) z = empty({M, N}, at::kBFloat16, a);
+    if (aux.defined()) {
+      aux = rowmajor2d(aux);
+      require(aux.size(0) == M && aux.size(1) == N && aux.scalar_type() == at::kBFloat16, "the auxiliary operand must be bf16 [M, N]");
+    }
+    for (const Tensor* v : {&bias, &scale})
+      if (v->defined()) require(v->scalar_type() == at::kFloat && v->numel() == N && v->is_contiguous(), "vectors must be contiguous fp32 [N]");
+    auto ld = [](const Tensor& t) { return t.defined() ? int(t.stride(0)) : 0; };
+    check("pnm_gemm_tn",
+          pnm_gemm_tn(ptr(a), ld(a), ptr(a2), ld(a2), ptr(a3), ld(a3), ptr(b), ld(b), ptr(out), ld(out), ptr(z), ld(z), ptr(aux), ld(aux), int(M),
+                      int(N), int(K), int(K1), int(K2), fptr(bias), fptr(scale), fptr(group_out), act, aux_mode, post, bn, cap, stream()));
+  }
   return z.defined() ? tuple_of({&out, &z}) : THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -143,19 +144,20 @@ PyObject* gemm_tn(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* gemm_nt(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 6);
-  const Tensor a = rowmajor2d(tensor(args[0])), b = rowmajor2d(tensor(args[1]));
-  Tensor out = optional(args[3]), sums = optional(args[4]);
-  const int64_t M = a.size(0), Na = a.size(1), Nb = b.size(1);
-  require(b.size(0) == M, "operands have different numbers of rows");
-  const auto f32 = at::TensorOptions().dtype(at::kFloat).device(a.device());
-  if (!out.defined()) out = at::zeros({Na, Nb}, f32);
-  if (!sums.defined() && truth(args[2])) sums = at::zeros({Na}, f32);
+  Tensor a = tensor(args[0]), b = tensor(args[1]), out = optional(args[3]), sums = optional(args[4]);
+  const bool want_sums = truth(args[2]);
   const int cap = int(integer(args[5]));
-  void* st = stream();
-  launch("pnm_gemm_nt", [&] {
-    return pnm_gemm_nt(ptr(a), int(a.stride(0)), ptr(b), int(b.stride(0)), fptr(out), int(out.stride(0)), fptr(sums), int(M), int(Na), int(Nb), cap,
-                       st);
-  });
+  {
+    const Unlocked unlocked;
+    a = rowmajor2d(a); b = rowmajor2d(b);
+    const int64_t M = a.size(0), Na = a.size(1), Nb = b.size(1);
+    require(b.size(0) == M, "operands have different numbers of rows");
+    const auto f32 = at::TensorOptions().dtype(at::kFloat).device(a.device());
+    if (!out.defined()) out = at::zeros({Na, Nb}, f32);
+    if (!sums.defined() && want_sums) sums = at::zeros({Na}, f32);
+    check("pnm_gemm_nt", pnm_gemm_nt(ptr(a), int(a.stride(0)), ptr(b), int(b.stride(0)), fptr(out), int(out.stride(0)), fptr(sums), int(M), int(Na),
+                                     int(Nb), cap, stream()));
+  }
   return sums.defined() ? tuple_of({&out, &sums}) : THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -166,13 +168,15 @@ PyObject* layernorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   need_args(n, 5);
   const Tensor x = tensor(args[0]), gamma = tensor(args[1]), beta = optional(args[2]), post = optional(args[4]);
   const float eps = float(real(args[3]));
-  require(x.dim() == 2, "expected a matrix");
-  const int64_t M = x.size(0), C = x.size(1);
-  const Tensor y = at::empty_like(x), mean = empty({M}, at::kFloat, x), rstd = empty({M}, at::kFloat, x);
-  void* st = stream();
-  launch("pnm_layernorm_fwd", [&] {
-    return pnm_layernorm_fwd(ptr(x), nullptr, fptr(gamma), fptr(beta), ptr(y), nullptr, fptr(mean), fptr(rstd), ptr(post), M, int(C), eps, st);
-  });
+  Tensor y, mean, rstd;
+  {
+    const Unlocked unlocked;
+    require(x.dim() == 2, "expected a matrix");
+    const int64_t M = x.size(0), C = x.size(1);
+    y = at::empty_like(x); mean = empty({M}, at::kFloat, x); rstd = empty({M}, at::kFloat, x);
+    check("pnm_layernorm_fwd", pnm_layernorm_fwd(ptr(x), nullptr, fptr(gamma), fptr(beta), ptr(y), nullptr, fptr(mean), fptr(rstd), ptr(post), M, int(C),
+                                                 eps, stream()));
+  }
   return tuple_of({&y, &mean, &rstd});
   END_HANDLE_TH_ERRORS
 }
@@ -240,29 +244,31 @@ PyObject* mlp3_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const void* w[3];
   for (int i = 0; i < 3; ++i) w[i] = tensor(PySequence_Fast_GET_ITEM(weights.get(), i)).data_ptr();
   Tensor vec[5];
-  for (int i = 0; i < 5; ++i) vec[i] = vector32(optional(PySequence_Fast_GET_ITEM(vectors.get(), i)));
+  for (int i = 0; i < 5; ++i) vec[i] = optional(PySequence_Fast_GET_ITEM(vectors.get(), i));
   const float eps = float(real(args[4]));
   const int act = int(integer(args[5]));
   const Tensor post = optional(args[6]);
   const int64_t m = integer(args[7]);
   const bool keep = truth(args[8]), relu = act == 3;
-  const Tensor y = empty({m, kWidth}, at::kBFloat16, table);
-  Tensor h1, h2, x3, mean, rstd, z1, z2;
-  if (keep) {
-    const Tensor h = empty({3, m, kWidth}, at::kBFloat16, table), s = empty({2, m}, at::kFloat, table);
-    h1 = h.select(0, 0); h2 = h.select(0, 1); x3 = h.select(0, 2);
-    mean = s.select(0, 0); rstd = s.select(0, 1);
-    if (!relu) {
-      const Tensor z = empty({2, (m + kRows - 1) / kRows, kRows * kWidth}, at::kBFloat16, table);     // whole tiles
-      z1 = z.select(0, 0); z2 = z.select(0, 1);
+  Tensor y, h1, h2, x3, mean, rstd, z1, z2;
+  {
+    const Unlocked unlocked;
+    for (Tensor& v : vec) v = vector32(v);
+    y = empty({m, kWidth}, at::kBFloat16, table);
+    if (keep) {
+      const Tensor h = empty({3, m, kWidth}, at::kBFloat16, table), s = empty({2, m}, at::kFloat, table);
+      h1 = h.select(0, 0); h2 = h.select(0, 1); x3 = h.select(0, 2);
+      mean = s.select(0, 0); rstd = s.select(0, 1);
+      if (!relu) {
+        const Tensor z = empty({2, (m + kRows - 1) / kRows, kRows * kWidth}, at::kBFloat16, table);     // whole tiles
+        z1 = z.select(0, 0); z2 = z.select(0, 1);
+      }
     }
+    check("pnm_mlp3_ln_fwd",
+          pnm_mlp3_ln_fwd(int(nsrc), src, rows, ld, idx, w[0], w[1], w[2], fptr(vec[0]), fptr(vec[1]), fptr(vec[2]), fptr(vec[3]), fptr(vec[4]), eps, act,
+                          ptr(post), post.defined() ? post.stride(0) : 0, ptr(y), kWidth, ptr(z1), ptr(z2), ptr(h1), ptr(h2), ptr(x3), fptr(mean),
+                          fptr(rstd), m, stream()));
   }
-  void* st = stream();
-  launch("pnm_mlp3_ln_fwd", [&] {
-    return pnm_mlp3_ln_fwd(int(nsrc), src, rows, ld, idx, w[0], w[1], w[2], fptr(vec[0]), fptr(vec[1]), fptr(vec[2]), fptr(vec[3]), fptr(vec[4]), eps,
-                           act, ptr(post), post.defined() ? post.stride(0) : 0, ptr(y), kWidth, ptr(z1), ptr(z2), ptr(h1), ptr(h2), ptr(x3), fptr(mean),
-                           fptr(rstd), m, st);
-  });
   if (!keep) return THPVariable_Wrap(y);
   return relu ? tuple_of({&y, &h1, &h2, &x3, &mean, &rstd}) : tuple_of({&y, &h1, &h2, &x3, &mean, &rstd, &z1, &z2});
   END_HANDLE_TH_ERRORS
@@ -273,16 +279,18 @@ PyObject* segment_sum(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 7);
   const Tensor x = tensor(args[0]), perm = tensor(args[1]), offsets = tensor(args[2]);
-  require(x.dim() == 2, "expected a matrix");
-  const int64_t segments = integer(args[3]), C = x.size(1);
+  const int64_t segments = integer(args[3]);
   const int accumulate = truth(args[4]), mean = truth(args[5]);
   Tensor out = optional(args[6]);
-  if (!out.defined()) out = empty({segments, C}, at::kBFloat16, x);
-  void* st = stream();
-  launch("pnm_segment_sum", [&] {
-    return pnm_segment_sum(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(perm)), static_cast<const int*>(ptr(offsets)), ptr(out),
-                           int(out.stride(0)), segments, int(C), accumulate, mean, st);
-  });
+  {
+    const Unlocked unlocked;
+    require(x.dim() == 2, "expected a matrix");
+    const int64_t C = x.size(1);
+    if (!out.defined()) out = empty({segments, C}, at::kBFloat16, x);
+    check("pnm_segment_sum",
+          pnm_segment_sum(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(perm)), static_cast<const int*>(ptr(offsets)), ptr(out),
+                          int(out.stride(0)), segments, int(C), accumulate, mean, stream()));
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -293,13 +301,14 @@ PyObject* gather_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   need_args(n, 4);
   const Tensor x = tensor(args[0]), index = tensor(args[1]), scale = optional(args[2]);
   Tensor out = optional(args[3]);
-  require(x.dim() == 2, "expected a matrix");
-  const int64_t E = index.numel(), C = x.size(1);
-  if (!out.defined()) out = empty({E, C}, at::kBFloat16, x);
-  void* st = stream();
-  launch("pnm_gather_rows", [&] {
-    return pnm_gather_rows(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(index)), fptr(scale), ptr(out), int(out.stride(0)), E, int(C), st);
-  });
+  {
+    const Unlocked unlocked;
+    require(x.dim() == 2, "expected a matrix");
+    const int64_t E = index.numel(), C = x.size(1);
+    if (!out.defined()) out = empty({E, C}, at::kBFloat16, x);
+    check("pnm_gather_rows", pnm_gather_rows(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(index)), fptr(scale), ptr(out), int(out.stride(0)), E,
+                                             int(C), stream()));
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -310,11 +319,14 @@ PyObject* conv2d_nhwc(PyObject*, PyObject* const* args, Py_ssize_t n) {
   need_args(n, 5);
   const Tensor x = tensor(args[0]), w = tensor(args[1]), bias = optional(args[2]);
   const int k = int(integer(args[3])), act = int(integer(args[4]));
-  require(x.dim() == 4, "expected an image [n, h, w, c]");
-  const int N = int(x.size(0)), H = int(x.size(1)), W = int(x.size(2)), cin = int(x.size(3)), cout = int(w.size(0));
-  const Tensor y = empty({N, H, W, cout}, at::kBFloat16, x);
-  void* st = stream();
-  launch("pnm_conv2d_nhwc", [&] { return pnm_conv2d_nhwc(ptr(x), ptr(w), ptr(y), N, H, W, cin, cout, k, fptr(bias), act, 0, 0, st); });
+  Tensor y;
+  {
+    const Unlocked unlocked;
+    require(x.dim() == 4, "expected an image [n, h, w, c]");
+    const int N = int(x.size(0)), H = int(x.size(1)), W = int(x.size(2)), cin = int(x.size(3)), cout = int(w.size(0));
+    y = empty({N, H, W, cout}, at::kBFloat16, x);
+    check("pnm_conv2d_nhwc", pnm_conv2d_nhwc(ptr(x), ptr(w), ptr(y), N, H, W, cin, cout, k, fptr(bias), act, 0, 0, stream()));
+  }
   return THPVariable_Wrap(y);
   END_HANDLE_TH_ERRORS
 }
@@ -324,13 +336,15 @@ PyObject* conv_pack_weight(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 4);
   const Tensor w = tensor(args[0]);
-  require(w.dim() == 4, "expected a filter [cout, cin, k, k]");
   const int rows = int(integer(args[1])), cols = int(integer(args[2])), flip = truth(args[3]);
-  const int cout = int(w.size(0)), cin = int(w.size(1)), k = int(w.size(2));
-  const Tensor out = empty({rows, int64_t(k) * k * cols}, at::kBFloat16, w);
-  void* st = stream();
-  launch("pnm_conv_pack_weight",
-         [&] { return pnm_conv_pack_weight(ptr(w), w.scalar_type() == at::kBFloat16, ptr(out), cout, cin, k, rows, cols, flip, st); });
+  Tensor out;
+  {
+    const Unlocked unlocked;
+    require(w.dim() == 4, "expected a filter [cout, cin, k, k]");
+    const int cout = int(w.size(0)), cin = int(w.size(1)), k = int(w.size(2));
+    out = empty({rows, int64_t(k) * k * cols}, at::kBFloat16, w);
+    check("pnm_conv_pack_weight", pnm_conv_pack_weight(ptr(w), w.scalar_type() == at::kBFloat16, ptr(out), cout, cin, k, rows, cols, flip, stream()));
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -342,16 +356,17 @@ PyObject* groupnorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const Tensor x = tensor(args[0]), gamma = tensor(args[1]), beta = tensor(args[2]);
   const int G = int(integer(args[3])), S = int(integer(args[4])), layout = int(integer(args[5])), dtype = int(integer(args[6])), silu = truth(args[7]);
   const float eps = float(real(args[8]));
-  require(x.dim() >= 2, "expected [batch, channels, ...]");
-  const int B = int(x.size(0)), C = int(x.size(1));
-  const long long hw = x.numel() / (int64_t(B) * C);
-  const Tensor y = at::empty_like(x), mean = empty({int64_t(B) * G}, at::kFloat, x), rstd = empty({int64_t(B) * G}, at::kFloat, x);
-  const Tensor scratch = empty({pnm_groupnorm_scratch_floats(B, C, G, S)}, at::kFloat, x);
-  void* st = stream();
-  launch("pnm_groupnorm_fwd", [&] {
-    return pnm_groupnorm_fwd(ptr(x), fptr(gamma), fptr(beta), ptr(y), fptr(mean), fptr(rstd), fptr(scratch), B, C, hw, G, S, layout, dtype, silu, eps,
-                             st);
-  });
+  Tensor y, mean, rstd;
+  {
+    const Unlocked unlocked;
+    require(x.dim() >= 2 && x.numel() > 0, "expected [batch, channels, ...]");
+    const int B = int(x.size(0)), C = int(x.size(1));
+    const long long hw = x.numel() / (int64_t(B) * C);
+    y = at::empty_like(x); mean = empty({int64_t(B) * G}, at::kFloat, x); rstd = empty({int64_t(B) * G}, at::kFloat, x);
+    const Tensor scratch = empty({pnm_groupnorm_scratch_floats(B, C, G, S)}, at::kFloat, x);
+    check("pnm_groupnorm_fwd", pnm_groupnorm_fwd(ptr(x), fptr(gamma), fptr(beta), ptr(y), fptr(mean), fptr(rstd), fptr(scratch), B, C, hw, G, S, layout,
+                                                 dtype, silu, eps, stream()));
+  }
   return tuple_of({&y, &mean, &rstd});
   END_HANDLE_TH_ERRORS
 }
@@ -362,14 +377,16 @@ PyObject* pa_prepare_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   need_args(n, 8);
   Tensor p[6];
   for (int i = 0; i < 6; ++i) p[i] = tensor(args[i]);
-  const int64_t H = integer(args[6]), D = integer(args[7]), C = p[0].size(1), HS = H * 64, inner = H * D;
-  const Tensor Wc = empty({HS, C}, at::kBFloat16, p[0]), bc = empty({HS}, at::kFloat, p[0]), inv_t = empty({HS}, at::kFloat, p[0]),
-               Wfx16 = empty({inner, C}, at::kBFloat16, p[0]), Wback = empty({C, HS + inner}, at::kBFloat16, p[0]);
-  void* st = stream();
-  launch("pnm_pa_prepare_fwd", [&] {
-    return pnm_pa_prepare_fwd(fptr(p[0]), fptr(p[1]), fptr(p[2]), fptr(p[3]), fptr(p[4]), fptr(p[5]), ptr(Wc), fptr(bc), fptr(inv_t), ptr(Wfx16),
-                              ptr(Wback), int(H), int(D), int(C), st);
-  });
+  const int64_t H = integer(args[6]), D = integer(args[7]), HS = H * 64, inner = H * D;
+  Tensor Wc, bc, inv_t, Wfx16, Wback;
+  {
+    const Unlocked unlocked;
+    const int64_t C = p[0].size(1);
+    Wc = empty({HS, C}, at::kBFloat16, p[0]); bc = empty({HS}, at::kFloat, p[0]); inv_t = empty({HS}, at::kFloat, p[0]);
+    Wfx16 = empty({inner, C}, at::kBFloat16, p[0]); Wback = empty({C, HS + inner}, at::kBFloat16, p[0]);
+    check("pnm_pa_prepare_fwd", pnm_pa_prepare_fwd(fptr(p[0]), fptr(p[1]), fptr(p[2]), fptr(p[3]), fptr(p[4]), fptr(p[5]), ptr(Wc), fptr(bc), fptr(inv_t),
+                                                   ptr(Wfx16), ptr(Wback), int(H), int(D), int(C), stream()));
+  }
   return tuple_of({&Wc, &bc, &inv_t, &Wfx16, &Wback});
   END_HANDLE_TH_ERRORS
 }
@@ -380,14 +397,22 @@ PyObject* empties(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n < 2) throw torch::TypeError("expected a tensor, a flag and shapes");
   const Tensor& like = tensor(args[0]);
   const at::ScalarType type = truth(args[1]) ? at::kBFloat16 : at::kFloat;
+  std::vector<std::vector<int64_t>> shapes(n - 2);
+  for (Py_ssize_t k = 2; k < n; ++k) {
+    if (!PyTuple_Check(args[k])) throw torch::TypeError("shapes are tuples of numbers");
+    for (Py_ssize_t d = 0; d < PyTuple_GET_SIZE(args[k]); ++d) shapes[k - 2].push_back(integer(PyTuple_GET_ITEM(args[k], d)));
+  }
+  std::vector<Tensor> tensors;
+  {
+    const Unlocked unlocked;
+    for (const auto& shape : shapes) tensors.push_back(empty(shape, type, like));
+  }
   THPObjectPtr result(PyList_New(n - 2));
   if (!result) throw python_error();
-  for (Py_ssize_t k = 2; k < n; ++k) {
-    if (!PyTuple_Check(args[k]) || PyTuple_GET_SIZE(args[k]) > 8) throw torch::TypeError("shapes are tuples of at most eight numbers");
-    int64_t sizes[8];
-    const Py_ssize_t dims = PyTuple_GET_SIZE(args[k]);
-    for (Py_ssize_t d = 0; d < dims; ++d) sizes[d] = integer(PyTuple_GET_ITEM(args[k], d));
-    PyList_SET_ITEM(result.get(), k - 2, THPVariable_Wrap(empty(at::IntArrayRef(sizes, size_t(dims)), type, like)));
+  for (Py_ssize_t k = 0; k < n - 2; ++k) {
+    PyObject* o = THPVariable_Wrap(tensors[k]);
+    if (!o) throw python_error();
+    PyList_SET_ITEM(result.get(), k, o);
   }
   return result.release();
   END_HANDLE_TH_ERRORS

@@ -1,4 +1,7 @@
 """Calls without gradients go to an autograd function's ``forward`` directly; the native host calls refuse what the Python code refused."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -50,6 +53,37 @@ def test_host_calls_refuse_bad_operands():
         host.gemm_tn(t, t[:, :64], None, None, 0, None, 0, None, None, False, None, None, False, 0, 0)
     with pytest.raises(AssertionError):                                  # not bf16
         host.gemm_tn(t.float(), t.float(), None, None, 0, None, 0, None, None, False, None, None, False, 0, 0)
+
+
+@pytest.mark.skipif(not _lib._HOST_PATH.exists(), reason="the kernel library is not built")
+def test_host_calls_copy_operands_without_the_interpreters_lock():
+    """Another thread runs while an operand is copied (or its memory allocated, which may wait for the device)."""
+    host, b = _lib.host(), torch.zeros(8, 16).bfloat16()
+    a = torch.zeros(8192, 8192).bfloat16().t()                           # read by columns: copied before its width is refused
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(1e-3)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        inside, threads = 0, torch.get_num_threads()
+        torch.set_num_threads(1)
+        for _ in range(3):
+            began = time.perf_counter()
+            with pytest.raises(AssertionError):
+                host.gemm_tn(a, b, None, None, 0, None, 0, None, None, False, None, None, False, 0, 0)
+            ended = time.perf_counter()
+            margin = 0.25 * (ended - began)                              # an end of the call may overlap with a tick that began outside
+            inside += sum(began + margin < t < ended - margin for t in ticks)
+    finally:
+        torch.set_num_threads(threads)
+        stop.set()
+        thread.join()
+    assert inside > 0
 
 
 @pytest.mark.gpu
