@@ -167,3 +167,20 @@ def test_group_norm_channels_last_on_two_streams():
             # the backward adds a channel's pixels with fp32 atomics: a rounding of bf16 (2^-9) at most, parameter gradients in fp32
             assert float((got[1].double() - want[1].double()).norm() / want[1].double().norm()) < 2.0 ** -9
             assert all(float((a - b).norm() / b.norm()) < 1e-5 for a, b in zip(got[2:], want[2:]))
+
+
+def test_build_passes_with_a_cpu_build_of_torch(monkeypatch):
+    import __graft_entry__ as entry
+
+    class Library:
+        def pnm_version(self):
+            return 100
+
+    def no_host():
+        raise RuntimeError("not built")
+
+    monkeypatch.setattr(torch.version, "cuda", None)
+    monkeypatch.setattr(_lib, "build", lambda force: _lib.lib_path())    # compiles the kernels only
+    monkeypatch.setattr(_lib, "load", lambda required=False: Library())
+    monkeypatch.setattr(_lib, "host", no_host)
+    entry.build()
