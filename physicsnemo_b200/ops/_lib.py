@@ -44,18 +44,22 @@ def _sources():
     return sorted(list(_SRC_DIR.glob("*.cu")) + list(_SRC_DIR.glob("*.cuh")) + list(_SRC_DIR.glob("*.h")))
 
 
-def needs_build() -> bool:
-    if not _LIB_PATH.exists():
-        return True
-    built = _LIB_PATH.stat().st_mtime
-    return any(s.stat().st_mtime > built for s in _sources()) or _host_needs_build()
+def _stale(target: Path, sources) -> bool:
+    return not target.exists() or any(p.stat().st_mtime > target.stat().st_mtime for p in sources)
+
+
+def _kernels_need_build() -> bool:
+    return _stale(_LIB_PATH, _sources())
 
 
 def _host_needs_build() -> bool:
     if torch.version.cuda is None:                           # nothing is launched without CUDA
         return False
-    return not _HOST_PATH.exists() or any(p.stat().st_mtime > _HOST_PATH.stat().st_mtime
-                                          for p in (_SRC_DIR / "host_calls.cpp", _SRC_DIR / "pnm_api.h"))
+    return _stale(_HOST_PATH, (_SRC_DIR / "host_calls.cpp", _SRC_DIR / "pnm_api.h"))
+
+
+def needs_build() -> bool:
+    return _kernels_need_build() or _host_needs_build()
 
 
 def _build_host() -> None:
@@ -77,13 +81,7 @@ def _build_host() -> None:
     os.replace(tmp_out, _HOST_PATH)
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile the kernel library in-tree; returns the path of the ``.so``."""
-    if not _SRC_DIR.exists():
-        raise FileNotFoundError(f"kernel sources not found at {_SRC_DIR}")
-    if not force and not needs_build():
-        return _LIB_PATH
-    _LIB_DIR.mkdir(parents=True, exist_ok=True)
+def _build_kernels(verbose: bool) -> None:
     nvcc = os.environ.get("NVCC", "nvcc")
     tmp_out = _LIB_DIR / f".libpnm_b200.{os.getpid()}.so.tmp"     # built aside, then moved into place in one step
     cmd = [nvcc, *NVCC_FLAGS, "-o", str(tmp_out), *[str(p) for p in sorted(_SRC_DIR.glob("*.cu"))]]
@@ -98,8 +96,17 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     os.replace(tmp_out, _LIB_PATH)
     if verbose:
         print(proc.stderr)
-    if torch.version.cuda is not None:
-        _build_host()
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Compile what is not up to date (``force``: all) of the kernel library and the host calls in-tree; returns the library's path."""
+    if not _SRC_DIR.exists():
+        raise FileNotFoundError(f"kernel sources not found at {_SRC_DIR}")
+    _LIB_DIR.mkdir(parents=True, exist_ok=True)
+    if force or _kernels_need_build():
+        _build_kernels(verbose)
+    if torch.version.cuda is not None and (force or _host_needs_build()):
+        _build_host()                                        # links the library
     return _LIB_PATH
 
 

@@ -184,3 +184,46 @@ def test_build_passes_with_a_cpu_build_of_torch(monkeypatch):
     monkeypatch.setattr(_lib, "load", lambda required=False: Library())
     monkeypatch.setattr(_lib, "host", no_host)
     entry.build()
+
+
+def _tree(tmp_path, monkeypatch):
+    """A tree of empty sources and built files that are up to date; the compilers' command lines are recorded."""
+    import os
+
+    src, out, ran = tmp_path / "csrc", tmp_path / "lib", []
+    src.mkdir()
+    out.mkdir()
+    monkeypatch.setattr(_lib, "_SRC_DIR", src)
+    monkeypatch.setattr(_lib, "_LIB_DIR", out)
+    monkeypatch.setattr(_lib, "_LIB_PATH", out / _lib._LIB_PATH.name)
+    monkeypatch.setattr(_lib, "_HOST_PATH", out / _lib._HOST_PATH.name)
+    monkeypatch.setattr(torch.version, "cuda", "12.8")
+    for k, name in enumerate(("kernels.cu", "kernels.cuh", "pnm_api.h", "host_calls.cpp")):
+        (src / name).touch()
+        os.utime(src / name, (1000 + k, 1000 + k))
+
+    def run(cmd, **kwargs):
+        ran.append(cmd[0])
+        target = next(t for f, t in zip(cmd, cmd[1:]) if f == "-o")
+        open(target, "w").close()
+        return type("Done", (), {"returncode": 0, "stdout": "", "stderr": ""})()
+
+    monkeypatch.setattr(_lib.subprocess, "run", run)
+    monkeypatch.setenv("NVCC", "nvcc")
+    monkeypatch.setenv("CXX", "g++")
+    _lib.build()
+    assert ran == ["nvcc", "g++"] and not _lib.needs_build()
+    ran.clear()
+    return src, ran
+
+
+@pytest.mark.parametrize("name,compilers", [("host_calls.cpp", ["g++"]), ("kernels.cuh", ["nvcc"]), ("pnm_api.h", ["nvcc", "g++"])])
+def test_only_what_is_out_of_date_is_built(tmp_path, monkeypatch, name, compilers):
+    import os
+
+    src, ran = _tree(tmp_path, monkeypatch)
+    later = time.time() + 60
+    os.utime(src / name, (later, later))
+    assert _lib.needs_build()
+    _lib.build()
+    assert ran == compilers
