@@ -4,8 +4,9 @@ The library is plain C ABI (see ``csrc/pnm_api.h``) bound through ``ctypes``: ev
 call passes raw device pointers and the current CUDA stream.  ``build()`` compiles the
 single translation unit ``csrc/pnm_lib.cu`` with
 ``nvcc -gencode arch=compute_100a,code=sm_100a`` (cross-compiles without a GPU), and the CPython
-extension ``_pnm_host.so`` from ``csrc/host_calls.cpp``: the host side of the hottest calls
-(operand checks, allocation, launch), without ctypes.
+extension ``_pnm_host.*.so`` from ``csrc/host_calls.cpp``: the host side of the hottest calls
+(operand checks, allocation, launch), without ctypes.  The library serves any Python; the extension serves the Python and the torch
+that its file name gives, and is built anew for others.
 On a machine with a CUDA device a missing library is an error, never a silent
 fallback.
 """
@@ -14,6 +15,7 @@ from __future__ import annotations
 import ctypes
 import os
 import subprocess
+import sysconfig
 import threading
 from pathlib import Path
 
@@ -24,7 +26,14 @@ _REPO = _PKG_DIR.parent
 _SRC_DIR = _REPO / "csrc"
 _LIB_DIR = _PKG_DIR / "lib"
 _LIB_PATH = _LIB_DIR / "libpnm_b200.so"
-_HOST_PATH = _LIB_DIR / "_pnm_host.so"
+
+
+def _host_path() -> Path:
+    """The extension's binary interface is that of one Python and one torch: its name says which."""
+    return _LIB_DIR / f"_pnm_host.torch-{torch.__version__}.{sysconfig.get_config_var('SOABI')}.so"
+
+
+_HOST_PATH = _host_path()
 _lock = threading.Lock()
 _lib = None
 _host = None
@@ -63,8 +72,6 @@ def needs_build() -> bool:
 
 
 def _build_host() -> None:
-    import sysconfig
-
     top = Path(torch.__file__).resolve().parent
     cuda = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
     include = [top / "include", top / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
@@ -171,7 +178,8 @@ def host():
         with _lock:
             if _host is None:
                 if not _HOST_PATH.exists():
-                    raise RuntimeError(f"{_HOST_PATH} not built; run `python -c 'import __graft_entry__ as g; g.build()'`")
+                    raise RuntimeError(f"{_HOST_PATH} not built for this Python and torch; run "
+                                       "`python -c 'import __graft_entry__ as g; g.build()'`")
                 spec = importlib.util.spec_from_file_location("_pnm_host", _HOST_PATH)
                 module = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(module)

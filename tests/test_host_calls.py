@@ -227,3 +227,30 @@ def test_only_what_is_out_of_date_is_built(tmp_path, monkeypatch, name, compiler
     assert _lib.needs_build()
     _lib.build()
     assert ran == compilers
+
+
+def test_host_calls_belong_to_one_python_and_one_torch(tmp_path, monkeypatch):
+    """Another torch or Python has an extension of its own and leaves the other's in place; the wheel is for one Python."""
+    import runpy
+    import sysconfig
+    from pathlib import Path
+
+    import setuptools
+
+    names = {_lib._HOST_PATH.name}
+    get = sysconfig.get_config_var
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.1")
+        names.add(_lib._host_path().name)
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-399-other" if name == "SOABI" else get(name))
+        names.add(_lib._host_path().name)
+    assert len(names) == 3
+    src, ran = _tree(tmp_path, monkeypatch)
+    monkeypatch.setattr(_lib, "_HOST_PATH", _lib._HOST_PATH.with_name(max(names - {_lib._HOST_PATH.name})))
+    assert _lib.needs_build()
+    _lib.build()
+    assert ran == ["g++"] and len(list(_lib._LIB_DIR.glob("_pnm_host.*"))) == 2
+    asked = {}
+    monkeypatch.setattr(setuptools, "setup", lambda **kwargs: asked.update(kwargs))
+    runpy.run_path(str(Path(__file__).resolve().parents[1] / "setup.py"))
+    assert asked["distclass"]().has_ext_modules()
