@@ -254,3 +254,20 @@ def test_host_calls_belong_to_one_python_and_one_torch(tmp_path, monkeypatch):
     monkeypatch.setattr(setuptools, "setup", lambda **kwargs: asked.update(kwargs))
     runpy.run_path(str(Path(__file__).resolve().parents[1] / "setup.py"))
     assert asked["distclass"]().has_ext_modules()
+
+
+def test_declared_functions_are_called():
+    """A function that the loader declares is called somewhere in the package (calls that went to the extension leave no declaration)."""
+    import re
+    from pathlib import Path
+
+    class Recorder:
+        def __getattr__(self, name):
+            return self.__dict__.setdefault(name, type("Function", (), {})())
+
+    lib = Recorder()
+    _lib._declare(lib)
+    own = Path(_lib.__file__)
+    text = "\n".join(f.read_text() for f in own.parents[1].rglob("*.py") if f != own) + own.read_text().split("def load(")[1]
+    entry = Path(__file__).resolve().parents[1] / "__graft_entry__.py"
+    assert vars(lib) and [name for name in vars(lib) if not re.search(rf"\.{name}\b", text + entry.read_text())] == []
