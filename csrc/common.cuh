@@ -27,6 +27,7 @@ enum : int {
 
 // Budget of one bounded wait, in nanoseconds of %globaltimer.
 constexpr unsigned long long kWaitBudgetNs = 2000000000ull;  // 2 s
+static_assert(kWaitBudgetNs < (1ull << 31), "mbar_wait compares it with the low word of the timer; the rest is for a thread that looks late");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -94,3 +94,15 @@ def test_no_thread_launches_before_the_attribute_is_set(tmp_path):
 @pytest.mark.skipif(not Path(NVCC).exists(), reason="no nvcc")
 def test_layernorm_plans_fit_the_sm(tmp_path):
     _run(tmp_path, PLAN)
+
+
+@pytest.mark.skipif(not Path(NVCC).exists(), reason="no nvcc")
+@pytest.mark.parametrize("budget,compiles", [("2000000000ull", True), ("5000000000ull", False)])
+def test_a_wait_budget_that_the_timers_low_word_cannot_hold_does_not_compile(tmp_path, budget, compiles):
+    text = (CSRC / "common.cuh").read_text()
+    assert "kWaitBudgetNs = 2000000000ull" in text
+    (tmp_path / "common.cuh").write_text(text.replace("kWaitBudgetNs = 2000000000ull", f"kWaitBudgetNs = {budget}"))
+    (tmp_path / "unit.cu").write_text('#include "common.cuh"\n')
+    built = subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(tmp_path), "-I", str(CSRC), "-c",
+                            "-o", str(tmp_path / "unit.o"), str(tmp_path / "unit.cu")], capture_output=True, text=True)
+    assert (built.returncode == 0) == compiles and (compiles or "low word" in built.stdout + built.stderr)
