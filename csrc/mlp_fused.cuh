@@ -400,6 +400,9 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
     const uint32_t base = tmem + (uint32_t(q * 32) << 16);
     // the moments of a half row lie in its own part of the A operand, whose last reader is the third product
     const uint32_t aop = base + 3 * kMlpW + grp * 64 + half * 32, other_aop = base + 3 * kMlpW + grp * 64 + (half ^ 1) * 32;
+    // A group meets accumulator `a` every other turn, always with the parity of `turn`: a wait for turn t + 2 would be over at once if
+    // turn t + 1 (the other group's tile n + 3) were not.  It is: one thread issues and commits the first products in the order of the
+    // tiles, so that of tile n + 3 has finished before that of n + 4, which this group has waited for before it comes to n + 6.
     uint32_t n = 0, uses = 0, a = 0, turn = 0;   // n = 3 turn + a
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++n, turn += a == 2, a = a == 2 ? 0 : a + 1) {
       if ((n & 1) != uint32_t(grp)) continue;

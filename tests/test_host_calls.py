@@ -86,6 +86,38 @@ def test_host_calls_copy_operands_without_the_interpreters_lock():
     assert inside > 0
 
 
+def _forms(t):
+    """The values of a matrix by columns, in rows of an odd stride, one element off a 16-byte boundary, and with a longer row stride."""
+    m, n = t.shape
+    odd, off, wide = t.new_empty(m, n + 1), t.new_empty(m * n + 1), t.new_empty(m, n + 8)
+    odd[:, :n], off[1:], wide[:, 8:] = t, t.reshape(-1), t
+    return [t.t().contiguous().t(), odd[:, :n], off[1:].view(m, n), wide[:, 8:]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [3, 130])
+def test_host_calls_copy_strided_and_misaligned_operands(rows):
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    bf = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    a, a2, b, aux, bias = bf(rows, 64), bf(rows, 128), bf(72, 192), bf(rows, 72), torch.randn(72, device="cuda")
+    want = G.gemm_tn(a, b, bias=bias, a2=a2, aux=aux, aux_mode=G.AUX_ADD)
+    for x, x2, w, r in zip(_forms(a), _forms(a2), _forms(b), _forms(aux)):
+        assert torch.equal(G.gemm_tn(x, w, bias=bias, a2=x2, aux=r, aux_mode=G.AUX_ADD), want)
+    ref, sums = a.double().t() @ a2.double(), a.double().sum(0)
+    for x, x2 in zip(_forms(a), _forms(a2)):
+        got, got_sums = G.gemm_nt(x, x2, colsum=True)
+        # exact products of bf16 values, at most 130 of them added in fp32
+        assert float((got - ref).abs().max()) < 1e-4 and float((got_sums - sums).abs().max()) < 1e-4
+    # parameter vectors of the one-kernel MLP: bf16, every other value of a longer vector, off a 16-byte boundary
+    x, w = bf(rows, 128), [bf(128, 128) / 11 for _ in range(3)]
+    vec = [torch.randn(128, device="cuda").bfloat16().float() for _ in range(5)]
+    want = mf._forward([x], [None], w, vec[:3], 2, *vec[3:], 1e-5, None, False)[0]
+    for form in (lambda v: v.bfloat16(), lambda v: v.repeat_interleave(2)[::2], lambda v: torch.cat([v[:1], v])[1:]):
+        v = [form(t) for t in vec]
+        assert torch.equal(mf._forward([x], [None], w, v[:3], 2, *v[3:], 1e-5, None, False)[0], want)
+
+
 @pytest.mark.gpu
 def test_host_calls_raise_for_tensors_without_storage():
     """The pointer is read where the interpreter's lock is released: its error arrives as an exception all the same."""
@@ -271,3 +303,19 @@ def test_declared_functions_are_called():
     text = "\n".join(f.read_text() for f in own.parents[1].rglob("*.py") if f != own) + own.read_text().split("def load(")[1]
     entry = Path(__file__).resolve().parents[1] / "__graft_entry__.py"
     assert vars(lib) and [name for name in vars(lib) if not re.search(rf"\.{name}\b", text + entry.read_text())] == []
+
+
+def test_mlps_with_an_identity_activation_stay_layer_by_layer():
+    """The fused chain takes Linear / activation / ... / Linear: an Identity between two layers is refused, no error."""
+    from torch import nn
+
+    from physicsnemo_b200.nn.module.gnn_layers.mesh_graph_mlp import MeshGraphMLP, _layers
+
+    lin = lambda: nn.Linear(8, 8)  # noqa: E731
+    assert _layers(nn.Sequential(lin(), nn.Identity(), lin())) is None
+    assert _layers(nn.Sequential(nn.SiLU(), lin())) is None and _layers(nn.Sequential(lin(), nn.SiLU(), nn.SiLU(), lin())) is None
+    model = nn.Sequential(lin(), nn.SiLU(), lin(), lin(), nn.LayerNorm(8))
+    weights, biases, acts, norm = _layers(model)
+    assert acts == [2, 0, 0] and weights[1] is model[2].weight and biases[2] is model[3].bias and norm is model[4]
+    m, x = MeshGraphMLP(8, 8, 8, 2, nn.Identity()), torch.randn(5, 8)
+    assert torch.equal(m(x), m.model(x))
