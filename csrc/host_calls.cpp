@@ -27,7 +27,8 @@ const Tensor& tensor(PyObject* o) {
   return THPVariable_Unpack(o);
 }
 // undefined for None
-Tensor optional(PyObject* o) { return o == Py_None ? Tensor() : tensor(o); }
+const Tensor kNone;
+const Tensor& optional(PyObject* o) { return o == Py_None ? kNone : tensor(o); }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
 long long integer(PyObject* o) {
@@ -69,20 +70,24 @@ void check(const char* name, int code) {
 }
 uintptr_t address(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); }
 // 2-D view whose last dim is contiguous, whose row stride is a multiple of 8 and that starts on a 16-byte boundary
-Tensor rowmajor2d(const Tensor& in) {
+// (the argument itself or a copy, which `own` holds: a second reference to a Python object's tensor costs 0.1 us)
+const Tensor& rowmajor2d(const Tensor& in, Tensor& own) {
   require(in.dim() == 2, "expected a matrix");
-  Tensor t = in;
-  if (t.stride(1) != 1 || t.stride(0) % 8 != 0) t = t.contiguous();
-  return address(t) % 16 == 0 ? t : t.clone();
+  const Tensor* t = &in;
+  if (t->stride(1) != 1 || t->stride(0) % 8 != 0) t = &(own = in.contiguous());
+  if (address(*t) % 16 != 0) t = &(own = t->clone());
+  return *t;
 }
 Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
   return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
 }
 // values of a parameter vector: fp32, contiguous, 16-byte aligned
-Tensor vector32(const Tensor& t) {
-  if (!t.defined()) return t;
-  Tensor v = t.scalar_type() == at::kFloat && t.is_contiguous() ? t : t.detach().to(at::kFloat).contiguous();
-  return address(v) % 16 == 0 ? v : v.detach().clone();
+const Tensor& vector32(const Tensor& in, Tensor& own) {
+  if (!in.defined()) return in;
+  const Tensor* t = &in;
+  if (t->scalar_type() != at::kFloat || !t->is_contiguous()) t = &(own = in.detach().to(at::kFloat).contiguous());
+  if (address(*t) % 16 != 0) t = &(own = t->detach().clone());
+  return *t;
 }
 PyObject* tuple_of(std::initializer_list<const Tensor*> tensors) {
   THPObjectPtr result(PyTuple_New(Py_ssize_t(tensors.size())));
@@ -100,21 +105,22 @@ PyObject* tuple_of(std::initializer_list<const Tensor*> tensors) {
 PyObject* gemm_tn(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 15);
-  Tensor a = tensor(args[0]), b = tensor(args[1]), aux = optional(args[5]), a2 = optional(args[7]), a3 = optional(args[8]), out = optional(args[10]), z;
-  const Tensor bias = optional(args[2]), scale = optional(args[3]), group_out = optional(args[11]);
+  const Tensor &a0 = tensor(args[0]), &b0 = tensor(args[1]), &bias = optional(args[2]), &scale = optional(args[3]), &aux0 = optional(args[5]),
+               &a20 = optional(args[7]), &a30 = optional(args[8]), &given = optional(args[10]), &group_out = optional(args[11]);
   const int act = int(integer(args[4])), aux_mode = int(integer(args[6])), post = truth(args[12]), bn = int(integer(args[13])),
             cap = int(integer(args[14]));
   const bool want_z = truth(args[9]);
+  Tensor own[5], made, z;
+  const Tensor& out = given.defined() ? given : made;
   {
     const Unlocked unlocked;
-    a = rowmajor2d(a); b = rowmajor2d(b);
+    const Tensor &a = rowmajor2d(a0, own[0]), &b = rowmajor2d(b0, own[1]);
+    const Tensor &a2 = a20.defined() ? rowmajor2d(a20, own[2]) : kNone, &a3 = a2.defined() && a30.defined() ? rowmajor2d(a30, own[3]) : kNone;
     const int64_t M = a.size(0), K1 = a.size(1), N = b.size(0), K = b.size(1);
     int64_t K2 = K;
     if (a2.defined()) {
-      a2 = rowmajor2d(a2);
       K2 = K1 + a2.size(1);
       if (a3.defined()) {
-        a3 = rowmajor2d(a3);
         require(a3.size(0) == M && K2 + a3.size(1) == K, "the column blocks of A do not match B");
       } else {
         require(a2.size(0) == M && K2 == K, "the column blocks of A do not match B");
@@ -123,10 +129,10 @@ PyObject* gemm_tn(PyObject*, PyObject* const* args, Py_ssize_t n) {
       require(K1 == K, "A and B have different numbers of columns");
     }
     require(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "operands must be bf16");
-    if (!out.defined()) out = empty({M, N}, at::kBFloat16, a);
+    if (!given.defined()) made = empty({M, N}, at::kBFloat16, a);
     if (want_z) z = empty({M, N}, at::kBFloat16, a);
+    const Tensor& aux = aux0.defined() ? rowmajor2d(aux0, own[4]) : kNone;
     if (aux.defined()) {
-      aux = rowmajor2d(aux);
       require(aux.size(0) == M && aux.size(1) == N && aux.scalar_type() == at::kBFloat16, "the auxiliary operand must be bf16 [M, N]");
     }
     for (const Tensor* v : {&bias, &scale})
@@ -144,17 +150,19 @@ PyObject* gemm_tn(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* gemm_nt(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 6);
-  Tensor a = tensor(args[0]), b = tensor(args[1]), out = optional(args[3]), sums = optional(args[4]);
+  const Tensor &a0 = tensor(args[0]), &b0 = tensor(args[1]), &given = optional(args[3]), &given_sums = optional(args[4]);
   const bool want_sums = truth(args[2]);
   const int cap = int(integer(args[5]));
+  Tensor own[2], made, made_sums;
+  const Tensor &out = given.defined() ? given : made, &sums = given_sums.defined() ? given_sums : made_sums;
   {
     const Unlocked unlocked;
-    a = rowmajor2d(a); b = rowmajor2d(b);
+    const Tensor &a = rowmajor2d(a0, own[0]), &b = rowmajor2d(b0, own[1]);
     const int64_t M = a.size(0), Na = a.size(1), Nb = b.size(1);
     require(b.size(0) == M, "operands have different numbers of rows");
     const auto f32 = at::TensorOptions().dtype(at::kFloat).device(a.device());
-    if (!out.defined()) out = at::zeros({Na, Nb}, f32);
-    if (!sums.defined() && want_sums) sums = at::zeros({Na}, f32);
+    if (!given.defined()) made = at::zeros({Na, Nb}, f32);
+    if (!given_sums.defined() && want_sums) made_sums = at::zeros({Na}, f32);
     check("pnm_gemm_nt", pnm_gemm_nt(ptr(a), int(a.stride(0)), ptr(b), int(b.stride(0)), fptr(out), int(out.stride(0)), fptr(sums), int(M), int(Na),
                                      int(Nb), cap, stream()));
   }
@@ -166,7 +174,7 @@ PyObject* gemm_nt(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* layernorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 5);
-  const Tensor x = tensor(args[0]), gamma = tensor(args[1]), beta = optional(args[2]), post = optional(args[4]);
+  const Tensor &x = tensor(args[0]), &gamma = tensor(args[1]), &beta = optional(args[2]), &post = optional(args[4]);
   const float eps = float(real(args[3]));
   Tensor y, mean, rstd;
   {
@@ -243,17 +251,17 @@ PyObject* mlp3_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const Tensor& table = tensor(PySequence_Fast_GET_ITEM(tables.get(), 0));
   const void* w[3];
   for (int i = 0; i < 3; ++i) w[i] = tensor(PySequence_Fast_GET_ITEM(weights.get(), i)).data_ptr();
-  Tensor vec[5];
-  for (int i = 0; i < 5; ++i) vec[i] = optional(PySequence_Fast_GET_ITEM(vectors.get(), i));
+  const Tensor* vec[5];
+  for (int i = 0; i < 5; ++i) vec[i] = &optional(PySequence_Fast_GET_ITEM(vectors.get(), i));
   const float eps = float(real(args[4]));
   const int act = int(integer(args[5]));
-  const Tensor post = optional(args[6]);
+  const Tensor& post = optional(args[6]);
   const int64_t m = integer(args[7]);
   const bool keep = truth(args[8]), relu = act == 3;
-  Tensor y, h1, h2, x3, mean, rstd, z1, z2;
+  Tensor own[5], y, h1, h2, x3, mean, rstd, z1, z2;
   {
     const Unlocked unlocked;
-    for (Tensor& v : vec) v = vector32(v);
+    for (int i = 0; i < 5; ++i) vec[i] = &vector32(*vec[i], own[i]);
     y = empty({m, kWidth}, at::kBFloat16, table);
     if (keep) {
       const Tensor h = empty({3, m, kWidth}, at::kBFloat16, table), s = empty({2, m}, at::kFloat, table);
@@ -265,8 +273,8 @@ PyObject* mlp3_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
       }
     }
     check("pnm_mlp3_ln_fwd",
-          pnm_mlp3_ln_fwd(int(nsrc), src, rows, ld, idx, w[0], w[1], w[2], fptr(vec[0]), fptr(vec[1]), fptr(vec[2]), fptr(vec[3]), fptr(vec[4]), eps, act,
-                          ptr(post), post.defined() ? post.stride(0) : 0, ptr(y), kWidth, ptr(z1), ptr(z2), ptr(h1), ptr(h2), ptr(x3), fptr(mean),
+          pnm_mlp3_ln_fwd(int(nsrc), src, rows, ld, idx, w[0], w[1], w[2], fptr(*vec[0]), fptr(*vec[1]), fptr(*vec[2]), fptr(*vec[3]), fptr(*vec[4]), eps,
+                          act, ptr(post), post.defined() ? post.stride(0) : 0, ptr(y), kWidth, ptr(z1), ptr(z2), ptr(h1), ptr(h2), ptr(x3), fptr(mean),
                           fptr(rstd), m, stream()));
   }
   if (!keep) return THPVariable_Wrap(y);
@@ -278,15 +286,16 @@ PyObject* mlp3_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* segment_sum(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 7);
-  const Tensor x = tensor(args[0]), perm = tensor(args[1]), offsets = tensor(args[2]);
+  const Tensor &x = tensor(args[0]), &perm = tensor(args[1]), &offsets = tensor(args[2]), &given = optional(args[6]);
   const int64_t segments = integer(args[3]);
   const int accumulate = truth(args[4]), mean = truth(args[5]);
-  Tensor out = optional(args[6]);
+  Tensor made;
+  const Tensor& out = given.defined() ? given : made;
   {
     const Unlocked unlocked;
     require(x.dim() == 2, "expected a matrix");
     const int64_t C = x.size(1);
-    if (!out.defined()) out = empty({segments, C}, at::kBFloat16, x);
+    if (!given.defined()) made = empty({segments, C}, at::kBFloat16, x);
     check("pnm_segment_sum",
           pnm_segment_sum(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(perm)), static_cast<const int*>(ptr(offsets)), ptr(out),
                           int(out.stride(0)), segments, int(C), accumulate, mean, stream()));
@@ -299,13 +308,14 @@ PyObject* segment_sum(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* gather_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 4);
-  const Tensor x = tensor(args[0]), index = tensor(args[1]), scale = optional(args[2]);
-  Tensor out = optional(args[3]);
+  const Tensor &x = tensor(args[0]), &index = tensor(args[1]), &scale = optional(args[2]), &given = optional(args[3]);
+  Tensor made;
+  const Tensor& out = given.defined() ? given : made;
   {
     const Unlocked unlocked;
     require(x.dim() == 2, "expected a matrix");
     const int64_t E = index.numel(), C = x.size(1);
-    if (!out.defined()) out = empty({E, C}, at::kBFloat16, x);
+    if (!given.defined()) made = empty({E, C}, at::kBFloat16, x);
     check("pnm_gather_rows", pnm_gather_rows(ptr(x), int(x.stride(0)), static_cast<const int*>(ptr(index)), fptr(scale), ptr(out), int(out.stride(0)), E,
                                              int(C), stream()));
   }
@@ -317,7 +327,7 @@ PyObject* gather_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* conv2d_nhwc(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 5);
-  const Tensor x = tensor(args[0]), w = tensor(args[1]), bias = optional(args[2]);
+  const Tensor &x = tensor(args[0]), &w = tensor(args[1]), &bias = optional(args[2]);
   const int k = int(integer(args[3])), act = int(integer(args[4]));
   Tensor y;
   {
@@ -335,7 +345,7 @@ PyObject* conv2d_nhwc(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* conv_pack_weight(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 4);
-  const Tensor w = tensor(args[0]);
+  const Tensor& w = tensor(args[0]);
   const int rows = int(integer(args[1])), cols = int(integer(args[2])), flip = truth(args[3]);
   Tensor out;
   {
@@ -353,7 +363,7 @@ PyObject* conv_pack_weight(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* groupnorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 9);
-  const Tensor x = tensor(args[0]), gamma = tensor(args[1]), beta = tensor(args[2]);
+  const Tensor &x = tensor(args[0]), &gamma = tensor(args[1]), &beta = tensor(args[2]);
   const int G = int(integer(args[3])), S = int(integer(args[4])), layout = int(integer(args[5])), dtype = int(integer(args[6])), silu = truth(args[7]);
   const float eps = float(real(args[8]));
   Tensor y, mean, rstd;
@@ -375,17 +385,17 @@ PyObject* groupnorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* pa_prepare_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 8);
-  Tensor p[6];
-  for (int i = 0; i < 6; ++i) p[i] = tensor(args[i]);
+  const Tensor* p[6];
+  for (int i = 0; i < 6; ++i) p[i] = &tensor(args[i]);
   const int64_t H = integer(args[6]), D = integer(args[7]), HS = H * 64, inner = H * D;
   Tensor Wc, bc, inv_t, Wfx16, Wback;
   {
     const Unlocked unlocked;
-    const int64_t C = p[0].size(1);
-    Wc = empty({HS, C}, at::kBFloat16, p[0]); bc = empty({HS}, at::kFloat, p[0]); inv_t = empty({HS}, at::kFloat, p[0]);
-    Wfx16 = empty({inner, C}, at::kBFloat16, p[0]); Wback = empty({C, HS + inner}, at::kBFloat16, p[0]);
-    check("pnm_pa_prepare_fwd", pnm_pa_prepare_fwd(fptr(p[0]), fptr(p[1]), fptr(p[2]), fptr(p[3]), fptr(p[4]), fptr(p[5]), ptr(Wc), fptr(bc), fptr(inv_t),
-                                                   ptr(Wfx16), ptr(Wback), int(H), int(D), int(C), stream()));
+    const int64_t C = p[0]->size(1);
+    Wc = empty({HS, C}, at::kBFloat16, *p[0]); bc = empty({HS}, at::kFloat, *p[0]); inv_t = empty({HS}, at::kFloat, *p[0]);
+    Wfx16 = empty({inner, C}, at::kBFloat16, *p[0]); Wback = empty({C, HS + inner}, at::kBFloat16, *p[0]);
+    check("pnm_pa_prepare_fwd", pnm_pa_prepare_fwd(fptr(*p[0]), fptr(*p[1]), fptr(*p[2]), fptr(*p[3]), fptr(*p[4]), fptr(*p[5]), ptr(Wc), fptr(bc),
+                                                   fptr(inv_t), ptr(Wfx16), ptr(Wback), int(H), int(D), int(C), stream()));
   }
   return tuple_of({&Wc, &bc, &inv_t, &Wfx16, &Wback});
   END_HANDLE_TH_ERRORS
