@@ -216,7 +216,7 @@ __device__ __forceinline__ CLThread cl_thread(const GNShape& sh, int s) {
 }
 
 // One counter per batch item, in the call's own scratch behind the folded sums: calls on other streams have theirs.  Zeroed on the
-// call's stream before the statistics kernel.
+// call's stream before the statistics kernel (2 us each: a U-Net block with attention, three calls, 414 -> 424 us; training without, 1992 -> 1998).
 static unsigned int* cl_counters(float2* folded, const GNShape& sh) { return reinterpret_cast<unsigned int*>(folded + (long long)sh.B * sh.G); }
 static cudaError_t cl_zero_counters(float2* folded, const GNShape& sh, cudaStream_t st) {
   return cudaMemsetAsync(cl_counters(folded, sh), 0, sh.B * sizeof(unsigned int), st);

@@ -3,8 +3,8 @@
 // A small call (a roll-out step of a mesh network, a block on a few thousand points) is bound by its host side: in Python one launch
 // took 15 to 50 us (attributes of every tensor, torch.empty, the foreign-function call with up to 40 arguments).  The
 // functions do what the Python code did, argument by argument; gradients, dispatch and weight copies stay in Python.  Together with calls
-// that skip the autograd function where no gradient is wanted: a message-passing step of 1 885 nodes (three launches) 151 -> 77 us, a Transolver
-// block of 4 096 points (eleven) 372 -> 227 us, an AFNO block (twelve) 314 -> 227 us, a U-Net block with attention 613 -> 416 us.
+// that skip the autograd function where no gradient is wanted: a message-passing step of 1 885 nodes (three launches) 150 -> 78 us, a Transolver
+// block of 4 096 points (eleven) 373 -> 231 us, an AFNO block (twelve) 305 -> 223 us, a U-Net block with attention 601 -> 427 us.
 // As there, the interpreter's lock is released not only for the launch but also where memory is allocated or copied (an allocation may wait
 // for the device): every function reads its arguments, works in an `Unlocked` scope and wraps its results.
 #include <Python.h>
@@ -70,7 +70,7 @@ void check(const char* name, int code) {
 }
 uintptr_t address(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); }
 // 2-D view whose last dim is contiguous, whose row stride is a multiple of 8 and that starts on a 16-byte boundary
-// (the argument itself or a copy, which `own` holds: a second reference to a Python object's tensor costs 0.1 us)
+// (the argument itself or a copy, which `own` holds: a second count on a Python object's tensor goes through the interpreter)
 const Tensor& rowmajor2d(const Tensor& in, Tensor& own) {
   require(in.dim() == 2, "expected a matrix");
   const Tensor* t = &in;

@@ -7,8 +7,8 @@
 // An edge row needs its own 256 bytes, two gathered node rows (mostly from L2) and 256 bytes of result; run layer by layer the
 // same chain moves fifteen such rows through HBM.  Here everything between the sources and the result stays on the SM, and what
 // is left is the chain of a tile (product, epilogue, product, epilogue, product, normalisation) and its instructions: 1.4 M rows from
-// three sources take 0.32 ms (0.53 ms before the points marked * below), where the rows' own traffic is worth 0.15 ms; with what the
-// backward needs (five more rows each, 0.33 ms) 0.55 ms (0.73).
+// three sources take 0.31 ms (0.55 ms before the points marked * below), where its own traffic (row in and out, node rows once, indices:
+// 0.80 GB at the 6.57 TB/s of a copy) is worth 0.12 ms; with what the backward needs (five more rows each, 1.82 GB, 0.28 ms) 0.59 ms (0.76).
 //   * W1, W2, W3 (96 + 32 + 32 KB in bf16 for three sources) are loaded once per persistent CTA and stay in shared memory;
 // * * gathered rows are copied 16 bytes at a time (cp.async), eight lanes to a row of 128 bytes, in the 128-byte swizzle of a plain
 //     tile, so no gathered copy of the node features exists;

@@ -2,7 +2,7 @@
 
 ``mlp3_ln``: ``LayerNorm(act(act(x W1^T + b1) W2^T + b2) W3^T + b3) (+ post)`` where ``x`` is the concatenation of up to
 three 128-wide tables, each read through an optional row index (``csrc/mlp_fused.cuh``): the edge update of a
-MeshGraphNet step reads its node rows by TMA gathers, the node update reads (aggregate, node).  Layer by layer the same
+MeshGraphNet step copies its node rows one by one, the node update reads tiles of (aggregate, node).  Layer by layer the same
 chain (``ops.gather_rows``, ``ops.mlp_chain``, ``ops.layer_norm``) writes and re-reads every intermediate row.
 """
 from __future__ import annotations
