@@ -43,6 +43,16 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
   return t;
 }
 
+// One lane of a converged warp, the same one at every call.  For the branches in which a single thread issues tensor-core products or
+// bulk copies: their operands live in uniform registers, and after elect.sync the compiler knows that one thread is active, where under
+// `lane == 0` it provides for several.  Four products of 128 x 64 x 16, a commit and a wait on a ready barrier took a thread 505 cycles
+// under `lane == 0` and take 260 here; the tensor cores need 256 for four of 128 x 128 x 16.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kFaThreads, 1) flash_fwd_kernel(const __grid_c
 
   if (warp == 8) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, TILE);
       for (int kb = 0; kb < KB; ++kb) tma_load_3d(sQ + kb * BLK, &g.tmQ, q_full, kb * 64, q0, bh);
       int issued = 0;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kFaThreads, 1) flash_fwd_kernel(const __grid_c
     }
   } else if (warp == 9) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(128, D, false, !VT);
       bool ok = mbar_wait(q_full, 0, abort_flag, g.err, ERR_WAIT_FULL);

@@ -106,7 +106,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool up_ready = false, down_ready = false;
       for (int kb = 0; kb < num_kb; ++kb) {
         const int s = kb % STAGES;
@@ -163,7 +163,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(128, BNB, true, true);
       constexpr uint32_t idesc1 = make_idesc_bf16(128, 16, true, false);
       // ones tile as a K-major, unswizzled operand: every element it can address is 1.0

@@ -73,7 +73,7 @@ gemm_nt_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool up_ready = false, down_ready = false;
       for (int kb = 0; kb < num_kb; ++kb) {
         const int s = kb % STAGES;
@@ -134,7 +134,7 @@ gemm_nt_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(256, BNB, true, true);
       constexpr uint32_t idesc1 = make_idesc_bf16(256, 16, true, false);
       // ones tile as a K-major, unswizzled operand: every element it can address is 1.0 (in both CTAs)

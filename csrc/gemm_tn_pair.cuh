@@ -151,7 +151,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool up_ready = false, down_ready = false;
       for (int tile = cluster_id; tile < num_tiles; tile += num_clusters) {
@@ -201,7 +201,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer (leader CTA)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(256, BN, false, false);
       uint32_t it = 0, tc = 0;
       bool ok = true;

@@ -325,7 +325,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
       }
     } else if (warp == kMlpProducers) {
       // ------------------------------------------------------------------------------------- first products, in order
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc = make_idesc_bf16(kMlpRows, kMlpW, false, false);
         const uint32_t wlo = desc_lo(smem_u32(wts)), rlo = desc_lo(smem_u32(ring));
         uint32_t slot = 0, phase = 0, a = 0, turn = 0;
@@ -352,7 +352,7 @@ mlp3_ln_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ 
       }
     } else {
       // ----------------------------------------------------- second and third products of both groups, as they become ready
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc = make_idesc_bf16(kMlpRows, kMlpW, false, false);
         int left = 2 * (tiles > int(blockIdx.x) ? (tiles - int(blockIdx.x) - 1) / int(gridDim.x) + 1 : 0);
         uint32_t arrivals[2] = {0, 0};           // phases of aready[grp] consumed so far: two per tile

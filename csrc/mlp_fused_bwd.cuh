@@ -82,7 +82,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
   const uint32_t tmem = *tmem_slot;              // accumulators of the groups at 0 and 128, dW3 at 256, dW2 at 384
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(wfull, 4 * kMlpChunk);
       for (int k = 0; k < 2; ++k) tma_load_2d(wts + k * kMlpChunk, &tmW3t, wfull, k * 64, 0);
       for (int k = 0; k < 2; ++k) tma_load_2d(wts + (2 + k) * kMlpChunk, &tmW2t, wfull, k * 64, 0);
@@ -182,7 +182,7 @@ mlp3_bwd_kernel(const __grid_constant__ CUtensorMap tmD, const __grid_constant__
       for (int i = 0; i < 4; ++i) { atomicAdd(g.db3 + col + i, s[0][i]); atomicAdd(g.db2 + col + i, s[1][i]); }
   } else if (warp == 3) {
     // --------------------------------------------------------------------------------------- dx3 and act(z2) tiles
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t issued[2] = {0, 0};
 #pragma unroll 1
       for (int n = 0; n < mine; ++n) {

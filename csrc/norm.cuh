@@ -167,7 +167,7 @@ layernorm_fwd_stream_kernel(const __nv_bfloat16* __restrict__ x, const float* __
   }
   __syncthreads();
   if (warp == kLnWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 1, issued = 0;
       for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -293,7 +293,7 @@ layernorm_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
 #pragma unroll
     for (int j = 0; j < 8; ++j) dg[v][j] = db[v][j] = 0.f;
   if (warp == kLnWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t ph = 1, issued = 0;
       for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
