@@ -9,6 +9,7 @@
 #include "gemm_tn_pair.cuh"
 #include "gemm_nt.cuh"
 #include "gemm_nt_pair.cuh"
+#include "conv3_wgrad.cuh"
 #include "norm.cuh"
 #include "graph.cuh"
 #include "peer.cuh"
@@ -309,6 +310,7 @@ int pnm_conv2d_wgrad_nhwc(const void* dy, const void* x, float* out, float* cols
   c.flag_up = reinterpret_cast<const uint32_t*>(flag_up); c.flag_down = reinterpret_cast<const uint32_t*>(flag_down);
   c.halo_epoch = epoch; c.halo_budget_s = budget_s;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (pnm::conv3_wgrad_applicable(c)) return pnm::launch_conv3_wgrad(c, g_num_sms, g_err_ptr, st);
   if (pair_gemm_enabled() && pnm::pair_gemm_nt_applicable(c)) {
     if ((9 * cin) % 256 == 0) return pnm::launch_gemm_nt_pair<256>(c, g_num_sms, g_err_ptr, st);
     return pnm::launch_gemm_nt_pair<128>(c, g_num_sms, g_err_ptr, st);

@@ -232,6 +232,27 @@ def test_conv2d_same_implicit_gemm(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 4, 16, 128, 128), (2, 33, 31, 64, 64), (1, 45, 50, 192, 72), (3, 29, 47, 128, 200),
+                                            (1, 64, 64, 320, 136), (1, 130, 126, 128, 256), (2, 24, 24, 512, 512)])
+def test_conv3x3_weight_gradient_by_columns_of_taps(n, h, w, cin, cout):
+    """Patches that the image's edges cut, one or two boxes of 64 input channels, ragged output channels; (1, 4, 16) is left to the
+    reduction GEMM.  A product of two bf16 values is exact in fp32 and 16 of them enter an accumulator together: each of the
+    pixels / 16 additions may lose 2^-23 of the sum."""
+    from physicsnemo_b200.ops import conv as C
+
+    g = torch.Generator(device="cuda").manual_seed(n * h + w)
+    x = torch.randn(n, h, w, cin, generator=g, device="cuda").bfloat16()
+    dy = torch.randn(n, h, w, cout, generator=g, device="cuda").bfloat16()
+    dw, db = C.wgrad3x3(dy, x, True)
+    ref = torch.nn.grad.conv2d_weight(x.permute(0, 3, 1, 2).double(), (cout, cin, 3, 3), dy.permute(0, 3, 1, 2).double(), padding=1)
+    ref, ref_b = ref.permute(0, 2, 3, 1).reshape(cout, -1), dy.double().sum((0, 1, 2))
+    bound = max(16, n * h * w / 16) * 2.0 ** -23
+    assert float((dw - ref).norm() / ref.norm()) < bound
+    assert float((db - ref_b).norm() / ref_b.norm()) < bound
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 512), (4000, 768, 1024), (32400, 1096, 768), (2304, 520, 584)])
 @pytest.mark.parametrize("mode", ["plain", "gelu_z", "add", "dgelu", "drelu"])
 def test_gemm_tn_cta_pair_tiles(M, N, K, mode):
