@@ -31,16 +31,29 @@ constexpr int kPairThreads = 320;
 
 // Two staging buffers per epilogue warp in every mode: a third buffer for the auxiliary operand costs a stage and
 // measured slower on K = 3072 (132 vs 124 us) and no faster on K = 768.
+//
+// MODE_CONV3 (3 x 3 convolutions, no halo rows of peers): the three taps of a filter column read windows of the image that differ by
+// whole rows of 16 pixels = 2048 bytes, so ONE box of 10 x 16 pixels holds the A operand of all three, each starting on a
+// 1024-byte boundary: 20 KB per three k-blocks instead of 48 KB.  A and B then come through rings of their own: a slot of A lasts three
+// k-blocks, a slot of B one.  One image 512 x 512, 128 -> 128 / 256 -> 128 / 128 -> 256 channels: 69 / 115 / 99 us (1.13 / 1.35 / 1.56
+// PFLOP/s; a box per tap 113 / 205 / 119 us); 2 x 256 x 256, 512 -> 256: 174 us (209); 64 x 64, 512 -> 512: 27 us (tiles of one CTA 57).
+constexpr int MODE_CONV3 = 3;
+constexpr int kConv3ABytes = (kConvTileH + 2) * kConvTileW * kBK * 2;
+
 template <int BN, int MODE>
 struct PairCfg {
+  static constexpr bool RINGS = MODE == MODE_CONV3;
   static constexpr int NBUF = 2;
   static constexpr int B_ROWS = BN / 2;                             // rows of B (output columns) this CTA loads
-  static constexpr int STAGE_BYTES = kBM * kBK * 2 + B_ROWS * kBK * 2;
+  static constexpr int B_BYTES = B_ROWS * kBK * 2;
+  static constexpr int STAGE_BYTES = kBM * kBK * 2 + B_BYTES;
   static constexpr int STAGING = 8 * NBUF * kChunkBytes;           // 8 epilogue warps x NBUF buffers x 4 KB
   static constexpr int BUDGET = 232448 - 1024 - 512;
   static constexpr int STAGES_RAW = (BUDGET - STAGING) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_RAW > 6 ? 6 : STAGES_RAW;
-  static constexpr int SMEM = 1024 + STAGES * STAGE_BYTES + STAGING + 512;
+  static constexpr int A_SLOTS = BN == 128 ? 4 : 3, B_SLOTS = BN == 128 ? 9 : 6;      // MODE_CONV3
+  static constexpr int STAGES = RINGS ? A_SLOTS + B_SLOTS : STAGES_RAW > 6 ? 6 : STAGES_RAW;      // pairs of full / empty barriers
+  static constexpr int OPERANDS = RINGS ? A_SLOTS * kConv3ABytes + B_SLOTS * B_BYTES : STAGES * STAGE_BYTES;
+  static constexpr int SMEM = 1024 + OPERANDS + STAGING + 512;
   static constexpr int TMEM_COLS = 2 * BN;                         // two accumulators
   static_assert(BN == 128 || BN == 256, "pair tile is 256 x 128 or 256 x 256");
   static_assert(STAGES >= 4 && SMEM <= 232448, "paired GEMM: shared memory budget");
@@ -117,9 +130,9 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int NBUF = Cfg::NBUF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* staging = base + STAGES * Cfg::STAGE_BYTES;
+  uint8_t* staging = base + Cfg::OPERANDS;
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + Cfg::STAGING);
-  uint64_t* full = bars;                              // leader's copies are the live ones
+  uint64_t* full = bars;                              // leader's copies are the live ones (MODE_CONV3: slots of A, then slots of B)
   uint64_t* empty = bars + STAGES;                    // per CTA, released by the leader's commits
   uint64_t* tfull = bars + 2 * STAGES;                // per CTA, published by the leader's commits
   uint64_t* tempty = tfull + 2;                       // leader's copies are the live ones (16 arrivals)
@@ -149,7 +162,33 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
+  if (MODE == MODE_CONV3 && warp == 0) {
+    // ------------------------------------- producer of the 3 x 3 convolution (both CTAs): columns of taps, see MODE_CONV3
+    if (elect_one()) {
+      uint8_t* b_slots = base + Cfg::A_SLOTS * kConv3ABytes;
+      uint32_t ia = 0, ib = 0;
+      bool ok = true;
+      for (int tile = cluster_id; ok && tile < num_tiles; tile += num_clusters) {
+        const int mt = tile / g.num_n_tiles, nt = tile % g.num_n_tiles;
+        const int col0 = nt * BN + int(rank) * Cfg::B_ROWS;
+        int cn, cy0, cx0;
+        conv_tile_origin(g, 2 * mt + int(rank), cn, cy0, cx0);
+        for (int c0 = 0; ok && c0 < g.cin; c0 += kBK)
+          for (int kx = 0; ok && kx < 3; ++kx, ++ia) {
+            const int sa = ia % Cfg::A_SLOTS;
+            if (!mbar_wait(&empty[sa], ((ia / Cfg::A_SLOTS) & 1) ^ 1, abort_flag, g.err, ERR_WAIT_EMPTY)) { ok = false; break; }
+            if (leader) mbar_expect_tx(&full[sa], 2 * kConv3ABytes);
+            tma_load_4d_pair(base + sa * kConv3ABytes, &tmA, map_to_cta(smem_u32(&full[sa]), 0), c0, cx0 + kx - 1, cy0 - 1, cn);
+            for (int ky = 0; ky < 3; ++ky, ++ib) {
+              const int sb = ib % Cfg::B_SLOTS, bar = Cfg::A_SLOTS + sb;
+              if (!mbar_wait(&empty[bar], ((ib / Cfg::B_SLOTS) & 1) ^ 1, abort_flag, g.err, ERR_WAIT_EMPTY)) { ok = false; break; }
+              if (leader) mbar_expect_tx(&full[bar], 2 * Cfg::B_BYTES);
+              tma_load_2d_pair(b_slots + sb * Cfg::B_BYTES, &tmB, map_to_cta(smem_u32(&full[bar]), 0), (3 * ky + kx) * g.cin + c0, col0);
+            }
+          }
+      }
+    }
+  } else if (warp == 0) {
     // ------------------------------------------------------------ producer (both CTAs)
     if (elect_one()) {
       uint32_t it = 0;
@@ -211,18 +250,36 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (!mbar_wait(&tempty[acc], aph ^ 1, abort_flag, g.err, ERR_WAIT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&full[s], ph, abort_flag, g.err, ERR_WAIT_FULL)) { ok = false; break; }
-          tc_fence_after();
-          uint8_t* sa = base + s * Cfg::STAGE_BYTES;
-          const uint64_t ad = make_smem_desc(smem_u32(sa), 16, 1024, 2);
-          const uint64_t bd = make_smem_desc(smem_u32(sa + kBM * kBK * 2), 16, 1024, 2);
+        if constexpr (MODE == MODE_CONV3) {
+          // `it` counts k-blocks: one slot of B each, one slot of A for three
+          for (int kb = 0; kb < num_kb; ++kb, ++it) {
+            const uint32_t ia = it / 3, ky = it % 3;
+            const int sa = ia % Cfg::A_SLOTS, sb = it % Cfg::B_SLOTS, bar = Cfg::A_SLOTS + sb;
+            if (ky == 0 && !mbar_wait(&full[sa], (ia / Cfg::A_SLOTS) & 1, abort_flag, g.err, ERR_WAIT_FULL)) { ok = false; break; }
+            if (!mbar_wait(&full[bar], (it / Cfg::B_SLOTS) & 1, abort_flag, g.err, ERR_WAIT_FULL)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t ad = make_smem_desc(smem_u32(base + sa * kConv3ABytes + ky * (kConvTileW * 128)), 16, 1024, 2);
+            const uint64_t bd = make_smem_desc(smem_u32(base + Cfg::A_SLOTS * kConv3ABytes + sb * Cfg::B_BYTES), 16, 1024, 2);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            umma_f16_pair(d, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair(&empty[s]);
+            for (int k = 0; k < kBK / 16; ++k)
+              umma_f16_pair(d, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit_pair(&empty[bar]);
+            if (ky == 2) umma_commit_pair(&empty[sa]);
+          }
+        } else {
+          for (int kb = 0; kb < num_kb; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t ph = (it / STAGES) & 1;
+            if (!mbar_wait(&full[s], ph, abort_flag, g.err, ERR_WAIT_FULL)) { ok = false; break; }
+            tc_fence_after();
+            uint8_t* sa = base + s * Cfg::STAGE_BYTES;
+            const uint64_t ad = make_smem_desc(smem_u32(sa), 16, 1024, 2);
+            const uint64_t bd = make_smem_desc(smem_u32(sa + kBM * kBK * 2), 16, 1024, 2);
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k)
+              umma_f16_pair(d, ad + 2 * k, bd + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_commit_pair(&empty[s]);
+          }
         }
         if (ok) umma_commit_pair(&tfull[acc]);
       }
@@ -415,6 +472,16 @@ inline bool pair_gemm_applicable(const GemmCall& c) {
   return c.Z != nullptr && c.K >= 256 && c.N >= 1024;
 }
 
+// Tile of a 3 x 3 convolution (MODE_CONV3): 256 or 128 output channels wide.  The wide tile reads fewer bytes per product (one image
+// 512 x 512, 128 -> 256 channels: 100 against 119 us), the narrow one splits a small map over more SMs (64 x 64, 512 -> 512: 26.6 against
+// 34.8 us; 120 x 120, 256 -> 256, 60 wide tiles: the same): rounds of tiles are compared, the narrow one's at 0.6 of the wide one's time.
+inline int conv3_tile_width(const GemmCall& c, int num_sms) {
+  const long long pairs = ((long long)c.img_n * ((c.img_h + kConvTileH - 1) / kConvTileH) * ((c.img_w + kConvTileW - 1) / kConvTileW) + 1) / 2;
+  const int clusters = num_sms / 2 > 0 ? num_sms / 2 : 1;
+  const long long wide = (pairs * ((c.N + 255) / 256) + clusters - 1) / clusters, narrow = (pairs * ((c.N + 127) / 128) + clusters - 1) / clusters;
+  return c.N > 128 && 10 * wide <= 6 * narrow ? 256 : 128;
+}
+
 template <int BN, int MODE>
 inline int launch_gemm_tn_pair(const GemmCall& c, int num_sms, int* err_word, cudaStream_t stream) {
   using Cfg = PairCfg<BN, MODE>;
@@ -425,8 +492,10 @@ inline int launch_gemm_tn_pair(const GemmCall& c, int num_sms, int* err_word, cu
   g.err = err_word;
   int tiles128 = (c.M + kBM - 1) / kBM;
   if (c.conv) {
-    if (MODE != MODE_PLAIN) return -19;
-    if (make_tmap_nhwc_b16(&tA, c.A, c.img_n, c.img_h, c.img_w, c.cin, kConvTileH, kConvTileW)) return -10;
+    if (MODE != MODE_PLAIN && MODE != MODE_CONV3) return -19;
+    if (MODE == MODE_CONV3 && (c.ksize != 3 || c.halo || c.cin % kBK)) return -19;
+    const int box_h = MODE == MODE_CONV3 ? kConvTileH + 2 : kConvTileH;
+    if (make_tmap_nhwc_b16(&tA, c.A, c.img_n, c.img_h, c.img_w, c.cin, box_h, kConvTileW)) return -10;
     if (make_tmap_nhwc_b16(&tC, c.C, c.img_n, c.img_h, c.img_w, c.N, 2, kConvTileW)) return -13;
     g.conv = 1; g.cin = c.cin; g.ksize = c.ksize; g.pad = c.ksize / 2; g.img_h = c.img_h; g.img_n = c.img_n;
     g.tiles_x = (c.img_w + kConvTileW - 1) / kConvTileW;

@@ -232,6 +232,24 @@ def test_conv2d_same_implicit_gemm(shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 1, 1, 64, 64), (1, 8, 16, 64, 72), (3, 7, 15, 128, 128), (1, 17, 33, 192, 136), (2, 41, 50, 64, 256),
+                                            (1, 64, 64, 512, 512), (1, 130, 126, 128, 384), (1, 200, 176, 128, 256)])
+def test_conv3x3_forward_by_columns_of_taps(n, h, w, cin, cout):
+    """One tile and less, an odd number of pixel tiles (half a pair is empty), ragged edges and channels, narrow and wide tiles.  Against
+    64 bits on the same bf16 operands only the rounding of the result is left: at most 2^-8 of a value."""
+    from physicsnemo_b200.ops import conv as C
+
+    g = torch.Generator(device="cuda").manual_seed(n * h + w)
+    x = torch.randn(n, cin, h, w, generator=g, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    wt = (torch.randn(cout, cin, 3, 3, generator=g, device="cuda") / (9 * cin) ** 0.5).bfloat16()
+    b = torch.randn(cout, generator=g, device="cuda")
+    y = C.conv2d_same(x, wt, b)
+    ref = torch.nn.functional.conv2d(x.double(), wt.double(), b.double(), padding=1)
+    assert float(((y - ref).abs() - 2.0 ** -8 * ref.abs()).max()) < 1e-4            # sums that cancel: 4 608 terms of fp32 rounding
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n,h,w,cin,cout", [(1, 4, 16, 128, 128), (2, 33, 31, 64, 64), (1, 45, 50, 192, 72), (3, 29, 47, 128, 200),
                                             (1, 64, 64, 320, 136), (1, 130, 126, 128, 256), (2, 24, 24, 512, 512)])
 def test_conv3x3_weight_gradient_by_columns_of_taps(n, h, w, cin, cout):
