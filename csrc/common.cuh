@@ -299,6 +299,11 @@ __device__ __forceinline__ float ex2_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float lg2_fast(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // 2^x on the FMA / ALU pipes (no special-function unit): round-to-nearest split x = n + f, f in [-0.5, 0.5], cubic for 2^f
 // (relative error 1e-4, below bf16 resolution), then n is added to the exponent field.  Inputs below -126 give 0.
 __device__ __forceinline__ float ex2_poly(float x) {
@@ -311,6 +316,38 @@ __device__ __forceinline__ float ex2_poly(float x) {
   const float r = __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
   return x < -126.f ? 0.f : r;
 }
+// Two fp32 values per instruction (add / mul / fma.rn.f32x2, the same roundings as one by one).
+__device__ __forceinline__ uint64_t f2_make(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f2_all(float a) { return f2_make(a, a); }
+__device__ __forceinline__ uint64_t f2_tanh(uint64_t v) {
+  const float2 x = f2_get(v);
+  return f2_make(tanh_fast(x.x), tanh_fast(x.y));
+}
+
 // GELU in its tanh form (|gelu_tanh - gelu_erf| < 1e-3, below bf16 resolution for O(1) values).
 __device__ __forceinline__ float gelu_f(float x) {
   const float u = x * (0.7978845608f + 0.0356774081f * x * x), h = 0.5f * x;
@@ -332,6 +369,30 @@ __device__ __forceinline__ float silu_grad_f(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
+// The four for two values: as above, operation by operation.
+__device__ __forceinline__ uint64_t gelu_f2(uint64_t x) {
+  const uint64_t x2 = f2_mul(x, x), h = f2_mul(x, f2_all(0.5f));
+  const uint64_t u = f2_mul(x, f2_fma(f2_all(0.0356774081f), x2, f2_all(0.7978845608f)));
+  return f2_fma(h, f2_tanh(u), h);
+}
+__device__ __forceinline__ uint64_t silu_f2(uint64_t x) {
+  const uint64_t h = f2_mul(x, f2_all(0.5f));
+  return f2_fma(h, f2_tanh(h), h);
+}
+// 0.5 (1 + t) + 0.5 x (1 - t^2) u'
+__device__ __forceinline__ uint64_t gelu_grad_f2(uint64_t x) {
+  const uint64_t x2 = f2_mul(x, x);
+  const uint64_t t = f2_tanh(f2_mul(x, f2_fma(f2_all(0.0356774081f), x2, f2_all(0.7978845608f))));
+  const uint64_t du = f2_fma(f2_all(0.1070322243f), x2, f2_all(0.7978845608f));
+  const uint64_t p = f2_fma(f2_mul(t, f2_all(-1.f)), t, f2_all(1.f));
+  return f2_fma(f2_mul(f2_mul(x, f2_all(0.5f)), p), du, f2_fma(t, f2_all(0.5f), f2_all(0.5f)));
+}
+// s (1 + x (1 - s))
+__device__ __forceinline__ uint64_t silu_grad_f2(uint64_t x) {
+  const uint64_t s = f2_fma(f2_tanh(f2_mul(x, f2_all(0.5f))), f2_all(0.5f), f2_all(0.5f));
+  return f2_mul(s, f2_fma(x, f2_fma(s, f2_all(-1.f), f2_all(1.f)), f2_all(1.f)));
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
@@ -339,6 +400,16 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(h);
+}
+
+__device__ __forceinline__ uint32_t f2_to_bf16x2(uint64_t v) {
+  const float2 f = f2_get(v);
+  return pack_bf16x2(f.x, f.y);
+}
+__device__ __forceinline__ uint64_t f2_from_bf16x2(uint32_t u) {      // the upper halves of two floats
+  uint32_t a, b;
+  a = u << 16; b = u & 0xffff0000u;
+  return f2_make(__uint_as_float(a), __uint_as_float(b));
 }
 
 }  // namespace pnm

@@ -6,9 +6,12 @@
 //   warps 2..   epilogue: TMEM -> registers -> fused math -> swizzled staging -> TMA store; one warp per 32 x 64 block of the
 //               tile, i.e. 8 warps for 128 columns and 16 for 256.  With 8 warps on 256 columns (two blocks each) the products
 //               with a heavy epilogue were bound by the latency of its instructions, not by memory or the tensor cores:
-//               1 M rows, softmax 256 -> 512 0.85 -> 0.57 ms.  With an auxiliary operand the tiles were 128 columns wide and
+//               1 M rows, softmax 256 -> 512 0.85 -> 0.53 ms.  With an auxiliary operand the tiles were 128 columns wide and
 //               read A twice as often: GELU' 256 -> 1024 1.40 -> 0.99 ms, softmax backward 512 -> 512 1.28 -> 0.83 ms.
 // Two TMEM accumulators let the epilogue of tile i overlap the main loop of tile i+1.
+// The arithmetic of an epilogue works on two columns per instruction (f2_*): one by one, a softmax took 20 instructions a value, its
+// backward 35, GELU' 20.  1 M rows, softmax 256 -> 512 532 -> 352 us (its writes alone are worth 262: a stream of writes runs at 3.9 TB/s
+// here), softmax backward 512 -> 512 986 -> 850 us (bound by the operands' way from L2, 448 KB a tile), GELU' 256 -> 1024 990 -> 950 us.
 //
 // Fused epilogues (all optional, all applied on fp32 values):
 //   x = (acc + bias[col]) * scale[col]            (scale before the activation unless scale_post)
@@ -130,46 +133,136 @@ struct GemmCfg {
   static_assert(STAGES >= 2, "not enough shared memory for a pipeline");
 };
 
-__device__ __forceinline__ void stage_write_row(uint8_t* buf, int lane, const float* v) {
-  // 64 fp32 -> 64 bf16 = 8 chunks of 16 bytes, chunk j of row r lands at (j ^ (r & 7)).
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    uint4 u;
-    u.x = pack_bf16x2(v[8 * j + 0], v[8 * j + 1]);
-    u.y = pack_bf16x2(v[8 * j + 2], v[8 * j + 3]);
-    u.z = pack_bf16x2(v[8 * j + 4], v[8 * j + 5]);
-    u.w = pack_bf16x2(v[8 * j + 6], v[8 * j + 7]);
-    *reinterpret_cast<uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4)) = u;
-  }
-}
-__device__ __forceinline__ void stage_write16(uint8_t* buf, int lane, int k, const float* x) {
+// The epilogues work on pairs of columns (f2_*, common.cuh): a row's values are an array of 32 pairs.
+// 64 columns -> 64 bf16 = 8 chunks of 16 bytes, chunk j of row r lands at (j ^ (r & 7)).
+__device__ __forceinline__ void stage_write16(uint8_t* buf, int lane, int k, const uint64_t* x) {
 #pragma unroll
   for (int j = 0; j < 2; ++j)
     *reinterpret_cast<uint4*>(buf + lane * 128 + (((2 * k + j) ^ (lane & 7)) << 4)) =
-        make_uint4(pack_bf16x2(x[8 * j], x[8 * j + 1]), pack_bf16x2(x[8 * j + 2], x[8 * j + 3]), pack_bf16x2(x[8 * j + 4], x[8 * j + 5]),
-                   pack_bf16x2(x[8 * j + 6], x[8 * j + 7]));
+        make_uint4(f2_to_bf16x2(x[4 * j]), f2_to_bf16x2(x[4 * j + 1]), f2_to_bf16x2(x[4 * j + 2]), f2_to_bf16x2(x[4 * j + 3]));
+}
+__device__ __forceinline__ void stage_write_row(uint8_t* buf, int lane, const uint64_t* v) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) stage_write16(buf, lane, k, v + 8 * k);
 }
 // columns [16 k, 16 k + 16) of a staged row
-__device__ __forceinline__ void stage_read16(const uint8_t* buf, int lane, int k, float* a) {
+__device__ __forceinline__ void stage_read16(const uint8_t* buf, int lane, int k, uint64_t* a) {
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const uint4 u = *reinterpret_cast<const uint4*>(buf + lane * 128 + (((2 * k + j) ^ (lane & 7)) << 4));
-    float2 f;
-    f = unpack_bf16x2(u.x); a[8 * j + 0] = f.x; a[8 * j + 1] = f.y;
-    f = unpack_bf16x2(u.y); a[8 * j + 2] = f.x; a[8 * j + 3] = f.y;
-    f = unpack_bf16x2(u.z); a[8 * j + 4] = f.x; a[8 * j + 5] = f.y;
-    f = unpack_bf16x2(u.w); a[8 * j + 6] = f.x; a[8 * j + 7] = f.y;
+    a[4 * j] = f2_from_bf16x2(u.x); a[4 * j + 1] = f2_from_bf16x2(u.y); a[4 * j + 2] = f2_from_bf16x2(u.z); a[4 * j + 3] = f2_from_bf16x2(u.w);
   }
 }
-__device__ __forceinline__ void stage_read_row(const uint8_t* buf, int lane, float* a) {
+// 32 columns of a row of the accumulator
+__device__ __forceinline__ void tmem_ld_pairs(uint32_t taddr, uint64_t* v) {
+  float t[32];
+  tmem_ld32(taddr, t);
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = f2_make(t[2 * j], t[2 * j + 1]);
+}
+// v <- v + p or v * p for the 2 NP columns from c0 on; p: vector of the columns (`vec`: whole and 16-byte aligned here), N of them
+template <int NP, bool MUL>
+__device__ __forceinline__ void epi_vector(uint64_t* v, const float* __restrict__ p, int c0, int N, bool vec) {
+  if (vec) {
+#pragma unroll
+    for (int j = 0; j < NP / 2; ++j) {
+      const float4 b = __ldg(reinterpret_cast<const float4*>(p + c0) + j);
+      v[2 * j] = MUL ? f2_mul(v[2 * j], f2_make(b.x, b.y)) : f2_add(v[2 * j], f2_make(b.x, b.y));
+      v[2 * j + 1] = MUL ? f2_mul(v[2 * j + 1], f2_make(b.z, b.w)) : f2_add(v[2 * j + 1], f2_make(b.z, b.w));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      const int c = c0 + 2 * j;
+      const uint64_t b = f2_make(c < N ? __ldg(p + c) : 0.f, c + 1 < N ? __ldg(p + c + 1) : 0.f);
+      v[j] = MUL ? f2_mul(v[j], b) : f2_add(v[j], b);
+    }
+  }
+}
+template <int NP>
+__device__ __forceinline__ void epi_act(uint64_t* v, int act) {
+  switch (act) {
+    case ACT_GELU:
+#pragma unroll
+      for (int j = 0; j < NP; ++j) v[j] = gelu_f2(v[j]);
+      break;
+    case ACT_SILU:
+#pragma unroll
+      for (int j = 0; j < NP; ++j) v[j] = silu_f2(v[j]);
+      break;
+    case ACT_RELU:
+#pragma unroll
+      for (int j = 0; j < NP; ++j) {
+        const float2 x = f2_get(v[j]);
+        v[j] = f2_make(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f));
+      }
+      break;
+    default: break;
+  }
+}
+// 16 columns with the auxiliary values of the same columns (all modes but the softmax backward)
+__device__ __forceinline__ void epi_aux16(uint64_t* v, const uint64_t* a, int mode) {
+  switch (mode) {
+    case AUX_ADD:
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = f2_add(v[j], a[j]);
+      break;
+    case AUX_DGELU:
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = f2_mul(v[j], gelu_grad_f2(a[j]));
+      break;
+    case AUX_DSILU:
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = f2_mul(v[j], silu_grad_f2(a[j]));
+      break;
+    case AUX_DRELU:
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 x = f2_get(v[j]), z = f2_get(a[j]);
+        v[j] = f2_make(z.x > 0.f ? x.x : 0.f, z.y > 0.f ? x.y : 0.f);
+      }
+      break;
+    default: break;
+  }
+}
+// softmax over a thread's 64 columns
+__device__ __forceinline__ void epi_softmax64(uint64_t* v) {
+  float m[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 x = f2_get(v[i]);
+    m[i] = fmaxf(x.x, x.y);
+  }
+#pragma unroll
+  for (int j = 4; j < 32; ++j) {
+    const float2 x = f2_get(v[j]);
+    m[j & 3] = fmaxf(m[j & 3], fmaxf(x.x, x.y));
+  }
+  const uint64_t neg = f2_all(-fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]))), log2e = f2_all(1.4426950409f);
+  uint64_t s[2] = {0, 0};
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const float2 x = f2_get(f2_mul(f2_add(v[j], neg), log2e));
+    v[j] = f2_make(ex2_fast(x.x), ex2_fast(x.y));
+    s[j & 1] = f2_add(s[j & 1], v[j]);
+  }
+  const float2 t = f2_get(f2_add(s[0], s[1]));
+  const uint64_t inv = f2_all(__frcp_rn(t.x + t.y));
+#pragma unroll
+  for (int j = 0; j < 32; ++j) v[j] = f2_mul(v[j], inv);
+}
+// softmax backward of 16 columns: v <- a (v - dot); the sum of v log2(a) where a group's sum is wanted.  Where a is 0, so is v: the
+// logarithm is that of the smallest normal number and the product 0.
+template <bool SUM>
+__device__ __forceinline__ void epi_dsoftmax16(uint64_t* v, const uint64_t* a, uint64_t neg_dot, uint64_t& sum) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    uint4 u = *reinterpret_cast<const uint4*>(buf + lane * 128 + ((j ^ (lane & 7)) << 4));
-    float2 f;
-    f = unpack_bf16x2(u.x); a[8 * j + 0] = f.x; a[8 * j + 1] = f.y;
-    f = unpack_bf16x2(u.y); a[8 * j + 2] = f.x; a[8 * j + 3] = f.y;
-    f = unpack_bf16x2(u.z); a[8 * j + 4] = f.x; a[8 * j + 5] = f.y;
-    f = unpack_bf16x2(u.w); a[8 * j + 6] = f.x; a[8 * j + 7] = f.y;
+    v[j] = f2_mul(a[j], f2_add(v[j], neg_dot));
+    if (SUM) {
+      const float2 p = f2_get(a[j]);
+      sum = f2_fma(v[j], f2_make(lg2_fast(fmaxf(p.x, 1.17549435e-38f)), lg2_fast(fmaxf(p.y, 1.17549435e-38f))), sum);
+    }
   }
 }
 
@@ -333,7 +426,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     auto issue_aux = [&](uint32_t item) {
       int r0, c0;
       if (!item_coords(item, r0, c0)) return;
-      if (lane == 0) {
+      if (elect_one()) {
         tma_store_wait_read<NBUF - 2 < 0 ? 0 : NBUF - 2>();
         const int b = item % NBUF;
         mbar_expect_tx(&mybar[b], kChunkBytes);
@@ -341,6 +434,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
     };
     if (MODE == MODE_AUX) issue_aux(0);
+    auto add_group = [&](uint64_t sum, int c0, bool wanted) {      // of v log2(a), over the warp's 32 rows
+      const float2 t = f2_get(sum);
+      float gs = t.x + t.y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+      if (lane == 0 && c0 < g.N && wanted) atomicAdd(g.group_out + (c0 >> 6), gs * 0.6931471806f);
+    };
 
     uint32_t item = 0;
     for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++tc) {
@@ -357,263 +457,170 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // 16 columns at a time, straight from TMEM into the staged auxiliary tile (which the result replaces): a row of 64 and
           // its auxiliary values do not fit the 96 registers of a thread.  The softmax backward reads the accumulator twice.
           const bool store_ok = (r0 < g.M) && (c0 < g.N), full_cols = (c0 + 64 <= g.N);
+          const bool scale_vec = full_cols && !(reinterpret_cast<uintptr_t>(g.scale) & 15);
           uint8_t* arow = stg + (item % NBUF) * kChunkBytes;
-          auto load16 = [&](int k, float* x) {
-            tmem_ld16(taddr + 16 * k, x);
+          auto load16 = [&](int k, uint64_t* x) {
+            float t[16];
+            tmem_ld16(taddr + 16 * k, t);
             tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = f2_make(t[2 * j], t[2 * j + 1]);
             const int c = c0 + 16 * k;
-            if (g.bias) {
-              if (full_cols) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + c) + j);
-                  x[4 * j] += b.x; x[4 * j + 1] += b.y; x[4 * j + 2] += b.z; x[4 * j + 3] += b.w;
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) if (c + j < g.N) x[j] += __ldg(g.bias + c + j);
-              }
-            }
-            if (g.scale && !g.scale_post) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) if (c + j < g.N) x[j] *= __ldg(g.scale + c + j);
-            }
-            if (g.act == ACT_GELU) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) x[j] = gelu_f(x[j]);
-            } else if (g.act == ACT_SILU) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) x[j] = silu_f(x[j]);
-            } else if (g.act == ACT_RELU) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) x[j] = fmaxf(x[j], 0.f);
-            }
+            if (g.bias) epi_vector<8, false>(x, g.bias, c, g.N, full_cols);
+            if (g.scale && !g.scale_post) epi_vector<8, true>(x, g.scale, c, g.N, scale_vec);
+            if (g.act) epi_act<8>(x, g.act);
           };
           if (!mbar_wait(&mybar[item % NBUF], (item / NBUF) & 1, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
-          float dot = 0.f, gs = 0.f;
+          uint64_t neg_dot = 0, gs = 0;
           if (g.aux_mode == AUX_DSOFTMAX) {
+            uint64_t d[2] = {0, 0};
 #pragma unroll 1
             for (int k = 0; k < 4; ++k) {
-              float x[16], a[16];
+              uint64_t x[8], a[8];
               load16(k, x);
               stage_read16(arow, lane, k, a);
 #pragma unroll
-              for (int j = 0; j < 16; ++j) dot += x[j] * a[j];
+              for (int j = 0; j < 8; ++j) d[j & 1] = f2_fma(x[j], a[j], d[j & 1]);
             }
+            const float2 t = f2_get(f2_add(d[0], d[1]));
+            neg_dot = f2_all(-(t.x + t.y));
           }
 #pragma unroll 1
           for (int k = 0; k < 4; ++k) {
-            float x[16], a[16];
+            uint64_t x[8], a[8];
             load16(k, x);
             stage_read16(arow, lane, k, a);
-            switch (g.aux_mode) {                // the modes that come here: those with arithmetic
-              case AUX_DGELU:
-#pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] *= gelu_grad_f(a[j]);
-                break;
-              case AUX_DSILU:
-#pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] *= silu_grad_f(a[j]);
-                break;
-              case AUX_DSOFTMAX:
-#pragma unroll
-                for (int j = 0; j < 16; ++j) x[j] = a[j] * (x[j] - dot);
-                if (g.group_out) {
-#pragma unroll
-                  for (int j = 0; j < 16; ++j) gs += (a[j] > 0.f) ? x[j] * __logf(a[j]) : 0.f;
-                }
-                break;
-              default: break;
-            }
-            if (g.scale && g.scale_post) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) if (c0 + 16 * k + j < g.N) x[j] *= __ldg(g.scale + c0 + 16 * k + j);
-            }
+            if (g.aux_mode != AUX_DSOFTMAX) epi_aux16(x, a, g.aux_mode);
+            else if (g.group_out) epi_dsoftmax16<true>(x, a, neg_dot, gs);
+            else epi_dsoftmax16<false>(x, a, neg_dot, gs);
+            if (g.scale && g.scale_post) epi_vector<8, true>(x, g.scale, c0 + 16 * k, g.N, scale_vec);
             stage_write16(arow, lane, k, x);
           }
           tc_fence_before();
           fence_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive(&tempty[acc]);
             if (store_ok) tma_store_2d(arow, &tmC, c0, r0);
             tma_store_commit();
           }
-          if (g.group_out) {                     // only the softmax backward has one
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
-            if (lane == 0 && c0 < g.N && g.aux_mode == AUX_DSOFTMAX) atomicAdd(g.group_out + (c0 >> 6), gs);
-          }
+          if (g.group_out) add_group(gs, c0, g.aux_mode == AUX_DSOFTMAX);      // only the softmax backward has one
           ++item;
           continue;
         }
-        float v[64];
-        tmem_ld32(taddr, v);
-        tmem_ld32(taddr + 32, v + 32);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[acc]);
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
         const bool full_cols = (c0 + 64 <= g.N);
         const int vo = g.batch_m_tiles ? (r0 / (kBM * g.batch_m_tiles)) * g.N : 0;   // offset of the problem's bias / scale
-        // ---- x = (acc + bias) * scale
-        if (g.bias) {
-          if (full_cols && !(vo & 3)) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + vo + c0) + j);
-              v[4 * j] += b.x; v[4 * j + 1] += b.y; v[4 * j + 2] += b.z; v[4 * j + 3] += b.w;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 64; ++j) if (c0 + j < g.N) v[j] += __ldg(g.bias + vo + c0 + j);
+        const bool scale_vec = full_cols && !(vo & 3) && !(reinterpret_cast<uintptr_t>(g.scale) & 15);
+        auto store = [&](uint8_t* buf) {          // the warp's block, written to `buf` by all lanes
+          fence_async_smem();
+          __syncwarp();
+          if (elect_one()) {
+            if (g.conv) {
+              // this warp's 32 rows are two image rows of 16 pixels: one 4-D box; the copy engine clips at the image edge
+              int n, y0, x0;
+              conv_tile_origin(g, r0 / kBM, n, y0, x0);
+              const int yy = y0 + 2 * q;
+              if (r0 < g.M && c0 < g.N && yy < g.img_h) tma_store_4d(buf, &tmC, c0, x0, yy, n);
+            } else if (store_ok) tma_store_2d(buf, &tmC, c0, r0);
+            tma_store_commit();
           }
+        };
+        if (BN == 256 && MODE == MODE_PLAIN && g.act != ACT_SOFTMAX64) {
+          // half a block at a time: with all 64 columns and the terms of an activation 96 registers spill
+          if (elect_one()) tma_store_wait_read<0>();
+          __syncwarp();
+#pragma unroll 1
+          for (int k = 0; k < 2; ++k) {
+            uint64_t v[16];
+            tmem_ld_pairs(taddr + 32 * k, v);
+            if (g.bias) epi_vector<16, false>(v, g.bias + vo, c0 + 32 * k, g.N, full_cols && !(vo & 3));
+            if (g.scale && !g.scale_post) epi_vector<16, true>(v, g.scale + vo, c0 + 32 * k, g.N, scale_vec);
+            if (g.act) epi_act<16>(v, g.act);
+            if (g.scale && g.scale_post) epi_vector<16, true>(v, g.scale + vo, c0 + 32 * k, g.N, scale_vec);
+            stage_write16(stg, lane, 2 * k, v);
+            stage_write16(stg, lane, 2 * k + 1, v + 8);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[acc]);
+          store(stg);
+          ++item;
+          continue;
         }
-        if (g.scale && !g.scale_post) {
-#pragma unroll
-          for (int j = 0; j < 64; ++j) if (c0 + j < g.N) v[j] *= __ldg(g.scale + vo + c0 + j);
-        }
+        uint64_t v[32];
+        tmem_ld_pairs(taddr, v);
+        tmem_ld_pairs(taddr + 32, v + 16);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[acc]);
+        // ---- x = (acc + bias) * scale
+        if (g.bias) epi_vector<32, false>(v, g.bias + vo, c0, g.N, full_cols && !(vo & 3));
+        if (g.scale && !g.scale_post) epi_vector<32, true>(v, g.scale + vo, c0, g.N, scale_vec);
         // ---- second output: pre-activation
         if (MODE == MODE_Z) {
           const int b = use % NBUF;
-          if (lane == 0) tma_store_wait_read<NBUF - 1>();
+          if (elect_one()) tma_store_wait_read<NBUF - 1>();
           __syncwarp();
           stage_write_row(stg + b * kChunkBytes, lane, v);
           fence_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             if (store_ok) tma_store_2d(stg + b * kChunkBytes, &tmX, c0, r0);
             tma_store_commit();
           }
           ++use;
         }
         // ---- activation
-        switch (g.act) {
-          case ACT_GELU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = gelu_f(v[j]);
-            break;
-          case ACT_SILU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = silu_f(v[j]);
-            break;
-          case ACT_RELU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = fmaxf(v[j], 0.f);
-            break;
-          case ACT_SOFTMAX64: {
-            float m = v[0];
-#pragma unroll
-            for (int j = 1; j < 64; ++j) m = fmaxf(m, v[j]);
-            float s = 0.f;
-#pragma unroll
-            for (int j = 0; j < 64; ++j) { v[j] = ex2_fast((v[j] - m) * 1.4426950409f); s += v[j]; }
-            const float inv = __frcp_rn(s);
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] *= inv;
-          } break;
-          default: break;
-        }
+        if (g.act == ACT_SOFTMAX64) epi_softmax64(v);
+        else if ((BN != 256 || MODE != MODE_PLAIN) && g.act) epi_act<32>(v, g.act);
         // ---- auxiliary operand
         int b = use % NBUF;
         if (MODE == MODE_AUX) {
           b = item % NBUF;
           const uint32_t bph = (item / NBUF) & 1;
           if (!mbar_wait(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
-          // read back 16 columns at a time: all 64 next to v[64] would not fit the registers of a 16-warp epilogue
+          // read back 16 columns at a time: all 64 next to v would not fit the registers of a 16-warp epilogue
           const uint8_t* arow = stg + b * kChunkBytes;
-          switch (g.aux_mode) {
-            case AUX_ADD:
+          if (g.aux_mode != AUX_DSOFTMAX) {
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
+            for (int k = 0; k < 4; ++k) {
+              uint64_t a[8];
+              stage_read16(arow, lane, k, a);
+              epi_aux16(v + 8 * k, a, g.aux_mode);
+            }
+          } else {
+            uint64_t d[2] = {0, 0}, gs = 0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[16 * k + j] += a[j];
-              }
-              break;
-            case AUX_DGELU:
+            for (int k = 0; k < 4; ++k) {
+              uint64_t a[8];
+              stage_read16(arow, lane, k, a);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
+              for (int j = 0; j < 8; ++j) d[j & 1] = f2_fma(v[8 * k + j], a[j], d[j & 1]);
+            }
+            const float2 t = f2_get(f2_add(d[0], d[1]));
+            const uint64_t neg_dot = f2_all(-(t.x + t.y));
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[16 * k + j] *= gelu_grad_f(a[j]);
-              }
-              break;
-            case AUX_DSILU:
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[16 * k + j] *= silu_grad_f(a[j]);
-              }
-              break;
-            case AUX_DRELU:
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[16 * k + j] = a[j] > 0.f ? v[16 * k + j] : 0.f;
-              }
-              break;
-            case AUX_DSOFTMAX: {
-              float dot = 0.f;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) dot += v[16 * k + j] * a[j];
-              }
-              float gs = 0.f;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                float a[16];
-                stage_read16(arow, lane, k, a);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  v[16 * k + j] = a[j] * (v[16 * k + j] - dot);
-                  gs += (a[j] > 0.f) ? v[16 * k + j] * __logf(a[j]) : 0.f;
-                }
-              }
-              if (g.group_out) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
-                if (lane == 0 && c0 < g.N) atomicAdd(g.group_out + (c0 >> 6), gs);
-              }
-            } break;
-            default: break;
+            for (int k = 0; k < 4; ++k) {
+              uint64_t a[8];
+              stage_read16(arow, lane, k, a);
+              if (g.group_out) epi_dsoftmax16<true>(v + 8 * k, a, neg_dot, gs);
+              else epi_dsoftmax16<false>(v + 8 * k, a, neg_dot, gs);
+            }
+            if (g.group_out) add_group(gs, c0, true);
           }
         } else {
-          if (lane == 0) tma_store_wait_read<NBUF - 1>();
+          if (elect_one()) tma_store_wait_read<NBUF - 1>();
           __syncwarp();
         }
-        if (g.scale && g.scale_post) {
-#pragma unroll
-          for (int j = 0; j < 64; ++j) if (c0 + j < g.N) v[j] *= __ldg(g.scale + vo + c0 + j);
-        }
+        if (g.scale && g.scale_post) epi_vector<32, true>(v, g.scale + vo, c0, g.N, scale_vec);
         stage_write_row(stg + b * kChunkBytes, lane, v);
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (g.conv) {
-            // this warp's 32 rows are two image rows of 16 pixels: one 4-D box; the copy engine clips at the image edge
-            int n, y0, x0;
-            conv_tile_origin(g, r0 / kBM, n, y0, x0);
-            const int yy = y0 + 2 * q;
-            if (r0 < g.M && c0 < g.N && yy < g.img_h) tma_store_4d(stg + b * kChunkBytes, &tmC, c0, x0, yy, n);
-          } else if (store_ok) tma_store_2d(stg + b * kChunkBytes, &tmC, c0, r0);
-          tma_store_commit();
-        }
+        store(stg + b * kChunkBytes);
         ++use;
         ++item;
       }
     }
-    if (lane == 0) tma_store_wait_all<0>();
+    if (elect_one()) tma_store_wait_all<0>();
     __syncwarp();
   }
   // ------------------------------------------------------------- teardown

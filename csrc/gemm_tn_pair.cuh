@@ -29,8 +29,8 @@ namespace pnm {
 
 constexpr int kPairThreads = 320;
 
-// Two staging buffers per epilogue warp in every mode: a third buffer for the auxiliary operand costs a stage and
-// measured slower on K = 3072 (132 vs 124 us) and no faster on K = 768.
+// Two staging buffers per epilogue warp: a third one for the auxiliary operand costs a stage and measured slower on K = 3072 (132 vs
+// 124 us) and no faster on K = 768.  Two outputs: two pairs of buffers, so that a block's outputs leave behind one fence.
 //
 // MODE_CONV3 (3 x 3 convolutions, no halo rows of peers): the three taps of a filter column read windows of the image that differ by
 // whole rows of 16 pixels = 2048 bytes, so ONE box of 10 x 16 pixels holds the A operand of all three, each starting on a
@@ -43,7 +43,7 @@ constexpr int kConv3ABytes = (kConvTileH + 2) * kConvTileW * kBK * 2;
 template <int BN, int MODE>
 struct PairCfg {
   static constexpr bool RINGS = MODE == MODE_CONV3;
-  static constexpr int NBUF = 2;
+  static constexpr int NBUF = MODE == MODE_Z ? 4 : 2;
   static constexpr int B_ROWS = BN / 2;                             // rows of B (output columns) this CTA loads
   static constexpr int B_BYTES = B_ROWS * kBK * 2;
   static constexpr int STAGE_BYTES = kBM * kBK * 2 + B_BYTES;
@@ -56,7 +56,7 @@ struct PairCfg {
   static constexpr int SMEM = 1024 + OPERANDS + STAGING + 512;
   static constexpr int TMEM_COLS = 2 * BN;                         // two accumulators
   static_assert(BN == 128 || BN == 256, "pair tile is 256 x 128 or 256 x 256");
-  static_assert(STAGES >= 4 && SMEM <= 232448, "paired GEMM: shared memory budget");
+  static_assert(STAGES >= 3 && SMEM <= 232448, "paired GEMM: shared memory budget");
 };
 
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
@@ -308,7 +308,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     auto issue_aux = [&](uint32_t item) {
       int r0, c0;
       if (!item_coords(item, r0, c0)) return;
-      if (lane == 0) {
+      if (elect_one()) {
         tma_store_wait_read<NBUF - 2>();               // the buffer's previous result has left
         const int b = item % NBUF;
         mbar_expect_tx(&mybar[b], kChunkBytes);
@@ -328,104 +328,61 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         int r0, c0;
         item_coords(item, r0, c0);
         if (MODE == MODE_AUX) issue_aux(item + 1);
-        float v[64];
+        uint64_t v[32];
         const uint32_t taddr = tmem_base + acc * BN + h * (BN / 2) + ci * 64 + (uint32_t(q * 32) << 16);
-        tmem_ld32(taddr, v);
-        tmem_ld32(taddr + 32, v + 32);
-        tmem_ld_wait();
+        tmem_ld_pairs(taddr, v);
+        tmem_ld_pairs(taddr + 32, v + 16);
         if (ci == CH - 1) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(tempty_leader[acc]);
         }
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
-        if (g.bias) {
-          if (c0 + 64 <= g.N) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(g.bias + c0) + j);
-              v[4 * j] += b.x; v[4 * j + 1] += b.y; v[4 * j + 2] += b.z; v[4 * j + 3] += b.w;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 64; ++j) if (c0 + j < g.N) v[j] += __ldg(g.bias + c0 + j);
-          }
-        }
-        if (MODE == MODE_Z) {                          // second output: the pre-activation
-          const int b = use % NBUF;
-          if (lane == 0) tma_store_wait_read<NBUF - 1>();
+        if (g.bias) epi_vector<32, false>(v, g.bias, c0, g.N, c0 + 64 <= g.N);
+        if (MODE == MODE_Z) {                          // second output: the pre-activation; both leave behind one fence
+          if (elect_one()) tma_store_wait_read<1>();
           __syncwarp();
-          stage_write_row(stg + b * kChunkBytes, lane, v);
-          fence_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (store_ok) tma_store_2d(stg + b * kChunkBytes, &tmX, c0, r0);
-            tma_store_commit();
-          }
-          ++use;
+          stage_write_row(stg + ((item & 1) * 2 + 1) * kChunkBytes, lane, v);
         }
-        switch (g.act) {
-          case ACT_GELU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = gelu_f(v[j]);
-            break;
-          case ACT_SILU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = silu_f(v[j]);
-            break;
-          case ACT_RELU:
-#pragma unroll
-            for (int j = 0; j < 64; ++j) v[j] = fmaxf(v[j], 0.f);
-            break;
-          default: break;
-        }
+        if (g.act) epi_act<32>(v, g.act);
         int b = use % NBUF;
         if (MODE == MODE_AUX) {
           b = item % NBUF;
           const uint32_t bph = (item / NBUF) & 1;
           if (!mbar_wait(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
-          float a[64];
-          stage_read_row(stg + b * kChunkBytes, lane, a);
-          switch (g.aux_mode) {
-            case AUX_ADD:
+          const uint8_t* arow = stg + b * kChunkBytes;
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] += a[j];
-              break;
-            case AUX_DGELU:
-#pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] *= gelu_grad_f(a[j]);
-              break;
-            case AUX_DSILU:
-#pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] *= silu_grad_f(a[j]);
-              break;
-            case AUX_DRELU:
-#pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] = a[j] > 0.f ? v[j] : 0.f;
-              break;
-            default: break;
+          for (int k = 0; k < 4; ++k) {
+            uint64_t a[8];
+            stage_read16(arow, lane, k, a);
+            epi_aux16(v + 8 * k, a, g.aux_mode);
           }
+        } else if (MODE == MODE_Z) {
+          b = (item & 1) * 2;
         } else {
-          if (lane == 0) tma_store_wait_read<NBUF - 1>();
+          if (elect_one()) tma_store_wait_read<NBUF - 1>();
           __syncwarp();
         }
         stage_write_row(stg + b * kChunkBytes, lane, v);
         fence_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           if (g.conv) {
             // this warp's 32 rows are two image rows of 16 pixels: one 4-D box; the copy engine clips at the image edge
             int n, y0, x0;
             conv_tile_origin(g, r0 / kBM, n, y0, x0);
             const int yy = y0 + 2 * q;
             if (store_ok && yy < g.img_h) tma_store_4d(stg + b * kChunkBytes, &tmC, c0, x0, yy, n);
-          } else if (store_ok) tma_store_2d(stg + b * kChunkBytes, &tmC, c0, r0);
+          } else if (store_ok) {
+            if (MODE == MODE_Z) tma_store_2d(stg + (b + 1) * kChunkBytes, &tmX, c0, r0);
+            tma_store_2d(stg + b * kChunkBytes, &tmC, c0, r0);
+          }
           tma_store_commit();
         }
         ++use;
       }
     }
-    if (lane == 0) tma_store_wait_all<0>();
+    if (elect_one()) tma_store_wait_all<0>();
     __syncwarp();
   }
   // ------------------------------------------------------------- teardown
