@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "pnm_api.h"
 #include "pnm_internal.h"
 
@@ -25,7 +27,7 @@ namespace pnm {
 
 constexpr int kPaS = 64;
 constexpr int kPaMaxD = 64;
-constexpr int kPaTokenThreads = 1024;   // the token kernels are latency-bound chains: 32 warps hide the shared-memory latency
+constexpr int kPaTokenThreads = 512;    // 4 x 4 outputs per thread: a product of a head has 128 to 384 tiles
 
 struct PaSrc {
   const float* p[kPeerMaxRanks];  // per rank: base of the partial-sum matrix (peer-mapped for r != rank)
@@ -89,224 +91,368 @@ struct PaSaved {        // per block, fp32, all [H][S][...]
   float* wcomb;         // [Cout][H*S]
 };
 
-// grid H, kPaTokenThreads threads, dynamic shared memory (see pa_fwd_smem).  One CTA per head: the work per head is a
-// chain of dependent 64 x 64 x D products, so the only parallelism to add inside a head is more warps per phase.
+// The token kernels: grid (H, slices).  Per head the work is a chain of products of 64 rows; every CTA of a head runs the chain and the
+// CTAs share what hangs at its ends, the rows of Wo (forward: Wcomb; backward: dWo, Bcat, BdT) in chunks of 64.  What bounds a product is
+// its reads of shared memory: with one output per thread two words per multiply-add (8 heads of width 32, Cout = 256: 43.5 us forward,
+// 101 us backward on 8 CTAs), so a thread computes 4 x 4 outputs from 16-byte vectors, half a word per multiply-add or less, and a head
+// has four CTAs: 17.7 / 44.3 us.  Every output is one sum in the order of k, as before, but for the sums along rows.
+constexpr int kPaChunk = 64;
+constexpr int kPaLp = kPaS + 4;          // row length of S x S matrices: 16-byte vectors of eight rows fall on different banks
+
+__device__ __forceinline__ float4 pa_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void pa_fma4(float (&acc)[4], float a, const float4& b) {
+  acc[0] = fmaf(a, b.x, acc[0]); acc[1] = fmaf(a, b.y, acc[1]); acc[2] = fmaf(a, b.z, acc[2]); acc[3] = fmaf(a, b.w, acc[3]);
+}
+// Tile t of out(i, j), i < I, j < J (multiples of 4, as is K):
+//   nt  sum_k A[i][k] B[j][k]     rows i = ib + r I / 4, j = jb + c J / 4
+//   nn  sum_k A[i][k] B[k][j]     rows i = ib + r I / 4, columns j = 4 jb + c
+//   tn  sum_k A[k][i] B[k][j]     columns i = 4 ib + r, j = 4 jb + c
+template <int I, int J, int K, int lda, int ldb>
+__device__ __forceinline__ void pa_nt(float (&acc)[4][4], const float* A, const float* B, int t) {
+  constexpr int ni = I >> 2, nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+  for (int k = 0; k < K; k += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) { a[r] = pa_ld4(A + (ib + r * ni) * lda + k); b[r] = pa_ld4(B + (jb + r * nj) * ldb + k); }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[r][c] = fmaf(a[r].w, b[c].w, fmaf(a[r].z, b[c].z, fmaf(a[r].y, b[c].y, fmaf(a[r].x, b[c].x, acc[r][c]))));
+  }
+}
+template <int I, int J, int K, int lda, int ldb>
+__device__ __forceinline__ void pa_nn(float (&acc)[4][4], const float* A, const float* B, int t) {
+  constexpr int ni = I >> 2, nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+  for (int k = 0; k < K; k += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) a[r] = pa_ld4(A + (ib + r * ni) * lda + k);
+    const float4 b0 = pa_ld4(B + k * ldb + 4 * jb), b1 = pa_ld4(B + (k + 1) * ldb + 4 * jb), b2 = pa_ld4(B + (k + 2) * ldb + 4 * jb),
+                 b3 = pa_ld4(B + (k + 3) * ldb + 4 * jb);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      pa_fma4(acc[r], a[r].x, b0); pa_fma4(acc[r], a[r].y, b1); pa_fma4(acc[r], a[r].z, b2); pa_fma4(acc[r], a[r].w, b3);
+    }
+  }
+}
+template <int J, int K, int lda, int ldb>
+__device__ __forceinline__ void pa_tn(float (&acc)[4][4], const float* A, const float* B, int t) {
+  constexpr int nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    const float4 a = pa_ld4(A + k * lda + 4 * ib), b = pa_ld4(B + k * ldb + 4 * jb);
+    pa_fma4(acc[0], a.x, b); pa_fma4(acc[1], a.y, b); pa_fma4(acc[2], a.z, b); pa_fma4(acc[3], a.w, b);
+  }
+}
+// f(i, j, value) for the outputs of a tile
+template <int I, int J, class F>
+__device__ __forceinline__ void pa_each_nt(const float (&acc)[4][4], int t, F f) {
+  constexpr int ni = I >> 2, nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) f(ib + r * ni, jb + c * nj, acc[r][c]);
+}
+template <int I, int J, class F>
+__device__ __forceinline__ void pa_each_nn(const float (&acc)[4][4], int t, F f) {
+  constexpr int ni = I >> 2, nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) f(ib + r * ni, 4 * jb + c, acc[r][c]);
+}
+template <int J, class F>
+__device__ __forceinline__ void pa_each_tn(const float (&acc)[4][4], int t, F f) {
+  constexpr int nj = J >> 2;
+  const int ib = t / nj, jb = t - ib * nj;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) f(4 * ib + r, 4 * jb + c, acc[r][c]);
+}
+__device__ __forceinline__ float pa_warp_sum(float v) {
+#pragma unroll
+  for (int x = 16; x > 0; x >>= 1) v += __shfl_xor_sync(0xffffffffu, v, x);
+  return v;
+}
+
+template <int Dp>                        // padded head width: loops and indexes are the compiler's
 __global__ void __launch_bounds__(kPaTokenThreads)
 pa_tokens_fwd_kernel(PaSrc src, long long norm_off, int ld_tok, const float* __restrict__ Wqkv, const float* __restrict__ Wo,
                      __nv_bfloat16* __restrict__ wcomb16, PaSaved sv, int H, int D, int Cout, float scale, PeerArgs peer, int* err) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   __shared__ int sh_ok;
-  const int S = kPaS, P1 = D + 1;
-  float* tok = sm;                 // [S][D+1]
-  float* q = tok + S * P1;
-  float* k = q + S * P1;
-  float* v = k + S * P1;
-  float* o = v + S * P1;
-  float* pr = o + S * P1;          // [S][S+1]
-  float* wq = pr + S * (S + 1);    // [3D][D+1]  padded rows: the q k v product reads one row per lane
-  float* wo_s = wq + 3 * D * P1;   // [Cout][D+1]  this head's columns of Wo
-  const int h = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+  constexpr int S = kPaS, L = Dp + 4, nt = kPaTokenThreads;
+  float* tok = sm;                 // [S][L]
+  float* q = tok + S * L;          // q, k, v follow one another
+  float* k = q + S * L;
+  float* v = k + S * L;
+  float* o = v + S * L;
+  float* pr = o + S * L;           // [S][kPaLp]
+  float* wq = pr + S * kPaLp;      // [3][Dp][L]
+  float* wo = wq + 3 * Dp * L;     // [kPaChunk][L]  rows of Wo, this head's columns
+  const int h = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, tid = threadIdx.x;
   const int HS = H * S, inner = H * D;
-  const bool ok = pa_wait(src, peer, err, &sh_ok);
+  const bool ok = pa_wait(src, peer, err, &sh_ok), first = slice == 0;
   const float nanv = __int_as_float(0x7fc00000);
-  for (int i = tid; i < 3 * D * D; i += nt) wq[(i / D) * P1 + (i % D)] = Wqkv[i];
-  for (int i = tid; i < Cout * D; i += nt) wo_s[(i / D) * P1 + (i % D)] = Wo[(size_t)(i / D) * inner + h * D + (i % D)];
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
-    const float nrm = ok ? pa_sum(src, norm_off + h * S + s) + 1e-2f : nanv;
-    const float t = ok ? pa_sum(src, (long long)(h * S + s) * ld_tok + h * D + d) : nanv;
-    const float tk = t / nrm;
-    tok[s * P1 + d] = tk;
-    sv.token[(size_t)(h * S + s) * D + d] = tk;
-    if (d == 0) sv.normp[h * S + s] = nrm;
+  auto load_wo = [&](int chunk) {
+#pragma unroll 4
+    for (int i = tid; i < kPaChunk * Dp; i += nt) {
+      const int r = i / Dp, d = i - r * Dp, c = chunk * kPaChunk + r;
+      wo[r * L + d] = c < Cout && d < D ? Wo[(size_t)c * inner + h * D + d] : 0.f;
+    }
+  };
+#pragma unroll 6
+  for (int i = tid; i < 3 * Dp * Dp; i += nt) {
+    const int j = i / Dp, d = i - j * Dp, part = j / Dp, r = j - part * Dp;
+    wq[j * L + d] = r < D && d < D ? Wqkv[(part * D + r) * D + d] : 0.f;
+  }
+  load_wo(slice);
+#pragma unroll 4
+  for (int i = tid; i < S * Dp; i += nt) {
+    const int s = i / Dp, d = i - s * Dp;
+    float tk = 0.f;
+    if (d < D) {
+      const float nrm = ok ? pa_sum(src, norm_off + h * S + s) + 1e-2f : nanv;
+      tk = (ok ? pa_sum(src, (long long)(h * S + s) * ld_tok + h * D + d) : nanv) / nrm;
+      if (first) sv.token[(size_t)(h * S + s) * D + d] = tk;
+      if (first && d == 0) sv.normp[h * S + s] = nrm;
+    }
+    tok[s * L + d] = tk;
   }
   __syncthreads();
-  for (int i = tid; i < S * 3 * D; i += nt) {
-    const int s = i / (3 * D), j = i % (3 * D);
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc += tok[s * P1 + d] * wq[j * P1 + d];
-    float* dst = j < D ? q : (j < 2 * D ? k : v);
-    float* gsv = j < D ? sv.q : (j < 2 * D ? sv.k : sv.v);
-    dst[s * P1 + (j % D)] = acc;
-    gsv[(size_t)(h * S + s) * D + (j % D)] = acc;
+  for (int t = tid; t < S * 3 * Dp / 16; t += nt) {
+    float acc[4][4] = {};
+    pa_nt<S, 3 * Dp, Dp, L, L>(acc, tok, wq, t);
+    pa_each_nt<S, 3 * Dp>(acc, t, [&](int s, int j, float x) {
+      const int part = j / Dp, d = j - part * Dp;
+      q[(part * S + s) * L + d] = x;
+      if (first && d < D) (part == 0 ? sv.q : part == 1 ? sv.k : sv.v)[(size_t)(h * S + s) * D + d] = x;
+    });
   }
   __syncthreads();
-  for (int i = tid; i < S * S; i += nt) {
-    const int s = i / S, t = i % S;
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc += q[s * P1 + d] * k[t * P1 + d];
-    pr[s * (S + 1) + t] = acc * scale;
+  for (int t = tid; t < S * S / 16; t += nt) {
+    float acc[4][4] = {};
+    pa_nt<S, S, Dp, L, L>(acc, q, k, t);
+    pa_each_nt<S, S>(acc, t, [&](int s, int u, float x) { pr[s * kPaLp + u] = x * scale; });
   }
   __syncthreads();
   {  // softmax over t: one warp per row, two columns per lane
     const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
     for (int s = warp; s < S; s += nw) {
-      float a = pr[s * (S + 1) + lane], b = pr[s * (S + 1) + lane + 32];
+      float a = pr[s * kPaLp + lane], b = pr[s * kPaLp + lane + 32];
       float m = fmaxf(a, b);
       for (int x = 16; x > 0; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
       a = __expf(a - m); b = __expf(b - m);
-      float z = a + b;
-      for (int x = 16; x > 0; x >>= 1) z += __shfl_xor_sync(0xffffffffu, z, x);
-      const float inv = 1.f / z;
-      pr[s * (S + 1) + lane] = a * inv;
-      pr[s * (S + 1) + lane + 32] = b * inv;
-      sv.prob[(size_t)(h * S + s) * S + lane] = a * inv;
-      sv.prob[(size_t)(h * S + s) * S + lane + 32] = b * inv;
+      const float inv = 1.f / pa_warp_sum(a + b);
+      pr[s * kPaLp + lane] = a * inv;
+      pr[s * kPaLp + lane + 32] = b * inv;
+      if (first) {
+        sv.prob[(size_t)(h * S + s) * S + lane] = a * inv;
+        sv.prob[(size_t)(h * S + s) * S + lane + 32] = b * inv;
+      }
     }
   }
   __syncthreads();
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
-    float acc = 0.f;
-    for (int t = 0; t < S; ++t) acc += pr[s * (S + 1) + t] * v[t * P1 + d];
-    o[s * P1 + d] = acc;
-    sv.out[(size_t)(h * S + s) * D + d] = acc;
+  for (int t = tid; t < S * Dp / 16; t += nt) {
+    float acc[4][4] = {};
+    pa_nn<S, Dp, S, kPaLp, L>(acc, pr, v, t);
+    pa_each_nn<S, Dp>(acc, t, [&](int s, int d, float x) {
+      o[s * L + d] = x;
+      if (first && d < D) sv.out[(size_t)(h * S + s) * D + d] = x;
+    });
   }
   __syncthreads();
-  for (int i = tid; i < Cout * S; i += nt) {
-    const int c = i / S, s = i % S;
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc += wo_s[c * P1 + d] * o[s * P1 + d];
-    wcomb16[(size_t)c * HS + h * S + s] = __float2bfloat16(acc);
-    sv.wcomb[(size_t)c * HS + h * S + s] = acc;
+  for (int chunk = slice; chunk * kPaChunk < Cout; chunk += slices) {
+    if (chunk != slice) {
+      __syncthreads();
+      load_wo(chunk);
+      __syncthreads();
+    }
+    for (int t = tid; t < kPaChunk * S / 16; t += nt) {
+      float acc[4][4] = {};
+      pa_nt<kPaChunk, S, Dp, L, L>(acc, wo, o, t);
+      pa_each_nt<kPaChunk, S>(acc, t, [&](int r, int s, float x) {
+        const int c = chunk * kPaChunk + r;
+        if (c < Cout) {
+          wcomb16[(size_t)c * HS + h * S + s] = __float2bfloat16(x);
+          sv.wcomb[(size_t)c * HS + h * S + s] = x;
+        }
+      });
+    }
   }
 }
 
-// grid H, kPaTokenThreads threads, dynamic shared memory
+template <int Dp>
 __global__ void __launch_bounds__(kPaTokenThreads)
 pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __restrict__ Wo, PaSaved sv,
                      float* __restrict__ dWo, float* __restrict__ dWqkv, float* __restrict__ d_norm,
                      __nv_bfloat16* __restrict__ Bcat, __nv_bfloat16* __restrict__ BdT, int H, int D, int Cout, float scale,
                      float share, PeerArgs peer, int* err) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   __shared__ int sh_ok;
-  const int S = kPaS, P1 = D + 1, SP = S + 1;
-  float* dwc = sm;                 // [Cout][S+1]   this head's columns of dWcomb
-  float* dout = dwc + Cout * SP;   // [S][D+1]
-  float* q = dout + S * P1;
-  float* k = q + S * P1;
-  float* v = k + S * P1;
-  float* tok = v + S * P1;
-  float* dq = tok + S * P1;
-  float* dk = dq + S * P1;
-  float* dv = dk + S * P1;
-  float* pr = dv + S * P1;         // [S][S+1]
-  float* ds = pr + S * SP;         // [S][S+1]
-  float* wq = ds + S * SP;         // [3D][D]
-  float* rowdot = wq + 3 * D * D;  // [S]
-  float* wo_s = rowdot + S;        // [Cout][D+1]  this head's columns of Wo
-  const int h = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-  const int HS = H * S, inner = H * D;
-  const bool ok = pa_wait(src, peer, err, &sh_ok);
+  constexpr int S = kPaS, L = Dp + 4, nt = kPaTokenThreads;
+  float* q = sm;                   // [S][L] each
+  float* k = q + S * L;
+  float* v = k + S * L;
+  float* tok = v + S * L;
+  float* dq = tok + S * L;         // dq, dk, dv follow one another; the attention output until dq takes its place
+  float* dk = dq + S * L;
+  float* dv = dk + S * L;
+  float* dout = dv + S * L;        // later: d token
+  float* pr = dout + S * L;        // [S][kPaLp]
+  float* ds = pr + S * kPaLp;
+  float* wq = ds + S * kPaLp;      // [3][Dp][L]
+  float* dwc = wq + 3 * Dp * L;    // [kPaChunk][kPaLp]  rows of dWcomb, this head's columns; later: of Wcomb
+  float* wo = dwc + kPaChunk * kPaLp;      // [kPaChunk][L]
+  float* inv_np = wo + kPaChunk * L;       // [S]
+  const int h = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  const int HS = H * S, inner = H * D, chunks = (Cout + kPaChunk - 1) / kPaChunk;
+  const bool ok = pa_wait(src, peer, err, &sh_ok), first = slice == 0;
   const float nanv = __int_as_float(0x7fc00000);
-  for (int i = tid; i < Cout * S; i += nt) {
-    const int c = i / S, s = i % S;
-    dwc[c * SP + s] = ok ? pa_sum(src, (long long)c * HS + h * S + s) : nanv;
+  // the next chunk's values are on their way while this one is worked on
+  constexpr int kPre = kPaChunk * kPaS / kPaTokenThreads;
+  float pre[kPre], pre_o[kPre];
+  auto fetch = [&](int chunk) {
+#pragma unroll
+    for (int n = 0; n < kPre; ++n) {
+      const int i = tid + n * kPaTokenThreads, c = chunk * kPaChunk + i / S, r = i / Dp, d = i - r * Dp, co = chunk * kPaChunk + r;
+      pre[n] = c >= Cout ? 0.f : ok ? pa_sum(src, (long long)c * HS + h * S + i % S) : nanv;
+      pre_o[n] = r < kPaChunk && co < Cout && d < D ? Wo[(size_t)co * inner + h * D + d] : 0.f;
+    }
+  };
+  fetch(0);
+#pragma unroll 6
+  for (int i = tid; i < 3 * Dp * Dp; i += nt) {
+    const int j = i / Dp, d = i - j * Dp, part = j / Dp, r = j - part * Dp;
+    wq[j * L + d] = r < D && d < D ? Wqkv[(part * D + r) * D + d] : 0.f;
   }
-  for (int i = tid; i < 3 * D * D; i += nt) wq[i] = Wqkv[i];
-  for (int i = tid; i < Cout * D; i += nt) wo_s[(i / D) * P1 + (i % D)] = Wo[(size_t)(i / D) * inner + h * D + (i % D)];
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
+#pragma unroll 4
+  for (int i = tid; i < S * Dp; i += nt) {
+    const int s = i / Dp, d = i - s * Dp, at = s * L + d;
     const size_t g = (size_t)(h * S + s) * D + d;
-    q[s * P1 + d] = sv.q[g]; k[s * P1 + d] = sv.k[g]; v[s * P1 + d] = sv.v[g]; tok[s * P1 + d] = sv.token[g];
-    dq[s * P1 + d] = sv.out[g];          // dq holds the attention output until the attention backward overwrites it
+    const bool in = d < D;
+    q[at] = in ? sv.q[g] : 0.f; k[at] = in ? sv.k[g] : 0.f; v[at] = in ? sv.v[g] : 0.f;
+    tok[at] = in ? sv.token[g] : 0.f; dq[at] = in ? sv.out[g] : 0.f;
   }
-  for (int i = tid; i < S * S; i += nt) pr[(i / S) * SP + (i % S)] = sv.prob[(size_t)h * S * S + i];
-  __syncthreads();
+#pragma unroll
+  for (int i = tid; i < S * S; i += nt) pr[(i / S) * kPaLp + (i % S)] = sv.prob[(size_t)h * S * S + i];
   // d out_tokens[s][d] = sum_c dWcomb[c][s] Wo[c][h D + d];  dWo[c][h D + d] = sum_s dWcomb[c][s] out[s][d]
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
-    float acc = 0.f;
-    for (int c = 0; c < Cout; ++c) acc += dwc[c * SP + s] * wo_s[c * P1 + d];
-    dout[s * P1 + d] = acc;
+  constexpr int tiles_sd = S * Dp / 16;                                  // at most 256: one tile per thread
+  float acc_o[4][4] = {};
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+#pragma unroll
+    for (int n = 0; n < kPre; ++n) {
+      const int i = tid + n * kPaTokenThreads, r = i / Dp;
+      dwc[(i / S) * kPaLp + i % S] = pre[n];
+      if (r < kPaChunk) wo[r * L + i - r * Dp] = pre_o[n];
+    }
+    __syncthreads();
+    if (chunk + 1 < chunks) fetch(chunk + 1);
+    if (tid < tiles_sd) pa_tn<Dp, kPaChunk, kPaLp, L>(acc_o, dwc, wo, tid);
+    if (chunk % slices == slice) {
+      const int t = tid - (nt - kPaChunk * Dp / 16);                 // the last threads
+      if (t >= 0) {
+        float acc[4][4] = {};
+        pa_nn<kPaChunk, Dp, S, kPaLp, L>(acc, dwc, dq, t);
+        pa_each_nn<kPaChunk, Dp>(acc, t, [&](int r, int d, float x) {
+          const int c = chunk * kPaChunk + r;
+          if (c < Cout && d < D) dWo[(size_t)c * inner + h * D + d] = x * share;
+        });
+      }
+    }
+    __syncthreads();
   }
-  for (int i = tid; i < Cout * D; i += nt) {
-    const int c = i / D, d = i % D;
-    float acc = 0.f;
-    for (int s = 0; s < S; ++s) acc += dwc[c * SP + s] * dq[s * P1 + d];
-    dWo[(size_t)c * inner + h * D + d] = acc * share;
-  }
+  if (tid < tiles_sd) pa_each_tn<Dp>(acc_o, tid, [&](int s, int d, float x) { dout[s * L + d] = x; });
   __syncthreads();
-  // dWcomb is consumed: its buffer now stages this head's Wcomb^T tile for the coalesced Bcat rows written at the end
-  for (int i = tid; i < Cout * S; i += nt) dwc[(i / S) * SP + (i % S)] = sv.wcomb[(size_t)(i / S) * HS + h * S + (i % S)];
   // dP = dout v^T ; dv = P^T dout
-  for (int i = tid; i < S * S; i += nt) {
-    const int s = i / S, t = i % S;
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc += dout[s * P1 + d] * v[t * P1 + d];
-    ds[s * SP + t] = acc;
-  }
-  for (int i = tid; i < S * D; i += nt) {
-    const int t = i / D, d = i % D;
-    float acc = 0.f;
-    for (int s = 0; s < S; ++s) acc += pr[s * SP + t] * dout[s * P1 + d];
-    dv[t * P1 + d] = acc;
+  for (int t = tid; t < S * S / 16 + tiles_sd; t += nt) {
+    float acc[4][4] = {};
+    if (t < S * S / 16) {
+      pa_nt<S, S, Dp, L, L>(acc, dout, v, t);
+      pa_each_nt<S, S>(acc, t, [&](int s, int u, float x) { ds[s * kPaLp + u] = x; });
+    } else {
+      pa_tn<Dp, S, kPaLp, L>(acc, pr, dout, t - S * S / 16);
+      pa_each_tn<Dp>(acc, t - S * S / 16, [&](int u, int d, float x) { dv[u * L + d] = x; });
+    }
   }
   __syncthreads();
-  if (tid < S) {
-    float acc = 0.f;
-    for (int t = 0; t < S; ++t) acc += ds[tid * SP + t] * pr[tid * SP + t];
-    rowdot[tid] = acc;
+  for (int s = warp; s < S; s += nw) {
+    const float p0 = pr[s * kPaLp + lane], p1 = pr[s * kPaLp + lane + 32], g0 = ds[s * kPaLp + lane], g1 = ds[s * kPaLp + lane + 32];
+    const float dot = pa_warp_sum(fmaf(g0, p0, g1 * p1));
+    ds[s * kPaLp + lane] = p0 * (g0 - dot) * scale;
+    ds[s * kPaLp + lane + 32] = p1 * (g1 - dot) * scale;
   }
   __syncthreads();
-  for (int i = tid; i < S * S; i += nt) {
-    const int s = i / S, t = i % S;
-    ds[s * SP + t] = pr[s * SP + t] * (ds[s * SP + t] - rowdot[s]) * scale;
+  // dq[s] = sum_t dS[s][t] k[t] ; dk[s] = sum_t dS[t][s] q[t]
+  for (int t = tid; t < 2 * tiles_sd; t += nt) {
+    float acc[4][4] = {};
+    if (t < tiles_sd) {
+      pa_nn<S, Dp, S, kPaLp, L>(acc, ds, k, t);
+      pa_each_nn<S, Dp>(acc, t, [&](int s, int d, float x) { dq[s * L + d] = x; });
+    } else {
+      pa_tn<Dp, S, kPaLp, L>(acc, ds, q, t - tiles_sd);
+      pa_each_tn<Dp>(acc, t - tiles_sd, [&](int s, int d, float x) { dk[s * L + d] = x; });
+    }
   }
   __syncthreads();
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
-    float a = 0.f, b = 0.f;
-    for (int t = 0; t < S; ++t) { a += ds[s * SP + t] * k[t * P1 + d]; b += ds[t * SP + s] * q[t * P1 + d]; }
-    dq[s * P1 + d] = a;   // dq[s] = sum_t dS[s][t] k[t]
-    dk[s * P1 + d] = b;   // dk[s] = sum_t dS[t][s] q[t]
+  // d token[s][d] = sum_j dqkv[s][j] Wqkv[j][d] (in dout's place);  dWqkv[j][d] += share * sum_s dqkv[s][j] token[s][d]
+  constexpr int tiles_w = Dp * Dp / 16;
+  for (int t = tid; t < tiles_sd + (first ? 3 * tiles_w : 0); t += nt) {
+    float acc[4][4] = {};
+    if (t < tiles_sd) {
+#pragma unroll 1
+      for (int part = 0; part < 3; ++part) pa_nn<S, Dp, Dp, L, L>(acc, dq + part * S * L, wq + part * Dp * L, t);
+      pa_each_nn<S, Dp>(acc, t, [&](int s, int d, float x) { dout[s * L + d] = x; });
+    } else {
+      const int part = (t - tiles_sd) / tiles_w, u = (t - tiles_sd) - part * tiles_w;
+      pa_tn<Dp, S, L, L>(acc, dq + part * S * L, tok, u);
+      pa_each_tn<Dp>(acc, u, [&](int j, int d, float x) {
+        if (j < D && d < D) atomicAdd(dWqkv + (part * D + j) * D + d, x * share);
+      });
+    }
   }
   __syncthreads();
-  // dWqkv[j][d] += share * sum_s dqkv[s][j] token[s][d]
-  for (int i = tid; i < 3 * D * D; i += nt) {
-    const int j = i / D, d = i % D;
-    const float* g = j < D ? dq : (j < 2 * D ? dk : dv);
-    const int jj = j % D;
-    float acc = 0.f;
-    for (int s = 0; s < S; ++s) acc += g[s * P1 + jj] * tok[s * P1 + d];
-    atomicAdd(dWqkv + i, acc * share);
-  }
-  // d token[s][d] = sum_j dqkv[s][j] Wqkv[j][d]  (reuses dout as storage)
-  __syncthreads();
-  for (int i = tid; i < S * D; i += nt) {
-    const int s = i / D, d = i % D;
-    float acc = 0.f;
-    for (int j = 0; j < D; ++j)
-      acc += dq[s * P1 + j] * wq[j * D + d] + dk[s * P1 + j] * wq[(D + j) * D + d] + dv[s * P1 + j] * wq[(2 * D + j) * D + d];
-    dout[s * P1 + d] = acc;
-  }
-  __syncthreads();
-  if (tid < S) {
-    const float np = sv.normp[h * S + tid];
-    float acc = 0.f;
-    for (int d = 0; d < D; ++d) acc += dout[tid * P1 + d] * tok[tid * P1 + d];
-    d_norm[h * S + tid] = -acc / np;
-    rowdot[tid] = 1.f / np;
+  for (int s = warp; s < S; s += nw) {
+    float dot = lane < Dp ? dout[s * L + lane] * tok[s * L + lane] : 0.f;
+    if (lane + 32 < Dp) dot = fmaf(dout[s * L + lane + 32], tok[s * L + lane + 32], dot);
+    dot = pa_warp_sum(dot);
+    const float np = sv.normp[h * S + s];
+    if (lane == 0) {
+      inv_np[s] = 1.f / np;
+      if (first) d_norm[h * S + s] = -dot / np;
+    }
   }
   __syncthreads();
   // Bcat rows h S + s: [Wcomb^T (Cout) | zeros ... d_tok[s][:] in block h ... zeros] ; BdT rows h D + d: d_tok[:, d] in block h
   const int ldc = Cout + inner;
-  for (int i = tid; i < S * ldc; i += nt) {
-    const int s = i / ldc, col = i % ldc;
-    float val;
-    if (col < Cout) val = dwc[col * SP + s];
-    else {
-      const int jd = col - Cout;
-      val = (jd / D == h) ? dout[s * P1 + (jd % D)] * rowdot[s] : 0.f;
+  for (int chunk = slice; chunk < chunks; chunk += slices) {
+#pragma unroll
+    for (int i = tid; i < kPaChunk * S; i += nt) {
+      const int c = chunk * kPaChunk + i / S;
+      dwc[(i / S) * kPaLp + i % S] = c < Cout ? sv.wcomb[(size_t)c * HS + h * S + i % S] : 0.f;
     }
-    Bcat[(size_t)(h * S + s) * ldc + col] = __float2bfloat16(val);
+    __syncthreads();
+#pragma unroll
+    for (int i = tid; i < S * kPaChunk; i += nt) {
+      const int s = i / kPaChunk, r = i % kPaChunk, c = chunk * kPaChunk + r;
+      if (c < Cout) Bcat[(size_t)(h * S + s) * ldc + c] = __float2bfloat16(dwc[r * kPaLp + s]);
+    }
+    __syncthreads();
   }
-  for (int i = tid; i < D * HS; i += nt) {
-    const int d = i / HS, col = i % HS;
-    const int s = col % S;
-    const float val = (col / S == h) ? dout[s * P1 + d] * rowdot[s] : 0.f;
-    BdT[(size_t)(h * D + d) * HS + col] = __float2bfloat16(val);
-  }
+  for (int s = slice; s < S; s += slices)
+    for (int jd = tid; jd < inner; jd += nt)
+      Bcat[(size_t)(h * S + s) * ldc + Cout + jd] = __float2bfloat16(jd / D == h ? dout[s * L + (jd % D)] * inv_np[s] : 0.f);
+  for (int d = slice; d < D; d += slices)
+    for (int col = tid; col < HS; col += nt)
+      BdT[(size_t)(h * D + d) * HS + col] = __float2bfloat16(col / S == h ? dout[(col % S) * L + d] * inv_np[col % S] : 0.f);
 }
 
 // grid inner + S * D / 8 + 1, 256 threads
@@ -358,12 +504,27 @@ pa_prepare_bwd_kernel(const float* __restrict__ dWc, const float* __restrict__ d
   }
 }
 
-static size_t pa_fwd_smem(int D, int Cout) {
-  return sizeof(float) * (5 * kPaS * (D + 1) + kPaS * (kPaS + 1) + 3 * D * (D + 1) + (size_t)Cout * (D + 1));
+static constexpr size_t pa_fwd_smem(size_t Dp) {
+  const size_t L = Dp + 4;
+  return sizeof(float) * (5 * kPaS * L + kPaS * kPaLp + 3 * Dp * L + kPaChunk * L);
 }
-static size_t pa_bwd_smem(int D, int Cout) {
-  return sizeof(float) * ((size_t)Cout * (kPaS + 1) + 9 * kPaS * (D + 1) + 2 * kPaS * (kPaS + 1) + 3 * D * D + kPaS +
-                          (size_t)Cout * (D + 1));
+static constexpr size_t pa_bwd_smem(size_t Dp) {
+  const size_t L = Dp + 4;
+  return sizeof(float) * (8 * kPaS * L + 2 * kPaS * kPaLp + 3 * Dp * L + kPaChunk * kPaLp + kPaChunk * L + kPaS);
+}
+// f(width) with the padded head width as a constant
+template <class F>
+static int pa_by_width(int D, F f) {
+  if (D <= 4) return f(std::integral_constant<int, 4>{});
+  if (D <= 8) return f(std::integral_constant<int, 8>{});
+  if (D <= 16) return f(std::integral_constant<int, 16>{});
+  if (D <= 32) return f(std::integral_constant<int, 32>{});
+  return f(std::integral_constant<int, 64>{});
+}
+// CTAs per head: one per chunk of Wo's rows, four at most (each repeats the head's chain)
+static int pa_slices(int Cout) {
+  const int chunks = (Cout + kPaChunk - 1) / kPaChunk;
+  return chunks < 4 ? chunks : 4;
 }
 
 static PaSrc make_src(const void* const* srcs, int world, int use_flags) {
@@ -403,15 +564,19 @@ int pnm_pa_tokens_fwd(const void* const* srcs, int world, int use_flags, long lo
   if (H <= 0 || D <= 0 || D > pnm::kPaMaxD || Cout <= 0 || world < 1 || world > pnm::kPeerMaxRanks) return -2;
   int* err = pnm::error_word_ptr();
   if (!err) return -1;
-  const size_t smem = pnm::pa_fwd_smem(D, Cout);
-  static pnm::DeviceMask smem_set{0};
-  if (!pnm::allow_smem(pnm::pa_tokens_fwd_kernel, 160 * 1024, smem_set)) return -4;
-  if (smem > 160 * 1024) return -2;
   pnm::PeerArgs p{};
   if (use_flags) p = pnm::make_peer_args(bases, rank, world, epoch, capacity_floats, budget_s, epoch_base);
-  pnm::pa_tokens_fwd_kernel<<<H, pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(pnm::make_src(srcs, world, use_flags), norm_off, ld_tok, Wqkv,
-                                                                   Wo, (__nv_bfloat16*)wcomb16, pnm::make_saved(saved), H, D,
-                                                                   Cout, scale, p, err);
+  auto launch = [&](auto width) {
+    constexpr int Dp = decltype(width)::value;
+    constexpr size_t smem = pnm::pa_fwd_smem(Dp);
+    static pnm::DeviceMask smem_set{0};
+    if (!pnm::allow_smem(pnm::pa_tokens_fwd_kernel<Dp>, smem, smem_set)) return -4;
+    pnm::pa_tokens_fwd_kernel<Dp><<<dim3(H, pnm::pa_slices(Cout)), pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(
+        pnm::make_src(srcs, world, use_flags), norm_off, ld_tok, Wqkv, Wo, (__nv_bfloat16*)wcomb16, pnm::make_saved(saved), H, D, Cout, scale, p, err);
+    return 0;
+  };
+  const int code = pnm::pa_by_width(D, launch);
+  if (code) return code;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -423,16 +588,23 @@ int pnm_pa_tokens_bwd(const void* const* srcs, int world, int use_flags, const f
   if (H <= 0 || D <= 0 || D > pnm::kPaMaxD || Cout <= 0 || world < 1 || world > pnm::kPeerMaxRanks) return -2;
   int* err = pnm::error_word_ptr();
   if (!err) return -1;
-  const size_t smem = pnm::pa_bwd_smem(D, Cout);
-  if (smem > 226 * 1024) return -2;
-  static pnm::DeviceMask smem_set{0};
-  if (!pnm::allow_smem(pnm::pa_tokens_bwd_kernel, 226 * 1024, smem_set)) return -4;
   pnm::PeerArgs p{};
   if (use_flags) p = pnm::make_peer_args(bases, rank, world, epoch, capacity_floats, budget_s, epoch_base);
-  pnm::pa_tokens_bwd_kernel<<<H, pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(pnm::make_src(srcs, world, use_flags), Wqkv, Wo,
-                                                                   pnm::make_saved(saved), dWo, dWqkv, d_norm,
-                                                                   (__nv_bfloat16*)Bcat16, (__nv_bfloat16*)BdT16, H, D, Cout,
-                                                                   scale, share, p, err);
+  auto launch = [&](auto width) {
+    constexpr int Dp = decltype(width)::value;
+    constexpr size_t smem = pnm::pa_bwd_smem(Dp);
+    if constexpr (smem > 226 * 1024) return -2;
+    else {
+      static pnm::DeviceMask smem_set{0};
+      if (!pnm::allow_smem(pnm::pa_tokens_bwd_kernel<Dp>, smem, smem_set)) return -4;
+      pnm::pa_tokens_bwd_kernel<Dp><<<dim3(H, pnm::pa_slices(Cout)), pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(
+          pnm::make_src(srcs, world, use_flags), Wqkv, Wo, pnm::make_saved(saved), dWo, dWqkv, d_norm, (__nv_bfloat16*)Bcat16, (__nv_bfloat16*)BdT16,
+          H, D, Cout, scale, share, p, err);
+      return 0;
+    }
+  };
+  const int code = pnm::pa_by_width(D, launch);
+  if (code) return code;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

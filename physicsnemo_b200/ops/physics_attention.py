@@ -15,7 +15,7 @@ every pass over the N points is a tcgen05 GEMM and everything else is four small
    raised, and the token kernel of every rank adds the P copies with direct peer loads in its
    prologue — no stand-alone collective.
 3. attention among the 64 tokens per head, the normalisation before it and the combined
-   de-slicing matrix after it are one kernel (``pnm_pa_tokens_fwd``), one CTA per head.
+   de-slicing matrix after it are one kernel (``pnm_pa_tokens_fwd``), up to four CTAs per head.
 4. de-slicing followed by ``out_linear`` is again one affine map:
    ``out = w @ Wcomb.T + bo (+ residual)`` with ``Wcomb = Wo @ blockdiag(out_tokens).T``.
 

@@ -61,3 +61,41 @@ def test_fused_batch_two():
     with torch.autocast("cuda", dtype=torch.bfloat16):
         out = model(fx, embedding=emb)
     assert _rel(out, ref(fx, embedding=emb)) < 3e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,D,cout", [(8, 32, 256), (8, 32, 264), (3, 16, 72), (4, 8, 200), (2, 4, 64), (3, 2, 40), (1, 1, 8)])
+def test_slice_token_kernels(H, D, cout):
+    """Slice-token attention and its backward, head widths below and at the tile, one to five chunks of 64 output channels (a head has at
+    most four CTAs), against autograd in 64 bits.  fp32 sums of at most 264 terms; bf16 results carry 2^-9 of a value."""
+    from physicsnemo_b200.ops import pa_small as P
+
+    S, g = P.S, torch.Generator(device="cuda").manual_seed(H * D + cout)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    sums, norm = rn(H * S, H * D) * 20, 5 + 10 * torch.rand(H * S, generator=g, device="cuda")
+    Wqkv, Wo, dwc = rn(3 * D, D) / D ** 0.5, rn(cout, H * D) / (H * D) ** 0.5, rn(cout, H * S)
+    buf = torch.cat((sums.reshape(-1), norm))
+    wcomb16, saved = P.tokens_fwd([buf.data_ptr()], sums.numel(), H * D, Wqkv, Wo, H, D)
+    dWo, dWqkv, d_norm, Bcat, BdT = P.tokens_bwd([dwc.data_ptr()], Wqkv, Wo, saved, H, D, 0.5)
+
+    eye = torch.eye(H, device="cuda", dtype=torch.float64)
+    raw = torch.stack([sums[h * S:(h + 1) * S, h * D:(h + 1) * D] for h in range(H)]).double().requires_grad_(True)
+    nrm, wq, wo = (t.double().requires_grad_(True) for t in (norm.reshape(H, S), Wqkv, Wo))
+    tok = raw / (nrm + 1e-2)[..., None]
+    q, k, v = (tok @ wq.t()).chunk(3, -1)
+    out = torch.softmax(q @ k.transpose(1, 2) * D ** -0.5, -1) @ v
+    wcomb = torch.einsum("chd,hsd->chs", wo.reshape(cout, H, D), out).reshape(cout, H * S)
+    draw, dn, dwq, dwo = torch.autograd.grad(wcomb, (raw, nrm, wq, wo), dwc.double())
+
+    def close(a, b, tol):
+        assert float((a.double() - b).norm() / b.norm()) < tol
+
+    close(saved[7], wcomb, 1e-5)
+    close(wcomb16, wcomb, 2.0 ** -8)
+    close(dWo, 0.5 * dwo, 1e-5)
+    close(dWqkv, 0.5 * dwq, 1e-5)
+    close(d_norm, dn.reshape(-1), 1e-4)                                  # a sum that partly cancels
+    blocks = torch.einsum("hsd,hg->hsgd", draw, eye).reshape(H * S, H * D)
+    close(Bcat, torch.cat((wcomb.t(), blocks), 1), 2.0 ** -8)
+    close(BdT, blocks.t(), 2.0 ** -8)
+    assert ops.device_error() == 0
