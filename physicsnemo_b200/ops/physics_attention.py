@@ -95,14 +95,16 @@ class _PhysAttnFn(torch.autograd.Function):
         dWo, dWqkv, d_norm, Bcat, BdT = P.tokens_bwd(srcs, Wqkv.detach(), Wo.detach(), saved, H, D, share, peer)
         # dw = [dout | fx] @ [Wcomb.T | blockdiag(d_tok)].T + d_norm ; softmax backward in the epilogue
         grp = torch.zeros(H, dtype=torch.float32, device=dev)
-        dlogit = G.gemm_tn(dout, Bcat, a2=fx, bias=d_norm, aux=w, aux_mode=G.AUX_DSOFTMAX, scale=inv_t, scale_post=True,
-                           group_out=grp)
-        dfx = G.gemm_tn(w, BdT)                                                # d fx = w @ blockdiag(d_tok)
-        dWc, dbc = G.gemm_nt(dlogit, xn, colsum=True)                         # (H*S, C), (H*S,)
-        dWfx, dbfx = G.gemm_nt(dfx, xn, colsum=True)                          # (H*D, C), (H*D,)
+        # side by side: what follows is one product over their columns each (rows of x once, one operand for the wide tiles)
+        both = torch.empty((xn.shape[0], HS + inner), dtype=torch.bfloat16, device=dev)
+        G.gemm_tn(dout, Bcat, a2=fx, bias=d_norm, aux=w, aux_mode=G.AUX_DSOFTMAX, scale=inv_t, scale_post=True, group_out=grp,
+                  out=both[:, :HS])                                           # d logits
+        G.gemm_tn(w, BdT, out=both[:, HS:])                                   # d fx = w @ blockdiag(d_tok)
+        dW, db = G.gemm_nt(both, xn, colsum=True)                             # (H*S + H*D, C), (H*S + H*D,)
+        dWc, dWfx, dbc, dbfx = dW[:HS], dW[HS:], db[:HS], db[HS:]             # dWc lives as long as its neighbour: 4 H S C bytes
         dWx, dbx, dWs, dbs, dtemp = P.prepare_bwd(dWc, dbc, grp, Wx.detach(), bx.detach(), Ws.detach(),
                                                   temp.detach().reshape(-1), H, D)
-        dxn = G.gemm_tn(dlogit, Wback, a2=dfx)                                # [dlogit | dfx] @ [Wc ; Wfx]
+        dxn = G.gemm_tn(both, Wback)                                          # [d logits | d fx] @ [Wc ; Wfx]
         dres = dout if ctx.has_res else None
         grads = [dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp.reshape(ctx.temp_shape), dWqkv, dWo, dbo]
         grads = [g if g.dtype == dt else g.to(dt) for g, dt in zip(grads, ctx.param_dtypes)]
