@@ -5,15 +5,20 @@
 // functions do what the Python code did, argument by argument; gradients, dispatch and weight copies stay in Python.  Together with calls
 // that skip the autograd function where no gradient is wanted: a message-passing step of 1 885 nodes (three launches) 150 -> 78 us, a Transolver
 // block of 4 096 points (eleven) 373 -> 231 us, an AFNO block (twelve) 305 -> 223 us, a U-Net block with attention 601 -> 427 us.
+// Where the Python around a launch took longer than the launch, it is native as well: the way from the modules of a message-passing MLP to
+// its kernel (mlp3_module), that MLP's backward of eight to fourteen launches (mlp3_bwd), the slice-token calls: the step of 1 885
+// nodes 77 -> 52 us, a network of fifteen steps 1 328 -> 1 005 us, a training step of 30 011 nodes 807 -> 660 us, the Transolver block 206 us.
 // As there, the interpreter's lock is released not only for the launch but also where memory is allocated or copied (an allocation may wait
 // for the device): every function reads its arguments, works in an `Unlocked` scope and wraps its results.
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
+#include <cmath>
 #include <vector>
 
 #include "pnm_api.h"
@@ -80,6 +85,12 @@ const Tensor& rowmajor2d(const Tensor& in, Tensor& own) {
 }
 Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
   return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+}
+// fp32 zeros; a memset costs a call 2 us less than the kernel behind at::zeros, and the device 0.5 us
+Tensor zeros32(at::IntArrayRef sizes, const Tensor& like) {
+  Tensor t = empty(sizes, at::kFloat, like);
+  if (t.numel()) check("pnm_zero", pnm_zero(t.data_ptr(), t.numel() * 4, stream()));
+  return t;
 }
 // values of a parameter vector: fp32, contiguous, 16-byte aligned
 const Tensor& vector32(const Tensor& in, Tensor& own) {
@@ -160,9 +171,13 @@ PyObject* gemm_nt(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Tensor &a = rowmajor2d(a0, own[0]), &b = rowmajor2d(b0, own[1]);
     const int64_t M = a.size(0), Na = a.size(1), Nb = b.size(1);
     require(b.size(0) == M, "operands have different numbers of rows");
-    const auto f32 = at::TensorOptions().dtype(at::kFloat).device(a.device());
-    if (!given.defined()) made = at::zeros({Na, Nb}, f32);
-    if (!given_sums.defined() && want_sums) made_sums = at::zeros({Na}, f32);
+    if (!given.defined() && !given_sums.defined() && want_sums) {          // the gradients of a layer: made and dropped together
+      const Tensor both = zeros32({Na * (Nb + 1)}, a);
+      made = both.narrow(0, 0, Na * Nb).view({Na, Nb}); made_sums = both.narrow(0, Na * Nb, Na);
+    } else {
+      if (!given.defined()) made = zeros32({Na, Nb}, a);
+      if (!given_sums.defined() && want_sums) made_sums = zeros32({Na}, a);
+    }
     check("pnm_gemm_nt", pnm_gemm_nt(ptr(a), int(a.stride(0)), ptr(b), int(b.stride(0)), fptr(out), int(out.stride(0)), fptr(sums), int(M), int(Na),
                                      int(Nb), cap, stream()));
   }
@@ -187,6 +202,14 @@ PyObject* layernorm_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   return tuple_of({&y, &mean, &rstd});
   END_HANDLE_TH_ERRORS
+}
+
+// contiguous and 16-byte aligned: the argument or a copy
+const Tensor& dense(const Tensor& in, Tensor& own) {
+  const Tensor* t = &in;
+  if (!t->is_contiguous()) t = &(own = in.contiguous());
+  if (address(*t) % 16 != 0) t = &(own = t->clone());
+  return *t;
 }
 
 constexpr int64_t kWidth = 128, kRows = 128;     // of the one-kernel MLP
@@ -279,6 +302,314 @@ PyObject* mlp3_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   if (!keep) return THPVariable_Wrap(y);
   return relu ? tuple_of({&y, &h1, &h2, &x3, &mean, &rstd}) : tuple_of({&y, &h1, &h2, &x3, &mean, &rstd, &z1, &z2});
+  END_HANDLE_TH_ERRORS
+}
+
+// Interned names of attributes.
+PyObject* name_of(const char* text) {
+  PyObject* o = PyUnicode_InternFromString(text);
+  if (!o) throw python_error();
+  return o;
+}
+// own attribute, or null (no error set) where there is none
+PyObject* attribute(PyObject* o, PyObject* name) {
+  PyObject* r = PyObject_GetAttr(o, name);
+  if (!r) {
+    if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw python_error();
+    PyErr_Clear();
+  }
+  return r;
+}
+PyObject* item(PyObject* dict, PyObject* key) {  // borrowed, or null where there is none
+  PyObject* r = PyDict_GetItemWithError(dict, key);
+  if (!r && PyErr_Occurred()) throw python_error();
+  return r;
+}
+bool same(PyObject* tuple, at::IntArrayRef v) {
+  if (!PyTuple_Check(tuple) || PyTuple_GET_SIZE(tuple) != Py_ssize_t(v.size())) return false;
+  for (size_t i = 0; i < v.size(); ++i)
+    if (integer(PyTuple_GET_ITEM(tuple, i)) != v[i]) return false;
+  return true;
+}
+// The bf16 copy that the weight cache holds of this parameter on this stream (a new reference), as the cache's own look-up finds it
+// (ops/gemm.py): an entry is ((version, address, shape, strides), copy, weak reference).  Null where there is none that is valid.
+PyObject* kept_copy(PyObject* w, PyObject* cache, PyObject* stream_handle, bool on_default) {
+  const Tensor& t = THPVariable_Unpack(w);
+  if (t.scalar_type() == at::kBFloat16) {
+    if (!t.is_contiguous() || address(t) % 16 != 0) return nullptr;
+    Py_INCREF(w);
+    return w;
+  }
+  if (t.is_view() || t.is_inference()) return nullptr;
+  THPObjectPtr id(PyLong_FromVoidPtr(w));
+  THPObjectPtr key(on_default ? PyTuple_Pack(2, id.get(), Py_False) : PyTuple_Pack(3, id.get(), Py_False, stream_handle));
+  if (!key) throw python_error();
+  PyObject* hit = item(cache, key.get());
+  if (!hit || !PyTuple_Check(hit) || PyTuple_GET_SIZE(hit) != 3) return nullptr;
+  PyObject *ver = PyTuple_GET_ITEM(hit, 0), *copy = PyTuple_GET_ITEM(hit, 1);
+  THPObjectPtr owner(PyObject_CallNoArgs(PyTuple_GET_ITEM(hit, 2)));
+  if (!owner) throw python_error();
+  if (owner.get() != w || !PyTuple_Check(ver) || PyTuple_GET_SIZE(ver) != 4 || integer(PyTuple_GET_ITEM(ver, 0)) != int64_t(t._version()) ||
+      PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(ver, 1)) != address(t) || !same(PyTuple_GET_ITEM(ver, 2), t.sizes()) ||
+      !same(PyTuple_GET_ITEM(ver, 3), t.strides()) || !THPVariable_Check(copy))
+    return nullptr;
+  Py_INCREF(copy);
+  return copy;
+}
+
+// mlp3_module(modules of a Sequential, tables, segment indices (or None each), post or None, weight cache, parameters of captured graphs,
+//   stream, (Linear, SiLU, ReLU, GELU, LayerNorm)) -> y, or None where the call has to go the general way.
+// The forward of Linear, act, Linear, act, Linear, LayerNorm without gradients: the walk over the modules, the checks of `supported`, the
+// look-up of the weights' bf16 copies and the launch.  Anything it does not know (other module types, a weight without a copy that is
+// up to date, a capture) is left to the Python code, which decides as before.
+PyObject* mlp3_module(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 8);
+  static PyObject *const k_parameters = name_of("_parameters"), *const k_weight = name_of("weight"), *const k_bias = name_of("bias"),
+                  *const k_eps = name_of("eps"), *const k_approximate = name_of("approximate"), *const k_index = name_of("index32"),
+                  *const k_items = name_of("num_items"), *const k_segments = name_of("num_segments");
+  PyObject *modules = args[0], *cache = args[4], *kinds = args[7];
+  THPObjectPtr tables(PySequence_Fast(args[1], "tables")), segs(PySequence_Fast(args[2], "segment indices"));
+  if (!tables || !segs) throw python_error();
+  const Py_ssize_t nsrc = PySequence_Fast_GET_SIZE(tables.get());
+  if (!PyDict_Check(modules) || PyDict_GET_SIZE(modules) != 6 || !PyDict_Check(cache) || !PyDict_Check(args[5]) || PyDict_GET_SIZE(args[5]) != 0 ||
+      !PyTuple_Check(kinds) || PyTuple_GET_SIZE(kinds) != 5 || nsrc < 1 || nsrc > 3 || PySequence_Fast_GET_SIZE(segs.get()) != nsrc)
+    Py_RETURN_NONE;
+  const long long handle = integer(args[6]);
+  if (handle != 0 && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
+
+  for (Py_ssize_t j = 0; j < nsrc; ++j)
+    if (!row_table(PySequence_Fast_GET_ITEM(tables.get(), j))) Py_RETURN_NONE;
+  const Tensor& table = THPVariable_Unpack(PySequence_Fast_GET_ITEM(tables.get(), 0));
+  const at::Device dev = table.device();
+  auto parameter = [&](PyObject* o) { return o && THPVariable_CheckExact(o) && THPVariable_Unpack(o).device() == dev; };
+  // ---- the modules: weights (as kept bf16 copies), vectors (b1, b2, b3, gamma, beta), activation
+  THPObjectPtr copies[3], vectors[5];            // owned: another thread may change the modules while this one launches
+  int act = 0;
+  double eps = 0;
+  Py_ssize_t at = 0;
+  PyObject *unused, *module;
+  for (int i = 0; PyDict_Next(modules, &at, &unused, &module); ++i) {
+    PyTypeObject* type = Py_TYPE(module);
+    auto is = [&](int k) { return reinterpret_cast<PyObject*>(type) == PyTuple_GET_ITEM(kinds, k); };
+    if (i == 1 || i == 3) {
+      int code = is(1) ? 2 : is(2) ? 3 : 0;
+      if (is(3)) {
+        THPObjectPtr form(attribute(module, k_approximate));
+        if (form && PyUnicode_Check(form.get()) && PyUnicode_CompareWithASCIIString(form.get(), "none") == 0) code = 1;
+      }
+      if (!code || (act && act != code)) Py_RETURN_NONE;
+      act = code;
+      continue;
+    }
+    if (i == 5 ? !PyType_Check(PyTuple_GET_ITEM(kinds, 4)) || !PyObject_TypeCheck(module, reinterpret_cast<PyTypeObject*>(PyTuple_GET_ITEM(kinds, 4))) : !is(0))
+      Py_RETURN_NONE;
+    THPObjectPtr own(attribute(module, k_parameters));
+    if (!own || !PyDict_Check(own.get())) Py_RETURN_NONE;
+    PyObject *w = item(own.get(), k_weight), *b = item(own.get(), k_bias);
+    if (!parameter(w) || !b || (b != Py_None && !parameter(b))) Py_RETURN_NONE;
+    const Tensor& t = THPVariable_Unpack(w);
+    if (i == 5) {
+      if (t.numel() != kWidth) Py_RETURN_NONE;
+      THPObjectPtr e(attribute(module, k_eps));
+      if (!e) Py_RETURN_NONE;
+      eps = real(e.get());
+      vectors[3] = Py_NewRef(w); vectors[4] = Py_NewRef(b);
+    } else {
+      if (t.dim() != 2 || t.size(0) != kWidth || t.size(1) != (i ? kWidth : kWidth * int64_t(nsrc))) Py_RETURN_NONE;
+      copies[i / 2] = kept_copy(w, cache, args[6], handle == 0);
+      if (!copies[i / 2]) Py_RETURN_NONE;
+      vectors[i / 2] = Py_NewRef(b);
+    }
+  }
+  // ---- rows
+  const void* src[3];
+  long long rows[3];
+  int ld[3];
+  const int* idx[3];
+  THPObjectPtr index[3];
+  int64_t m = -1;
+  Py_ssize_t post_at = -1;
+  for (Py_ssize_t j = 0; j < nsrc; ++j) {
+    PyObject *o = PySequence_Fast_GET_ITEM(tables.get(), j), *seg = PySequence_Fast_GET_ITEM(segs.get(), j);
+    const Tensor& t = THPVariable_Unpack(o);
+    int64_t count = t.size(0);
+    src[j] = t.data_ptr(); rows[j] = count; ld[j] = int(t.stride(0)); idx[j] = nullptr;
+    if (t.device() != dev) Py_RETURN_NONE;
+    if (seg != Py_None) {
+      THPObjectPtr items(attribute(seg, k_items)), parts(attribute(seg, k_segments));
+      index[j] = attribute(seg, k_index);
+      if (!items || !parts || !index[j] || integer(parts.get()) != count) Py_RETURN_NONE;
+      count = integer(items.get());
+      idx[j] = static_cast<const int*>(tensor(index[j].get()).data_ptr());
+    } else if (o == args[3] && post_at < 0) {
+      post_at = j;
+    }
+    if (count == 0 || (m >= 0 && m != count)) Py_RETURN_NONE;
+    m = count;
+  }
+  if (args[3] != Py_None && post_at < 0) Py_RETURN_NONE;
+  const Tensor& post = args[3] == Py_None ? kNone : THPVariable_Unpack(args[3]);
+  const void* w[3];
+  for (int i = 0; i < 3; ++i) w[i] = tensor(copies[i].get()).data_ptr();
+  const Tensor* vec[5];
+  for (int i = 0; i < 5; ++i) vec[i] = &optional(vectors[i].get());
+  Tensor own[5], y;
+  {
+    const Unlocked unlocked;
+    for (int i = 0; i < 5; ++i) vec[i] = &vector32(*vec[i], own[i]);
+    y = empty({m, kWidth}, at::kBFloat16, table);
+    check("pnm_mlp3_ln_fwd",
+          pnm_mlp3_ln_fwd(int(nsrc), src, rows, ld, idx, w[0], w[1], w[2], fptr(*vec[0]), fptr(*vec[1]), fptr(*vec[2]), fptr(*vec[3]), fptr(*vec[4]),
+                          float(eps), act, ptr(post), post.defined() ? post.stride(0) : 0, ptr(y), kWidth, nullptr, nullptr, nullptr, nullptr, nullptr,
+                          nullptr, nullptr, m, stream()));
+  }
+  return THPVariable_Wrap(y);
+  END_HANDLE_TH_ERRORS
+}
+
+// mlp3_bwd(dy, tables, segment indices (or None each), groups of indexed tables that are one tensor, gradients wanted (per table), post, act,
+//   (w1t [128 n, 128], w2t, w3t), gamma, (h1, h2, x3, mean, rstd, z1, z2))
+//   -> ([gradient of a table or None], dw1, dw2, dw3, db1, db2, db3, dgamma, dbeta, launches)
+// The launches of the backward in their order; see ops/mlp_fused.py for what they compute.
+PyObject* mlp3_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 10);
+  THPObjectPtr tables(PySequence_Fast(args[1], "tables")), segs(PySequence_Fast(args[2], "segment indices")), groups(PySequence_Fast(args[3], "groups")),
+      wanted(PySequence_Fast(args[4], "flags")), weights(PySequence_Fast(args[7], "weights")), kept(PySequence_Fast(args[9], "kept"));
+  if (!tables || !segs || !groups || !wanted || !weights || !kept) throw python_error();
+  const Py_ssize_t nsrc = PySequence_Fast_GET_SIZE(tables.get());
+  if (nsrc < 1 || nsrc > 3 || PySequence_Fast_GET_SIZE(segs.get()) != nsrc || PySequence_Fast_GET_SIZE(wanted.get()) < nsrc ||
+      PySequence_Fast_GET_SIZE(weights.get()) != 3 || PySequence_Fast_GET_SIZE(kept.get()) != 7)
+    throw torch::TypeError("one to three tables, as many indices and flags, three weights, seven kept tensors");
+  const Tensor& dy0 = tensor(args[0]);
+  const Py_ssize_t post = args[5] == Py_None ? -1 : Py_ssize_t(integer(args[5]));
+  const int act = int(integer(args[6]));
+  const Tensor *src[3], *wt[3], *saved[7], &gamma0 = tensor(args[8]);
+  bool want[3];
+  THPObjectPtr held[3][2];
+  const Tensor *perm[3] = {}, *offsets[3] = {};
+  static PyObject *const k_perm = name_of("perm"), *const k_offsets = name_of("offsets");
+  for (Py_ssize_t j = 0; j < nsrc; ++j) {
+    src[j] = &tensor(PySequence_Fast_GET_ITEM(tables.get(), j));
+    want[j] = truth(PySequence_Fast_GET_ITEM(wanted.get(), j));
+    PyObject* seg = PySequence_Fast_GET_ITEM(segs.get(), j);
+    if (seg == Py_None) continue;
+    held[j][0] = PyObject_GetAttr(seg, k_perm); held[j][1] = PyObject_GetAttr(seg, k_offsets);
+    if (!held[j][0] || !held[j][1]) throw python_error();
+    perm[j] = &tensor(held[j][0].get()); offsets[j] = &tensor(held[j][1].get());
+  }
+  for (int i = 0; i < 3; ++i) wt[i] = &tensor(PySequence_Fast_GET_ITEM(weights.get(), i));
+  for (int i = 0; i < 7; ++i) saved[i] = &tensor(PySequence_Fast_GET_ITEM(kept.get(), i));
+  std::vector<std::vector<int>> group;
+  for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(groups.get()); ++k) {
+    THPObjectPtr members(PySequence_Fast(PySequence_Fast_GET_ITEM(groups.get(), k), "members"));
+    if (!members) throw python_error();
+    group.emplace_back();
+    for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(members.get()); ++i) {
+      const long long j = integer(PySequence_Fast_GET_ITEM(members.get(), i));
+      if (j < 0 || j >= nsrc || !perm[j]) throw torch::TypeError("groups name indexed tables");
+      group.back().push_back(int(j));
+    }
+  }
+  const Tensor &h1 = *saved[0], &h2 = *saved[1], &x3 = *saved[2], &mean = *saved[3], &rstd = *saved[4], &z1 = *saved[5], &z2 = *saved[6];
+  Tensor own[2], dsrc[3], dw[3], db[3], dgamma, dbeta;
+  int launches = 3;
+  {
+    const Unlocked unlocked;
+    void* const st = stream();
+    const int64_t W = kWidth, m = x3.size(0), N = nsrc;
+    const Tensor &dy = dense(dy0, own[0]), &gamma = vector32(gamma0, own[1]);
+    require(dy.dim() == 2 && dy.size(0) == m && dy.size(1) == W && dy.scalar_type() == at::kBFloat16, "the gradient must be bf16 [rows, 128]");
+    // All gradients of parameters in one zeroed buffer, and nothing else: it lives as long as they do.  Before them, in a buffer of its
+    // own, the sums against each table's pairs.
+    const Tensor grads = zeros32({(N + 2) * W * W + 5 * W}, x3);
+    int64_t at = 0;
+    auto take = [&](int64_t count) { at += count; return grads.narrow(0, at - count, count); };
+    dw[0] = take(N * W * W).view({W, N * W}); dw[1] = take(W * W).view({W, W}); dw[2] = take(W * W).view({W, W});
+    for (int i = 0; i < 3; ++i) db[i] = take(W);
+    dgamma = take(W); dbeta = take(W);
+    const Tensor rows = empty({2, m, W}, at::kBFloat16, x3);
+    void *const dx3 = rows.data_ptr(), *const g1 = static_cast<char*>(rows.data_ptr()) + m * W * 2;
+    {
+      const Tensor scratch = empty({pnm_layernorm_bwd_scratch_floats(m, int(W))}, at::kFloat, x3);
+      check("pnm_layernorm_bwd", pnm_layernorm_bwd(ptr(dy), ptr(x3), fptr(gamma), fptr(mean), fptr(rstd), nullptr, dx3, fptr(dgamma), fptr(dbeta),
+                                                   fptr(scratch), m, int(W), st));
+    }
+    check("pnm_mlp3_bwd", pnm_mlp3_bwd(dx3, ptr(z2), ptr(z1), ptr(h2), ptr(h1), ptr(*wt[2]), ptr(*wt[1]), act, g1, fptr(dw[2]), fptr(dw[1]), fptr(db[2]),
+                                       fptr(db[1]), m, st));
+    float* const dw1 = fptr(dw[0]);
+    auto data_gradient = [&](const void* a, int64_t count, int64_t k, const void* b, const Tensor& aux) {
+      Tensor out = empty({count, W}, at::kBFloat16, x3);
+      check("pnm_gemm_tn", pnm_gemm_tn(a, int(k), nullptr, 0, nullptr, 0, b, int(k), ptr(out), int(W), nullptr, 0, ptr(aux), aux.defined() ? int(W) : 0,
+                                       int(count), int(W), int(k), int(k), int(k), nullptr, nullptr, nullptr, 0, aux.defined() ? 1 : 0, 0, 0, 0, st));
+      ++launches;
+      return out;
+    };
+    bool summed = false;                         // the bias' gradient: of one source's product
+    for (int j = 0; j < N; ++j) {
+      if (perm[j]) continue;
+      if (want[j]) dsrc[j] = data_gradient(g1, m, W, static_cast<char*>(ptr(*wt[0])) + j * W * W * 2, post == j ? dy : kNone);
+      Tensor copy;
+      const Tensor& x = rowmajor2d(*src[j], copy);
+      check("pnm_gemm_nt", pnm_gemm_nt(g1, int(W), ptr(x), int(x.stride(0)), dw1 + j * W, int(N * W), summed ? nullptr : fptr(db[0]), int(m), int(W), int(W), 0, st));
+      ++launches;
+      summed = true;
+    }
+    for (const std::vector<int>& js : group) {
+      const int64_t L = js.size(), cols = 2 * W * L;
+      Tensor copy;
+      const Tensor& x = rowmajor2d(*src[js[0]], copy);
+      const int64_t count = offsets[js[0]]->numel() - 1;
+      const Tensor pairs = empty({count, cols}, at::kBFloat16, x3);
+      for (int k = 0; k < L; ++k) {
+        check("pnm_segment_sum_split",
+              pnm_segment_sum_split(g1, static_cast<const int*>(ptr(*perm[js[k]])), static_cast<const int*>(ptr(*offsets[js[k]])),
+                                    static_cast<char*>(pairs.data_ptr()) + 4 * k * W, cols, count, int(W), st));
+        ++launches;
+      }
+      const Tensor both = zeros32({cols * (W + 1)}, x3);
+      check("pnm_gemm_nt", pnm_gemm_nt(ptr(pairs), int(cols), ptr(x), int(x.stride(0)), fptr(both), int(W), summed ? nullptr : fptr(both) + cols * W,
+                                       int(count), int(cols), int(W), 0, st));
+      ++launches;
+      const Tensor halves = both.narrow(0, 0, cols * W).view({L, 2, W, W});
+      for (int k = 0; k < L; ++k) {
+        Tensor block = dw[0].narrow(1, js[k] * W, W);
+        at::add_out(block, halves.select(0, k).select(0, 0), halves.select(0, k).select(0, 1));
+      }
+      if (!summed) {
+        db[0] = both.narrow(0, cols * W, cols).view({L, 2, W}).select(0, 0).sum(0);
+        summed = true;
+      }
+      bool any = false;
+      for (int j : js) any = any || want[j];
+      if (any) {
+        std::vector<Tensor> parts;
+        for (int j : js)
+          for (int half = 0; half < 2; ++half) parts.push_back(wt[0]->narrow(0, j * W, W));
+        const Tensor b = at::cat(parts, 1);
+        dsrc[js[0]] = data_gradient(ptr(pairs), count, cols, ptr(b), kNone);
+      }
+    }
+  }
+  THPObjectPtr result(PyTuple_New(10)), list(PyList_New(nsrc));
+  if (!result || !list) throw python_error();
+  for (Py_ssize_t j = 0; j < nsrc; ++j) {
+    PyObject* o = dsrc[j].defined() ? THPVariable_Wrap(dsrc[j]) : Py_NewRef(Py_None);
+    if (!o) throw python_error();
+    PyList_SET_ITEM(list.get(), j, o);
+  }
+  PyTuple_SET_ITEM(result.get(), 0, list.release());
+  const Tensor* out[8] = {&dw[0], &dw[1], &dw[2], &db[0], &db[1], &db[2], &dgamma, &dbeta};
+  for (int i = 0; i < 8; ++i) {
+    PyObject* o = THPVariable_Wrap(*out[i]);
+    if (!o) throw python_error();
+    PyTuple_SET_ITEM(result.get(), i + 1, o);
+  }
+  PyObject* count = PyLong_FromLong(launches);
+  if (!count) throw python_error();
+  PyTuple_SET_ITEM(result.get(), 9, count);
+  return result.release();
   END_HANDLE_TH_ERRORS
 }
 
@@ -401,36 +732,91 @@ PyObject* pa_prepare_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// empties(like, is_bf16, shape, shape, ...) -> list of tensors on like's device (many small results of one launch)
-PyObject* empties(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  HANDLE_TH_ERRORS
-  if (n < 2) throw torch::TypeError("expected a tensor, a flag and shapes");
-  const Tensor& like = tensor(args[0]);
-  const at::ScalarType type = truth(args[1]) ? at::kBFloat16 : at::kFloat;
-  std::vector<std::vector<int64_t>> shapes(n - 2);
-  for (Py_ssize_t k = 2; k < n; ++k) {
-    if (!PyTuple_Check(args[k])) throw torch::TypeError("shapes are tuples of numbers");
-    for (Py_ssize_t d = 0; d < PyTuple_GET_SIZE(args[k]); ++d) shapes[k - 2].push_back(integer(PyTuple_GET_ITEM(args[k], d)));
+// floats of what the forward of the slice-token kernel keeps: token, norm, q, k, v, probabilities, out, Wcomb one after the other
+struct TokenParts {
+  int64_t count[8], total = 0;
+  TokenParts(int64_t H, int64_t D, int64_t cout) : count{H * 64 * D, H * 64, H * 64 * D, H * 64 * D, H * 64 * D, H * 64 * 64, H * 64 * D, cout * H * 64} {
+    for (int64_t c : count) total += c;
   }
-  std::vector<Tensor> tensors;
+  void addresses(float* base, void** out) const {
+    for (int i = 0; i < 8; base += count[i++]) out[i] = base;
+  }
+};
+
+// pa_tokens_fwd(address of the token sums, offset of the norms, row length, Wqkv, Wo, heads, head width) -> (Wcomb bf16, kept)
+PyObject* pa_tokens_fwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 7);
+  const void* const src = reinterpret_cast<const void*>(uintptr_t(integer(args[0])));
+  const long long norm_off = integer(args[1]);
+  const int ld = int(integer(args[2])), H = int(integer(args[5])), D = int(integer(args[6]));
+  const Tensor &Wqkv = tensor(args[3]), &Wo = tensor(args[4]);
+  Tensor wcomb, kept;
   {
     const Unlocked unlocked;
-    for (const auto& shape : shapes) tensors.push_back(empty(shape, type, like));
+    const int64_t cout = Wo.size(0);
+    const TokenParts parts(H, D, cout);
+    kept = empty({parts.total}, at::kFloat, Wo);
+    wcomb = empty({cout, int64_t(H) * 64}, at::kBFloat16, Wo);
+    void* saved[8];
+    parts.addresses(fptr(kept), saved);
+    check("pnm_pa_tokens_fwd", pnm_pa_tokens_fwd(&src, 1, 0, norm_off, ld, fptr(Wqkv), fptr(Wo), ptr(wcomb), saved, H, D, int(cout),
+                                                 float(1.0 / std::sqrt(double(D))), nullptr, 0, 0, 0, 1.0, nullptr, stream()));
   }
-  THPObjectPtr result(PyList_New(n - 2));
-  if (!result) throw python_error();
-  for (Py_ssize_t k = 0; k < n - 2; ++k) {
-    PyObject* o = THPVariable_Wrap(tensors[k]);
-    if (!o) throw python_error();
-    PyList_SET_ITEM(result.get(), k, o);
+  return tuple_of({&wcomb, &kept});
+  END_HANDLE_TH_ERRORS
+}
+
+// pa_tokens_bwd(address of dWcomb, Wqkv, Wo, kept, heads, head width, share) -> (dWo, dWqkv, d_norm, Bcat, BdT)
+PyObject* pa_tokens_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 7);
+  const void* const src = reinterpret_cast<const void*>(uintptr_t(integer(args[0])));
+  const Tensor &Wqkv = tensor(args[1]), &Wo = tensor(args[2]), &kept = tensor(args[3]);
+  const int H = int(integer(args[4])), D = int(integer(args[5]));
+  const float share = float(real(args[6]));
+  Tensor dWo, dWqkv, d_norm, Bcat, BdT;
+  {
+    const Unlocked unlocked;
+    const int64_t cout = Wo.size(0), inner = int64_t(H) * D, HS = int64_t(H) * 64;
+    const TokenParts parts(H, D, cout);
+    require(kept.numel() == parts.total && kept.is_contiguous(), "kept values of another layer");
+    dWo = empty({cout, inner}, at::kFloat, Wo); dWqkv = zeros32({3 * int64_t(D), D}, Wo); d_norm = empty({HS}, at::kFloat, Wo);
+    Bcat = empty({HS, cout + inner}, at::kBFloat16, Wo); BdT = empty({inner, HS}, at::kBFloat16, Wo);
+    void* saved[8];
+    parts.addresses(fptr(kept), saved);
+    check("pnm_pa_tokens_bwd", pnm_pa_tokens_bwd(&src, 1, 0, fptr(Wqkv), fptr(Wo), saved, fptr(dWo), fptr(dWqkv), fptr(d_norm), ptr(Bcat), ptr(BdT), H, D,
+                                                 int(cout), float(1.0 / std::sqrt(double(D))), share, nullptr, 0, 0, 0, 1.0, nullptr, stream()));
   }
-  return result.release();
+  return tuple_of({&dWo, &dWqkv, &d_norm, &Bcat, &BdT});
+  END_HANDLE_TH_ERRORS
+}
+
+// pa_prepare_bwd(dWc, dbc, per-head sums, Wx, bx, Ws, temperature, heads, head width) -> (dWx, dbx, dWs, dbs, dtemp)
+PyObject* pa_prepare_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need_args(n, 9);
+  const Tensor* p[7];
+  for (int i = 0; i < 7; ++i) p[i] = &tensor(args[i]);
+  const int64_t H = integer(args[7]), D = integer(args[8]);
+  Tensor dWx, dbx, dWs, dbs, dtemp;
+  {
+    const Unlocked unlocked;
+    const Tensor& like = *p[3];
+    const int64_t C = like.size(1);
+    dWx = empty({H * D, C}, at::kFloat, like); dbx = empty({H * D}, at::kFloat, like); dWs = empty({64, D}, at::kFloat, like);
+    dbs = empty({64}, at::kFloat, like); dtemp = empty({H}, at::kFloat, like);
+    check("pnm_pa_prepare_bwd", pnm_pa_prepare_bwd(fptr(*p[0]), fptr(*p[1]), fptr(*p[2]), fptr(*p[3]), fptr(*p[4]), fptr(*p[5]), fptr(*p[6]), fptr(dWx),
+                                                   fptr(dbx), fptr(dWs), fptr(dbs), fptr(dtemp), int(H), int(D), int(C), stream()));
+  }
+  return tuple_of({&dWx, &dbx, &dWs, &dbs, &dtemp});
   END_HANDLE_TH_ERRORS
 }
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {FAST(gemm_tn),     FAST(gemm_nt),     FAST(layernorm_fwd),    FAST(mlp3_operands_ok), FAST(mlp3_fwd),       FAST(segment_sum),
-                         FAST(gather_rows), FAST(conv2d_nhwc), FAST(conv_pack_weight), FAST(groupnorm_fwd),    FAST(pa_prepare_fwd), FAST(empties),
+PyMethodDef methods[] = {FAST(gemm_tn),     FAST(gemm_nt),     FAST(layernorm_fwd),    FAST(mlp3_operands_ok), FAST(mlp3_module),    FAST(mlp3_bwd), FAST(mlp3_fwd),       FAST(segment_sum),
+                         FAST(gather_rows), FAST(conv2d_nhwc), FAST(conv_pack_weight), FAST(groupnorm_fwd),    FAST(pa_prepare_fwd), FAST(pa_tokens_fwd),
+                         FAST(pa_tokens_bwd), FAST(pa_prepare_bwd),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pnm_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -12,6 +12,9 @@ int pnm_num_sms();
 int pnm_get_error();    // synchronising read of the device error word (0 = none)
 int pnm_reset_error();
 
+// Zeros on the stream (a memset, also under capture).
+int pnm_zero(void* p, long long bytes, void* stream);
+
 // C[M,N] = epilogue(A[M,K] * B[N,K]^T); bf16 in/out, fp32 accumulate.  See gemm_tn.cuh.
 int pnm_gemm_tn(const void* A, int lda, const void* A2, int lda2, const void* A3, int lda3, const void* B, int ldb, void* C, int ldc, void* Z,
                 int ldz, const void* AUX, int ldaux, int M, int N, int K, int K1, int K2, const float* bias,

@@ -89,6 +89,10 @@ int pnm_reset_error() {
   return cudaMemset(g_err_ptr, 0, sizeof(int)) == cudaSuccess ? 0 : -1;
 }
 
+int pnm_zero(void* p, long long bytes, void* stream) {
+  return cudaMemsetAsync(p, 0, size_t(bytes), reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess ? 0 : -1;
+}
+
 int pnm_gemm_tn(const void* A, int lda, const void* A2, int lda2, const void* A3, int lda3, const void* B, int ldb, void* C, int ldc, void* Z,
                 int ldz, const void* AUX, int ldaux, int M, int N, int K, int K1, int K2, const float* bias,
                 const float* scale, float* group_out, int act, int aux_mode, int scale_post, int bn, int max_ctas,

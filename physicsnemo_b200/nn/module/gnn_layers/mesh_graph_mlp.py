@@ -67,10 +67,13 @@ def _one_kernel(layers, srcs, segs, post: Optional[Tensor]) -> Optional[Tensor]:
 
 def _chain(model: nn.Sequential, x, post: Optional[Tensor] = None) -> Optional[Tensor]:
     """Run ``model`` (Linear/act…/[LayerNorm]) on the fused kernels; ``None`` if it cannot be fused."""
+    srcs = list(x) if isinstance(x, (tuple, list)) else [x]
+    y = _mlp_fused.module_call(model, srcs, [None] * len(srcs), post)
+    if y is not None:
+        return y
     layers = _layers(model)
     if layers is None:
         return None
-    srcs = list(x) if isinstance(x, (tuple, list)) else [x]
     y = _one_kernel(layers, srcs, [None] * len(srcs), post)
     if y is not None:
         return y
@@ -131,10 +134,14 @@ class MeshGraphEdgeMLPConcat(MeshGraphMLP):
     def forward(self, efeat: Tensor, nfeat, graph, post: Optional[Tensor] = None) -> Tensor:
         if ops.fused_path_enabled(efeat) and efeat.dtype == torch.bfloat16:
             srcs, segs = edge_sources(nfeat, graph)
-            layers = _layers(self.model) if isinstance(self.model, nn.Sequential) else None
-            y = None if layers is None else _one_kernel(layers, [efeat, *srcs], [None, *segs], post)
-            if y is not None:
-                return y
+            if isinstance(self.model, nn.Sequential):
+                y = _mlp_fused.module_call(self.model, [efeat, *srcs], [None, *segs], post)
+                if y is not None:
+                    return y
+                layers = _layers(self.model)
+                y = None if layers is None else _one_kernel(layers, [efeat, *srcs], [None, *segs], post)
+                if y is not None:
+                    return y
             gathered = [t if s is None else ops.gather_rows(t, s) for t, s in zip(srcs, segs)]
             return super().forward((efeat, *gathered), post=post)
         return super().forward(concat_efeat(efeat, nfeat, graph), post=post)

@@ -22,6 +22,7 @@ _ACTS = (_g.ACT_GELU, _g.ACT_SILU, _g.ACT_RELU)
 
 
 def _lib_mlp():
+    """The library with the signatures of the two calls that are launched by themselves (by tests; a backward launches natively)."""
     lib = _lib.load(required=True)
     if not getattr(lib, "_mlp3_declared", False):
         c = ctypes
@@ -52,14 +53,6 @@ def supported(srcs: Sequence[torch.Tensor], segs: Sequence, weights, biases, act
             return False
         rows = n
     return post is None or segs[post] is None
-
-
-def _vec(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """fp32 contiguous, 16-byte aligned values of a parameter vector, for a launch: the parameter itself where it is that already."""
-    if t is None:
-        return None
-    t = _g._f32(t)
-    return t if t.data_ptr() % 16 == 0 else t.detach().clone()
 
 
 def _forward(srcs, segs, weights, biases, act, gamma, beta, eps, post, save: bool):
@@ -94,69 +87,31 @@ class _Mlp3LnFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        segs, post = ctx.segs, ctx.post
-        n = len(segs)
+        n = len(ctx.segs)
         saved = ctx.saved_tensors                            # read once: activation checkpointing allows no second time
         srcs, (w1, w2, w3, gamma, h1, h2, x3, mean, rstd, *z) = saved[:n], saved[n:]
         z1, z2 = z or (h1, h2)
-        m, dev = x3.shape[0], x3.device
-        dy = _g._aligned(dy.contiguous())
-        lib = _lib_mlp()
-        # all gradients of parameters in one zeroed buffer, and nothing else: it lives as long as they do
-        sizes = [n * WIDTH * WIDTH, WIDTH * WIDTH, WIDTH * WIDTH] + [WIDTH] * 5
-        dw1, dw2, dw3, db1, db2, db3, dgamma, dbeta = torch.zeros(sum(sizes), dtype=torch.float32, device=dev).split(sizes)
-        dw1, dw2, dw3 = dw1.view(WIDTH, -1), dw2.view(WIDTH, WIDTH), dw3.view(WIDTH, WIDTH)
-        block = [dw1[:, j * WIDTH:(j + 1) * WIDTH] for j in range(n)]            # of source j
-        rows = torch.empty((2, m, WIDTH), dtype=torch.bfloat16, device=dev)
-        dx3, g1 = rows[0], rows[1]
-        scratch = torch.empty(lib.pnm_layernorm_bwd_scratch_floats(m, WIDTH), dtype=torch.float32, device=dev)
-        code = lib.pnm_layernorm_bwd(dy.data_ptr(), x3.data_ptr(), _vec(gamma).data_ptr(), mean.data_ptr(), rstd.data_ptr(), None,
-                                     dx3.data_ptr(), dgamma.data_ptr(), dbeta.data_ptr(), scratch.data_ptr(), m, WIDTH,
-                                     _g._stream())
-        _g._check(code, "pnm_layernorm_bwd")
-        w3t, w2t = _w_t(w3), _w_t(w2)                        # held: the second look-up may empty the cache
-        code = lib.pnm_mlp3_bwd(dx3.data_ptr(), z2.data_ptr(), z1.data_ptr(), h2.data_ptr(), h1.data_ptr(), w3t.data_ptr(), w2t.data_ptr(),
-                                ctx.act, g1.data_ptr(), dw3.data_ptr(), dw2.data_ptr(), db3.data_ptr(), db2.data_ptr(), m, _g._stream())
-        _g._check(code, "pnm_mlp3_bwd")
-        _g.launch_count += 3
-        need = ctx.needs_input_grad[5:]
-        w1t = _w_t(w1)                                       # [128 n, 128]: rows j * 128 .. belong to source j
-        dsrc = [None] * n
-        summed_bias = False
-        for j in range(n):
-            if segs[j] is None:
-                if need[j]:
-                    own = {"aux": dy, "aux_mode": _g.AUX_ADD} if post == j else {}
-                    dsrc[j] = _g.gemm_tn(g1, w1t[j * WIDTH:(j + 1) * WIDTH], **own)
-                _g.gemm_nt(g1, srcs[j], out=block[j], colsum_out=None if summed_bias else db1)
-                summed_bias = True
-        # An indexed source: sum g1 over the rows that read a table row FIRST (the products are linear), then one small product
-        # per table instead of one per row of M.  The fp32 sums go into the products as a bf16 pair (hi + lo).
-        for js in ctx.tables:
-            src, rows = srcs[js[0]], segs[js[0]].num_segments
-            pairs = torch.empty((rows, 2 * WIDTH * len(js)), dtype=torch.bfloat16, device=dev)
-            for k, j in enumerate(js):
-                part = pairs[:, 2 * k * WIDTH:]
-                code = lib.pnm_segment_sum_split(g1.data_ptr(), segs[j].perm.data_ptr(), segs[j].offsets.data_ptr(), part.data_ptr(),
-                                                 pairs.stride(0), rows, WIDTH, _g._stream())
-                _g._check(code, "pnm_segment_sum_split")
-                _g.launch_count += 1
-            # every sum against the table in one product; the two halves of a sum are added afterwards
-            both = torch.zeros(pairs.shape[1] * (WIDTH + 1), dtype=torch.float32, device=dev)
-            part = both[:pairs.shape[1] * WIDTH].view(-1, WIDTH)
-            _g.gemm_nt(pairs, src, out=part, colsum_out=None if summed_bias else both[part.numel():])
-            halves = part.view(len(js), 2, WIDTH, WIDTH)
-            for k, j in enumerate(js):
-                torch.add(halves[k, 0], halves[k, 1], out=block[j])
-            if not summed_bias:
-                db1 = both[part.numel():].view(len(js), 2, WIDTH)[0].sum(0)
-                summed_bias = True
-            if any(need[j] for j in js):
-                wt = torch.cat([w1t[j * WIDTH:(j + 1) * WIDTH] for j in js for _ in range(2)], 1)
-                dsrc[js[0]] = _g.gemm_tn(pairs, wt)
-        grads = [dw1, dw2, dw3, db1, db2, db3, dgamma, dbeta]
+        # An indexed source: the gradient is summed over the rows that read a table row FIRST (the products are linear), then one small
+        # product per table instead of one per row of M.  The fp32 sums go into the products as a bf16 pair (hi + lo): every sum
+        # against the table in one product, and the two halves of a sum are added afterwards.
+        dsrc, *grads, launches = _lib.host().mlp3_bwd(dy, srcs, ctx.segs, ctx.tables, ctx.needs_input_grad[5:], ctx.post, ctx.act,
+                                                      (_w_t(w1), _w_t(w2), _w_t(w3)), gamma, (h1, h2, x3, mean, rstd, z1, z2))
+        _g.launch_count += launches
         grads = [None if dt is None else (t if t.dtype == dt else t.to(dt)) for t, dt in zip(grads, ctx.dtypes)]
         return (None, None, None, None, None, *dsrc, *grads)
+
+
+_KINDS = (torch.nn.Linear, torch.nn.SiLU, torch.nn.ReLU, torch.nn.GELU, torch.nn.LayerNorm)
+
+
+def module_call(model: torch.nn.Sequential, srcs, segs, post: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """The kernel's result for a call without gradients, straight from the modules; ``None`` where the general way has to decide."""
+    if torch.is_grad_enabled() or _g.call_is_observed():
+        return None
+    y = _lib.host().mlp3_module(model._modules, srcs, segs, post, _g._wcache, _g._captured, _lib.stream(), _KINDS)
+    if y is not None:
+        _g.launch_count += 1
+    return y
 
 
 def mlp3_ln(srcs: Sequence[torch.Tensor], segs: Sequence[Optional["_graph.SegmentIndex"]], weights, biases, act: int, gamma, beta,

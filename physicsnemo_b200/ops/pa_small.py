@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import math
 from typing import List, Optional, Sequence
 
 import torch
@@ -19,8 +20,7 @@ def _lib_pa():
         vp, i, u, ll, f, d = c.c_void_p, c.c_int, c.c_uint, c.c_longlong, c.c_float, c.c_double
         lib.pnm_pa_tokens_fwd.argtypes = [vp, i, i, ll, i, vp, vp, vp, vp, i, i, i, f, vp, i, u, ll, d, vp, vp]
         lib.pnm_pa_tokens_bwd.argtypes = [vp, i, i, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, f, vp, i, u, ll, d, vp, vp]
-        lib.pnm_pa_prepare_bwd.argtypes = [vp] * 12 + [i, i, i, vp]
-        for n in ("pnm_pa_tokens_fwd", "pnm_pa_tokens_bwd", "pnm_pa_prepare_bwd"):
+        for n in ("pnm_pa_tokens_fwd", "pnm_pa_tokens_bwd"):
             getattr(lib, n).restype = i
         lib._pasmall_declared = True
     return lib
@@ -46,9 +46,15 @@ def prepare_fwd(Wx, bx, Wfx, Ws, bs, temp, H: int, D: int):
     return res
 
 
-def new_saved(H: int, D: int, Cout: int, like: torch.Tensor) -> List[torch.Tensor]:
+def _saved_shapes(H: int, D: int, Cout: int) -> tuple:
+    """What the forward keeps, one after the other in one fp32 buffer: token, norm, q, k, v, probabilities, out, Wcomb."""
     t = (H, S, D)
-    return _lib.host().empties(like, False, t, (H, S), t, t, t, (H, S, S), t, (Cout, H * S))
+    return t, (H, S), t, t, t, (H, S, S), t, (Cout, H * S)
+
+
+def saved_parts(saved: torch.Tensor, H: int, D: int, Cout: int) -> List[torch.Tensor]:
+    shapes = _saved_shapes(H, D, Cout)
+    return [p.view(s) for p, s in zip(saved.split([math.prod(s) for s in shapes]), shapes)]
 
 
 def tokens_fwd(src_ptrs: Sequence[int], norm_off: int, ld_tok: int, Wqkv, Wo, H: int, D: int, peer: Optional[tuple] = None):
@@ -56,22 +62,25 @@ def tokens_fwd(src_ptrs: Sequence[int], norm_off: int, ld_tok: int, Wqkv, Wo, H:
 
     ``peer``: ``PeerRuntime.peer_args(epoch)`` when the sources are peers' buffers whose flags must be awaited.
     """
+    _g.launch_count += 1
+    if peer is None and len(src_ptrs) == 1:
+        return _lib.host().pa_tokens_fwd(src_ptrs[0], norm_off, ld_tok, Wqkv, Wo, H, D)
     Cout = Wo.shape[0]
-    saved = new_saved(H, D, Cout, Wo)
+    saved = torch.empty(sum(math.prod(s) for s in _saved_shapes(H, D, Cout)), dtype=torch.float32, device=Wo.device)
     wcomb16 = torch.empty(Cout, H * S, dtype=torch.bfloat16, device=Wo.device)
-    world = len(src_ptrs)
-    use_flags = int(peer is not None)
     bases, rank, _w, epoch, cap, budget, ebase = peer if peer is not None else (None, 0, 1, 0, 0, 1.0, None)
-    err = _lib_pa().pnm_pa_tokens_fwd(_ptr_array(src_ptrs), world, use_flags, norm_off, ld_tok, Wqkv.data_ptr(), Wo.data_ptr(),
-                                      wcomb16.data_ptr(), _ptr_array([t.data_ptr() for t in saved]), H, D, Cout,
+    err = _lib_pa().pnm_pa_tokens_fwd(_ptr_array(src_ptrs), len(src_ptrs), int(peer is not None), norm_off, ld_tok, Wqkv.data_ptr(), Wo.data_ptr(),
+                                      wcomb16.data_ptr(), _ptr_array([t.data_ptr() for t in saved_parts(saved, H, D, Cout)]), H, D, Cout,
                                       float(D) ** -0.5, bases, rank, epoch, cap, budget, ebase, _st())
     _g._check(err, "pnm_pa_tokens_fwd")
-    _g.launch_count += 1
     return wcomb16, saved
 
 
 def tokens_bwd(src_ptrs: Sequence[int], Wqkv, Wo, saved, H: int, D: int, share: float, peer: Optional[tuple] = None):
     """``(dWo, dWqkv, d_norm [H*S], Bcat bf16 [H*S, Cout + H*D], BdT bf16 [H*D, H*S])``."""
+    _g.launch_count += 1
+    if peer is None and len(src_ptrs) == 1:
+        return _lib.host().pa_tokens_bwd(src_ptrs[0], Wqkv, Wo, saved, H, D, share)
     Cout = Wo.shape[0]
     dev = Wo.device
     inner = H * D
@@ -80,28 +89,17 @@ def tokens_bwd(src_ptrs: Sequence[int], Wqkv, Wo, saved, H: int, D: int, share: 
     d_norm = torch.empty(H * S, dtype=torch.float32, device=dev)
     Bcat = torch.empty(H * S, Cout + inner, dtype=torch.bfloat16, device=dev)
     BdT = torch.empty(inner, H * S, dtype=torch.bfloat16, device=dev)
-    world = len(src_ptrs)
-    use_flags = int(peer is not None)
     bases, rank, _w, epoch, cap, budget, ebase = peer if peer is not None else (None, 0, 1, 0, 0, 1.0, None)
-    err = _lib_pa().pnm_pa_tokens_bwd(_ptr_array(src_ptrs), world, use_flags, Wqkv.data_ptr(), Wo.data_ptr(),
-                                      _ptr_array([t.data_ptr() for t in saved]), dWo.data_ptr(), dWqkv.data_ptr(),
+    err = _lib_pa().pnm_pa_tokens_bwd(_ptr_array(src_ptrs), len(src_ptrs), int(peer is not None), Wqkv.data_ptr(), Wo.data_ptr(),
+                                      _ptr_array([t.data_ptr() for t in saved_parts(saved, H, D, Cout)]), dWo.data_ptr(), dWqkv.data_ptr(),
                                       d_norm.data_ptr(), Bcat.data_ptr(), BdT.data_ptr(), H, D, Cout, float(D) ** -0.5,
                                       float(share), bases, rank, epoch, cap, budget, ebase, _st())
     _g._check(err, "pnm_pa_tokens_bwd")
-    _g.launch_count += 1
     return dWo, dWqkv, d_norm, Bcat, BdT
 
 
 def prepare_bwd(dWc, dbc, grp, Wx, bx, Ws, temp, H: int, D: int):
     """``(dWx, dbx, dWs, dbs, dtemp)`` from the gradients of the combined projection."""
-    C = Wx.shape[1]
-    dev = Wx.device
-    f = dict(dtype=torch.float32, device=dev)
-    dWx, dbx = torch.empty(H * D, C, **f), torch.empty(H * D, **f)
-    dWs, dbs, dtemp = torch.empty(S, D, **f), torch.empty(S, **f), torch.empty(H, **f)
-    err = _lib_pa().pnm_pa_prepare_bwd(dWc.data_ptr(), dbc.data_ptr(), grp.data_ptr(), Wx.data_ptr(), bx.data_ptr(),
-                                       Ws.data_ptr(), temp.data_ptr(), dWx.data_ptr(), dbx.data_ptr(), dWs.data_ptr(),
-                                       dbs.data_ptr(), dtemp.data_ptr(), H, D, C, _st())
-    _g._check(err, "pnm_pa_prepare_bwd")
+    res = _lib.host().pa_prepare_bwd(dWc, dbc, grp, Wx, bx, Ws, temp, H, D)
     _g.launch_count += 1
-    return dWx, dbx, dWs, dbs, dtemp
+    return res

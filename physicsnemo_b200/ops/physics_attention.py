@@ -66,7 +66,7 @@ class _PhysAttnFn(torch.autograd.Function):
         peer = ex.publish()
         Wcomb16, saved = P.tokens_fwd(srcs, HS * inner, inner, Wqkv.detach(), Wo.detach(), H, D, peer)
         out = G.gemm_tn(w, Wcomb16, bias=bo.detach().float(), aux=res, aux_mode=G.AUX_ADD if res is not None else G.AUX_NONE)
-        ctx.save_for_backward(xn, fx, w, Wx, bx, Ws, temp, Wqkv, Wo, inv_t, Wback, *saved)
+        ctx.save_for_backward(xn, fx, w, Wx, bx, Ws, temp, Wqkv, Wo, inv_t, Wback, saved)
         ctx.dims = (H, D, S)
         ctx.exchange = ex
         ctx.has_res = res is not None
@@ -76,7 +76,7 @@ class _PhysAttnFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        xn, fx, w, Wx, bx, Ws, temp, Wqkv, Wo, inv_t, Wback, *saved = ctx.saved_tensors
+        xn, fx, w, Wx, bx, Ws, temp, Wqkv, Wo, inv_t, Wback, saved = ctx.saved_tensors
         H, D, S = ctx.dims
         ex = ctx.exchange
         HS, inner = H * S, H * D

@@ -378,3 +378,60 @@ def test_mlp3_ln_many_tiles_per_cta(act):
             assert _rel(a, b) < (0.06 if act == 3 else 0.02)
     torch.cuda.synchronize()
     assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", [torch.nn.SiLU, torch.nn.ReLU, torch.nn.GELU])
+@pytest.mark.parametrize("nsrc,post", [(1, None), (2, 1), (3, 0)])
+def test_call_from_the_modules_is_the_general_call(act, nsrc, post):
+    """The native walk over a Sequential gives what ``mlp3_ln`` gives, bit for bit, and declines what it does not know: a first call
+    (no copies of the weights yet), weights changed in place, another stream, a subclass, another form of an activation."""
+    from torch import nn
+
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import gemm as G
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    torch.manual_seed(nsrc)
+    mods = [nn.Linear(nsrc * W, W), act(), nn.Linear(W, W), act(), nn.Linear(W, W), nn.LayerNorm(W)]
+    model = nn.Sequential(*mods).cuda()
+    n, m = 300, 777
+    srcs = [torch.randn(m if j == 0 else n, W, device="cuda").bfloat16() for j in range(nsrc)] if nsrc == 3 else \
+        [torch.randn(m, W, device="cuda").bfloat16() for _ in range(nsrc)]
+    segs = [None] + [ops.SegmentIndex(torch.randint(0, n, (m,), device="cuda"), n) for _ in range(2)] if nsrc == 3 else [None] * nsrc
+    p = None if post is None else srcs[post]
+    code = {nn.SiLU: G.ACT_SILU, nn.ReLU: G.ACT_RELU, nn.GELU: G.ACT_GELU}[act]
+    lin = [mods[0], mods[2], mods[4]]
+
+    def general():
+        return mf.mlp3_ln(srcs, segs, [q.weight for q in lin], [q.bias for q in lin], code, mods[5].weight, mods[5].bias, mods[5].eps, post)
+
+    with torch.no_grad():
+        assert mf.module_call(model, srcs, segs, p) is None                     # no copies yet
+        want = general()
+        assert torch.equal(mf.module_call(model, srcs, segs, p), want)
+        mods[2].weight.mul_(1.5)
+        assert mf.module_call(model, srcs, segs, p) is None                     # the copy is of the values before
+        want = general()
+        assert torch.equal(mf.module_call(model, srcs, segs, p), want)
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            assert mf.module_call(model, srcs, segs, p) is None                 # each stream has its own copies
+        torch.cuda.current_stream().wait_stream(side)
+        if p is not None:
+            assert mf.module_call(model, srcs, segs, p.clone()) is None         # the residual is none of the tables
+        assert mf.module_call(model, [t[:, :64] for t in srcs], segs, None) is None
+        if act is nn.GELU:
+            mods[1].approximate = "tanh"
+            assert mf.module_call(model, srcs, segs, p) is None
+            mods[1].approximate = "none"
+
+        class Other(nn.Linear):
+            pass
+
+        model[4] = Other(W, W).cuda()
+        assert mf.module_call(model, srcs, segs, p) is None
+    with torch.enable_grad():
+        assert mf.module_call(model, srcs, segs, p) is None
+    assert ops.device_error() == 0
