@@ -119,7 +119,7 @@ afno_rows_c2r_kernel(const float2* __restrict__ X, TokenPtrs tok, AfGeom g, int 
   extern __shared__ float sm[];
   float2* xs = reinterpret_cast<float2*>(sm);                    // [KX][Cb]
   float2* tw = xs + (size_t)g.KX * g.Cb;                         // [W]
-  __nv_bfloat16* ys = reinterpret_cast<__nv_bfloat16*>(tw + g.W);  // [W][Cb]
+  __nv_bfloat16* ys = reinterpret_cast<__nv_bfloat16*>(tw + g.W + (g.W & 1));  // [W][Cb], read by 16-byte vectors
   const int row = blockIdx.x, j = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
   const int ldx = g.nblk * g.Cb;
   for (int i = tid; i < g.W; i += nt) {
@@ -885,7 +885,7 @@ int pnm_afno_rows_c2r(const void* X, const void* const* tokens, const int* geom,
       return cudaGetLastError() == cudaSuccess ? 0 : -3;
     }
   }
-  const size_t smem = sizeof(float2) * ((size_t)g.KX * g.Cb + g.W) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
+  const size_t smem = sizeof(float2) * ((size_t)g.KX * g.Cb + g.W + (g.W & 1)) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
   static pnm::DeviceMask mask{0};
   if (int rc = pnm::af_smem_attr(pnm::afno_rows_c2r_kernel, smem, mask)) return rc;
   pnm::afno_rows_c2r_kernel<<<dim3(g.B * g.H, g.nblk), 2 * g.Cb, smem, (cudaStream_t)stream>>>((const float2*)X, pnm::make_tok(tokens),

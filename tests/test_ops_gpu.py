@@ -585,6 +585,44 @@ def test_afno_spectral_filter_kernels(shape, mlp):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,H,W,C,nb,kept", [(1, 3, 7, 64, 8, 3), (1, 3, 5, 8, 1, 2), (2, 5, 16, 200, 5, 8), (1, 4, 34, 144, 2, 9), (1, 30, 60, 768, 8, 16),
+                                             (2, 45, 90, 768, 8, 46), (3, 4, 255, 64, 1, 20), (1, 2, 256, 64, 1, 40), (1, 2, 300, 64, 1, 10), (1, 160, 20, 256, 2, 10)])
+def test_afno_row_transforms(B, H, W, C, nb, kept):
+    """Odd and even rows, rows and modes that fill no tile, channels that fill no box of 64, rows too long for one box: to the spectrum, a
+    sum of W fp32 terms, and back to bf16 tokens, with and without addends."""
+    import math
+
+    from physicsnemo_b200 import ops
+    from physicsnemo_b200.ops import _lib
+    from physicsnemo_b200.ops import afno_spectral as A
+
+    lib, st, g = A._lib_af(), _lib.stream(), A.FilterGeometry(B, H, W, C, nb, kept)
+    gen = torch.Generator(device="cuda").manual_seed(W + C)
+    x = torch.randn(B * H, W, C, generator=gen, device="cuda").bfloat16()
+    weight = torch.full((g.KX,), 2.0, device="cuda", dtype=torch.double)
+    weight[0] = 1.0
+    for kw in (0, 1):
+        Y = torch.full((B * H, g.KX, C, 2), float("nan"), device="cuda")
+        assert lib.pnm_afno_rows_r2c(A._ptrs8([x.data_ptr()]), Y.data_ptr(), g.arr, g.Tp, kw, 0, None, 0, 1, 0, 0, 1.0, None, st) == 0
+        ref = torch.fft.rfft(x.double(), dim=1, norm="ortho")[:, :g.KX] * (weight if kw else torch.ones_like(weight))[:, None]
+        assert float((torch.view_as_complex(Y.double()) - ref).norm() / ref.norm()) < max(W, 16) * 2.0 ** -24
+    S = torch.randn(B * H, g.KX, C, 2, generator=gen, device="cuda")
+    adds = [torch.randn(B * H, W, C, generator=gen, device="cuda").bfloat16() for _ in range(2)]
+    k, w = torch.arange(g.KX, device="cuda"), torch.arange(W, device="cuda")
+    angle = 2 * math.pi * ((w[:, None] * k) % W).double() / W
+    plain = (torch.einsum("wk,rkc->rwc", angle.cos() * weight, S[..., 0].double())
+             - torch.einsum("wk,rkc->rwc", angle.sin() * weight, S[..., 1].double())) / math.sqrt(W)
+    for n in range(3):
+        out = torch.full((B * H, W, C), float("nan"), device="cuda", dtype=torch.bfloat16)
+        A._rows_c2r_local(lib, S, out, adds[:n], g, 1, st)
+        ref = plain + sum(a.double() for a in adds[:n])
+        # the result is rounded (2^-8 of a value), with addends the transform before them too and for odd rows every partial sum
+        bound = 2.0 ** -8 * (ref.abs() + 2 * (plain.abs() + sum(a.double().abs() for a in adds[:n])) * (n > 0)) + 1e-5
+        assert float(((out.double() - ref).abs() - bound).max()) < 0
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(2, 90, 46, 96, 2), (1, 12, 5, 32, 1)])
 def test_afno_column_transforms(dims):
     """Column DFT into the bf16 [real | imag] layout (with the soft-shrink mask of the backward) and its inverse
