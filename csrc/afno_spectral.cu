@@ -780,6 +780,13 @@ afno_cols_dft_v2_kernel(const float2* __restrict__ Y, __nv_bfloat16* __restrict_
     *reinterpret_cast<uint32_t*>(E + o) = pack_bf16x2(v.x, v.z);
     *reinterpret_cast<uint32_t*>(E + o + g.Cb) = pack_bf16x2(v.y, v.w);
   }
+  // the rows that pad a block to the GEMM's tile, shared out among the modes: zeros (a fill of their own is a launch)
+  for (int m = g.B * g.KX * g.H + bk; m < Mp; m += gridDim.x)
+    for (int c = 2 * tid; c < CH; c += 2 * nt) {
+      const size_t o = ((size_t)j * Mp + m) * (2 * g.Cb) + coff + c;
+      *reinterpret_cast<uint32_t*>(E + o) = 0u;
+      *reinterpret_cast<uint32_t*>(E + o + g.Cb) = 0u;
+    }
 }
 
 __global__ void __launch_bounds__(256)

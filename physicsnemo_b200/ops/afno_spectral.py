@@ -125,8 +125,6 @@ class _AfnoFilterTcFn(torch.autograd.Function):
         Y = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
         Y2 = torch.empty_like(Y)
         Z = torch.empty(g.nblk, g.Mp, cb2, dtype=torch.bfloat16, device=dev)
-        if g.Mp > g.Mb:
-            Z[:, g.Mb:].zero_()                                   # rows that pad a block to the GEMM's M tile
         O1, O2 = torch.empty_like(Z), torch.empty_like(Z)
         w1e, b1e, w2e, b2e = _expand_parameters(w1, b1, w2, b2, g)
 
@@ -165,9 +163,7 @@ class _AfnoFilterTcFn(torch.autograd.Function):
         rows, ld, cb2 = g.B * g.H, g.nblk * g.Cb, 2 * g.Cb
         dY2 = torch.empty(rows, g.KX, ld, 2, dtype=torch.float32, device=dev)
         dY = torch.empty_like(dY2)
-        G2 = torch.empty_like(Z)
-        if g.Mp > g.Mb:
-            G2[:, g.Mb:].zero_()          # zero padding rows: they then contribute nothing to the weight gradients
+        G2 = torch.empty_like(Z)          # its padding rows are zeroed by the transform: they add nothing to the weight gradients
         G1, dZ = torch.empty_like(Z), torch.empty_like(Z)
         # the four accumulators of the weight / bias gradients as views of ONE zero-filled buffer (one fill kernel, not four)
         nw, nbias = g.nblk * cb2 * cb2, g.nblk * cb2
