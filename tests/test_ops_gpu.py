@@ -885,6 +885,17 @@ def test_conv_weight_packing_matches_the_tensor_operations(cout, cin, k, cin_p, 
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cout,cin,cin_p,cout_p", [(3, 4, 64, 64), (72, 68, 128, 72), (65, 132, 192, 128), (520, 64, 64, 520)])
+def test_conv3x3_weight_packing_at_the_edges(cout, cin, cin_p, cout_p):
+    """3 x 3 filters in fp32 by vectors: rows and columns that fill no block, padding on both sides."""
+    from physicsnemo_b200.ops import conv
+
+    w = torch.randn(cout, cin, 3, 3, generator=torch.Generator().manual_seed(cout))
+    assert torch.equal(conv._forward_operand(w.cuda(), cin_p, cout_p).cpu(), conv._pack_weight(w, cin_p, cout_p))
+    assert torch.equal(conv._backward_operand(w.cuda(), cin_p, cout_p).cpu(), conv._pack_weight(w.flip(2, 3).transpose(0, 1), cout_p, cin_p))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("nb,cb,blk0,nblk", [(1, 8, 0, 1), (8, 96, 0, 8), (8, 96, 6, 2), (3, 40, 0, 3), (4, 128, 2, 1)])
 def test_afno_parameter_kernels_match_the_tensor_operations(nb, cb, blk0, nblk):
     """A permutation, a sign and one rounding: equal; the folded gradients are the same fp32 sums."""
