@@ -885,6 +885,13 @@ int pnm_afno_rows_c2r(const void* X, const void* const* tokens, const int* geom,
   if (pnm::af_check(g) || (signal && !counter)) return -2;
   pnm::PeerArgs p{};
   if (signal) p = pnm::make_peer_args(bases, rank, world, epoch, capacity_floats, 1.0, epoch_base);
+  if (!signal && g.Tp == (long long)g.B * g.H * g.W && g.blk0 == 0 && g.nblk * g.Cb == g.C) {
+    int* err = pnm::error_word_ptr();
+    if (!err) return -1;
+    const int code = pnm::launch_rows_c2r_tc((const float2*)X, const_cast<void*>(tokens[0]), nullptr, nullptr, g.B * g.H, g.W, g.C, g.KX, kweight,
+                                             pnm::num_sms(), err, (cudaStream_t)stream);
+    if (code <= 0) return code;
+  }
   if (g.W % 2 == 0 && g.W >= 4) {
     const pnm::RowPlan rp = pnm::row_plan(g.W / 2 + 1, g.Cb);
     const size_t smem2 = sizeof(float2) * ((size_t)g.KX * g.Cb + (size_t)g.KX * rp.pad) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
@@ -912,6 +919,12 @@ int pnm_afno_rows_c2r_add(const void* X, void* out, const void* add0, const void
                           void* stream) {
   pnm::AfGeom g{geom[0], geom[1], geom[2], geom[3], geom[4], geom[5], geom[6], geom[7], Tp, geom[8], geom[9]};
   if (pnm::af_check(g) || !out || !add0) return -2;
+  if (g.Tp == (long long)g.B * g.H * g.W && g.blk0 == 0 && g.nblk * g.Cb == g.C) {
+    int* err = pnm::error_word_ptr();
+    if (!err) return -1;
+    const int code = pnm::launch_rows_c2r_tc((const float2*)X, out, add0, add1, g.B * g.H, g.W, g.C, g.KX, kweight, pnm::num_sms(), err, (cudaStream_t)stream);
+    if (code <= 0) return code;
+  }
   if (g.W % 2 || g.W < 4) return -2;
   const pnm::RowPlan rp = pnm::row_plan(g.W / 2 + 1, g.Cb);
   const size_t smem2 = sizeof(float2) * ((size_t)g.KX * g.Cb + (size_t)g.KX * rp.pad) + sizeof(__nv_bfloat16) * (size_t)g.W * g.Cb;
