@@ -30,20 +30,22 @@ namespace pnm {
 constexpr int kPairThreads = 320;
 
 // Two staging buffers per epilogue warp: a third one for the auxiliary operand costs a stage and measured slower on K = 3072 (132 vs
-// 124 us) and no faster on K = 768.  Two outputs: two pairs of buffers, so that a block's outputs leave behind one fence.
+// 124 us) and no faster on K = 768.  With two outputs each has one and both leave behind one fence (two pairs of buffers leave three
+// stages of five: Z_FIGS).
 //
 // MODE_CONV3 (3 x 3 convolutions, no halo rows of peers): the three taps of a filter column read windows of the image that differ by
 // whole rows of 16 pixels = 2048 bytes, so ONE box of 10 x 16 pixels holds the A operand of all three, each starting on a
 // 1024-byte boundary: 20 KB per three k-blocks instead of 48 KB.  A and B then come through rings of their own: a slot of A lasts three
 // k-blocks, a slot of B one.  One image 512 x 512, 128 -> 128 / 256 -> 128 / 128 -> 256 channels: 69 / 115 / 99 us (1.13 / 1.35 / 1.56
 // PFLOP/s; a box per tap 113 / 205 / 119 us); 2 x 256 x 256, 512 -> 256: 174 us (209); 64 x 64, 512 -> 512: 27 us (tiles of one CTA 57).
-constexpr int MODE_CONV3 = 3;
+constexpr int MODE_CONV3 = 3, MODE_Z4 = 4;
 constexpr int kConv3ABytes = (kConvTileH + 2) * kConvTileW * kBK * 2;
 
 template <int BN, int MODE>
 struct PairCfg {
   static constexpr bool RINGS = MODE == MODE_CONV3;
-  static constexpr int NBUF = MODE == MODE_Z ? 4 : 2;
+  static constexpr bool TWO = MODE == MODE_Z || MODE == MODE_Z4;           // outputs
+  static constexpr int NBUF = MODE == MODE_Z4 ? 4 : 2;
   static constexpr int B_ROWS = BN / 2;                             // rows of B (output columns) this CTA loads
   static constexpr int B_BYTES = B_ROWS * kBK * 2;
   static constexpr int STAGE_BYTES = kBM * kBK * 2 + B_BYTES;
@@ -339,10 +341,10 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
         if (g.bias) epi_vector<32, false>(v, g.bias, c0, g.N, c0 + 64 <= g.N);
-        if (MODE == MODE_Z) {                          // second output: the pre-activation; both leave behind one fence
-          if (elect_one()) tma_store_wait_read<1>();
+        if (Cfg::TWO) {                                // second output: the pre-activation; both leave behind one fence
+          if (elect_one()) tma_store_wait_read<NBUF / 2 - 1>();
           __syncwarp();
-          stage_write_row(stg + ((item & 1) * 2 + 1) * kChunkBytes, lane, v);
+          stage_write_row(stg + (2 * (item % (NBUF / 2)) + 1) * kChunkBytes, lane, v);
         }
         if (g.act) epi_act<32>(v, g.act);
         int b = use % NBUF;
@@ -357,8 +359,8 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             stage_read16(arow, lane, k, a);
             epi_aux16(v + 8 * k, a, g.aux_mode);
           }
-        } else if (MODE == MODE_Z) {
-          b = (item & 1) * 2;
+        } else if (Cfg::TWO) {
+          b = 2 * (item % (NBUF / 2));
         } else {
           if (elect_one()) tma_store_wait_read<NBUF - 1>();
           __syncwarp();
@@ -374,7 +376,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             const int yy = y0 + 2 * q;
             if (store_ok && yy < g.img_h) tma_store_4d(stg + b * kChunkBytes, &tmC, c0, x0, yy, n);
           } else if (store_ok) {
-            if (MODE == MODE_Z) tma_store_2d(stg + (b + 1) * kChunkBytes, &tmX, c0, r0);
+            if (Cfg::TWO) tma_store_2d(stg + (b + 1) * kChunkBytes, &tmX, c0, r0);
             tma_store_2d(stg + b * kChunkBytes, &tmC, c0, r0);
           }
           tma_store_commit();
@@ -475,7 +477,7 @@ inline int launch_gemm_tn_pair(const GemmCall& c, int num_sms, int* err_word, cu
     if (make_tmap_2d_b16(&tC, c.C, c.M, c.N, c.ldc, 32, 64)) return -13;
   }
   if (make_tmap_2d_b16(&tB, c.B, c.N, c.K, c.ldb, Cfg::B_ROWS, kBK)) return -12;
-  if (MODE == MODE_Z) { if (make_tmap_2d_b16(&tX, c.Z, c.M, c.N, c.ldz, 32, 64)) return -14; }
+  if (Cfg::TWO) { if (make_tmap_2d_b16(&tX, c.Z, c.M, c.N, c.ldz, 32, 64)) return -14; }
   else if (MODE == MODE_AUX) { if (make_tmap_2d_b16(&tX, c.AUX, c.M, c.N, c.ldaux, 32, 64)) return -15; }
   else if (c.conv && c.halo && c.down_rows) { if (make_tmap_nhwc_b16(&tX, c.down_rows, c.img_n, 1, c.img_w, c.cin, 1, kConvTileW)) return -15; }
   else tX = tC;

@@ -271,6 +271,20 @@ def test_conv3x3_weight_gradient_by_columns_of_taps(n, h, w, cin, cout):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(2048, 1024, 256), (2999, 1096, 264), (2304, 1032, 504), (2100, 1024, 512)])
+def test_gemm_tn_two_outputs_of_short_products(M, N, K):
+    """Two outputs on CTA pairs below K = 512 keep two pairs of staging buffers: ragged edges, several blocks per warp."""
+    a, b, bias = _rand(M, K), _rand(N, K, scale=K ** -0.5), torch.randn(N, device="cuda")
+    y, z = G.gemm_tn(a, b, bias=bias, act=G.ACT_GELU, z_out=True)
+    zr = a.double() @ b.double().t() + bias.double()
+    assert float(((z - zr).abs() - 2.0 ** -8 * zr.abs()).max()) < 1e-4            # rounded once
+    # the kernels' GELU is the tanh form: within 1e-3 of the erf form
+    yr = torch.nn.functional.gelu(zr, approximate="tanh")
+    assert float(((y - yr).abs() - 2.0 ** -8 * yr.abs()).max()) < 2e-3
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 512), (4000, 768, 1024), (32400, 1096, 768), (2304, 520, 584)])
 @pytest.mark.parametrize("mode", ["plain", "gelu_z", "add", "dgelu", "drelu"])
 def test_gemm_tn_cta_pair_tiles(M, N, K, mode):
