@@ -457,6 +457,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           // 16 columns at a time, straight from TMEM into the staged auxiliary tile (which the result replaces): a row of 64 and
           // its auxiliary values do not fit the 96 registers of a thread.  The softmax backward reads the accumulator twice.
           const bool store_ok = (r0 < g.M) && (c0 < g.N), full_cols = (c0 + 64 <= g.N);
+          const bool bias_vec = full_cols && !(reinterpret_cast<uintptr_t>(g.bias) & 15);
           const bool scale_vec = full_cols && !(reinterpret_cast<uintptr_t>(g.scale) & 15);
           uint8_t* arow = stg + (item % NBUF) * kChunkBytes;
           auto load16 = [&](int k, uint64_t* x) {
@@ -466,7 +467,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = f2_make(t[2 * j], t[2 * j + 1]);
             const int c = c0 + 16 * k;
-            if (g.bias) epi_vector<8, false>(x, g.bias, c, g.N, full_cols);
+            if (g.bias) epi_vector<8, false>(x, g.bias, c, g.N, bias_vec);
             if (g.scale && !g.scale_post) epi_vector<8, true>(x, g.scale, c, g.N, scale_vec);
             if (g.act) epi_act<8>(x, g.act);
           };
@@ -511,6 +512,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
         const bool full_cols = (c0 + 64 <= g.N);
         const int vo = g.batch_m_tiles ? (r0 / (kBM * g.batch_m_tiles)) * g.N : 0;   // offset of the problem's bias / scale
+        // a vector may be a slice of a flat buffer that starts anywhere
+        const bool bias_vec = full_cols && !(vo & 3) && !(reinterpret_cast<uintptr_t>(g.bias) & 15);
         const bool scale_vec = full_cols && !(vo & 3) && !(reinterpret_cast<uintptr_t>(g.scale) & 15);
         auto store = [&](uint8_t* buf) {          // the warp's block, written to `buf` by all lanes
           fence_async_smem();
@@ -534,7 +537,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int k = 0; k < 2; ++k) {
             uint64_t v[16];
             tmem_ld_pairs(taddr + 32 * k, v);
-            if (g.bias) epi_vector<16, false>(v, g.bias + vo, c0 + 32 * k, g.N, full_cols && !(vo & 3));
+            if (g.bias) epi_vector<16, false>(v, g.bias + vo, c0 + 32 * k, g.N, bias_vec);
             if (g.scale && !g.scale_post) epi_vector<16, true>(v, g.scale + vo, c0 + 32 * k, g.N, scale_vec);
             if (g.act) epi_act<16>(v, g.act);
             if (g.scale && g.scale_post) epi_vector<16, true>(v, g.scale + vo, c0 + 32 * k, g.N, scale_vec);
@@ -555,7 +558,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[acc]);
         // ---- x = (acc + bias) * scale
-        if (g.bias) epi_vector<32, false>(v, g.bias + vo, c0, g.N, full_cols && !(vo & 3));
+        if (g.bias) epi_vector<32, false>(v, g.bias + vo, c0, g.N, bias_vec);
         if (g.scale && !g.scale_post) epi_vector<32, true>(v, g.scale + vo, c0, g.N, scale_vec);
         // ---- second output: pre-activation
         if (MODE == MODE_Z) {

@@ -340,7 +340,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (lane == 0) mbar_arrive_cluster(tempty_leader[acc]);
         }
         const bool store_ok = (r0 < g.M) && (c0 < g.N);
-        if (g.bias) epi_vector<32, false>(v, g.bias, c0, g.N, c0 + 64 <= g.N);
+        if (g.bias) epi_vector<32, false>(v, g.bias, c0, g.N, c0 + 64 <= g.N && !(reinterpret_cast<uintptr_t>(g.bias) & 15));
         if (Cfg::TWO) {                                // second output: the pre-activation; both leave behind one fence
           if (elect_one()) tma_store_wait_read<NBUF / 2 - 1>();
           __syncwarp();

@@ -285,6 +285,33 @@ def test_gemm_tn_two_outputs_of_short_products(M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("skip", [1, 2, 3])
+@pytest.mark.parametrize("M,N,K", [(300, 128, 72), (300, 320, 64), (90000, 128, 64), (40000, 256, 128), (2048, 1024, 256), (2304, 576, 512)])
+def test_vectors_that_start_off_a_16_byte_boundary(M, N, K, skip):
+    """Bias and scale as slices of a flat buffer, `skip` elements from its start, on every kind of tile and with every kind of epilogue, and
+    in a convolution: what an aligned copy gives, bit for bit."""
+    from physicsnemo_b200.ops import conv as C
+
+    a, b, aux = _rand(M, K), _rand(N, K, scale=K ** -0.5), _rand(M, N)
+    flat = torch.randn(2 * N + 8, device="cuda")
+    bias, scale = flat[skip:skip + N], flat[N + 4 + skip:2 * N + 4 + skip]
+    assert bias.data_ptr() % 16 == scale.data_ptr() % 16 == 4 * skip
+    forms = [dict(bias=bias), dict(bias=bias, act=G.ACT_GELU), dict(bias=bias, scale=scale), dict(bias=bias, scale=scale, scale_post=True),
+             dict(bias=bias, act=G.ACT_SILU, z_out=True), dict(bias=bias, aux=aux, aux_mode=G.AUX_ADD), dict(bias=bias, aux=aux, aux_mode=G.AUX_DGELU)]
+    if N % 64 == 0:
+        forms += [dict(bias=bias, scale=scale, act=G.ACT_SOFTMAX64), dict(bias=bias, scale=scale, scale_post=True, aux=aux, aux_mode=G.AUX_DSOFTMAX)]
+    for form in forms:
+        own = {k: v.clone() if k in ("bias", "scale") else v for k, v in form.items()}
+        out, want = G.gemm_tn(a, b, **form), G.gemm_tn(a, b, **own)
+        for u, v in zip(*((t if isinstance(t, tuple) else (t,)) for t in (out, want))):
+            assert torch.equal(u, v)
+    x = _rand(1, 64, 24, 40).contiguous(memory_format=torch.channels_last)
+    for k in (1, 3):
+        w = _rand(N, 64, k, k, scale=0.05)
+        assert torch.equal(C.conv2d_same(x, w, bias), C.conv2d_same(x, w, bias.clone()))
+    assert ops.device_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(2048, 256, 512), (4000, 768, 1024), (32400, 1096, 768), (2304, 520, 584)])
 @pytest.mark.parametrize("mode", ["plain", "gelu_z", "add", "dgelu", "drelu"])
 def test_gemm_tn_cta_pair_tiles(M, N, K, mode):
