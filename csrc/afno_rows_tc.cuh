@@ -128,8 +128,7 @@ afno_rows_r2c_tc_kernel(const __grid_constant__ CUtensorMap tmX, const RowTcArgs
     uint32_t it = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
       const int a = it & 1, row = t / g.tiles_c, c = (t - row * g.tiles_c) * 128 + q * 32 + lane;
-      const bool ok = mbar_wait(&tfull[a], (it >> 1) & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL);
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!mbar_wait_warp(&tfull[a], (it >> 1) & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       float2* dst = g.Y + (long long)row * g.KX * g.C + c;
       for (int j = half; j < g.n16 / 16; j += 2) {           // eight modes
@@ -283,8 +282,7 @@ __global__ void __launch_bounds__(kRowInvThreads, 1) afno_rows_c2r_tc_kernel(con
           if (kx < g.KX && c < g.C) v[n] = __ldcs(reinterpret_cast<const float4*>(g.X + ((long long)row * g.KX + kx) * g.C + c));
         }
         if (first == 0) {                        // the first loads are on their way meanwhile
-          ok = mbar_wait(&aempty, (it & 1) ^ 1, abort_flag, g.err, ERR_WAIT_EMPTY);
-          ok = __all_sync(0xffffffffu, ok);
+          ok = mbar_wait_warp(&aempty, (it & 1) ^ 1, abort_flag, g.err, ERR_WAIT_EMPTY);
           if (!ok) break;
         }
 #pragma unroll
@@ -351,8 +349,7 @@ __global__ void __launch_bounds__(kRowInvThreads, 1) afno_rows_c2r_tc_kernel(con
           if (g.add1 && inside(i)) b1[n] = __ldg(reinterpret_cast<const uint4*>(g.add1 + address(i)));
         }
       };
-      bool ok = mbar_wait(&tfull[a], (it >> 1) & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
+      const bool ok = mbar_wait_warp(&tfull[a], (it >> 1) & 1, abort_flag, g.err, ERR_WAIT_TMEM_FULL);
       tc_fence_after();
       const uint32_t acc = tmem + a * 256 + (uint32_t(q * 32) << 16);
       // A thread has one channel; with its neighbour's values of the same two positions it stores two channels of one of them.

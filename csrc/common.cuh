@@ -118,6 +118,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The wait of a whole warp, one answer for all its lanes: what follows needs the warp together (elect.sync, TMEM loads, shuffles), and
+// where a wait runs out one lane may still have seen the phase end and another not.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err_word, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err_word, code));
+}
+
 // Bounded wait that never raises the abort flag: lets a copy in flight land before the CTA leaves.  `parity` is that of the phase
 // that the copy completes and must be the barrier's last: any wait for the other parity is over at once.
 __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {

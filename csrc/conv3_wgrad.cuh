@@ -115,7 +115,7 @@ conv3_wgrad_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     // Two warps per lane quarter, every second tap each; a lane's 64 sums leave as one bulk reduction of 256 bytes from the shared
     // memory of the finished stages (a warp's red instructions touch 32 rows each: 16 bytes of a sector at a time).
     const int q = warp & 3, half = (warp - 2) >> 2;
-    if (mbar_wait(tfull, 0, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) {
+    if (mbar_wait_warp(tfull, 0, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) {
       tc_fence_after();
       const int row = ta * 128 + q * 32 + lane;                    // output channel
       const uint32_t lanes = tmem_base + (uint32_t(q * 32) << 16);

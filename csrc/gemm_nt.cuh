@@ -189,7 +189,7 @@ gemm_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (num_kb > 0) {
     const int q = warp & 3;
-    if (mbar_wait(tfull, 0, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) {
+    if (mbar_wait_warp(tfull, 0, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) {
       tc_fence_after();
       const int row = ta * 128 + q * 32 + lane;  // output row (column of A)
       for (int c = 0; c < BNB; c += 32) {

@@ -446,7 +446,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++tc) {
       const int acc = tc & 1;
       const uint32_t aph = (tc >> 1) & 1;
-      if (!mbar_wait(&tfull[acc], aph, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
+      if (!mbar_wait_warp(&tfull[acc], aph, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
       {
         int r0, c0;
@@ -471,7 +471,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (g.scale && !g.scale_post) epi_vector<8, true>(x, g.scale, c, g.N, scale_vec);
             if (g.act) epi_act<8>(x, g.act);
           };
-          if (!mbar_wait(&mybar[item % NBUF], (item / NBUF) & 1, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
+          if (!mbar_wait_warp(&mybar[item % NBUF], (item / NBUF) & 1, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
           uint64_t neg_dot = 0, gs = 0;
           if (g.aux_mode == AUX_DSOFTMAX) {
             uint64_t d[2] = {0, 0};
@@ -582,7 +582,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (MODE == MODE_AUX) {
           b = item % NBUF;
           const uint32_t bph = (item / NBUF) & 1;
-          if (!mbar_wait(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
+          if (!mbar_wait_warp(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
           // read back 16 columns at a time: all 64 next to v would not fit the registers of a 16-warp epilogue
           const uint8_t* arow = stg + b * kChunkBytes;
           if (g.aux_mode != AUX_DSOFTMAX) {

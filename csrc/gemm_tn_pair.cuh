@@ -323,7 +323,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     for (int tile = cluster_id; ok && tile < num_tiles; tile += num_clusters, ++tc) {
       const int acc = tc & 1;
       const uint32_t aph = (tc >> 1) & 1;
-      if (!mbar_wait(&tfull[acc], aph, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
+      if (!mbar_wait_warp(&tfull[acc], aph, abort_flag, g.err, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int ci = 0; ci < CH; ++ci, ++item) {
@@ -351,7 +351,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (MODE == MODE_AUX) {
           b = item % NBUF;
           const uint32_t bph = (item / NBUF) & 1;
-          if (!mbar_wait(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
+          if (!mbar_wait_warp(&mybar[b], bph, abort_flag, g.err, ERR_WAIT_AUX)) { ok = false; break; }
           const uint8_t* arow = stg + b * kChunkBytes;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {

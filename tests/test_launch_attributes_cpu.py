@@ -1,4 +1,5 @@
 """Host side of the launchers: the once-per-device kernel attributes (with a stand-in for the CUDA call) and the LayerNorm plan."""
+import re
 import shutil
 import subprocess
 from pathlib import Path
@@ -106,3 +107,11 @@ def test_a_wait_budget_that_the_timers_low_word_cannot_hold_does_not_compile(tmp
     built = subprocess.run([NVCC, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(tmp_path), "-I", str(CSRC), "-c",
                             "-o", str(tmp_path / "unit.o"), str(tmp_path / "unit.cu")], capture_output=True, text=True)
     assert (built.returncode == 0) == compiles and (compiles or "low word" in built.stdout + built.stderr)
+
+
+@pytest.mark.parametrize("name", ["gemm_tn.cuh", "gemm_tn_pair.cuh", "gemm_nt.cuh", "gemm_nt_pair.cuh", "conv3_wgrad.cuh", "afno_rows_tc.cuh"])
+def test_whole_warps_take_the_end_of_a_wait_together(name):
+    """An epilogue warp goes on to elect.sync and TMEM loads, for which its lanes must be together: also where a wait ran out, which no
+    test can bring about."""
+    waits = re.findall(r"\b(mbar_wait\w*)\(&?(?:tfull|mybar)\b", (CSRC / name).read_text())
+    assert waits and set(waits) == {"mbar_wait_warp"}
