@@ -289,6 +289,15 @@ pa_tokens_fwd_kernel(PaSrc src, long long norm_off, int ld_tok, const float* __r
   }
 }
 
+// Heads wider than 32 would want 255 KB in the backward: there Wqkv, which is read after the last chunk of dWcomb and Wo and before the
+// chunks of Wcomb, takes their place (221 KB).  4 heads of width 64, Cout = 256: 39 / 77 us event to event, 8 heads, Cout = 512: 43 / 108 us.
+__host__ __device__ constexpr bool pa_bwd_shares(int Dp) { return Dp > 32; }
+// floats of Wqkv and of a chunk of dWcomb and Wo
+__host__ __device__ constexpr int pa_bwd_weights(int Dp) {
+  const int wq = 3 * Dp * (Dp + 4), chunk = kPaChunk * (kPaLp + Dp + 4);
+  return pa_bwd_shares(Dp) ? (wq > chunk ? wq : chunk) : wq + chunk;
+}
+
 template <int Dp>
 __global__ void __launch_bounds__(kPaTokenThreads)
 pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __restrict__ Wo, PaSaved sv,
@@ -309,9 +318,9 @@ pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __r
   float* pr = dout + S * L;        // [S][kPaLp]
   float* ds = pr + S * kPaLp;
   float* wq = ds + S * kPaLp;      // [3][Dp][L]
-  float* dwc = wq + 3 * Dp * L;    // [kPaChunk][kPaLp]  rows of dWcomb, this head's columns; later: of Wcomb
+  float* dwc = wq + (pa_bwd_shares(Dp) ? 0 : 3 * Dp * L);      // [kPaChunk][kPaLp]  rows of dWcomb, this head's columns; later: of Wcomb
   float* wo = dwc + kPaChunk * kPaLp;      // [kPaChunk][L]
-  float* inv_np = wo + kPaChunk * L;       // [S]
+  float* inv_np = ds + S * kPaLp + pa_bwd_weights(Dp);         // [S]
   const int h = blockIdx.x, slice = blockIdx.y, slices = gridDim.y, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   const int HS = H * S, inner = H * D, chunks = (Cout + kPaChunk - 1) / kPaChunk;
@@ -329,11 +338,14 @@ pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __r
     }
   };
   fetch(0);
+  auto load_wq = [&] {
 #pragma unroll 6
-  for (int i = tid; i < 3 * Dp * Dp; i += nt) {
-    const int j = i / Dp, d = i - j * Dp, part = j / Dp, r = j - part * Dp;
-    wq[j * L + d] = r < D && d < D ? Wqkv[(part * D + r) * D + d] : 0.f;
-  }
+    for (int i = tid; i < 3 * Dp * Dp; i += nt) {
+      const int j = i / Dp, d = i - j * Dp, part = j / Dp, r = j - part * Dp;
+      wq[j * L + d] = r < D && d < D ? Wqkv[(part * D + r) * D + d] : 0.f;
+    }
+  };
+  if (!pa_bwd_shares(Dp)) load_wq();
 #pragma unroll 4
   for (int i = tid; i < S * Dp; i += nt) {
     const int s = i / Dp, d = i - s * Dp, at = s * L + d;
@@ -370,6 +382,7 @@ pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __r
     }
     __syncthreads();
   }
+  if (pa_bwd_shares(Dp)) load_wq();                                      // the chunks are done with: all threads have met behind the last
   if (tid < tiles_sd) pa_each_tn<Dp>(acc_o, tid, [&](int s, int d, float x) { dout[s * L + d] = x; });
   __syncthreads();
   // dP = dout v^T ; dv = P^T dout
@@ -430,7 +443,7 @@ pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __r
       if (first) d_norm[h * S + s] = -dot / np;
     }
   }
-  __syncthreads();
+  __syncthreads();                         // also: Wqkv has been read where its memory is that of the chunks
   // Bcat rows h S + s: [Wcomb^T (Cout) | zeros ... d_tok[s][:] in block h ... zeros] ; BdT rows h D + d: d_tok[:, d] in block h
   const int ldc = Cout + inner;
   for (int chunk = slice; chunk < chunks; chunk += slices) {
@@ -510,8 +523,9 @@ static constexpr size_t pa_fwd_smem(size_t Dp) {
 }
 static constexpr size_t pa_bwd_smem(size_t Dp) {
   const size_t L = Dp + 4;
-  return sizeof(float) * (8 * kPaS * L + 2 * kPaS * kPaLp + 3 * Dp * L + kPaChunk * kPaLp + kPaChunk * L + kPaS);
+  return sizeof(float) * (8 * kPaS * L + 2 * kPaS * kPaLp + pa_bwd_weights(int(Dp)) + kPaS);
 }
+static_assert(pa_bwd_smem(kPaMaxD) <= 226 * 1024, "the widest head that is accepted fits");
 // f(width) with the padded head width as a constant
 template <class F>
 static int pa_by_width(int D, F f) {
@@ -593,15 +607,12 @@ int pnm_pa_tokens_bwd(const void* const* srcs, int world, int use_flags, const f
   auto launch = [&](auto width) {
     constexpr int Dp = decltype(width)::value;
     constexpr size_t smem = pnm::pa_bwd_smem(Dp);
-    if constexpr (smem > 226 * 1024) return -2;
-    else {
-      static pnm::DeviceMask smem_set{0};
-      if (!pnm::allow_smem(pnm::pa_tokens_bwd_kernel<Dp>, smem, smem_set)) return -4;
-      pnm::pa_tokens_bwd_kernel<Dp><<<dim3(H, pnm::pa_slices(Cout)), pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(
-          pnm::make_src(srcs, world, use_flags), Wqkv, Wo, pnm::make_saved(saved), dWo, dWqkv, d_norm, (__nv_bfloat16*)Bcat16, (__nv_bfloat16*)BdT16,
-          H, D, Cout, scale, share, p, err);
-      return 0;
-    }
+    static pnm::DeviceMask smem_set{0};
+    if (!pnm::allow_smem(pnm::pa_tokens_bwd_kernel<Dp>, smem, smem_set)) return -4;
+    pnm::pa_tokens_bwd_kernel<Dp><<<dim3(H, pnm::pa_slices(Cout)), pnm::kPaTokenThreads, smem, (cudaStream_t)stream>>>(
+        pnm::make_src(srcs, world, use_flags), Wqkv, Wo, pnm::make_saved(saved), dWo, dWqkv, d_norm, (__nv_bfloat16*)Bcat16, (__nv_bfloat16*)BdT16,
+        H, D, Cout, scale, share, p, err);
+    return 0;
   };
   const int code = pnm::pa_by_width(D, launch);
   if (code) return code;

@@ -64,10 +64,11 @@ def test_fused_batch_two():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("H,D,cout", [(8, 32, 256), (8, 32, 264), (3, 16, 72), (4, 8, 200), (2, 4, 64), (3, 2, 40), (1, 1, 8)])
+@pytest.mark.parametrize("H,D,cout", [(8, 32, 256), (8, 32, 264), (3, 16, 72), (4, 8, 200), (2, 4, 64), (3, 2, 40), (1, 1, 8), (8, 64, 512), (2, 64, 264),
+                                      (1, 64, 64)])
 def test_slice_token_kernels(H, D, cout):
     """Slice-token attention and its backward, head widths below and at the tile, one to five chunks of 64 output channels (a head has at
-    most four CTAs), against autograd in 64 bits.  fp32 sums of at most 264 terms; bf16 results carry 2^-9 of a value."""
+    most four CTAs), against autograd in 64 bits.  fp32 sums of at most 512 terms; bf16 results carry 2^-9 of a value."""
     from physicsnemo_b200.ops import pa_small as P
 
     S, g = P.S, torch.Generator(device="cuda").manual_seed(H * D + cout)
@@ -99,3 +100,34 @@ def test_slice_token_kernels(H, D, cout):
     close(Bcat, torch.cat((wcomb.t(), blocks), 1), 2.0 ** -8)
     close(BdT, blocks.t(), 2.0 ** -8)
     assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,heads,dim_head", [(256, 8, 64), (128, 1, 64)])
+def test_training_call_of_the_module(dim, heads, dim_head):
+    """Whatever the fused path takes forward it takes backward: the module's default head width, against the plain path in fp32.  Gradients
+    are compared as in the test of a block."""
+    from physicsnemo_b200.nn.module.physics_attention import PhysicsAttentionIrregularMesh
+
+    torch.manual_seed(dim)
+    mod = PhysicsAttentionIrregularMesh(dim, heads=heads, dim_head=dim_head, slice_num=64, use_te=False).cuda()
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.add_(torch.randn_like(p) * 0.02)
+    ref = copy.deepcopy(mod)
+    x = torch.randn(1, 3001, dim, device="cuda")
+    g = torch.randn_like(x)
+    xs = [x.clone().requires_grad_(True) for _ in range(2)]
+    before = ops.kernel_launches()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        out = mod(xs[0])
+    out.float().backward(g)
+    assert ops.kernel_launches() - before >= 10, "fused kernels were not used"
+    want = ref(xs[1])
+    want.backward(g)
+    assert ops.device_error() == 0
+    assert _rel(out, want) < 3e-2
+    assert _rel(xs[0].grad, xs[1].grad) < 3e-2
+    total = torch.sqrt(sum(q.grad.float().pow(2).sum() for q in ref.parameters())).item()
+    for (name, p), (_, q) in zip(mod.named_parameters(), ref.named_parameters()):
+        assert (p.grad.float() - q.grad.float()).norm().item() < 2e-2 * (q.grad.float().norm().item() + 1e-2 * total), name
