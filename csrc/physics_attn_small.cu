@@ -512,7 +512,7 @@ pa_prepare_bwd_kernel(const float* __restrict__ dWc, const float* __restrict__ d
   } else {
     for (int h = tid; h < H; h += blockDim.x) {
       const float T = temp[h];
-      dtemp[h] = (T > 0.5f && T < 5.f) ? -grp[h] / T : 0.f;
+      dtemp[h] = (T >= 0.5f && T <= 5.f) ? -grp[h] / T : 0.f;      // torch.clamp passes the gradient at its ends; 0.5 is the initial value
     }
   }
 }

@@ -131,3 +131,19 @@ def test_training_call_of_the_module(dim, heads, dim_head):
     total = torch.sqrt(sum(q.grad.float().pow(2).sum() for q in ref.parameters())).item()
     for (name, p), (_, q) in zip(mod.named_parameters(), ref.named_parameters()):
         assert (p.grad.float() - q.grad.float()).norm().item() < 2e-2 * (q.grad.float().norm().item() + 1e-2 * total), name
+
+
+@pytest.mark.gpu
+def test_temperatures_at_the_ends_of_their_range_have_gradients():
+    """The initial temperature is the lower end of the clamp, where torch passes the gradient on."""
+    from physicsnemo_b200.ops import pa_small as P
+
+    temp = torch.tensor([0.4, 0.5, 0.7, 5.0, 5.1], device="cuda")
+    H, D, C = temp.numel(), 8, 64
+    rn = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
+    sums = rn(H)                                                         # of d(logit / T) logit / T
+    dtemp = P.prepare_bwd(rn(H * P.S, C), rn(H * P.S), sums, rn(H * D, C), rn(H * D), rn(P.S, D), temp, H, D)[-1]
+    t = temp.double().requires_grad_(True)
+    (want,) = torch.autograd.grad((-sums.double() * torch.log(torch.clamp(t, min=0.5, max=5))).sum(), t)
+    assert torch.allclose(dtemp.double(), want, rtol=1e-6, atol=0)
+    assert ops.device_error() == 0
