@@ -97,7 +97,8 @@ class _PhysAttnFn(torch.autograd.Function):
         grp = torch.zeros(H, dtype=torch.float32, device=dev)
         # side by side: what follows is one product over their columns each (rows of x once, one operand for the wide tiles)
         both = torch.empty((xn.shape[0], HS + inner), dtype=torch.bfloat16, device=dev)
-        G.gemm_tn(dout, Bcat, a2=fx, bias=d_norm, aux=w, aux_mode=G.AUX_DSOFTMAX, scale=inv_t, scale_post=True, group_out=grp,
+        a, a2 = (dout, fx) if Cout % 64 == 0 else (torch.cat((dout, fx), 1), None)       # a second operand starts on a block of 64 columns
+        G.gemm_tn(a, Bcat, a2=a2, bias=d_norm, aux=w, aux_mode=G.AUX_DSOFTMAX, scale=inv_t, scale_post=True, group_out=grp,
                   out=both[:, :HS])                                           # d logits
         G.gemm_tn(w, BdT, out=both[:, HS:])                                   # d fx = w @ blockdiag(d_tok)
         dW, db = G.gemm_nt(both, xn, colsum=True)                             # (H*S + H*D, C), (H*S + H*D,)

@@ -103,10 +103,10 @@ def test_slice_token_kernels(H, D, cout):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dim,heads,dim_head", [(256, 8, 64), (128, 1, 64)])
+@pytest.mark.parametrize("dim,heads,dim_head", [(256, 8, 64), (128, 1, 64), (72, 4, 16), (200, 8, 32)])
 def test_training_call_of_the_module(dim, heads, dim_head):
-    """Whatever the fused path takes forward it takes backward: the module's default head width, against the plain path in fp32.  Gradients
-    are compared as in the test of a block."""
+    """Whatever the fused path takes forward it takes backward: the module's default head width, widths that are no multiple of 64, against
+    the plain path in fp32.  Gradients are compared as in the test of a block."""
     from physicsnemo_b200.nn.module.physics_attention import PhysicsAttentionIrregularMesh
 
     torch.manual_seed(dim)
