@@ -171,13 +171,9 @@ PyObject* gemm_nt(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Tensor &a = rowmajor2d(a0, own[0]), &b = rowmajor2d(b0, own[1]);
     const int64_t M = a.size(0), Na = a.size(1), Nb = b.size(1);
     require(b.size(0) == M, "operands have different numbers of rows");
-    if (!given.defined() && !given_sums.defined() && want_sums) {          // the gradients of a layer: made and dropped together
-      const Tensor both = zeros32({Na * (Nb + 1)}, a);
-      made = both.narrow(0, 0, Na * Nb).view({Na, Nb}); made_sums = both.narrow(0, Na * Nb, Na);
-    } else {
-      if (!given.defined()) made = zeros32({Na, Nb}, a);
-      if (!given_sums.defined() && want_sums) made_sums = zeros32({Na}, a);
-    }
+    // two buffers: a weight's gradient and its bias' are held, saved and changed one without the other
+    if (!given.defined()) made = zeros32({Na, Nb}, a);
+    if (!given_sums.defined() && want_sums) made_sums = zeros32({Na}, a);
     check("pnm_gemm_nt", pnm_gemm_nt(ptr(a), int(a.stride(0)), ptr(b), int(b.stride(0)), fptr(out), int(out.stride(0)), fptr(sums), int(M), int(Na),
                                      int(Nb), cap, stream()));
   }
@@ -792,24 +788,26 @@ PyObject* pa_tokens_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// pa_prepare_bwd(dWc, dbc, per-head sums, Wx, bx, Ws, temperature, heads, head width) -> (dWx, dbx, dWs, dbs, dtemp)
+// pa_prepare_bwd(dW [64 H + H D, C], db, per-head sums, Wx, bx, Ws, temperature, heads, head width) -> (dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp)
 PyObject* pa_prepare_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   need_args(n, 9);
   const Tensor* p[7];
   for (int i = 0; i < 7; ++i) p[i] = &tensor(args[i]);
   const int64_t H = integer(args[7]), D = integer(args[8]);
-  Tensor dWx, dbx, dWs, dbs, dtemp;
+  Tensor dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp;
   {
     const Unlocked unlocked;
     const Tensor& like = *p[3];
-    const int64_t C = like.size(1);
-    dWx = empty({H * D, C}, at::kFloat, like); dbx = empty({H * D}, at::kFloat, like); dWs = empty({64, D}, at::kFloat, like);
-    dbs = empty({64}, at::kFloat, like); dtemp = empty({H}, at::kFloat, like);
+    const int64_t C = like.size(1), inner = H * D, rows = H * 64 + inner;
+    require(p[0]->numel() == rows * C && p[1]->numel() == rows && p[0]->is_contiguous() && p[1]->is_contiguous(), "gradients of another layer");
+    dWx = empty({inner, C}, at::kFloat, like); dbx = empty({inner}, at::kFloat, like); dWfx = empty({inner, C}, at::kFloat, like);
+    dbfx = empty({inner}, at::kFloat, like); dWs = empty({64, D}, at::kFloat, like); dbs = empty({64}, at::kFloat, like);
+    dtemp = empty({H}, at::kFloat, like);
     check("pnm_pa_prepare_bwd", pnm_pa_prepare_bwd(fptr(*p[0]), fptr(*p[1]), fptr(*p[2]), fptr(*p[3]), fptr(*p[4]), fptr(*p[5]), fptr(*p[6]), fptr(dWx),
-                                                   fptr(dbx), fptr(dWs), fptr(dbs), fptr(dtemp), int(H), int(D), int(C), stream()));
+                                                   fptr(dbx), fptr(dWfx), fptr(dbfx), fptr(dWs), fptr(dbs), fptr(dtemp), int(H), int(D), int(C), stream()));
   }
-  return tuple_of({&dWx, &dbx, &dWs, &dbs, &dtemp});
+  return tuple_of({&dWx, &dbx, &dWfx, &dbfx, &dWs, &dbs, &dtemp});
   END_HANDLE_TH_ERRORS
 }
 

@@ -9,7 +9,7 @@
 //   pa_tokens_bwd    dWcomb (sum over ranks in the prologue) -> d out_tokens, dWo -> attention backward -> d tokens,
 //                    dWqkv -> the operands of the point-sized backward GEMMs: Bcat = [Wcomb^T | blockdiag(d_tok)],
 //                    BdT = blockdiag(d_tok)^T (bf16), d_norm
-//   pa_prepare_bwd   dWx, dbx, dWs, dbs, dT from dWc, dbc and the per-head temperature sums
+//   pa_prepare_bwd   dWx, dbx, dWs, dbs, dT from dWc, dbc and the per-head temperature sums; dWfx, dbfx out of the rows behind dWc, dbc
 //
 // Cross-rank sums: the producers (gemm_nt) write into a region of this rank's symmetric buffer, a signal kernel raises
 // the flags, and the token kernels add the P copies with direct peer loads after a bounded wait -- there is no
@@ -472,13 +472,14 @@ pa_tokens_bwd_kernel(PaSrc src, const float* __restrict__ Wqkv, const float* __r
 __global__ void __launch_bounds__(256)
 pa_prepare_bwd_kernel(const float* __restrict__ dWc, const float* __restrict__ dbc, const float* __restrict__ grp,
                       const float* __restrict__ Wx, const float* __restrict__ bx, const float* __restrict__ Ws,
-                      const float* __restrict__ temp, float* __restrict__ dWx, float* __restrict__ dbx,
-                      float* __restrict__ dWs, float* __restrict__ dbs, float* __restrict__ dtemp, int H, int D, int C) {
-  const int S = kPaS, inner = H * D;
+                      const float* __restrict__ temp, float* __restrict__ dWx, float* __restrict__ dbx, float* __restrict__ dWfx,
+                      float* __restrict__ dbfx, float* __restrict__ dWs, float* __restrict__ dbs, float* __restrict__ dtemp, int H, int D, int C) {
+  const int S = kPaS, inner = H * D, HS = H * S;
   const int b = blockIdx.x, tid = threadIdx.x;
   if (b < inner) {
     const int h = b / D, d = b % D;
     for (int c = tid; c < C; c += blockDim.x) {
+      dWfx[(size_t)b * C + c] = dWc[(size_t)(HS + b) * C + c];
       float acc = 0.f;
       for (int s = 0; s < S; ++s) acc += Ws[s * D + d] * dWc[(size_t)(h * S + s) * C + c];
       dWx[(size_t)b * C + c] = acc;
@@ -487,6 +488,7 @@ pa_prepare_bwd_kernel(const float* __restrict__ dWc, const float* __restrict__ d
       float acc = 0.f;
       for (int s = 0; s < S; ++s) acc += Ws[s * D + d] * dbc[h * S + s];
       dbx[b] = acc;
+      dbfx[b] = dbc[HS + b];
     }
   } else if (b < inner + (S * D) / 8) {
     // dWs[s][d] = sum_h ( sum_c dWc[h S + s][c] Wx[h D + d][c] + dbc[h S + s] bx[h D + d] ): one warp per (s, d), lanes over c
@@ -619,12 +621,14 @@ int pnm_pa_tokens_bwd(const void* const* srcs, int world, int use_flags, const f
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+// dWc [H*S + H*D, C], dbc [H*S + H*D]: gradients of the combined projection, then those of the values' projection, which are copied out
+// (a parameter's gradient is a buffer of its own).
 int pnm_pa_prepare_bwd(const float* dWc, const float* dbc, const float* grp, const float* Wx, const float* bx, const float* Ws,
-                       const float* temp, float* dWx, float* dbx, float* dWs, float* dbs, float* dtemp, int H, int D, int C,
-                       void* stream) {
+                       const float* temp, float* dWx, float* dbx, float* dWfx, float* dbfx, float* dWs, float* dbs, float* dtemp, int H, int D,
+                       int C, void* stream) {
   if (H <= 0 || D <= 0 || D > pnm::kPaMaxD || C <= 0) return -2;
-  pnm::pa_prepare_bwd_kernel<<<H * D + (pnm::kPaS * D) / 8 + 1, 256, 0, (cudaStream_t)stream>>>(dWc, dbc, grp, Wx, bx, Ws, temp, dWx, dbx,
-                                                                                      dWs, dbs, dtemp, H, D, C);
+  pnm::pa_prepare_bwd_kernel<<<H * D + (pnm::kPaS * D) / 8 + 1, 256, 0, (cudaStream_t)stream>>>(dWc, dbc, grp, Wx, bx, Ws, temp, dWx, dbx, dWfx,
+                                                                                      dbfx, dWs, dbs, dtemp, H, D, C);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

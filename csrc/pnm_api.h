@@ -286,7 +286,7 @@ int pnm_resample2x_nhwc(const void* x, void* y, int n, int h, int w, int c, int 
 int pnm_pa_prepare_fwd(const float* Wx, const float* bx, const float* Wfx, const float* Ws, const float* bs, const float* temp, void* Wc16, float* bc, float* inv_t, void* Wfx16, void* Wback16, int H, int D, int C, void* stream);
 int pnm_pa_tokens_fwd(const void* const* srcs, int world, int use_flags, long long norm_off, int ld_tok, const float* Wqkv, const float* Wo, void* wcomb16, void* const* saved, int H, int D, int Cout, float scale, const void* const* bases, int rank, unsigned int epoch, long long capacity_floats, double budget_s, const void* epoch_base, void* stream);
 int pnm_pa_tokens_bwd(const void* const* srcs, int world, int use_flags, const float* Wqkv, const float* Wo, void* const* saved, float* dWo, float* dWqkv, float* d_norm, void* Bcat16, void* BdT16, int H, int D, int Cout, float scale, float share, const void* const* bases, int rank, unsigned int epoch, long long capacity_floats, double budget_s, const void* epoch_base, void* stream);
-int pnm_pa_prepare_bwd(const float* dWc, const float* dbc, const float* grp, const float* Wx, const float* bx, const float* Ws, const float* temp, float* dWx, float* dbx, float* dWs, float* dbs, float* dtemp, int H, int D, int C, void* stream);
+int pnm_pa_prepare_bwd(const float* dWc, const float* dbc, const float* grp, const float* Wx, const float* bx, const float* Ws, const float* temp, float* dWx, float* dbx, float* dWfx, float* dbfx, float* dWs, float* dbs, float* dtemp, int H, int D, int C, void* stream);
 int pnm_graph_halo_publish(const void* in, int ldi, const int* send_idx, void* mailbox, long long n_send, int C, const void* const* bases, int rank, int world, unsigned int epoch, long long capacity_floats, const void* epoch_base, void* counter, void* stream);
 int pnm_graph_gather_halo(const void* in, int ldi, const int* idx, int n_local, const int* halo_owner, const int* halo_slot, const void* const* mailboxes, void* out, int ldo, long long E, int C, int wait, const void* const* bases, int rank, int world, unsigned int epoch, long long capacity_floats, double budget_s, const void* epoch_base, void* stream);
 int pnm_graph_halo_pull_add(void* dn, int ldn, const int* bnd_row, const int* bnd_off, const int* ent_peer, const int* ent_slot, const void* const* mailboxes, long long n_bnd, int C, int wait, const void* const* bases, int rank, int world, unsigned int epoch, long long capacity_floats, double budget_s, const void* epoch_base, void* stream);

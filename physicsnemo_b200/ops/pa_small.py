@@ -98,8 +98,8 @@ def tokens_bwd(src_ptrs: Sequence[int], Wqkv, Wo, saved, H: int, D: int, share: 
     return dWo, dWqkv, d_norm, Bcat, BdT
 
 
-def prepare_bwd(dWc, dbc, grp, Wx, bx, Ws, temp, H: int, D: int):
-    """``(dWx, dbx, dWs, dbs, dtemp)`` from the gradients of the combined projection."""
-    res = _lib.host().pa_prepare_bwd(dWc, dbc, grp, Wx, bx, Ws, temp, H, D)
+def prepare_bwd(dW, db, grp, Wx, bx, Ws, temp, H: int, D: int):
+    """``(dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp)`` from the gradients of the combined projection and, below them, of the values' projection."""
+    res = _lib.host().pa_prepare_bwd(dW, db, grp, Wx, bx, Ws, temp, H, D)
     _g.launch_count += 1
     return res

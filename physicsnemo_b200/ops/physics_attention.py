@@ -102,9 +102,8 @@ class _PhysAttnFn(torch.autograd.Function):
                   out=both[:, :HS])                                           # d logits
         G.gemm_tn(w, BdT, out=both[:, HS:])                                   # d fx = w @ blockdiag(d_tok)
         dW, db = G.gemm_nt(both, xn, colsum=True)                             # (H*S + H*D, C), (H*S + H*D,)
-        dWc, dWfx, dbc, dbfx = dW[:HS], dW[HS:], db[:HS], db[HS:]             # dWc lives as long as its neighbour: 4 H S C bytes
-        dWx, dbx, dWs, dbs, dtemp = P.prepare_bwd(dWc, dbc, grp, Wx.detach(), bx.detach(), Ws.detach(),
-                                                  temp.detach().reshape(-1), H, D)
+        dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp = P.prepare_bwd(dW, db, grp, Wx.detach(), bx.detach(), Ws.detach(),
+                                                              temp.detach().reshape(-1), H, D)
         dxn = G.gemm_tn(both, Wback)                                          # [d logits | d fx] @ [Wc ; Wfx]
         dres = dout if ctx.has_res else None
         grads = [dWx, dbx, dWfx, dbfx, dWs, dbs, dtemp.reshape(ctx.temp_shape), dWqkv, dWo, dbo]

@@ -89,6 +89,19 @@ def test_gemm_nt(M, Na, Nb):
     assert ops.device_error() == 0
 
 
+def test_gradients_of_a_weight_and_its_bias_are_two_buffers():
+    """A bias' gradient that is held or saved holds no weight's, and neither notices what is done to the other in place."""
+    x = torch.randn(300, 128, device="cuda").bfloat16()
+    params = [torch.randn(256, 128, device="cuda", requires_grad=True), torch.randn(256, device="cuda", requires_grad=True)]
+    ops.mlp_chain(x, params[:1], params[1:], [G.ACT_NONE]).float().sum().backward()
+    for p in params:
+        assert p.grad.untyped_storage().nbytes() == p.grad.nbytes
+    dw, db = ops.gemm_nt(x, x, colsum=True)
+    before = dw._version
+    db.add_(1)
+    assert dw._version == before and dw.untyped_storage().data_ptr() != db.untyped_storage().data_ptr()
+
+
 @pytest.mark.parametrize("P,Mp,N,K", [(8, 8320, 192, 192), (3, 256, 64, 64), (2, 384, 264, 136)])
 def test_gemm_stacked_batches(P, Mp, N, K):
     """`P` equal problems in one launch: forward with bias + ReLU, data gradient with the ReLU mask, weight gradient

@@ -131,6 +131,7 @@ def test_training_call_of_the_module(dim, heads, dim_head):
     total = torch.sqrt(sum(q.grad.float().pow(2).sum() for q in ref.parameters())).item()
     for (name, p), (_, q) in zip(mod.named_parameters(), ref.named_parameters()):
         assert (p.grad.float() - q.grad.float()).norm().item() < 2e-2 * (q.grad.float().norm().item() + 1e-2 * total), name
+        assert p.grad.untyped_storage().nbytes() == p.grad.nbytes, name          # a buffer of its own: held and saved alone
 
 
 @pytest.mark.gpu
@@ -142,7 +143,7 @@ def test_temperatures_at_the_ends_of_their_range_have_gradients():
     H, D, C = temp.numel(), 8, 64
     rn = lambda *s: torch.randn(*s, device="cuda")  # noqa: E731
     sums = rn(H)                                                         # of d(logit / T) logit / T
-    dtemp = P.prepare_bwd(rn(H * P.S, C), rn(H * P.S), sums, rn(H * D, C), rn(H * D), rn(P.S, D), temp, H, D)[-1]
+    dtemp = P.prepare_bwd(rn(H * (P.S + D), C), rn(H * (P.S + D)), sums, rn(H * D, C), rn(H * D), rn(P.S, D), temp, H, D)[-1]
     t = temp.double().requires_grad_(True)
     (want,) = torch.autograd.grad((-sums.double() * torch.log(torch.clamp(t, min=0.5, max=5))).sum(), t)
     assert torch.allclose(dtemp.double(), want, rtol=1e-6, atol=0)
