@@ -182,7 +182,9 @@ int pnm_conv2d_nhwc(const void* x, const void* weight, void* y, int n, int h, in
   c.max_ctas = max_ctas;
   c.conv = 1; c.img_n = n; c.img_h = h; c.img_w = w; c.cin = cin; c.ksize = ksize;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (ksize == 3 && !max_ctas && ((bn == 0 && pair_gemm_enabled()) || bn == 1128 || bn == 1256)) {     // 1128, 1256: tile by name
+  const bool named = bn == 1128 || bn == 1256;   // a tile of columns of taps by its width: for comparisons of the two
+  if (named && (ksize != 3 || max_ctas)) return -2;
+  if (ksize == 3 && !max_ctas && (named || (bn == 0 && pair_gemm_enabled()))) {
     if (bn == 1256 || (bn == 0 && pnm::conv3_tile_width(c, g_num_sms) == 256))
       return pnm::launch_gemm_tn_pair<256, pnm::MODE_CONV3>(c, g_num_sms, g_err_ptr, st);
     return pnm::launch_gemm_tn_pair<128, pnm::MODE_CONV3>(c, g_num_sms, g_err_ptr, st);

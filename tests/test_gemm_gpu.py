@@ -262,6 +262,35 @@ def test_conv3x3_forward_by_columns_of_taps(n, h, w, cin, cout):
     assert ops.device_error() == 0
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 1, 1, 64, 64), (3, 7, 15, 128, 128), (1, 17, 33, 192, 136), (2, 41, 50, 64, 264), (1, 64, 64, 512, 512),
+                                            (1, 130, 126, 128, 384)])
+def test_conv3x3_tiles_of_both_widths(n, h, w, cin, cout):
+    """Every shape on tiles of 128 and of 256 output channels, whichever the rule would take; a tile that does not apply is refused."""
+    import ctypes as c
+
+    from physicsnemo_b200.ops import _lib
+    from physicsnemo_b200.ops import conv as C
+
+    conv = _lib.load(required=True)["pnm_conv2d_nhwc"]
+    conv.argtypes, conv.restype = [c.c_void_p] * 3 + [c.c_int] * 6 + [c.c_void_p] + [c.c_int] * 3 + [c.c_void_p], c.c_int
+    g = torch.Generator(device="cuda").manual_seed(n * h + w)
+    x = torch.randn(n, h, w, cin, generator=g, device="cuda").bfloat16()
+    wt = (torch.randn(cout, cin, 3, 3, generator=g, device="cuda") / (9 * cin) ** 0.5).bfloat16()
+    b = torch.randn(cout, generator=g, device="cuda")
+    packed = C._forward_operand(wt, cin, cout)
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), wt.double(), b.double(), padding=1).permute(0, 2, 3, 1)
+    for bn in (1128, 1256):
+        y = torch.full((n, h, w, cout), float("nan"), device="cuda", dtype=torch.bfloat16)
+
+        def call(ksize, max_ctas):
+            return conv(x.data_ptr(), packed.data_ptr(), y.data_ptr(), n, h, w, cin, cout, ksize, b.data_ptr(), 0, bn, max_ctas, _lib.stream())
+
+        assert call(3, 0) == 0
+        assert float(((y - ref).abs() - 2.0 ** -8 * ref.abs()).max()) < 1e-4        # as above
+        assert call(1, 0) == call(3, 4) == -2
+    assert ops.device_error() == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,h,w,cin,cout", [(1, 4, 16, 128, 128), (2, 33, 31, 64, 64), (1, 45, 50, 192, 72), (3, 29, 47, 128, 200),
                                             (1, 64, 64, 320, 136), (1, 130, 126, 128, 256), (2, 24, 24, 512, 512)])
