@@ -201,12 +201,16 @@ __device__ __forceinline__ void epi_act(uint64_t* v, int act) {
     default: break;
   }
 }
-// 16 columns with the auxiliary values of the same columns (all modes but the softmax backward)
+// 16 columns with the auxiliary values of the same columns (all modes but the softmax backward; `ALL` false: those with arithmetic on
+// the auxiliary values, the only ones that come to the 256-column tiles of one CTA)
+template <bool ALL>
 __device__ __forceinline__ void epi_aux16(uint64_t* v, const uint64_t* a, int mode) {
   switch (mode) {
     case AUX_ADD:
+      if (ALL) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = f2_add(v[j], a[j]);
+        for (int j = 0; j < 8; ++j) v[j] = f2_add(v[j], a[j]);
+      }
       break;
     case AUX_DGELU:
 #pragma unroll
@@ -217,10 +221,12 @@ __device__ __forceinline__ void epi_aux16(uint64_t* v, const uint64_t* a, int mo
       for (int j = 0; j < 8; ++j) v[j] = f2_mul(v[j], silu_grad_f2(a[j]));
       break;
     case AUX_DRELU:
+      if (ALL) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2 x = f2_get(v[j]), z = f2_get(a[j]);
-        v[j] = f2_make(z.x > 0.f ? x.x : 0.f, z.y > 0.f ? x.y : 0.f);
+        for (int j = 0; j < 8; ++j) {
+          const float2 x = f2_get(v[j]), z = f2_get(a[j]);
+          v[j] = f2_make(z.x > 0.f ? x.x : 0.f, z.y > 0.f ? x.y : 0.f);
+        }
       }
       break;
     default: break;
@@ -491,7 +497,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint64_t x[8], a[8];
             load16(k, x);
             stage_read16(arow, lane, k, a);
-            if (g.aux_mode != AUX_DSOFTMAX) epi_aux16(x, a, g.aux_mode);
+            if (g.aux_mode != AUX_DSOFTMAX) epi_aux16<false>(x, a, g.aux_mode);
             else if (g.group_out) epi_dsoftmax16<true>(x, a, neg_dot, gs);
             else epi_dsoftmax16<false>(x, a, neg_dot, gs);
             if (g.scale && g.scale_post) epi_vector<8, true>(x, g.scale, c0 + 16 * k, g.N, scale_vec);
@@ -590,7 +596,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int k = 0; k < 4; ++k) {
               uint64_t a[8];
               stage_read16(arow, lane, k, a);
-              epi_aux16(v + 8 * k, a, g.aux_mode);
+              epi_aux16<true>(v + 8 * k, a, g.aux_mode);
             }
           } else {
             uint64_t d[2] = {0, 0}, gs = 0;

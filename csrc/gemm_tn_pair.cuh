@@ -357,7 +357,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           for (int k = 0; k < 4; ++k) {
             uint64_t a[8];
             stage_read16(arow, lane, k, a);
-            epi_aux16(v + 8 * k, a, g.aux_mode);
+            epi_aux16<true>(v + 8 * k, a, g.aux_mode);
           }
         } else if (Cfg::TWO) {
           b = 2 * (item % (NBUF / 2));
