@@ -30,8 +30,10 @@ namespace pnm {
 constexpr int kPairThreads = 320;
 
 // Two staging buffers per epilogue warp: a third one for the auxiliary operand costs a stage and measured slower on K = 3072 (132 vs
-// 124 us) and no faster on K = 768.  With two outputs each has one and both leave behind one fence (two pairs of buffers leave three
-// stages of five: Z_FIGS).
+// 124 us) and no faster on K = 768.  With two outputs each has one and both leave behind one fence.  MODE_Z4 has two pairs of buffers and
+// three operand stages instead of five, which pays for the shortest products only.  GELU and its argument, one pair / two pairs:
+//   262 144 rows -> 1024   K = 256 269 / 243 us, 320 269 / 261, 384 245 / 271, 448 253 / 312, 512 273 / 320, 768 366 / 423
+//    32 400 rows -> 3072   K = 256  93 /  87 us, 320  93 /  97, 384  95 / 103, 448  99 / 118, 512 104 / 120, 768 132 / 155
 //
 // MODE_CONV3 (3 x 3 convolutions, no halo rows of peers): the three taps of a filter column read windows of the image that differ by
 // whole rows of 16 pixels = 2048 bytes, so ONE box of 10 x 16 pixels holds the A operand of all three, each starting on a

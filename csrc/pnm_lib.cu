@@ -117,7 +117,7 @@ int pnm_gemm_tn(const void* A, int lda, const void* A2, int lda2, const void* A3
   if (bn == 0 && pair_gemm_enabled() && pnm::pair_gemm_applicable(c)) {
     // compute-bound shapes: 256 x 256 tiles on CTA pairs (tcgen05.mma.cta_group::2)
     if (AUX) return pnm::launch_gemm_tn_pair<256, pnm::MODE_AUX>(c, g_num_sms, g_err_ptr, st);
-    if (Z && K < 512) return pnm::launch_gemm_tn_pair<256, pnm::MODE_Z4>(c, g_num_sms, g_err_ptr, st);
+    if (Z && K <= 256) return pnm::launch_gemm_tn_pair<256, pnm::MODE_Z4>(c, g_num_sms, g_err_ptr, st);      // see there
     if (Z) return pnm::launch_gemm_tn_pair<256, pnm::MODE_Z>(c, g_num_sms, g_err_ptr, st);
     return pnm::launch_gemm_tn_pair<256, pnm::MODE_PLAIN>(c, g_num_sms, g_err_ptr, st);
   }

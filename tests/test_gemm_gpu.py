@@ -315,7 +315,7 @@ def test_conv3x3_weight_gradient_by_columns_of_taps(n, h, w, cin, cout):
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K", [(2048, 1024, 256), (2999, 1096, 264), (2304, 1032, 504), (2100, 1024, 512)])
 def test_gemm_tn_two_outputs_of_short_products(M, N, K):
-    """Two outputs on CTA pairs below K = 512 keep two pairs of staging buffers: ragged edges, several blocks per warp."""
+    """Two outputs on CTA pairs, two pairs of staging buffers at K = 256 and one above: ragged edges, several blocks per warp."""
     a, b, bias = _rand(M, K), _rand(N, K, scale=K ** -0.5), torch.randn(N, device="cuda")
     y, z = G.gemm_tn(a, b, bias=bias, act=G.ACT_GELU, z_out=True)
     zr = a.double() @ b.double().t() + bias.double()
