@@ -589,7 +589,9 @@ def test_afno_spectral_filter_kernels(shape, mlp):
                                              (2, 45, 90, 768, 8, 46), (3, 4, 255, 64, 1, 20), (1, 2, 256, 64, 1, 40), (1, 2, 300, 64, 1, 10), (1, 160, 20, 256, 2, 10)])
 def test_afno_row_transforms(B, H, W, C, nb, kept):
     """Odd and even rows, rows and modes that fill no tile, channels that fill no box of 64, rows too long for one box: to the spectrum, a
-    sum of W fp32 terms, and back to bf16 tokens, with and without addends."""
+    sum of W fp32 terms, and back to bf16 tokens, with and without addends.  Up to 256 positions the spectrum has to be closer than a
+    transform whose twiddles lack their third bf16 term: 1.9e-6 off, 1.0e-6 where only the positions past 64 of 90 or past 192 of 255
+    lack it.  The sums themselves: 3 W / 16 additions, each off by 2^-24 of the sum, add up like a random walk to at most 4e-7."""
     import math
 
     from physicsnemo_b200 import ops
@@ -605,7 +607,7 @@ def test_afno_row_transforms(B, H, W, C, nb, kept):
         Y = torch.full((B * H, g.KX, C, 2), float("nan"), device="cuda")
         assert lib.pnm_afno_rows_r2c(A._ptrs8([x.data_ptr()]), Y.data_ptr(), g.arr, g.Tp, kw, 0, None, 0, 1, 0, 0, 1.0, None, st) == 0
         ref = torch.fft.rfft(x.double(), dim=1, norm="ortho")[:, :g.KX] * (weight if kw else torch.ones_like(weight))[:, None]
-        assert float((torch.view_as_complex(Y.double()) - ref).norm() / ref.norm()) < max(W, 16) * 2.0 ** -24
+        assert float((torch.view_as_complex(Y.double()) - ref).norm() / ref.norm()) < (5e-7 if W <= 256 else W * 2.0 ** -24)
     S = torch.randn(B * H, g.KX, C, 2, generator=gen, device="cuda")
     adds = [torch.randn(B * H, W, C, generator=gen, device="cuda").bfloat16() for _ in range(2)]
     k, w = torch.arange(g.KX, device="cuda"), torch.arange(W, device="cuda")
