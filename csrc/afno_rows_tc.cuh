@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kRowInvThreads, 1) afno_rows_c2r_tc_kernel(con
           const int i = i0 + n * kStride;
           if (!inside(i) || !ok) continue;
           uint4 u = *reinterpret_cast<const uint4*>(ys + (i >> 4) * kRowInvLd + 8 * (i & 15));
-          if (g.add0) {                          // residual terms of the surrounding block, summed in fp32 and rounded once
+          if (g.add0) {                          // residual terms of the surrounding block: added in fp32 to the rounded transform, rounded again
             uint64_t f[4] = {f2_from_bf16x2(u.x), f2_from_bf16x2(u.y), f2_from_bf16x2(u.z), f2_from_bf16x2(u.w)};
             auto add = [&](const uint4& b) {
               f[0] = f2_add(f[0], f2_from_bf16x2(b.x)); f[1] = f2_add(f[1], f2_from_bf16x2(b.y));

@@ -380,7 +380,7 @@ afno_rows_c2r_v2_kernel(const float2* __restrict__ X, TokenPtrs tok, AfGeom g, i
     const int w = it.row, v = it.col;
     uint4 u = *reinterpret_cast<const uint4*>(ys + w * g.Cb + v * 8);
     if (add0) {
-      // residual terms of the surrounding block (local [T, C] token layout), summed in fp32 and rounded once
+      // residual terms of the surrounding block (local [T, C] token layout): added in fp32 to the rounded transform, rounded again
       const long long at = ((long long)row * g.W + w) * g.C + c0 + v * 8;
       float f[8], a[8];
       sm_unpack8(u, f);

@@ -179,6 +179,10 @@ inline int launch_conv3_wgrad(const NtCall& c, int num_sms, int* err_word, cudaS
   g.tiles_a = (c.Na + 127) / 128;
   g.tiles_c = (c.cin + 127) / 128;
   const int tiles = g.tiles_a * g.tiles_c * 3;
+  // Whole parts only: 75 to 147 tiles leave SMs idle, 149 and more make rounds of whole tiles.  It is still the sooner kernel there (us,
+  // reduction GEMM / this; 16 x 16, 64 x 64, 128 x 128 pixels): 640 -> 640 channels, 75 tiles, 24 / 16, 114 / 49, 323 / 150; 512 -> 896, 84
+  // tiles, 24 / 16, 85 / 49, 221 / 150; 896 -> 896, 147 tiles, 34 / 21, 171 / 55, 636 / 156; 1024 -> 1024, 192 tiles, 40 / 29, 163 / 94,
+  // 431 / 289; 1280 -> 1280, 300 tiles, 54 / 37, 298 / 135, 833 / 442.
   int splits = num_sms / tiles;            // also few patches: 64 in 24 parts 16.4 us, in 8 18.4 us (256 -> 128 channels, 64 x 64 pixels)
   if (splits < 1) splits = 1;
   if (splits > g.patches) splits = g.patches;

@@ -96,6 +96,8 @@ struct PaSaved {        // per block, fp32, all [H][S][...]
 // its reads of shared memory: with one output per thread two words per multiply-add (8 heads of width 32, Cout = 256: 43.5 us forward,
 // 101 us backward on 8 CTAs), so a thread computes 4 x 4 outputs from 16-byte vectors, half a word per multiply-add or less, and a head
 // has four CTAs: 17.7 / 44.3 us.  Every output is one sum in the order of k, as before, but for the sums along rows.
+// With P ranks every CTA adds the P copies of its head's sums for itself, four times the peer reads of one CTA per head: backward, at the
+// sizes above, (P - 1) x 2 MB per rank, by the link's 770 GB/s 2.7 us a peer (estimated; not measured on several GPUs).
 constexpr int kPaChunk = 64;
 constexpr int kPaLp = kPaS + 4;          // row length of S x S matrices: 16-byte vectors of eight rows fall on different banks
 
