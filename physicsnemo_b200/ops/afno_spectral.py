@@ -135,12 +135,12 @@ class _AfnoFilterTcFn(torch.autograd.Function):
             _g._check(lib.pnm_afno_cols_idft(O2.data_ptr(), Y2.data_ptr(), g.arr, g.Mp, float(lam), st), "pnm_afno_cols_idft")
 
         if exchange is None:
-            src = tokens.contiguous()
+            src = _g._aligned(tokens.contiguous())
             out = torch.empty_like(src)
             rc = lib.pnm_afno_rows_r2c(_ptrs8([src.data_ptr()]), Y.data_ptr(), g.arr, g.Tp, 0, 0, None, 0, 1, 0, 0, 1.0, None, st)
             _g._check(rc, "pnm_afno_rows_r2c")
             cols()
-            addends = ([src] if add_input else []) + ([residual.contiguous()] if residual is not None else [])
+            addends = ([src] if add_input else []) + ([_g._aligned(residual.contiguous())] if residual is not None else [])
             _rows_c2r_local(lib, Y2, out, addends, g, 1, st)
         else:
             if add_input or residual is not None:
@@ -181,7 +181,7 @@ class _AfnoFilterTcFn(torch.autograd.Function):
             _g.gemm_tn_stacked(G1, w1t, out=dZ)
             _g._check(lib.pnm_afno_cols_idft(dZ.data_ptr(), dY.data_ptr(), g.arr, g.Mp, 0.0, st), "pnm_afno_cols_idft")
 
-        d = dout.to(torch.bfloat16).contiguous()
+        d = _g._aligned(dout.to(torch.bfloat16).contiguous())
         if exchange is None:
             dx = torch.empty_like(d)
             rc = lib.pnm_afno_rows_r2c(_ptrs8([d.data_ptr()]), dY2.data_ptr(), g.arr, g.Tp, 1, 0, None, 0, 1, 0, 0, 1.0, None, st)
@@ -251,7 +251,7 @@ class _AfnoFilterFn(torch.autograd.Function):
         sv = [torch.empty(g.B * g.KX, g.nblk, g.H, g.Cb, 2, dtype=torch.float32, device=dev) for _ in range(3)]
         w1f, b1f, w2f, b2f = (t.detach().float().contiguous() for t in (w1, b1, w2, b2))
         if exchange is None:
-            src = tokens.contiguous()
+            src = _g._aligned(tokens.contiguous())
             out = torch.empty_like(src)
             rc = lib.pnm_afno_rows_r2c(_ptrs8([src.data_ptr()]), Y.data_ptr(), g.arr, g.Tp, 0, 0, None, 0, 1, 0, 0, 1.0, None, st)
             _g._check(rc, "pnm_afno_rows_r2c")
@@ -289,7 +289,7 @@ class _AfnoFilterFn(torch.autograd.Function):
                                        w2f.data_ptr(), dw1.data_ptr(), db1.data_ptr(), dw2.data_ptr(), db2.data_ptr(), g.nb, g.arr, st)
             _g._check(rc, "pnm_afno_cols_bwd")
 
-        d = dout.to(torch.bfloat16).contiguous()
+        d = _g._aligned(dout.to(torch.bfloat16).contiguous())
         if exchange is None:
             dx = torch.empty_like(d)
             # adjoint of the weighted c2r = r2c with the same weights; adjoint of the r2c = unweighted c2r

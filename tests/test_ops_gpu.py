@@ -887,6 +887,32 @@ def test_conv_weight_packing_matches_the_tensor_operations(cout, cin, k, cin_p, 
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mlp", ["bf16", "fp32"])
+def test_afno_filter_of_tensors_off_a_16_byte_boundary(mlp):
+    """Tokens, residual and gradient as slices of flat buffers, four elements from their start: the row kernels read vectors of eight."""
+    from physicsnemo_b200.ops import afno_spectral as A
+
+    g = A.FilterGeometry(1, 6, 12, 64, 4, 6)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    params = [0.1 * rn(2, 4, 16, 16), 0.1 * rn(2, 4, 16), 0.1 * rn(2, 4, 16, 16), 0.1 * rn(2, 4, 16)]
+    flat = [rn(72 * 64 + 4).bfloat16() for _ in range(3)]
+    off = [t[4:].view(72, 64) for t in flat]
+    results = []
+    for x, res, dy in (off, [t.clone() for t in off]):
+        assert x.data_ptr() % 16 == (8 if x is off[0] else 0)
+        own = [p.clone().requires_grad_(True) for p in params]
+        xg = x.detach().requires_grad_(True)
+        y = A.afno_filter(xg, *own, g, 0.01, mlp=mlp, add_input=True, residual=res)
+        y.backward(dy)
+        results.append([y.detach(), xg.grad])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    from physicsnemo_b200 import ops
+
+    assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cout,cin,cin_p,cout_p", [(3, 4, 64, 64), (72, 68, 128, 72), (65, 132, 192, 128), (520, 64, 64, 520)])
 def test_conv3x3_weight_packing_at_the_edges(cout, cin, cin_p, cout_p):
     """3 x 3 filters in fp32 by vectors: rows and columns that fill no block, padding on both sides."""
