@@ -236,11 +236,12 @@ PyObject* mlp3_operands_ok(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const Tensor& w = THPVariable_Unpack(o);
     if (w.dim() != 2 || w.size(0) != kWidth || w.size(1) != (i ? kWidth : kWidth * int64_t(nsrc))) Py_RETURN_FALSE;
   }
+  auto vector = [&](PyObject* o) { return parameter(o) && THPVariable_Unpack(o).numel() == kWidth; };
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(biases.get()); ++i) {
     PyObject* o = PySequence_Fast_GET_ITEM(biases.get(), i);
-    if (o != Py_None && !parameter(o)) Py_RETURN_FALSE;
+    if (o != Py_None && !vector(o)) Py_RETURN_FALSE;
   }
-  if (!parameter(args[3]) || THPVariable_Unpack(args[3]).numel() != kWidth || (args[4] != Py_None && !parameter(args[4]))) Py_RETURN_FALSE;
+  if (!vector(args[3]) || (args[4] != Py_None && !vector(args[4]))) Py_RETURN_FALSE;
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }
@@ -403,7 +404,7 @@ PyObject* mlp3_module(PyObject*, PyObject* const* args, Py_ssize_t n) {
     THPObjectPtr own(attribute(module, k_parameters));
     if (!own || !PyDict_Check(own.get())) Py_RETURN_NONE;
     PyObject *w = item(own.get(), k_weight), *b = item(own.get(), k_bias);
-    if (!parameter(w) || !b || (b != Py_None && !parameter(b))) Py_RETURN_NONE;
+    if (!parameter(w) || !b || (b != Py_None && (!parameter(b) || THPVariable_Unpack(b).numel() != kWidth))) Py_RETURN_NONE;
     const Tensor& t = THPVariable_Unpack(w);
     if (i == 5) {
       if (t.numel() != kWidth) Py_RETURN_NONE;

@@ -435,3 +435,26 @@ def test_call_from_the_modules_is_the_general_call(act, nsrc, post):
     with torch.enable_grad():
         assert mf.module_call(model, srcs, segs, p) is None
     assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("at", ["bias", "beta"])
+def test_vectors_of_another_length_are_declined(at):
+    """The kernel reads 128 values of every vector: a shorter one is left to the general way, from the modules and by `supported`."""
+    from torch import nn
+
+    from physicsnemo_b200.ops import gemm as G
+    from physicsnemo_b200.ops import mlp_fused as mf
+
+    model = nn.Sequential(nn.Linear(W, W), nn.SiLU(), nn.Linear(W, W), nn.SiLU(), nn.Linear(W, W), nn.LayerNorm(W)).cuda()
+    lin, norm, x = [model[0], model[2], model[4]], model[5], torch.randn(40, W, device="cuda").bfloat16()
+
+    def supported():
+        return mf.supported([x], [None], [q.weight for q in lin], [q.bias for q in lin], (G.ACT_SILU, G.ACT_SILU, 0), norm.weight, norm.bias, None)
+
+    with torch.no_grad():
+        assert supported()
+        mf.mlp3_ln([x], [None], [q.weight for q in lin], [q.bias for q in lin], G.ACT_SILU, norm.weight, norm.bias, norm.eps, None)
+        assert mf.module_call(model, [x], [None], None) is not None
+        (norm if at == "beta" else lin[1]).bias = nn.Parameter(torch.zeros(1, device="cuda"))
+        assert not supported() and mf.module_call(model, [x], [None], None) is None
