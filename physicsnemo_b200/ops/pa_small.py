@@ -36,7 +36,7 @@ def _ptr_array(ptrs: Sequence[int]):
 
 def supported(H: int, D: int, slices: int, C: int, params: Sequence[torch.Tensor]) -> bool:
     return (slices == S and 0 < D <= 64 and 256 % D == 0 and (H * D) % 8 == 0 and C % 8 == 0
-            and all(p.dtype == torch.float32 and p.is_cuda for p in params))
+            and all(p.dtype == torch.float32 and p.is_cuda and p.is_contiguous() for p in params))      # read as they lie
 
 
 def prepare_fwd(Wx, bx, Wfx, Ws, bs, temp, H: int, D: int):

@@ -112,7 +112,7 @@ class _PhysAttnFn(torch.autograd.Function):
 
 
 def fused_supported(mod) -> bool:
-    """The kernels cover fp32 parameters, 64 slices and head widths that divide 256."""
+    """The kernels cover contiguous fp32 parameters, 64 slices and head widths that divide 256."""
     params = [mod.in_project_x.weight, mod.in_project_x.bias, mod.in_project_fx.weight, mod.in_project_fx.bias,
               mod.in_project_slice.weight, mod.in_project_slice.bias, mod.temperature, mod.qkv_project.weight,
               mod.out_linear.weight, mod.out_linear.bias]

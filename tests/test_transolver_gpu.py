@@ -148,3 +148,21 @@ def test_temperatures_at_the_ends_of_their_range_have_gradients():
     (want,) = torch.autograd.grad((-sums.double() * torch.log(torch.clamp(t, min=0.5, max=5))).sum(), t)
     assert torch.allclose(dtemp.double(), want, rtol=1e-6, atol=0)
     assert ops.device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["in_project_x", "in_project_fx", "qkv_project", "out_linear"])
+def test_parameters_that_lie_by_columns(name):
+    """A weight given as a transposed view is the same weight: the kernels, which read parameters as they lie, leave it to the plain path."""
+    from physicsnemo_b200.nn.module.physics_attention import PhysicsAttentionIrregularMesh
+
+    torch.manual_seed(7)
+    mod = PhysicsAttentionIrregularMesh(64, heads=2, dim_head=32, slice_num=64, use_te=False).cuda()
+    x = torch.randn(1, 500, 64, device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        want = mod(x)
+        layer = getattr(mod, name)
+        layer.weight = torch.nn.Parameter(layer.weight.t().contiguous().t())
+        assert not layer.weight.is_contiguous()
+        assert _rel(mod(x), want) < 2e-2
+    assert ops.device_error() == 0
